@@ -93,11 +93,25 @@ gf_status ensure_multipliers(gf_ctx *ctx)
 {
     if (ctx->d_mult) return GF_OK;
     const std::vector<uint32_t> &mult = gfh::multipliers();
-    GF_TRY(dev_alloc(&ctx->d_mult, GF_MAX_STREAMS));
-    GF_CUDA(cudaMemcpy(ctx->d_mult, mult.data(), 4 * (size_t)GF_MAX_STREAMS, cudaMemcpyHostToDevice));
-    GF_TRY(dev_alloc(&ctx->jt.lo, (size_t)GF_MAX_STREAMS * 32));
-    GF_TRY(dev_alloc(&ctx->jt.hi, (size_t)GF_MAX_STREAMS * GF_JUMP_HI));
-    GF_CUDA(gfk::launch_jump_tables(ctx->d_mult, GF_MAX_STREAMS, ctx->jt.lo, ctx->jt.hi, ctx->stream));
+    /* the context takes the three tables together, when all are there: a failed
+     * allocation leaves none, and the next call makes them again */
+    uint32_t *d_mult = nullptr;
+    JumpTables jt = {nullptr, nullptr};
+    auto make = [&]() -> gf_status {
+        GF_TRY(dev_alloc(&d_mult, GF_MAX_STREAMS));
+        GF_TRY(dev_alloc(&jt.lo, (size_t)GF_MAX_STREAMS * 32));
+        GF_TRY(dev_alloc(&jt.hi, (size_t)GF_MAX_STREAMS * GF_JUMP_HI));
+        GF_CUDA(cudaMemcpy(d_mult, mult.data(), 4 * (size_t)GF_MAX_STREAMS, cudaMemcpyHostToDevice));
+        GF_CUDA(gfk::launch_jump_tables(d_mult, GF_MAX_STREAMS, jt.lo, jt.hi, ctx->stream));
+        return GF_OK;
+    };
+    const gf_status st = make();
+    if (st != GF_OK) {
+        dev_free(d_mult); dev_free(jt.lo); dev_free(jt.hi);
+        return st;
+    }
+    ctx->d_mult = d_mult;
+    ctx->jt = jt;
     return GF_OK;
 }
 
@@ -1243,7 +1257,7 @@ static gf_status module_feh(gf_ctx *ctx, const gf_feh_config *fp, const gf_gauss
     const int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_FEH);
-    GF_CUDA(gfk::launch_feh(fp, gp, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_feh(fp, gp, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     return GF_OK;
 }
 
@@ -1260,7 +1274,7 @@ gf_status gf_module_multiples(gf_ctx *ctx, const gf_multiples_config *cfg, gf_ta
     const int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_FEH);
-    GF_CUDA(gfk::launch_multiples(*cfg, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_multiples(*cfg, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     t->systems = 1;
     return GF_OK;
 }
@@ -1286,7 +1300,7 @@ gf_status gf_module_bond2010(gf_ctx *ctx, const gf_bond2010_config *cfg, gf_tabl
     int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_BOND2010);
-    GF_CUDA(gfk::launch_bond2010(*cfg, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_bond2010(*cfg, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     return GF_OK;
 }
 

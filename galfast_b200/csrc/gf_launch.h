@@ -110,10 +110,17 @@ cudaError_t launch_tie_place_multi(const LaunchPlaceMulti &L, const int64_t *row
 cudaError_t launch_clipper(const gf_footprint &foot, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
 cudaError_t launch_poisson_stream(uint32_t *st, const float *mu, int32_t n, uint32_t *out, cudaStream_t s);
 /* os_FeH (fp) or os_GaussianFeH (gp): the one that is not NULL */
-cudaError_t launch_feh(const gf_feh_config *fp, const gf_gaussfeh_config *gp, uint32_t *rng, int32_t NS, gf_table t,
+/* the context's multipliers and their powers, with which a warp jumps along a stream */
+struct StreamPowers {
+    JumpTables jt;
+    const uint32_t *mult;
+};
+cudaError_t launch_feh(const gf_feh_config *fp, const gf_gaussfeh_config *gp, const StreamPowers &pw,
+    uint32_t *rng, int32_t NS, gf_table t,
                        int64_t begin, int64_t end, cudaStream_t s);
 cudaError_t launch_fixedfeh(const gf_fixedfeh_config &c, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
-cudaError_t launch_bond2010(const gf_bond2010_config &c, uint32_t *rng, int32_t rng_nstreams, gf_table t,
+cudaError_t launch_bond2010(const gf_bond2010_config &c, const StreamPowers &pw,
+    uint32_t *rng, int32_t rng_nstreams, gf_table t,
                             int64_t begin, int64_t end, cudaStream_t s);
 struct PhotTables {
     int32_t nbands, bidx, nFeH, nMr;
@@ -124,7 +131,8 @@ struct PhotTables {
     uint32_t comp_mask;
 };
 cudaError_t launch_photometry(const PhotTables &c, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
-cudaError_t launch_multiples(const gf_multiples_config &c, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
+cudaError_t launch_multiples(const gf_multiples_config &c, const StreamPowers &pw,
+    uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
                              cudaStream_t s);
 struct PerrTables {
     int32_t nbands, nknots;
@@ -248,13 +256,16 @@ struct MultiRows {
 };
 cudaError_t launch_clipper_multi(const gf_footprint *foot_by_job, MultiRows R, gf_table t, int64_t begin, int64_t end,
                                  cudaStream_t s);
-cudaError_t launch_bond2010_multi(const gf_bond2010_config &c, uint32_t *rng_all, int32_t NS, MultiRows R,
+cudaError_t launch_bond2010_multi(const gf_bond2010_config &c, const StreamPowers &pw,
+    uint32_t *rng_all, int32_t NS, MultiRows R,
                                   const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks,
                                   const int64_t *slot_rows, gf_table t, cudaStream_t s);
-cudaError_t launch_feh_multi(const gf_feh_config *fp, const gf_gaussfeh_config *gp, uint32_t *rng_all, int32_t NS,
+cudaError_t launch_feh_multi(const gf_feh_config *fp, const gf_gaussfeh_config *gp, const StreamPowers &pw,
+    uint32_t *rng_all, int32_t NS,
                              MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks,
                              const int64_t *slot_rows, gf_table t, cudaStream_t s);
-cudaError_t launch_multiples_multi(const gf_multiples_config &c, uint32_t *rng_all, int32_t NS, MultiRows R,
+cudaError_t launch_multiples_multi(const gf_multiples_config &c, const StreamPowers &pw,
+    uint32_t *rng_all, int32_t NS, MultiRows R,
                                    const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks, const int64_t *slot_rows,
                                    gf_table t, cudaStream_t s);
 cudaError_t launch_photoerrors_multi(const PerrTables &c, const uint64_t *seed_by_job, const int64_t *catalog_offset_by_job,

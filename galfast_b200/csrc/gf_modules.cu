@@ -6,9 +6,11 @@
  *
  *   clipper_kernel     os_clipper::process (src/skygen/os_skygen.cpp:999-1044), analytic footprints
  *   fixedfeh_kernel    os_fixedFeH_kernel (src/modules/fixedFeH_gpu.cu.h:34-50)
- *   feh_kernel<0>      os_FeH_kernel (src/modules/FeH_gpu.cu.h:43-87)
- *   feh_kernel<1>      os_GaussianFeH_kernel (src/modules/GaussianFeH_gpu.cu.h:42-73)
- *   bond2010_kernel    os_Bond2010_kernel (src/modules/Bond2010_gpu.cu.h:81-218)
+ *   stream_rows_kernel with
+ *     BondOps          os_Bond2010_kernel (src/modules/Bond2010_gpu.cu.h:81-218)
+ *     FehOps           os_FeH_kernel (src/modules/FeH_gpu.cu.h:43-87)
+ *     GaussFehOps      os_GaussianFeH_kernel (src/modules/GaussianFeH_gpu.cu.h:42-73)
+ *     MultOps          os_unresolvedMultiples_kernel (src/modules/unresolvedMultiples_gpu.cu.h:36-123)
  *   photometry_kernel  os_photometry_kernel (src/modules/photometry_gpu.cu.h:87-174)
  *   photoerr_kernel    os_photometricErrors::process (photometricErrors_host.cpp:112-131)
  *   vel2pm_kernel      os_vel2pm_kernel (src/modules/vel2pm_gpu.cu.h:253-301)
@@ -128,6 +130,321 @@ cudaError_t launch_fixedfeh(const gf_fixedfeh_config &c, gf_table t, int64_t beg
     return cudaGetLastError();
 }
 
+/* ---------------- rows that draw from a stream, 256 to a stream ---------------- */
+/* The reference gives each stream 256 consecutive rows, one thread walking them: the
+ * uniforms a row takes depend on the rejections of the rows before it.  What depends on
+ * the order is only where each row's uniforms begin; so one warp takes a stream and
+ *   1  generates a run of W = 32 R uniforms, R to a lane: the MWC is a Lehmer generator,
+ *      and lane l starts at the state times a^(l R);
+ *   2  marks the positions where a Gaussian's pair is accepted and finds for every
+ *      position where a Gaussian (next), and a row's NG Gaussians (fh), begun there end;
+ *   3  walks the rows through fh, one shared-memory read a row;
+ *   4  forms the rows' values, 32 rows at a time, reading and writing whole lines.
+ * A row that the run ends in begins the next run.  Measured (Bond2010): 20001 rows 0.73 ms as one thread
+ * a stream, 0.06 ms now (latency of one chunk); 4.0e6 rows 0.94 -> 0.39 ms, 6.2e7 rows 5.7 -> 6.0 ms
+ * (instruction issue: 56 % of slots, 16e3 warp instructions a chunk, half of them the rows' functions).
+ */
+#define GF_RUN_LANE 26                  /* uniforms of a lane in a run (even): three runs serve 256 rows of three Gaussians */
+#define GF_RUN_PITCH 33
+#define GF_RUN_END 0xffffu
+
+/* Position p of a run of 32 R uniforms (lane p / R holds it, as its (p mod R)-th) is kept at
+ * (p mod R) 33 + p / R: a lane's run is a column, and the run's end (p = 32 R) has an index of its own.
+ * The tables hold such indexes, so following them takes no arithmetic. */
+struct RowStream {
+    float u[GF_RUN_PITCH * GF_RUN_LANE];
+    uint16_t next[GF_RUN_PITCH * GF_RUN_LANE];      /* end of the Gaussian that begins here */
+    uint16_t fh[GF_RUN_PITCH * GF_RUN_LANE];        /* end of the NG Gaussians that begin here (from the next position when every row leads with a uniform) */
+    uint16_t start[256];
+    uint16_t list[256];                 /* the rows that draw: row | kind << 8 */
+};
+
+template <int R>
+__device__ __forceinline__ int run_forward(int q) { return q < (R - 1) * GF_RUN_PITCH ? q + GF_RUN_PITCH : q - (R - 1) * GF_RUN_PITCH + 1; }
+template <int R>
+__device__ __forceinline__ int run_back(int q) { return q >= GF_RUN_PITCH ? q - GF_RUN_PITCH : q + (R - 1) * GF_RUN_PITCH - 1; }
+
+__device__ __forceinline__ float row_step(uint64_t &v, uint32_t a)
+{
+    const uint64_t t = (uint64_t)a * (uint32_t)v + (v >> 32);
+    v = t;
+    return GF_MWC_SCALE * (float)(uint32_t)t;
+}
+
+/* a chunk's stream: its multiplier, and the powers that jump it */
+struct RowJump {
+    const uint64_t *lo, *hi;            /* the context's tables of stream th, or null (another multiplier was set) */
+    uint32_t a;
+    bool ok;                            /* the multiplier is within the bounds of mwc_fold3 */
+};
+
+__device__ __forceinline__ RowJump row_jump(const JumpTables &jt, const uint32_t *mult, const uint32_t *rng, int64_t th)
+{
+    RowJump j;
+    j.a = rng[th];
+    const bool same = j.a == mult[th];
+    j.lo = same ? jt.lo + (size_t)th * 32 : nullptr;
+    j.hi = same ? jt.hi + (size_t)th * GF_JUMP_HI : nullptr;
+    j.ok = j.a >= 16u && j.a <= 0xfffffff0u;
+    return j;
+}
+
+/* the state of the lane's part of a run, lane R steps after v; false when v is not a residue of the Lehmer
+ * generator modulo p = a 2^32 - 1 (0 < v < p).  mwc_mulmod_scaled(x, y) = x y a^3 mod p, so s(n) = a^(n-3)
+ * jumps n steps and s(n + m) = mulmod(s(n), s(m)); s(1) = a^-2 = 2^64 mod p. */
+template <int R>
+__device__ __forceinline__ bool stream_runs(const RowJump &j, uint64_t v, int lane, uint64_t &w)
+{
+    const uint64_t p = ((uint64_t)j.a << 32) - 1;
+    if (!j.ok || v == 0 || v >= p) return false;
+    const int n = lane * R;
+    w = v;
+    if (j.hi) {
+        w = gfr::mwc_mulmod_scaled(__ldg(j.hi + (n >> 5)), w, j.a, p);
+        w = gfr::mwc_mulmod_scaled(__ldg(j.lo + (n & 31)), w, j.a, p);
+    } else {
+        uint64_t m = (0ull - p) % p;
+        for (int k = n; k; k >>= 1) {
+            if (k & 1) w = gfr::mwc_mulmod_scaled(m, w, j.a, p);
+            m = gfr::mwc_mulmod_scaled(m, m, j.a, p);
+        }
+    }
+    return true;
+}
+
+/* the stream's state at index q of the run (the run's end included), given each lane's start w0 */
+template <int R>
+__device__ __forceinline__ uint64_t stream_state_at(uint32_t a, uint64_t w0, int q, int lane)
+{
+    int steps = q / GF_RUN_PITCH, src = q - steps * GF_RUN_PITCH;
+    if (src == 32) { src = 31; steps = R; }
+    uint64_t w = w0;
+    for (int s = 0; s < steps; s++) (void)row_step(w, a);
+    const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)w, src), hi = __shfl_sync(0xffffffffu, (uint32_t)(w >> 32), src);
+    return ((uint64_t)hi << 32) | lo;
+}
+
+/* gaussian()'s test of a pair of uniforms (cuda_rng.h:165-182) */
+__device__ __forceinline__ float pair_r2(float u0, float u1, float &y)
+{
+    const float x = -1.f + 2.f * u0;
+    y = -1.f + 2.f * u1;
+    return x * x + y * y;
+}
+__device__ __forceinline__ bool pair_accepted(float r2) { return !(r2 > 1.0f || r2 == 0.f || r2 == 4.f); }
+
+/* One run of 32 R uniforms: the places of the rows from r0 on that it holds (S.start, S.next, S.u).  lead:
+ * every row's kind, or -1 when they differ.  Returns the row after the last one, with v the state there; r0
+ * when none fits or v cannot be jumped. */
+template <int NG, int R>
+__device__ __forceinline__ int rows_of_run(const RowJump &j, uint64_t &v, int r0, int na, int lead, RowStream &S, int lane)
+{
+    constexpr unsigned full = 0xffffffffu;
+    uint64_t w0;
+    if (!stream_runs<R>(j, v, lane, w0)) return r0;
+    /* the uniforms, and the accepted pairs that begin in the lane's part */
+    uint32_t acc = 0;
+    {
+        uint64_t w = w0;
+        float y, prev = row_step(w, j.a);
+        const float first = prev;
+        S.u[lane] = prev;
+#pragma unroll 5
+        for (int s = 1; s < R; s++) {
+            const float u = row_step(w, j.a);
+            S.u[s * GF_RUN_PITCH + lane] = u;
+            if (pair_accepted(pair_r2(prev, u, y))) acc |= 1u << (s - 1);
+            prev = u;
+        }
+        const float after = __shfl_down_sync(full, first, 1);
+        if (lane < 31 && pair_accepted(pair_r2(prev, after, y))) acc |= 1u << (R - 1);
+    }
+    /* the end of the first accepted pair of each parity in the lanes after this one (R is even) */
+    uint32_t later[2];
+#pragma unroll
+    for (int par = 0; par < 2; par++) {
+        const uint32_t mine = acc & (0x55555555u << par);
+        const int at = run_forward<R>(run_forward<R>((__ffs(mine) - 1) * GF_RUN_PITCH + lane));
+        const unsigned has = __ballot_sync(full, mine != 0) & (0xfffffffeu << lane);
+        const int there = __shfl_sync(full, at, has ? __ffs(has) - 1 : lane);
+        later[par] = has ? (uint32_t)there : GF_RUN_END;
+    }
+    uint32_t even = later[0], odd = later[1];
+    int at = (R - 1) * GF_RUN_PITCH + lane;           /* the odd position of a pair of positions */
+#pragma unroll 2
+    for (int s = R - 2; s >= 0; s -= 2, at -= 2 * GF_RUN_PITCH) {
+        if ((acc >> s) & 2u) odd = (uint32_t)run_forward<R>(run_forward<R>(at));
+        if ((acc >> s) & 1u) even = (uint32_t)run_forward<R>(at);
+        S.next[at] = (uint16_t)odd;
+        S.next[at - GF_RUN_PITCH] = (uint16_t)even;
+    }
+    __syncwarp();
+    /* the indexes of whole rows; the run's end is at column 32 and ends every chain */
+    if (NG > 1 || lead == 1) {
+#pragma unroll 2
+        for (int s = 0; s < R; s++) {
+            int q = s * GF_RUN_PITCH + lane;
+            if (lead == 1) q = run_forward<R>(q);
+#pragma unroll
+            for (int g = 0; g < NG; g++) q = (q < R * GF_RUN_PITCH && q != 32) ? S.next[q] : (int)GF_RUN_END;
+            S.fh[s * GF_RUN_PITCH + lane] = (uint16_t)q;
+        }
+        __syncwarp();
+    }
+    /* where each row begins */
+    const uint16_t *fh = (NG > 1 || lead == 1) ? S.fh : S.next;
+    int q = 0, r = r0;
+    if (lead >= 0) {
+        while (r < na && q != 32) {
+            const int e = fh[q];
+            if (e == (int)GF_RUN_END) break;
+            if (lane == 0) S.start[r] = (uint16_t)q;
+            q = e;
+            r++;
+        }
+    } else {
+        while (r < na && q != 32) {
+            const int b = (S.list[r] >> 8) ? run_forward<R>(q) : q;
+            const int e = b != 32 ? fh[b] : (int)GF_RUN_END;
+            if (e == (int)GF_RUN_END) break;
+            if (lane == 0) S.start[r] = (uint16_t)q;
+            q = e;
+            r++;
+        }
+    }
+    if (r > r0) v = stream_state_at<R>(j.a, w0, q, lane);
+    return r;
+}
+
+/* the rows [begin + 256 th, ...) of one chunk with stream th, on one warp */
+template <class Ops>
+__device__ __forceinline__ void chunk_rows(const Ops &ops, const JumpTables &jt, const uint32_t *mult, uint32_t *rng, int32_t NS,
+                                           gf_table &t, int64_t begin, int64_t end, int64_t th, RowStream &S)
+{
+    constexpr int NG = Ops::NG, R = GF_RUN_LANE;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int64_t rb = begin + 256 * th;
+    const int nrow = (int)(end - rb < 256 ? end - rb : 256);
+    int na = 0, leads = 0;
+    for (int q = 0; q < nrow; q += 32) {
+        const int i = q + lane;
+        const int kind = i < nrow ? ops.kind(t, rb + i) : -1;
+        const unsigned m = __ballot_sync(full, kind >= 0);
+        if (kind >= 0) S.list[na + __popc(m & ((1u << lane) - 1u))] = (uint16_t)(i | (kind << 8));
+        na += __popc(m);
+        leads += __popc(__ballot_sync(full, kind == 1));
+    }
+    __syncwarp();
+    if (na == 0) return;
+    const int lead = leads == na ? 1 : leads == 0 ? 0 : -1;
+    const RowJump j = row_jump(jt, mult, rng, th);
+    uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
+    int r0 = 0;
+    while (r0 < na) {
+        int r = rows_of_run<NG, R>(j, v, r0, na, lead, S, lane);
+        if (r == r0) {
+            /* a state outside the Lehmer range, or a row longer than a run: its uniforms one after
+             * another, the accepted ones laid out as the first of a run */
+            const int kind = S.list[r0] >> 8;
+            int q = 0;
+            if (kind) {
+                S.u[0] = row_step(v, j.a);
+                q = GF_RUN_PITCH;
+            }
+            for (int g = 0; g < NG; g++, q += 2 * GF_RUN_PITCH) {
+                float u0, u1, y;
+                do {
+                    u0 = row_step(v, j.a);
+                    u1 = row_step(v, j.a);
+                } while (!pair_accepted(pair_r2(u0, u1, y)));
+                S.u[q] = u0;
+                S.u[q + GF_RUN_PITCH] = u1;
+                S.next[q] = (uint16_t)(q + 2 * GF_RUN_PITCH);
+            }
+            S.start[r0] = 0;
+            r = r0 + 1;
+        }
+        __syncwarp();
+        for (int i = r0 + lane; i < r; i += 32) {
+            const int entry = S.list[i], kind = entry >> 8;
+            int b = S.start[i];
+            float pu = 0.f;
+            if (kind) {
+                pu = S.u[b];
+                b = run_forward<R>(b);
+            }
+            float ys[NG], ss[NG];
+#pragma unroll
+            for (int g = 0; g < NG; g++) {
+                b = S.next[b];
+                const int b1 = run_back<R>(b);
+                const float r2 = pair_r2(S.u[run_back<R>(b1)], S.u[b1], ys[g]);
+                ss[g] = sqrtf(-2.0f * gfm::logf_(r2) / r2);
+            }
+            ops.apply(t, rb + (entry & 0xff), kind, pu, ys, ss);
+        }
+        r0 = r;
+        __syncwarp();
+    }
+    if (lane == 0) {
+        rng[NS + th] = (uint32_t)(v >> 32);
+        rng[2 * NS + th] = (uint32_t)v;
+    }
+}
+
+#define GF_ROW_WARPS 4
+
+template <class Ops>
+__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_kernel(const Ops ops, JumpTables jt, const uint32_t *mult, uint32_t *rng, int32_t NS, gf_table t,
+                                                                        int64_t begin, int64_t end, int64_t nchunks)
+{
+    __shared__ RowStream S[GF_ROW_WARPS];
+    const int64_t th = (int64_t)blockIdx.x * GF_ROW_WARPS + (threadIdx.x >> 5);
+    if (th >= nchunks) return;
+    chunk_rows(ops, jt, mult, rng, NS, t, begin, end, th, S[threadIdx.x >> 5]);
+}
+
+/* the 256-row chunks of every request of a pass, each drawing from its request's streams */
+template <class Ops>
+__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel(const Ops ops, JumpTables jt, const uint32_t *mult, uint32_t *rng_all, int32_t NS,
+                                                                              MultiRows R, const int64_t *slot_chunk_begin,
+                                                                              int32_t nslots, int64_t nchunks,
+                                                                              const int64_t *slot_rows, gf_table t)
+{
+    __shared__ RowStream S[GF_ROW_WARPS];
+    const int64_t c = (int64_t)blockIdx.x * GF_ROW_WARPS + (threadIdx.x >> 5);
+    if (c >= nchunks) return;
+    int lo = 0, hi = nslots - 1;          /* last slot whose first chunk is <= c */
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    const int64_t b = R.slot_row_begin[lo];
+    chunk_rows(ops, jt, mult, rng_all + (size_t)R.slot_job[lo] * 3 * NS, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo],
+               S[threadIdx.x >> 5]);
+}
+
+template <class Ops>
+cudaError_t launch_stream_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
+                               int64_t nchunks, cudaStream_t s)
+{
+    stream_rows_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
+        ops, pw.jt, pw.mult, rng, NS, t, begin, end, nchunks);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+template <class Ops>
+cudaError_t launch_stream_rows_multi(const Ops &ops, const StreamPowers &pw, uint32_t *rng_all, int32_t NS, MultiRows R, const int64_t *slot_chunk_begin,
+                                     int32_t nslots, int64_t nchunks, const int64_t *slot_rows, gf_table t, cudaStream_t s)
+{
+    stream_rows_multi_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
+        ops, pw.jt, pw.mult, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 /* ---------------- Bond2010 kinematics ---------------- */
 __device__ __forceinline__ float modfun(float Rsquared, float Z, const float *val)
 {
@@ -135,7 +452,7 @@ __device__ __forceinline__ float modfun(float Rsquared, float Z, const float *va
     return val[0] + val[1] * gfm::powf_(fabsf(Z), val[2]) + val[3] * gfm::powf_(Rsquared, (float)(0.5 * (double)val[4]));
 }
 
-__device__ __forceinline__ void trivar_gauss(float y[3], const float sg[6], gfr::Mwc &rng)
+__device__ __forceinline__ void trivar_gauss(float y[3], const float sg[6], const float z[3])
 {
     /* Cholesky draw, Bond2010_gpu.cu.h:81-103 */
     float s11 = sg[0], s12 = sg[1], s13 = sg[2], s22 = sg[3], s23 = sg[4], s33 = sg[5];
@@ -147,48 +464,48 @@ __device__ __forceinline__ void trivar_gauss(float y[3], const float sg[6], gfr:
     float a20 = b20 * oneDivA00;
     float a21 = (b21 - a20 * a10) / a11;
     float a22 = sqrtf(b22 - a20 * a20 - a21 * a21);
-    float z0 = rng.gaussian(1.0f);
-    float z1 = rng.gaussian(1.0f);
-    float z2 = rng.gaussian(1.0f);
-    y[0] += a00 * z0;
-    y[1] += a10 * z0 + a11 * z1;
-    y[2] += a20 * z0 + a21 * z1 + a22 * z2;
+    y[0] += a00 * z[0];
+    y[1] += a10 * z[0] + a11 * z[1];
+    y[2] += a20 * z[0] + a21 * z[1] + a22 * z[2];
 }
 
-__device__ __forceinline__ void draw_moments(float v[3], float R2, float Z, const gf_vmoments &mo, bool disk, gfr::Mwc &rng)
+__device__ __forceinline__ void draw_moments(float v[3], float R2, float Z, const gf_vmoments &mo, bool disk, const float z[3])
 {
     for (int i = 0; i < 3; i++) v[i] = modfun(R2, Z, mo.m[i]);
     if (disk && v[1] > 0.f) v[1] = 0.f;
     float sg[6];
     for (int i = 0; i < 6; i++) sg[i] = modfun(R2, Z, mo.ss[i]);
-    trivar_gauss(v, sg, rng);
+    trivar_gauss(v, sg, z);
 }
 
-/* rows [begin + 256 th, min(begin + 256 (th + 1), end)) with stream th (Bond2010_gpu.cu.h:179, 217) */
-__device__ __forceinline__ void bond2010_chunk(const gf_bond2010_config &par, uint32_t *rng, int32_t NS, gf_table &t,
-                                               int64_t begin, int64_t end, int64_t th)
-{
-    const int64_t P = t.capacity;
-    gfr::Mwc r;
-    r.a = rng[th]; r.c = rng[NS + th]; r.x = rng[2 * NS + th];
-    int64_t rb = begin + 256 * th, re = begin + 256 * (th + 1);
-    if (re > end) re = end;
-    for (int64_t row = rb; row < re; row++) {
-        if (t.hidden[row]) continue;
+/* os_Bond2010_kernel's row (Bond2010_gpu.cu.h:140-215): disk stars draw the disk
+ * component's uniform, then three Gaussians; halo stars three Gaussians */
+struct BondOps {
+    gf_bond2010_config par;
+    static constexpr int NG = 3;
+
+    __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
+    {
+        if (t.hidden[row]) return -1;
         const int cmp = t.comp[row];
+        if (((par.comp_thin | par.comp_thick) >> cmp) & 1u) return 1;
+        return ((par.comp_halo >> cmp) & 1u) ? 0 : -1;
+    }
+    __device__ __forceinline__ void apply(gf_table &t, int64_t row, int kind, float pu, const float *y, const float *s) const
+    {
+        const int64_t P = t.capacity;
         float vx = t.XYZ[row] + par.T[0], vy = t.XYZ[P + row] + par.T[1], vz = t.XYZ[2 * P + row] + par.T[2];
         float wx = par.M[0] * vx + par.M[1] * vy + par.M[2] * vz;
         float wy = par.M[3] * vx + par.M[4] * vy + par.M[5] * vz;
         float wz = par.M[6] * vx + par.M[7] * vy + par.M[8] * vz;
         const float R2 = (float)(1e-6 * (double)(wx * wx + wy * wy));
         const float Z = (float)(1e-3 * (double)wz);
+        const float z[3] = {y[0] * s[0], y[1] * s[1], y[2] * s[2]};
         float v[3];
-        if (((par.comp_thin | par.comp_thick) >> cmp) & 1u) {
-            float pu = r.uniform();
-            const gf_vmoments &disk = pu < par.fk ? par.disk_1 : par.disk_2;
-            draw_moments(v, R2, Z, disk, true, r);
-        } else if ((par.comp_halo >> cmp) & 1u) {
-            draw_moments(v, R2, Z, par.halo, false, r);
+        if (kind == 1) {
+            draw_moments(v, R2, Z, pu < par.fk ? par.disk_1 : par.disk_2, true, z);
+        } else {
+            draw_moments(v, R2, Z, par.halo, false, z);
             float invR = 1.f / sqrtf(R2 + Z * Z);
             float cosa = sqrtf(R2) * invR;
             float sina = Z * invR;
@@ -197,81 +514,55 @@ __device__ __forceinline__ void bond2010_chunk(const gf_bond2010_config &par, ui
             v[0] = vR;
             v[1] = v[2];
             v[2] = vZ;
-        } else {
-            continue;
         }
         t.vcyl[row] = v[0];
         t.vcyl[P + row] = v[1];
         t.vcyl[2 * P + row] = v[2];
     }
-    rng[NS + th] = r.c;
-    rng[2 * NS + th] = r.x;
-}
+};
 
-__global__ void __launch_bounds__(128) bond2010_kernel(const gf_bond2010_config par, uint32_t *rng, int32_t NS, gf_table t,
-                                                        int64_t begin, int64_t end, int64_t nchunks)
-{
-    int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (th >= nchunks) return;
-    bond2010_chunk(par, rng, NS, t, begin, end, th);
-}
-
-/* the 256-row chunks of every request, each drawing from its request's streams */
-__global__ void __launch_bounds__(128) bond2010_multi_kernel(const gf_bond2010_config par, uint32_t *rng_all, int32_t NS,
-                                                              MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots,
-                                                              int64_t nchunks, const int64_t *slot_rows, gf_table t)
-{
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    int lo = 0, hi = nslots - 1;          /* last slot whose first chunk is <= c */
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const int64_t b = R.slot_row_begin[lo];
-    bond2010_chunk(par, rng_all + (size_t)R.slot_job[lo] * 3 * NS, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo]);
-}
-
-cudaError_t launch_bond2010_multi(const gf_bond2010_config &c, uint32_t *rng_all, int32_t NS, MultiRows R,
+cudaError_t launch_bond2010_multi(const gf_bond2010_config &c, const StreamPowers &pw, uint32_t *rng_all, int32_t NS, MultiRows R,
                                   const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks,
                                   const int64_t *slot_rows, gf_table t, cudaStream_t s)
 {
     if (nchunks <= 0) return cudaSuccess;
-    bond2010_multi_kernel<<<(unsigned)((nchunks + 127) / 128), 128, 0, s>>>(c, rng_all, NS, R, slot_chunk_begin, nslots,
-                                                                          nchunks, slot_rows, t);
-    count_launches(1);
-    return cudaGetLastError();
+    BondOps o;
+    o.par = c;
+    return launch_stream_rows_multi(o, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t, s);
 }
 
-cudaError_t launch_bond2010(const gf_bond2010_config &c, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
+cudaError_t launch_bond2010(const gf_bond2010_config &c, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
                             cudaStream_t s)
 {
     if (end <= begin) return cudaSuccess;
     int64_t n = end - begin;
     int64_t nchunks = n / 256 + (n % 256 ? 1 : 0);
     if (nchunks > NS) return cudaErrorInvalidValue;
-    bond2010_kernel<<<(int)((nchunks + 127) / 128), 128, 0, s>>>(c, rng, NS, t, begin, end, nchunks);
-    count_launches(1);
-    return cudaGetLastError();
+    BondOps o;
+    o.par = c;
+    return launch_stream_rows(o, pw, rng, NS, t, begin, end, nchunks, s);
 }
 
 /* ---------------- FeH (Ivezic et al. 2008) and GaussianFeH ---------------- */
 
-/* os_FeH_kernel (FeH_gpu.cu.h:43-87) on rows [begin + 256 th, ...) with stream th */
-__device__ __forceinline__ void feh_chunk(const gf_feh_config &par, uint32_t *rng, int32_t NS, gf_table &t, int64_t begin,
-                                          int64_t end, int64_t th)
-{
-    const int64_t P = t.capacity;
-    gfr::Mwc r;
-    r.a = rng[th]; r.c = rng[NS + th]; r.x = rng[2 * NS + th]; r.used = 0;
-    int64_t rb = begin + 256 * th, re = begin + 256 * (th + 1);
-    if (re > end) re = end;
-    for (int64_t row = rb; row < re; row++) {
-        if (t.hidden[row]) continue;
+/* os_FeH_kernel's row (FeH_gpu.cu.h:43-87): disk stars draw the Gaussian's number, then it; halo stars one Gaussian */
+struct FehOps {
+    gf_feh_config par;
+    static constexpr int NG = 1;
+
+    __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
+    {
+        if (t.hidden[row]) return -1;
         const int cmp = t.comp[row];
-        if (((par.comp_thin | par.comp_thick) >> cmp) & 1u) {
+        if (((par.comp_thin | par.comp_thick) >> cmp) & 1u) return 1;
+        return ((par.comp_halo >> cmp) & 1u) ? 0 : -1;
+    }
+    __device__ __forceinline__ void apply(gf_table &t, int64_t row, int kind, float pu, const float *y, const float *s) const
+    {
+        const int64_t P = t.capacity;
+        if (kind == 1) {
             /* the Gaussian to draw from */
-            const float p = r.uniform() * (par.A[0] + par.A[1]);
+            const float p = pu * (par.A[0] + par.A[1]);
             const int i = p < par.A[0] ? 0 : 1;
             /* the star's place in the disk */
             const float vx = t.XYZ[row] + par.T[0], vy = t.XYZ[P + row] + par.T[1], vz = t.XYZ[2 * P + row] + par.T[2];
@@ -279,101 +570,63 @@ __device__ __forceinline__ void feh_chunk(const gf_feh_config &par, uint32_t *rn
             /* Bond et al. A2; exp in single precision through the portable expf */
             const float muD = par.muInf + par.DeltaMu * gfm::expf_(-fabsf(wz) / par.Hmu);
             const float aZ = muD - 0.067f;
-            const float feh = r.gaussian(par.sigma[i]) + aZ + par.offs[i];
-            t.FeH[row] = feh;
-        } else if ((par.comp_halo >> cmp) & 1u) {
-            const float feh = par.offs[2] + r.gaussian(par.sigma[2]);
-            t.FeH[row] = feh;
+            t.FeH[row] = par.sigma[i] * y[0] * s[0] + aZ + par.offs[i];
+        } else {
+            t.FeH[row] = par.offs[2] + par.sigma[2] * y[0] * s[0];
         }
     }
-    rng[NS + th] = r.c;
-    rng[2 * NS + th] = r.x;
-}
+};
 
-/* os_GaussianFeH_kernel (GaussianFeH_gpu.cu.h:42-73) on rows [begin + 256 th, ...) with stream th */
-__device__ __forceinline__ void gaussfeh_chunk(const gf_gaussfeh_config &par, uint32_t *rng, int32_t NS, gf_table &t,
-                                               int64_t begin, int64_t end, int64_t th)
-{
-    gfr::Mwc r;
-    r.a = rng[th]; r.c = rng[NS + th]; r.x = rng[2 * NS + th]; r.used = 0;
-    int64_t rb = begin + 256 * th, re = begin + 256 * (th + 1);
-    if (re > end) re = end;
-    for (int64_t row = rb; row < re; row++) {
-        if (t.hidden[row]) continue;
-        const int cmp = t.comp[row];
-        if (!((par.comp_mask >> cmp) & 1u)) continue;
+/* os_GaussianFeH_kernel's row (GaussianFeH_gpu.cu.h:42-73): the component's uniform when there
+ * are several, then one Gaussian */
+struct GaussFehOps {
+    gf_gaussfeh_config par;
+    static constexpr int NG = 1;
+
+    __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
+    {
+        if (t.hidden[row] || !((par.comp_mask >> t.comp[row]) & 1u)) return -1;
+        return par.ncomp != 1 ? 1 : 0;
+    }
+    __device__ __forceinline__ void apply(gf_table &t, int64_t row, int kind, float u, const float *y, const float *s) const
+    {
         int at = 0;
-        if (par.ncomp != 1) {
-            const float u = r.uniform();
+        if (kind == 1)
             while (par.pcum[at] < u) ++at;
-        }
-        t.FeH[row] = par.mean[at] + r.gaussian(par.sigma[at]);
+        t.FeH[row] = par.mean[at] + par.sigma[at] * y[0] * s[0];
         t.FeH_comp[row] = at;
     }
-    rng[NS + th] = r.c;
-    rng[2 * NS + th] = r.x;
-}
+};
 
-template <int KIND>
-__global__ void __launch_bounds__(128) feh_kernel(const gf_feh_config fp, const gf_gaussfeh_config gp, uint32_t *rng,
-                                                  int32_t NS, gf_table t, int64_t begin, int64_t end, int64_t nchunks)
-{
-    const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (th >= nchunks) return;
-    if (KIND == 0) feh_chunk(fp, rng, NS, t, begin, end, th);
-    else gaussfeh_chunk(gp, rng, NS, t, begin, end, th);
-}
-
-/* the 256-row chunks of every request of a multi-request pass, each with its request's streams */
-template <int KIND>
-__global__ void __launch_bounds__(128) feh_multi_kernel(const gf_feh_config fp, const gf_gaussfeh_config gp,
-                                                        uint32_t *rng_all, int32_t NS, MultiRows R,
-                                                        const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks,
-                                                        const int64_t *slot_rows, gf_table t)
-{
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    int lo = 0, hi = nslots - 1;          /* last slot whose first chunk is <= c */
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const int64_t b = R.slot_row_begin[lo];
-    uint32_t *rng = rng_all + (size_t)R.slot_job[lo] * 3 * NS;
-    if (KIND == 0) feh_chunk(fp, rng, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo]);
-    else gaussfeh_chunk(gp, rng, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo]);
-}
-
-cudaError_t launch_feh(const gf_feh_config *fp, const gf_gaussfeh_config *gp, uint32_t *rng, int32_t NS, gf_table t,
+cudaError_t launch_feh(const gf_feh_config *fp, const gf_gaussfeh_config *gp, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t,
                        int64_t begin, int64_t end, cudaStream_t s)
 {
     if (end <= begin) return cudaSuccess;
     const int64_t n = end - begin, nchunks = n / 256 + (n % 256 ? 1 : 0);
     if (nchunks > NS) return cudaErrorInvalidValue;
-    gf_feh_config f = {};
-    gf_gaussfeh_config g = {};
-    if (fp) f = *fp;
-    if (gp) g = *gp;
-    if (fp) feh_kernel<0><<<(int)((nchunks + 127) / 128), 128, 0, s>>>(f, g, rng, NS, t, begin, end, nchunks);
-    else feh_kernel<1><<<(int)((nchunks + 127) / 128), 128, 0, s>>>(f, g, rng, NS, t, begin, end, nchunks);
-    count_launches(1);
-    return cudaGetLastError();
+    if (fp) {
+        FehOps o;
+        o.par = *fp;
+        return launch_stream_rows(o, pw, rng, NS, t, begin, end, nchunks, s);
+    }
+    GaussFehOps o;
+    o.par = *gp;
+    return launch_stream_rows(o, pw, rng, NS, t, begin, end, nchunks, s);
 }
 
-cudaError_t launch_feh_multi(const gf_feh_config *fp, const gf_gaussfeh_config *gp, uint32_t *rng_all, int32_t NS,
+cudaError_t launch_feh_multi(const gf_feh_config *fp, const gf_gaussfeh_config *gp, const StreamPowers &pw, uint32_t *rng_all, int32_t NS,
                              MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks,
                              const int64_t *slot_rows, gf_table t, cudaStream_t s)
 {
     if (nchunks <= 0) return cudaSuccess;
-    gf_feh_config f = {};
-    gf_gaussfeh_config g = {};
-    if (fp) f = *fp;
-    if (gp) g = *gp;
-    const unsigned blocks = (unsigned)((nchunks + 127) / 128);
-    if (fp) feh_multi_kernel<0><<<blocks, 128, 0, s>>>(f, g, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
-    else feh_multi_kernel<1><<<blocks, 128, 0, s>>>(f, g, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
-    count_launches(1);
-    return cudaGetLastError();
+    if (fp) {
+        FehOps o;
+        o.par = *fp;
+        return launch_stream_rows_multi(o, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t, s);
+    }
+    GaussFehOps o;
+    o.par = *gp;
+    return launch_stream_rows_multi(o, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t, s);
 }
 
 /* ---------------- unresolved multiple systems ---------------- */
@@ -387,104 +640,139 @@ __device__ __forceinline__ float mult_tex(const float *tab, int n, float x0, flo
     return tab[(uint32_t)xi];
 }
 
-/* draw_companion (unresolvedMultiples_gpu.cu.h:46-77) */
-__device__ __forceinline__ bool mult_companion(const gf_multiples_config &c, float M1, gfr::Mwc &r, float &M2)
-{
-    const float psec = mult_tex(c.secprob, c.nsec, c.sec_x0, c.sec_inv_dx, M1);
-    float u = r.uniform();
-    if (u > psec) return false;
-    if (c.algo == GF_MULT_EQUAL_MASS) { M2 = M1; return true; }
-    const float pprim = mult_tex(c.cumlf, c.ncum, c.cum_x0, c.cum_inv_dx, M1);
-    u = r.uniform();
-    /* fainter than the primary: u rescaled into [pprim, 1] in double, as written */
-    if (c.algo == GF_MULT_LF_M2_GT_M1) u = (float)((double)pprim + (double)u * (1. - (double)pprim));
-    M2 = mult_tex(c.invcumlf, c.ninv, c.inv_x0, c.inv_inv_dx, u);
-    if (c.algo == GF_MULT_LF_M2_GT_M1 && M2 < M1) M2 = M1;
-    return true;
-}
+/* os_unresolvedMultiples_kernel's row (unresolvedMultiples_gpu.cu.h:46-123) with two system
+ * components: a uniform against the binary fraction and, for a companion drawn from the
+ * luminosity function, a second one */
+struct MultOps {
+    gf_multiples_config c;
 
-/* os_unresolvedMultiples_kernel (unresolvedMultiples_gpu.cu.h:80-123) on rows
- * [begin + 256 th, ...) with stream th; two system components (absmagSys[2]) */
-__device__ __forceinline__ void multiples_chunk(const gf_multiples_config &c, uint32_t *rng, int32_t NS, gf_table &t,
-                                                int64_t begin, int64_t end, int64_t th)
-{
-    const int64_t P = t.capacity;
-    gfr::Mwc r;
-    r.a = rng[th]; r.c = rng[NS + th]; r.x = rng[2 * NS + th]; r.used = 0;
-    int64_t rb = begin + 256 * th, re = begin + 256 * (th + 1);
-    if (re > end) re = end;
-    for (int64_t row = rb; row < re; row++) {
+    __device__ __forceinline__ bool active(const gf_table &t, int64_t row) const
+    {
+        return !t.hidden[row] && ((c.comp_mask >> t.comp[row]) & 1u);
+    }
+    __device__ __forceinline__ float fraction(const gf_table &t, int64_t row) const
+    {
+        return mult_tex(c.secprob, c.nsec, c.sec_x0, c.sec_inv_dx, t.absmag[row]);
+    }
+    __device__ __forceinline__ void single(gf_table &t, int64_t row) const
+    {
+        t.absmagSys[row] = t.absmag[row];
+        t.absmagSys[t.capacity + row] = 99.999f;
+        t.absmagSysNcomp[row] = 1;
+    }
+    /* companion: whether one was drawn; u: its uniform (not used by equal-mass pairs) */
+    __device__ __forceinline__ void apply(gf_table &t, int64_t row, bool companion, float u) const
+    {
+        const int64_t P = t.capacity;
         const float M1 = t.absmag[row];
-        if (t.hidden[row] || !((c.comp_mask >> t.comp[row]) & 1u)) {
-            /* a single star */
-            t.absmagSys[row] = M1;
-            t.absmagSys[P + row] = 99.999f;
-            t.absmagSysNcomp[row] = 1;
-            continue;
-        }
         t.absmagSys[row] = M1;
         float Ltot = gfm::exp10f_(-0.4f * M1);
         int ncomps = 1;
-        float M2 = 0.f;
-        if (mult_companion(c, M1, r, M2)) {
-            t.absmagSys[P + row] = M2;
+        float M2 = 99.999f;
+        if (companion) {
+            if (c.algo == GF_MULT_EQUAL_MASS) {
+                M2 = M1;
+            } else {
+                const float pprim = mult_tex(c.cumlf, c.ncum, c.cum_x0, c.cum_inv_dx, M1);
+                /* fainter than the primary: u rescaled into [pprim, 1] in double, as written */
+                if (c.algo == GF_MULT_LF_M2_GT_M1) u = (float)((double)pprim + (double)u * (1. - (double)pprim));
+                M2 = mult_tex(c.invcumlf, c.ninv, c.inv_x0, c.inv_inv_dx, u);
+                if (c.algo == GF_MULT_LF_M2_GT_M1 && M2 < M1) M2 = M1;
+            }
             Ltot += gfm::exp10f_(-0.4f * M2);
             ncomps++;
-        } else {
-            t.absmagSys[P + row] = 99.999f;
         }
+        t.absmagSys[P + row] = M2;
         /* -2.5 is a double: the product is formed in double and stored as float */
         t.absmag[row] = (float)(-2.5 * (double)gfm::log10f_(Ltot));
         t.absmagSysNcomp[row] = ncomps;
     }
-    rng[NS + th] = r.c;
-    rng[2 * NS + th] = r.x;
-}
+};
 
-__global__ void __launch_bounds__(128) multiples_kernel(const gf_multiples_config c, uint32_t *rng, int32_t NS, gf_table t,
-                                                        int64_t begin, int64_t end, int64_t nchunks)
+/* rows [begin + 256 th, ...) with stream th on one warp: at most two uniforms a row, so one run of 512 serves
+ * the chunk; the walk over the rows only counts them, the magnitudes are formed by all lanes */
+__device__ __forceinline__ void chunk_rows(const MultOps &ops, const JumpTables &jt, const uint32_t *mult, uint32_t *rng,
+                                           int32_t NS, gf_table &t, int64_t begin, int64_t end, int64_t th, RowStream &S)
 {
-    const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (th >= nchunks) return;
-    multiples_chunk(c, rng, NS, t, begin, end, th);
-}
-
-__global__ void __launch_bounds__(128) multiples_multi_kernel(const gf_multiples_config c, uint32_t *rng_all, int32_t NS,
-                                                              MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots,
-                                                              int64_t nchunks, const int64_t *slot_rows, gf_table t)
-{
-    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nchunks) return;
-    int lo = 0, hi = nslots - 1;          /* last slot whose first chunk is <= k */
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (slot_chunk_begin[mid] <= k) lo = mid; else hi = mid - 1;
+    const int lane = threadIdx.x & 31;
+    const int64_t rb = begin + 256 * th;
+    const int nrow = (int)(end - rb < 256 ? end - rb : 256);
+    float *psec = (float *)S.next;                     /* binary fraction of each active row */
+    int na = 0;
+    for (int q = 0; q < nrow; q += 32) {
+        const int i = q + lane;
+        const bool in = i < nrow, on = in && ops.active(t, rb + i);
+        const unsigned m = __ballot_sync(0xffffffffu, on);
+        if (on) {
+            const int k = na + __popc(m & ((1u << lane) - 1u));
+            S.list[k] = (uint16_t)i;
+            psec[k] = ops.fraction(t, rb + i);
+        } else if (in) {
+            ops.single(t, rb + i);
+        }
+        na += __popc(m);
     }
-    const int64_t b = R.slot_row_begin[lo];
-    uint32_t *rng = rng_all + (size_t)R.slot_job[lo] * 3 * NS;
-    multiples_chunk(c, rng, NS, t, b, b + slot_rows[lo], k - slot_chunk_begin[lo]);
+    if (na == 0) return;
+    const bool two = ops.c.algo != GF_MULT_EQUAL_MASS;
+    const RowJump j = row_jump(jt, mult, rng, th);
+    uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
+    constexpr int R = 16;
+    uint64_t w0;
+    const bool run = stream_runs<R>(j, v, lane, w0);
+    if (run) {
+        uint64_t w = w0;
+#pragma unroll 4
+        for (int s = 0; s < R; s++) S.u[s * GF_RUN_PITCH + lane] = row_step(w, j.a);
+    }
+    __syncwarp();
+    int q = 0;
+    for (int r = 0; r < na; r++) {
+        /* (a state outside the Lehmer range: its uniforms one after another, from every lane's copy of v) */
+        const float u = run ? S.u[q] : row_step(v, j.a);
+        const bool companion = !(u > psec[r]);
+        const float u2 = run || !(companion && two) ? 0.f : row_step(v, j.a);
+        if (lane == 0) {
+            S.start[r] = (uint16_t)(q | (companion ? 0x8000 : 0));
+            if (!run) S.u[256 + r] = u2;
+        }
+        q = run_forward<R>(q);
+        if (companion && two) q = run_forward<R>(q);
+        if (!run) q = r + 1;
+    }
+    __syncwarp();
+    for (int r = lane; r < na; r += 32) {
+        const int st = S.start[r];
+        const bool companion = (st & 0x8000) != 0;
+        float u2 = 0.f;
+        if (companion && two) u2 = run ? S.u[run_forward<R>(st & 0x7fff)] : S.u[256 + r];
+        ops.apply(t, rb + S.list[r], companion, u2);
+    }
+    const uint64_t ve = run ? stream_state_at<R>(j.a, w0, q, lane) : v;
+    if (lane == 0) {
+        rng[NS + th] = (uint32_t)(ve >> 32);
+        rng[2 * NS + th] = (uint32_t)ve;
+    }
 }
 
-cudaError_t launch_multiples(const gf_multiples_config &c, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
+cudaError_t launch_multiples(const gf_multiples_config &c, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
                              cudaStream_t s)
 {
     if (end <= begin) return cudaSuccess;
     const int64_t n = end - begin, nchunks = n / 256 + (n % 256 ? 1 : 0);
     if (nchunks > NS) return cudaErrorInvalidValue;
-    multiples_kernel<<<(int)((nchunks + 127) / 128), 128, 0, s>>>(c, rng, NS, t, begin, end, nchunks);
-    count_launches(1);
-    return cudaGetLastError();
+    MultOps o;
+    o.c = c;
+    return launch_stream_rows(o, pw, rng, NS, t, begin, end, nchunks, s);
 }
 
-cudaError_t launch_multiples_multi(const gf_multiples_config &c, uint32_t *rng_all, int32_t NS, MultiRows R,
+cudaError_t launch_multiples_multi(const gf_multiples_config &c, const StreamPowers &pw, uint32_t *rng_all, int32_t NS, MultiRows R,
                                    const int64_t *slot_chunk_begin, int32_t nslots, int64_t nchunks, const int64_t *slot_rows,
                                    gf_table t, cudaStream_t s)
 {
     if (nchunks <= 0) return cudaSuccess;
-    multiples_multi_kernel<<<(unsigned)((nchunks + 127) / 128), 128, 0, s>>>(c, rng_all, NS, R, slot_chunk_begin, nslots,
-                                                                             nchunks, slot_rows, t);
-    count_launches(1);
-    return cudaGetLastError();
+    MultOps o;
+    o.c = c;
+    return launch_stream_rows_multi(o, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t, s);
 }
 
 /* ---------------- photometry ---------------- */

@@ -1315,6 +1315,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             GF_TRY(gfa::zero_module_rows(ctx, &out, total));
             out.systems = J0.multiples ? 1 : 0;
             /* the module chain in pipeline order (pipeline.h:75-88) over every request's rows */
+            const gfk::StreamPowers powers = {ctx->jt, ctx->d_mult};
             gfk::MultiRows MR;
             MR.row_slot = row_slot.p; MR.slot_row_begin = d_row_begin; MR.slot_job = d_slot_job;
             if (total > 0) {
@@ -1326,20 +1327,20 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 if (J0.feh_ivezic || J0.feh_gauss) {
                     ProfScope ps(ctx, GF_PROF_FEH);
                     if (J0.feh_ivezic)
-                        GF_CUDA(gfk::launch_feh_multi(J0.feh_ivezic, nullptr, d_rng, NS, MR, d_chunk_begin, nslots, nchunks,
+                        GF_CUDA(gfk::launch_feh_multi(J0.feh_ivezic, nullptr, powers, d_rng, NS, MR, d_chunk_begin, nslots, nchunks,
                                                       d_slot_rows, out, st));
                     if (J0.feh_gauss)
-                        GF_CUDA(gfk::launch_feh_multi(nullptr, J0.feh_gauss, d_rng, NS, MR, d_chunk_begin, nslots, nchunks,
+                        GF_CUDA(gfk::launch_feh_multi(nullptr, J0.feh_gauss, powers, d_rng, NS, MR, d_chunk_begin, nslots, nchunks,
                                                       d_slot_rows, out, st));
                 }
                 if (J0.multiples) {
                     ProfScope ps(ctx, GF_PROF_FEH);
-                    GF_CUDA(gfk::launch_multiples_multi(*J0.multiples, d_rng, NS, MR, d_chunk_begin, nslots, nchunks, d_slot_rows,
+                    GF_CUDA(gfk::launch_multiples_multi(*J0.multiples, powers, d_rng, NS, MR, d_chunk_begin, nslots, nchunks, d_slot_rows,
                                                         out, st));
                 }
                 if (J0.kin) {
                     ProfScope ps(ctx, GF_PROF_BOND2010);
-                    GF_CUDA(gfk::launch_bond2010_multi(*J0.kin, d_rng, NS, MR, d_chunk_begin, nslots, nchunks, d_slot_rows, out, st));
+                    GF_CUDA(gfk::launch_bond2010_multi(*J0.kin, powers, d_rng, NS, MR, d_chunk_begin, nslots, nchunks, d_slot_rows, out, st));
                 }
                 int s0 = 0;
                 while (s0 < nslots) {
