@@ -9,25 +9,24 @@
  * The arrangement is this library's, for requests whose nm * nM is a multiple
  * of 10 (so every pixel's blocks start at local indices 0, 10, 20, ...):
  *
- *   slot densities  (warp per pixel) the model density at each slot distance of
- *                   the request's anchor plan along the pixel's direction: the
- *                   anchor quantity that depends on the pixel.  The anchor of any
- *                   bin is then a table lookup: block-start anchors through the
- *                   plan's per-block slot, diagonal starts through its
- *                   per-diagonal slot.
- *   draw            one warp per 32 consecutive streams, one lane per stream.
- *                   The lanes' blocks at the same step are consecutive blocks of
- *                   one pixel (stream t + L takes block t + L + r N at step r), so
- *                   the plan and slot-density loads coalesce.  Each lane computes
- *                   mu of its block's 10 bins in registers and walks them with
- *                   plain MWC steps; the lanes whose bin has stars run the
- *                   reference's Poisson sampler and the star uniforms together,
- *                   record the bin (an event: its k and the stream state at its
- *                   first star) and walk on from the state after the stars.
+ *   block words     the model density at each slot distance of the request's anchor plan
+ *                   along the pixel's direction (the anchor quantity that depends on the
+ *                   pixel), and from them one 32-bit word per block of 10 bins and row of
+ *                   up to 4 neighbouring pixels with the same cut: how many bins are live
+ *                   (not cut), and a threshold that no uniform of an empty block's bins
+ *                   reaches in any of the row's pixels.
+ *   draw            one warp per 32 consecutive streams, one lane per stream.  Stream t
+ *                   takes blocks t, t + N, t + 2N, ... of the request: a step loads the
+ *                   word of the lane's next block, steps the MWC over the live bins and
+ *                   compares the largest uniform with the threshold.  A lane whose block
+ *                   may hold stars parks; when enough lanes are parked they find their
+ *                   first candidate bin together, test it exactly, run the reference's
+ *                   Poisson sampler and the star uniforms, record the bin (an event: its k
+ *                   and the stream state at its first star) and go on with the bins after it.
  *   expand          (thread per event) the star records of each event, regenerated
  *                   from its stream state, at offsets from a scan over k.
- * The stream states left behind are the reference's, for the modules that
- * continue the streams (Bond2010).
+ *
+ * The streams' final states are written back for the modules that continue them (Bond2010).
  */
 #include "gf_crawl.cuh"
 #include "gf_launch.h"
@@ -39,14 +38,11 @@ namespace gfk {
 namespace {
 
 #define BD_FULL 0xffffffffu
-#define GF_EVBUF 32                /* events staged in shared memory per warp */
-
-__device__ __forceinline__ float bd_mwc_step(uint64_t &v, uint32_t a)
-{
-    const uint64_t t = (uint64_t)a * (uint32_t)v + (v >> 32);
-    v = t;
-    return GF_MWC_SCALE * (float)(uint32_t)t;
-}
+#define GF_EVBUF 64                /* events staged in shared memory per warp (a pass over the parked lanes adds at most 32) */
+#define GF_BINS 0x3ffu             /* the bins of a block as bits */
+#define GF_NLIVE 0xfu              /* a block word: number of live bins below, threshold / 16 above */
+#define GF_DEAD_WORD 0xfffffff0u   /* no live bins, nothing reaches the threshold */
+#define GF_END_WORD 0xffffffffu    /* past the stream's last block */
 
 /* one MWC step; returns the new x (the uniform is 2^-32 x) */
 __device__ __forceinline__ uint32_t bd_mwc_x(uint64_t &v, uint32_t a)
@@ -68,138 +64,19 @@ __device__ __forceinline__ bool bd_has_stars(float u, float mu)
     return mu > 10.f || gfr::exceeds_exp_neg(u, mu);
 }
 
-/* a request's view for the draw walk (per warp, in shared memory) */
-struct DrawJobView {
-    const uint32_t *blk, *binfo;
-    const uint16_t *bslot, *dslot;
-    const float *slotD;
-    const float2 *ms2;             /* per pixel: (density, D^3) of each slot, then (first cut row, K) */
-    const uint4 *brec;             /* per block: blk, binfo, bslot | first diagonal-start slot << 16, LF max */
-    const gf_pencil_beam *pixels;
-    int nslots, Bp, npix, x, y, N;
-    int QN, RN;                    /* N = QN Bp + RN: a stream's step in (pixel, block) */
-    float norm, dmin, dmax;
-    bool dlim, bound;
-};
-
 template <class T>
 __device__ __forceinline__ const T *plan_at(const unsigned char *plan, int off)
 {
     return (const T *)(plan + off);
 }
 
-template <int MODEL>
-__global__ void __launch_bounds__(256) slot_density_kernel(SlotDensityParams P)
-{
-    const int lane = threadIdx.x & 31;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
-    for (int p = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < P.total_pix; p += nwarps) {
-        int lo = 0, hi = P.njobs;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (P.pix_off[mid] <= p) lo = mid; else hi = mid;
-        }
-        const int job = P.job_list[lo];
-        const int ilb = p - P.pix_off[lo];
-        const CrawlJob &J = P.jobs[job];
-        const unsigned char *plan = P.plans[job];
-        const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
-        const int nslots = h->nslots;
-        const float *slotD = plan_at<float>(plan, h->off_slot);
-        const gf_pencil_beam pix = J.g.pixels[ilb];
-        float2 *row = P.ms[job] + (size_t)ilb * (nslots + 1);
-        for (int s = lane; s < nslots; s += 32) {
-            const float D = slotD[s];
-            const float px = D * pix.cl * pix.cb;
-            const float py = D * pix.sl * pix.cb;
-            const float pz = D * pix.sb;
-            /* D^3 with the reference's float product (skygen.cu.h:554) */
-            row[s] = make_float2(gfc::model_rho<MODEL>(J.m, px, py, pz), D * D * D);
-        }
-        /* the pixel's first cut apparent-magnitude row (m0 + dm im + Am > m1; increasing in im)
-         * and its volume factor K = dA * POGSON * dm * dM */
-        const SkyModel &m = J.m;
-        const float Am = gfc::beam_extinction(J.g, pix);
-        int icut = m.nm;
-        for (int i = lane; i < m.nm; i += 32)
-            if (m.m0 + m.dm * (float)i + Am > m.m1) { icut = i; break; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const int t = __shfl_xor_sync(0xffffffffu, icut, o);
-            icut = t < icut ? t : icut;
-        }
-        if (lane == 0) row[nslots] = make_float2(__int_as_float(icut), pix.dA * GF_POGSON * m.dm * m.dM);
-    }
-}
-
-/* A bin with stars, on the lane (stream) that found it: the reference's Poisson
- * sampler from the bin's stream state wb, then the stars' uniforms (draw_stars:
- * x, y, and M, m unless x^2 + y^2 > 2).  Returns the number of stars and the
- * stream state after them; fills the event record when there are stars. */
-__device__ __forceinline__ int draw_event(uint32_t a, uint64_t wb, float mu, const gf_pencil_beam *pp, uint64_t &vnew,
-                                       uint64_t &v_star)
-{
-    gfr::Mwc r;
-    r.a = a;
-    r.set_v(wb);
-    r.used = 0;
-    const int k = (int)r.poisson(mu);
-    v_star = r.v();
-    if (k > 0) {
-        const float X = pp->X, Y = pp->Y, dx = pp->dx;
-        for (int n = 0; n < k; n++) {
-            const float u0 = r.uniform();
-            const float u1 = r.uniform();
-            float xx = X, yy = Y;
-            xx += dx * (u0 - 0.5f);
-            yy += dx * (u1 - 0.5f);
-            if (!(xx * xx + yy * yy > 2.f)) {
-                r.uniform();
-                r.uniform();
-            }
-        }
-    }
-    vnew = r.v();
-    return k;
-}
-
-/* stage one event from divergent code (any lanes of the warp) */
-__device__ __forceinline__ void stage_event(const BatchDrawParams &P, EventRecord *evb, int *nev, const EventRecord &e)
-{
-    const int q = atomicAdd(nev, 1);
-    if (q < GF_EVBUF) {
-        evb[q] = e;
-    } else {
-        const unsigned long long sl = atomicAdd(P.ev_count, 1ull);
-        if (sl < (unsigned long long)P.ev_capacity) P.ev[sl] = e;
-    }
-}
-
-/* write the warp's staged events to the global list (all lanes) */
-__device__ __forceinline__ void flush_events(const BatchDrawParams &P, EventRecord *evb, int *nev, int lane)
-{
-    __syncwarp();
-    const int n = *nev < GF_EVBUF ? *nev : GF_EVBUF;     /* events past the buffer went straight to the list */
-    if (n == 0) {
-        if (lane == 0) *nev = 0;
-        __syncwarp();
-        return;
-    }
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(P.ev_count, (unsigned long long)n);
-    base = __shfl_sync(BD_FULL, base, 0);
-    for (int q = lane; q < n; q += 32)
-        if (base + q < (unsigned long long)P.ev_capacity) P.ev[base + q] = evb[q];
-    __syncwarp();
-    if (lane == 0) *nev = 0;
-    __syncwarp();
-}
-
-/* Per request of a chunk and block of its grid, the record the bound walk loads
- * in one piece: the block's first bin (i | j << 16), its binfo word, its
- * block-start slot | the slot of its first diagonal start << 16, and the largest
- * LF value over its 10 bins (the same LF(M) samples the draw's shared table
- * holds; negative values count as 0). */
+/* Per request of a chunk and block of its grid: the block's first bin (i | j << 16), its
+ * binfo word, its block-start slot | the slot of its first diagonal start << 16, and a bound
+ * C of LF(M) D^3 norm over its 10 bins (negative values count as 0; NaN where the
+ * bound does not hold: a negative density factor or normalisation).  A bin's expected count
+ * (((LF ms) norm) D^3) K, four rounded products of non-negative factors, is at most
+ * (1 + 2^-24)^4 its exact value, and C ms K with ms the largest density of the block's
+ * slots is at least (1 - 2^-24)^6 (1 + 1e-6) times that: the factor 1 + 1e-6 covers all ten. */
 __global__ void __launch_bounds__(256) block_records_kernel(BlockLfParams P)
 {
     for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < P.total; f += (long long)gridDim.x * blockDim.x) {
@@ -213,45 +90,292 @@ __global__ void __launch_bounds__(256) block_records_kernel(BlockLfParams P)
         const SkyModel &m = P.jobs[job].m;
         const unsigned char *plan = P.plans[job];
         const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
+        const float *slotD = plan_at<float>(plan, h->off_slot);
+        const uint16_t *dslot = plan_at<uint16_t>(plan, h->off_dslot);
         const uint32_t bij = plan_at<uint32_t>(plan, h->off_blk)[b];
         int i = (int)(bij & 0xffffu), j = (int)(bij >> 16);
         const uint32_t bi = plan_at<uint32_t>(plan, h->off_binfo)[b];
-        const uint32_t wm = (bi >> 16) & 0x3ffu;
+        const uint32_t wm = (bi >> 16) & GF_BINS;
         const uint32_t s0 = plan_at<uint16_t>(plan, h->off_bslot)[b];
-        const uint32_t s1 = wm ? plan_at<uint16_t>(plan, h->off_dslot)[i + j + 1] : 0u;
+        const uint32_t s1 = wm ? dslot[i + j + 1] : 0u;
+        float D = slotD[s0];
         float mx = gfc::lf_sample(m, m.lf, m.M1 - (float)j * m.dM);
         for (int s = 1; s < GF_BLOCK; s++) {
-            gfc::step_in_pixel(i, j, m.nm, m.nM);
+            if (gfc::step_in_pixel(i, j, m.nm, m.nM)) D = fmaxf(D, slotD[dslot[i + j]]);
             mx = fmaxf(mx, gfc::lf_sample(m, m.lf, m.M1 - (float)j * m.dM));
         }
-        P.brec[job][b] = make_uint4(bij, bi, s0 | (s1 << 16), __float_as_uint(fmaxf(mx, 0.f)));
+        float C = fmaxf(mx, 0.f) * m.norm;
+        C *= D * D * D;
+        C *= 1.0f + 1.0e-6f;
+        if (!(m.f >= 0.f && m.norm >= 0.f)) C = __int_as_float(0x7fffffff);
+        P.brec[job][b] = make_uint4(bij, bi, s0 | (s1 << 16), __float_as_uint(C));
+        /* a request's threads also sample its LF(M) at every absolute-magnitude row */
+        for (int q = b; q < m.nM; q += h->nblocks) P.lfm[job][q] = gfc::lf_sample(m, m.lf, m.M1 - (float)q * m.dM);
     }
 }
 
-/* One warp per 32 consecutive streams of a request, one lane per stream.  Lane L
- * walks its stream block by block: the blocks of the 32 streams at the same step
- * are 32 consecutive blocks of (mostly) one pixel, so the table loads coalesce.
- * Lanes whose bin has stars run the sampler together and go on from the state
- * after the stars.  BOUND: every request of the launch takes the block bound
- * (non-negative densities, no distance limits, per-block LF maxima present);
- * otherwise every bin's expected count is formed and tested exactly. */
-template <int MODEL, bool BOUND>
-__global__ void __launch_bounds__(256, 4) batch_draw_kernel(BatchDrawParams P)
+/* The live bins of a block: im below the pixel's cut row, and the anchor's distance inside [dmin, dmax).
+ * At most one diagonal start (bin p): bins before it continue the first diagonal (im = i0 + s), bins from it
+ * on the next one from im = max(0, d + 1 - (nM - 1)); each run's live bins are a prefix of it. */
+__device__ __forceinline__ uint32_t block_live(const uint4 &br, int icut, int nM)
+{
+    const int i0 = (int)(br.x & 0xffffu), j0 = (int)(br.x >> 16);
+    if ((int)(br.y & 0xffffu) < icut) return GF_BINS;                       /* the block's largest im */
+    const uint32_t wm = (br.y >> 16) & GF_BINS;
+    if (!(wm & (wm - 1u))) {
+        const int p = wm ? __ffs(wm) - 1 : GF_BLOCK;
+        const int iB = max(0, i0 + j0 + 1 - (nM - 1));
+        uint32_t live = (1u << min(p, max(0, icut - i0))) - 1u;
+        if (wm) live |= ((1u << min(GF_BLOCK - p, max(0, icut - iB))) - 1u) << p;
+        return live;
+    }
+    /* several diagonal starts (short diagonals at the grid's corners) */
+    int ii = i0, dd = i0 + j0;
+    uint32_t live = ii < icut ? 1u : 0u;
+    for (int s = 1; s < GF_BLOCK; s++) {
+        if ((wm >> s) & 1u) {
+            dd++;
+            ii = max(0, dd - (nM - 1));
+        } else {
+            ii++;
+        }
+        live |= ii < icut ? (1u << s) : 0u;
+    }
+    return live;
+}
+
+/* the bins of a block whose anchor lies in [dmin, dmax) */
+__device__ __noinline__ uint32_t block_inside(const uint4 &br, const float *slotD, const uint16_t *dslot, float dmin, float dmax)
+{
+    const uint32_t wm = (br.y >> 16) & GF_BINS;
+    int d = (int)(br.x & 0xffffu) + (int)(br.x >> 16);
+    float D = slotD[br.z & 0xffffu];
+    uint32_t in = 0;
+    for (int s = 0; s < GF_BLOCK; s++) {
+        if ((wm >> s) & 1u) D = slotD[dslot[++d]];
+        in |= (dmin > D || dmax <= D) ? 0u : 1u << s;
+    }
+    return in;
+}
+
+/* A CTA takes up to P.tile rows of one request: the slot densities of their pixels (a warp a
+ * row) into the request's tables, for the exact tests of candidate bins, and each slot's largest
+ * in the row into shared memory; then every block's word, a thread's block for all the tile's
+ * rows (the block record is decoded once).  Pixels of a row are neighbours: their densities
+ * differ by a few percent, and so do the thresholds' candidates from each pixel's own. */
+template <int MODEL>
+__global__ void __launch_bounds__(256) block_words_kernel(BlockWordParams P)
+{
+    extern __shared__ __align__(16) float s_ms[];      /* [tile][nslots] */
+    __shared__ SkyModel m;
+    __shared__ int s_icut[GF_WORD_TILE];
+    __shared__ float s_K[GF_WORD_TILE];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int loaded = -1;
+    for (int unit = blockIdx.x; unit < P.total_tiles; unit += gridDim.x) {
+        int lo = 0, hi = P.njobs;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (P.tile_off[mid] <= unit) lo = mid; else hi = mid;
+        }
+        const int job = P.job_list[lo];
+        const CrawlJob &J = P.jobs[job];
+        const DrawJob &V = P.view[job];
+        const int q0 = (unit - P.tile_off[lo]) * P.tile;             /* within the segment's rows */
+        const int nr = min(V.nrows - q0, P.tile);
+        __syncthreads();
+        if (job != loaded) {
+            for (int w = tid; w < (int)(sizeof(SkyModel) / 4); w += blockDim.x) ((uint32_t *)&m)[w] = ((const uint32_t *)&J.m)[w];
+            loaded = job;
+            __syncthreads();
+        }
+        const int nslots = V.nslots;
+        for (int q = warp; q < nr; q += 8) {
+            const int row = V.row0 + q0 + q;
+            const int pa = max(V.rowpx[row], V.px0), pb = min(V.rowpx[row + 1], V.px0 + V.npx);
+            float K = 0.f;
+            for (int p = pa; p < pb; p++) {
+                const gf_pencil_beam pix = J.g.pixels[p];
+                K = fmaxf(K, pix.dA * GF_POGSON * m.dm * m.dM);
+                if (lane == 0) V.roff[p - V.px0] = (uint32_t)(q0 + q) * (uint32_t)V.Bp;
+                float *ms_row = V.ms + (size_t)(p - V.px0) * nslots;
+                for (int s = lane; s < nslots; s += 32) {
+                    const float D = V.slotD[s];
+                    const float px = D * pix.cl * pix.cb;
+                    const float py = D * pix.sl * pix.cb;
+                    const float pz = D * pix.sb;
+                    const float ms = gfc::model_rho<MODEL>(m, px, py, pz);
+                    ms_row[s] = ms;
+                    s_ms[q * nslots + s] = p == pa ? ms : fmaxf(s_ms[q * nslots + s], ms);
+                }
+            }
+            if (lane == 0) {
+                s_icut[q] = (int)(V.prow[pa].y & 0xffffu);
+                s_K[q] = K;
+            }
+        }
+        __syncthreads();
+        const bool dlim = m.dmin != 0.f || m.dmax != 0.f;
+        uint32_t *words = V.words + (size_t)q0 * V.Bp;
+        for (int lb = tid; lb < V.Bp; lb += blockDim.x) {
+            const uint4 br = __ldg(V.brec + lb);
+            const uint32_t wm = (br.y >> 16) & GF_BINS;
+            const bool several = (wm & (wm - 1u)) != 0;
+            const int s0 = (int)(br.z & 0xffffu), s1 = wm ? (int)(br.z >> 16) : s0;
+            const float C = __uint_as_float(br.w);
+            const uint32_t in = dlim ? block_inside(br, V.slotD, V.dslot, m.dmin, m.dmax) : GF_BINS;
+            int icut = -1;
+            uint32_t n = 0;
+            for (int q = 0; q < nr; q++) {
+                if (s_icut[q] != icut) {
+                    icut = s_icut[q];
+                    n = __popc(block_live(br, icut, m.nM) & in);
+                }
+                const float *ms = s_ms + q * nslots;
+                float msmax = fmaxf(ms[s0], ms[s1]);
+                if (several) {
+                    int d = (int)(br.x & 0xffffu) + (int)(br.x >> 16) + 1;
+                    for (uint32_t mm = wm & (wm - 1u); mm; mm &= mm - 1u) msmax = fmaxf(msmax, ms[V.dslot[++d]]);
+                }
+                const float mub = C * msmax * s_K[q];
+                /* u <= 1 - mub - 3e-7 proves a bin empty; x <= X implies it (uniform_threshold_lower), and the
+                 * word keeps X rounded down to 16s: a bin is a candidate when x >= that (conversion of a
+                 * negative or NaN threshold gives 0: every bin is one; so it is without a bound, C NaN) */
+                const uint32_t X = __float2uint_rz(((1.0f - mub) - 3.0e-7f) * 4294967296.0f * 0.99999976f);
+                words[(size_t)q * V.Bp + lb] = n ? (X & ~GF_NLIVE) | n : GF_DEAD_WORD;
+            }
+        }
+    }
+}
+
+/* A candidate bin on the lane (stream) that found it: whether its stars k > 0, from the first
+ * uniform u (drawn from state wb; w the state after it).  The reference's Poisson sampler: the
+ * product of uniforms against exp(-mu), bracketed as in Mwc::poisson_small, or for large means its
+ * gamma and binomial stages from wb.  w becomes the state after the sampler. */
+__device__ __forceinline__ int draw_count(uint32_t a, uint64_t wb, float u, float mu, uint64_t &w)
+{
+    if (mu >= GF_FASTEXP_MIN_MU && mu <= 10.f) {
+        const float ea = __expf(-mu);
+        const float lo = ea * (1.0f - GF_FASTEXP_MARGIN), hi = ea * (1.0f + GF_FASTEXP_MARGIN);
+        float prod = u;
+        int k = 0;
+        for (;;) {
+            if (prod <= lo) break;
+            if (!(prod > hi) && !(prod > gfm::expf_(-mu))) break;
+            k++;
+            prod *= GF_MWC_SCALE * (float)bd_mwc_x(w, a);
+        }
+        return k;
+    }
+    if (!bd_has_stars(u, mu)) return 0;
+    gfr::Mwc r;
+    r.a = a;
+    r.set_v(wb);
+    r.used = 0;
+    const int k = (int)r.poisson(mu);
+    w = r.v();
+    return k;
+}
+
+/* the state after the uniforms of k stars (draw_stars: x, y, and M, m unless x^2 + y^2 > 2) */
+__device__ __forceinline__ uint64_t skip_stars(uint32_t a, uint64_t w, int k, bool edge, const gf_pencil_beam *pix)
+{
+    if (!edge) {
+        /* no point of the pixel lies beyond x^2 + y^2 = 2 */
+        for (int n = 0; n < 4 * k; n++) (void)bd_mwc_x(w, a);
+        return w;
+    }
+    const float X = pix->X, Y = pix->Y, dx = pix->dx;
+    for (int n = 0; n < k; n++) {
+        const float u0 = GF_MWC_SCALE * (float)bd_mwc_x(w, a);
+        const float u1 = GF_MWC_SCALE * (float)bd_mwc_x(w, a);
+        float xx = X, yy = Y;
+        xx += dx * (u0 - 0.5f);
+        yy += dx * (u1 - 0.5f);
+        if (!(xx * xx + yy * yy > 2.f)) {
+            (void)bd_mwc_x(w, a);
+            (void)bd_mwc_x(w, a);
+        }
+    }
+    return w;
+}
+
+/* write the warp's staged events to the global list (all lanes) */
+__device__ __forceinline__ void flush_events(const BatchDrawParams &P, EventRecord *evb, int *nev, int lane)
+{
+    __syncwarp();
+    const int n = *nev;
+    if (n == 0) return;
+    unsigned long long base = 0;
+    if (lane == 0) base = atomicAdd(P.ev_count, (unsigned long long)n);
+    base = __shfl_sync(BD_FULL, base, 0);
+    for (int q = lane; q < n; q += 32)
+        if (base + q < (unsigned long long)P.ev_capacity) P.ev[base + q] = evb[q];
+    __syncwarp();
+    if (lane == 0) *nev = 0;
+    __syncwarp();
+}
+
+/* n (at most 10) MWC steps from (c, x); returns the largest x of them.  Every lane takes the
+ * first six unconditionally (most) when all have as many bins: on this chip a step is a wide
+ * multiply-add, a move and a maximum, 7 cycles of a scheduler, and 5 more when predicated or
+ * selected.  Lanes with fewer bins are blocks that the magnitude cut crosses. */
+__device__ __forceinline__ uint32_t walk_bins(uint32_t &x, uint32_t &c, uint32_t a, uint32_t n)
+{
+    uint32_t mx = 0;
+    auto step = [&](uint32_t &xs, uint32_t &cs) {
+        asm("{\n\t.reg .u64 t;\n\tmov.b64 t, {%1, %4};\n\tmad.wide.u32 t, %2, %3, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
+            : "=r"(xs), "+r"(cs) : "r"(xs), "r"(a), "r"(0u));
+    };
+    if (__all_sync(BD_FULL, n >= 6u)) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            step(x, c);
+            mx = max(mx, x);
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            uint32_t x1 = x, c1 = c;
+            step(x1, c1);
+            const bool on = s < (int)n;
+            x = on ? x1 : x;
+            c = on ? c1 : c;
+            mx = max(mx, on ? x1 : 0u);
+        }
+    }
+#pragma unroll
+    for (int s = 6; s < GF_BLOCK; s++) {
+        uint32_t x1 = x, c1 = c;
+        step(x1, c1);
+        const bool on = s < (int)n;
+        x = on ? x1 : x;
+        c = on ? c1 : c;
+        mx = max(mx, on ? x1 : 0u);
+    }
+    return mx;
+}
+
+/* One warp per 32 consecutive streams of a request, one lane per stream.  A step of a lane
+ * is one block: its word (loaded three steps ahead), at most 10 MWC steps, one comparison.
+ * Almost every block is empty, and the few lanes that find a candidate bin would hold up
+ * the others if the warp served each at once; so they park and are served together, when
+ * their waiting has cost about what a service does (whatever the rate of candidates, that is
+ * within twice the best choice).  The lanes drift apart by the steps they waited; their words
+ * come from a table small enough for the caches.
+ * Bound by the integer pipes: a step takes about 160 scheduler cycles (104 of them the walk), a
+ * service about 430.  Measured, three models: 256 beams of 0.5-5 deg (5.1e9 blocks, 6.2e7 stars)
+ * 34 ms, against 64 ms when each warp bounded its blocks itself and walked those with candidates
+ * again at once; 64 beams 27 -> 11 ms.  With 64 registers (4 CTAs an SM) 38 ms at 256 beams; one vote
+ * per step or two instead of four, or three times the patience: 35 to 41 ms. */
+__global__ void __launch_bounds__(256, 3) batch_draw_kernel(BatchDrawParams P)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned char *mine = smem + (size_t)wib * P.warp_bytes;
-    SkyModel &m = *(SkyModel *)mine;
-    float *LFM = (float *)(mine + P.off_tab);
-    EventRecord *evb = (EventRecord *)(mine + P.off_ev);
+    EventRecord *evb = (EventRecord *)(smem + (size_t)wib * (sizeof(EventRecord) * GF_EVBUF + 16));
     int *nev = (int *)(evb + GF_EVBUF);
     if (lane == 0) *nev = 0;
     __syncwarp();
-
-    /* the request's tables and scalars live in the warp's shared memory, not in
-     * registers: the walk keeps its registers for the stream state and the block */
-    DrawJobView &V = *(DrawJobView *)(mine + P.off_view);
-    int loaded = -1;
 
     for (;;) {
         int it = 0;
@@ -260,356 +384,141 @@ __global__ void __launch_bounds__(256, 4) batch_draw_kernel(BatchDrawParams P)
         if (it >= P.nitems) break;
         const uint32_t wi = P.items[it];
         const int job = (int)(wi >> 16), t = (int)(wi & 0xffffu) + lane;
-        const CrawlJob &J = P.jobs[job];
-        if (job != loaded) {
-            __syncwarp();
-            const uint32_t *src = (const uint32_t *)&J.m;
-            for (int w = lane; w < (int)(sizeof(SkyModel) / 4); w += 32) ((uint32_t *)&m)[w] = src[w];
-            __syncwarp();
-            for (int q = lane; q < m.nM; q += 32) LFM[q] = gfc::lf_sample(m, m.lf, m.M1 - (float)q * m.dM);
-            if (lane == 0) {
-                const unsigned char *plan = P.plans[job];
-                const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
-                V.x = m.nm; V.y = m.nM; V.N = m.nthreads;
-                V.nslots = h->nslots;
-                V.Bp = h->nblocks;
-                V.QN = V.N / V.Bp;
-                V.RN = V.N - V.QN * V.Bp;
-                V.slotD = plan_at<float>(plan, h->off_slot);
-                V.blk = plan_at<uint32_t>(plan, h->off_blk);
-                V.bslot = plan_at<uint16_t>(plan, h->off_bslot);
-                V.dslot = plan_at<uint16_t>(plan, h->off_dslot);
-                V.binfo = plan_at<uint32_t>(plan, h->off_binfo);
-                V.ms2 = P.ms[job];
-                V.pixels = J.g.pixels;
-                V.npix = J.g.npixels;
-                V.norm = m.norm;
-                V.dmin = m.dmin;
-                V.dmax = m.dmax;
-                V.dlim = m.dmin != 0.f || m.dmax != 0.f;
-                V.brec = P.brec ? P.brec[job] : nullptr;
-                /* the block bound needs non-negative densities (f >= 0) and normalisation */
-                V.bound = V.brec && !V.dlim && m.f >= 0.f && m.norm >= 0.f;
-            }
-            __syncwarp();
-            loaded = job;
-        }
-        if (BOUND && !V.bound) {
-            /* the host put a request that needs the exact test into the bound launch */
-            if (lane == 0) atomicOr(P.err, 2ull);
-            continue;
-        }
-        const int NS = J.rng_nstreams;
-        uint32_t *rng = J.rng;
+        const DrawJob &V = P.view[job];
+        const uint32_t Bp = (uint32_t)V.Bp;
         const bool stream_ok = t < V.N;
+        const int NS = V.rng_nstreams;
+        uint32_t *rng = V.rng;
         const uint32_t a = stream_ok ? rng[t] : 0u;
         uint64_t w = stream_ok ? (((uint64_t)rng[NS + t] << 32) | rng[2 * NS + t]) : 0ull;
-        const int sid = (job << 16) | t;
-        /* block r of stream t is the (t + r N)-th block of the request */
-        int pix = stream_ok ? t / V.Bp : V.npix, lb = stream_ok ? t - (t / V.Bp) * V.Bp : 0;
-        int nst = 0;
-        bool stop = !stream_ok;
+        const uint32_t *words = V.words, *roff = V.roff;
+        const uint32_t npx = (uint32_t)V.npx, QN = (uint32_t)V.QN, RN = (uint32_t)V.RN;
+        uint32_t x = (uint32_t)w, c = (uint32_t)(w >> 32);
+        /* the block whose word is loaded next: pixel, block in the pixel, the words of the pixel's row.
+         * The stream's first block of the segment (block r of stream t is the request's t + r N -th): */
+        uint32_t lb = (uint32_t)(t >= V.first ? t - V.first : t - V.first + V.N);
+        uint32_t px = (__umulhi(lb, V.fB.mul) + lb) >> V.fB.shift;
+        lb -= px * Bp;
+        if (!stream_ok) px = npx;
+        uint32_t ro = px < npx ? __ldg(roff + px) : 0u;
+        auto next_word = [&]() {
+            const uint32_t word = px < npx ? __ldg(words + (ro + lb)) : GF_END_WORD;
+            px += QN;
+            lb += RN;
+            if (lb >= Bp) { lb -= Bp; px++; }
+            ro = px < npx ? __ldg(roff + px) : 0u;
+            return word;
+        };
+        uint32_t c0 = next_word(), c1 = next_word(), c2 = next_word();
+        int skip = 0;                  /* live bins of the current block that are done */
+        bool parked = false;
+        int idle = 0;                  /* rounds of four steps that parked lanes have waited */
         for (;;) {
-            const bool valid = !stop && pix < V.npix;
-            if (!__any_sync(BD_FULL, valid)) break;
-            if constexpr (BOUND) {
-                /* Upper bound of the block's expected counts: the reference's float product
-                 * with each factor at its largest over the block (correctly rounded products of
-                 * non-negative factors are monotone).  u <= 1 - bound - 3e-7 proves a bin
-                 * empty, so the walk only steps the stream over the block's live bins and
-                 * compares the largest uniform with the threshold; a block whose largest
-                 * uniform exceeds it is walked again with the exact expected counts. */
-                uint32_t live = 0;
-                bool any = false;
-                int64_t xthr = -1;             /* uniform u = 2^-32 x passes the bound iff x <= xthr */
-                uint4 br = make_uint4(0u, 0u, 0u, 0u);
-                const float2 *row = V.ms2;
-                float K = 0.f;
-                const uint64_t w0 = w;
-                if (valid) {
-                    br = __ldg(V.brec + lb);
-                    const int i0 = (int)(br.x & 0xffffu), j0 = (int)(br.x >> 16);
-                    const int imax = (int)(br.y & 0xffffu);
-                    const uint32_t wm = (br.y >> 16) & 0x3ffu;
-                    row = V.ms2 + (size_t)pix * (V.nslots + 1);
-                    const float2 ik = row[V.nslots];
-                    const int icut = __float_as_int(ik.x);
-                    K = ik.y;
-                    const float2 q0 = row[br.z & 0xffffu];
-                    float msmax = q0.x, D3max = q0.y;
-                    if (wm) {
-                        const float2 q1 = row[br.z >> 16];
-                        msmax = fmaxf(msmax, q1.x);
-                        D3max = fmaxf(D3max, q1.y);
-                        /* further diagonal starts in the block (short diagonals only) */
-                        int d = i0 + j0 + 1;
-                        for (uint32_t mm = wm & (wm - 1u); mm; mm &= mm - 1u) {
-                            d++;
-                            const float2 q2 = row[__ldg(V.dslot + d)];
-                            msmax = fmaxf(msmax, q2.x);
-                            D3max = fmaxf(D3max, q2.y);
-                        }
-                    }
-                    float mub = __uint_as_float(br.w) * msmax;
-                    mub *= V.norm;
-                    mub *= D3max;
-                    mub *= K;
-                    xthr = gfr::uniform_threshold_lower((1.0f - mub) - 3.0e-7f);
-                    if (imax < icut) {
-                        live = (1u << GF_BLOCK) - 1u;
-                    } else if (!(wm & (wm - 1u))) {
-                        /* At most one diagonal start (bin p): bins before it continue the
-                         * first diagonal (im = i0 + s), bins from it on the next one from
-                         * im = max(0, d + 1 - (y - 1)); a bin is live while im < icut, so
-                         * each run's live bins are a prefix of it. */
-                        const int p = wm ? __ffs(wm) - 1 : GF_BLOCK;
-                        live = (1u << min(p, max(0, icut - i0))) - 1u;
-                        if (wm) {
-                            const int dB = i0 + j0 + 1;
-                            const int iB = dB - (V.y - 1) > 0 ? dB - (V.y - 1) : 0;
-                            live |= ((1u << min(GF_BLOCK - p, max(0, icut - iB))) - 1u) << p;
-                        }
-                    } else {
-                        /* several diagonal starts (short diagonals at the grid's corners) */
-                        int ii = i0, dd = i0 + j0;
-                        live = ii < icut ? 1u : 0u;
-                        for (int s = 1; s < GF_BLOCK; s++) {
-                            if ((wm >> s) & 1u) {
-                                dd++;
-                                ii = dd - (V.y - 1) > 0 ? dd - (V.y - 1) : 0;
-                            } else {
-                                ii++;
-                            }
-                            live |= ii < icut ? (1u << s) : 0u;
-                        }
-                    }
-                    if (xthr < 0) {
-                        any = live != 0;               /* the bound proves nothing: exact test throughout */
-                    } else {
-                        /* one predicated walk for full and partial blocks alike (no divergence) */
-                        uint32_t mx = 0;
 #pragma unroll
-                        for (int s = 0; s < GF_BLOCK; s++)
-                            if ((live >> s) & 1u) mx = max(mx, bd_mwc_x(w, a));
-                        any = mx > (uint32_t)xthr;
+            for (int u = 0; u < 4; u++) {
+                const bool act = !parked && c0 != GF_END_WORD;
+                uint32_t x1 = x, cc = c;
+                const uint32_t mx = walk_bins(x1, cc, a, act ? c0 & GF_NLIVE : (uint32_t)GF_BLOCK);
+                if (act) {
+                    if (mx >= (c0 & ~GF_NLIVE)) {
+                        parked = true;
+                    } else {
+                        x = x1;
+                        c = cc;
+                        skip = 0;
+                        c0 = c1;
+                        c1 = c2;
+                        c2 = next_word();
                     }
                 }
-                if (any) {
-                    /* The candidate bins (uniform above the threshold), the first of them and the
-                     * stream state before it.  While no star is drawn the uniforms are the bound
-                     * walk's, so once no candidate is left the walk's end state stands. */
-                    const uint64_t w_end = w;
-                    const bool walked = xthr >= 0;
-                    uint32_t cand = 0;
-                    int s = -1;
-                    {
-                        uint64_t ww = w0, wf = w0;
-#pragma unroll
-                        for (int q = 0; q < GF_BLOCK; q++) {
-                            if ((live >> q) & 1u) {
-                                const uint64_t wb = ww;
-                                const uint32_t x = bd_mwc_x(ww, a);
-                                if (!walked || (int64_t)x > xthr) {
-                                    cand |= 1u << q;
-                                    if (s < 0) { s = q; wf = wb; }
-                                }
-                            }
-                        }
-                        w = wf;
-                    }
-                    const int i0 = (int)(br.x & 0xffffu), j0 = (int)(br.x >> 16);
-                    const uint32_t wm = (br.y >> 16) & 0x3ffu;
-                    const int sl0 = (int)(br.z & 0xffffu);
-                    /* exact tests from the first candidate bin s on; the bin's position
-                     * follows from the block's diagonal starts (wm), as step_in_pixel walks it */
-                    const uint32_t starts = wm & ((2u << s) - 2u);         /* diagonal starts in bins 1..s */
-                    int d = i0 + j0 + __popc(starts), i, j, slot;
-                    if (starts) {
-                        const int s1 = 31 - __clz(starts);
-                        i = d - (V.y - 1) > 0 ? d - (V.y - 1) : 0;
-                        i += s - s1;
-                        j = d - i;
-                        slot = __ldg(V.dslot + d);
-                    } else {
-                        i = i0 + s;
-                        j = j0 - s;
-                        slot = sl0;
-                    }
-                    float2 q = row[slot];
-                    float ms = q.x, D3 = q.y;
-                    bool star = false;
-                    for (const int s0 = s; s < GF_BLOCK; s++) {
-                        if (s > s0) {
-                            if ((wm >> s) & 1u) {
-                                d++;
-                                i = d - (V.y - 1) > 0 ? d - (V.y - 1) : 0;
-                                j = d - i;
-                                slot = __ldg(V.dslot + d);
-                                q = row[slot];
-                                ms = q.x;
-                                D3 = q.y;
-                            } else {
-                                i++;
-                                j--;
-                            }
-                        }
-                        if (!((live >> s) & 1u)) continue;
-                        if (walked && !star && !(cand >> s)) { w = w_end; break; }
-                        const uint64_t wb = w;
-                        const uint32_t xs = bd_mwc_x(w, a);
-                        if ((int64_t)xs <= xthr) continue;
-                        const float u = GF_MWC_SCALE * (float)xs;
-                        float r = LFM[j] * ms;
-                        r *= V.norm;
-                        r *= D3;
-                        r *= K;
-                        if (bd_surely_empty(u, r) || !bd_has_stars(u, r)) continue;
-                        if (!(r < 3.0e38f)) {
-                            /* an infinite expected count would never leave the sampler's gamma loop */
-                            atomicOr(P.err, 1ull);
-                            stop = true;
-                            break;
-                        }
-                        uint64_t v_star = 0;
-                        const int k = draw_event(a, wb, r, V.pixels + pix, w, v_star);
-                        star = true;
-                        if (k > 0) {
-                            EventRecord e;
-                            e.stream = sid;
-                            e.ilb = pix;
-                            e.im = (int16_t)i;
-                            e.iM = (int16_t)j;
-                            e.k = k;
-                            e.nstars = nst;
-                            e.pad = 0;
-                            e.v_star = v_star;
-                            stage_event(P, evb, nev, e);
-                            nst += k;
-                        }
-                    }
-                }
-                __syncwarp();
-                if (*nev >= GF_EVBUF / 2) flush_events(P, evb, nev, lane);
-                pix += V.QN;
-                lb += V.RN;
-                if (lb >= V.Bp) { lb -= V.Bp; pix++; }
-                continue;
-            } else {
-            float mu[GF_BLOCK];
-            uint32_t live = 0;
-            int i0 = 0, j0 = 0;
-            if (valid) {
-                const uint32_t bij = __ldg(V.blk + lb);
-                i0 = (int)(bij & 0xffffu);
-                j0 = (int)(bij >> 16);
-                int slot = __ldg(V.bslot + lb);
-                const float2 *row = V.ms2 + (size_t)pix * (V.nslots + 1);
-                const float2 ik = row[V.nslots];
-                const int icut = __float_as_int(ik.x);
-                const float K = ik.y;
-                float2 q = row[slot];
-                float ms = q.x, D3 = q.y;
-                float D = V.dlim ? __ldg(V.slotD + slot) : 0.f;
-                bool dc = V.dlim && (V.dmin > D || V.dmax <= D);      /* anchor outside [V.dmin, V.dmax): Am = inf */
-                int i = i0, j = j0;
-#pragma unroll
-                for (int s = 0; s < GF_BLOCK; s++) {
-                    if (s > 0 && gfc::step_in_pixel(i, j, V.x, V.y)) {
-                        slot = __ldg(V.dslot + i + j);
-                        q = row[slot];
-                        ms = q.x;
-                        D3 = q.y;
-                        D = V.dlim ? __ldg(V.slotD + slot) : 0.f;
-                        dc = V.dlim && (V.dmin > D || V.dmax <= D);
-                    }
-                    float r = LFM[j] * ms;
-                    r *= V.norm;
-                    r *= D3;
-                    r *= K;
-                    mu[s] = r;
-                    live |= (i < icut && !dc) ? (1u << s) : 0u;
-                }
-            } else {
-#pragma unroll
-                for (int s = 0; s < GF_BLOCK; s++) mu[s] = 0.f;
             }
-            uint32_t todo = live;
-            for (;;) {
-                /* walk the lane's remaining bins up to the first with stars */
-                int ev_s = -1;
-                uint64_t wb_ev = 0;
-                float mu_ev = 0.f;
-                for (;;) {
-                    int c = -1;
-                    uint64_t cwb = 0;
-                    float cu = 0.f, cmu = 0.f;
-#pragma unroll
-                    for (int s = 0; s < GF_BLOCK; s++) {
-                        if (c < 0 && ((todo >> s) & 1u)) {
-                            const uint64_t wb = w;
-                            const float u = bd_mwc_step(w, a);
-                            if (!bd_surely_empty(u, mu[s])) { c = s; cwb = wb; cu = u; cmu = mu[s]; }
-                        }
-                    }
-                    if (c < 0) { todo = 0; break; }
-                    todo &= ~((2u << c) - 1u);
-                    if (bd_has_stars(cu, cmu)) {
-                        ev_s = c;
-                        wb_ev = cwb;
-                        mu_ev = cmu;
-                        break;
-                    }
+            const unsigned waiting = __ballot_sync(BD_FULL, parked), left = __ballot_sync(BD_FULL, c0 != GF_END_WORD);
+            if (left == 0) break;
+            /* serve the parked lanes when they have waited, together, as long as a service holds up the lanes left */
+            idle += __popc(waiting);
+            if (waiting == 0 || (2 * idle < __popc(left) && waiting != left)) continue;
+            idle = 0;
+            if (parked) {
+                parked = false;
+                /* the block, three steps behind the next word's */
+                uint32_t pixel = px - 3 * QN;
+                int lbc = (int)lb - 3 * (int)RN;
+                while (lbc < 0) { lbc += (int)Bp; pixel--; }
+                const uint4 br = __ldg(V.brec + lbc);
+                const uint2 cut = __ldg(V.prow + V.px0 + pixel);
+                const gf_pencil_beam *pix = V.pixels + V.px0 + pixel;
+                const float dA = __ldg(&pix->dA);
+                /* its first candidate bin, the states before and after it */
+                const uint32_t n = c0 & GF_NLIVE, T = c0 & ~GF_NLIVE;
+                uint32_t k = 0, xk = 0;
+                w = ((uint64_t)c << 32) | x;
+                uint64_t wb = w;
+                for (; k < n; k++) {
+                    wb = w;
+                    xk = bd_mwc_x(w, a);
+                    if (xk >= T) break;
                 }
-                const bool ev = ev_s >= 0;
-                if (!__any_sync(BD_FULL, ev)) break;
-                int k = 0;
-                uint64_t v_star = 0;
-                int ei = 0, ej = 0;
-                if (ev) {
-                    if (!(mu_ev < 3.0e38f)) {
+                const float K = dA * GF_POGSON * V.dm * V.dM;
+                uint32_t live = block_live(br, (int)(cut.y & 0xffffu), V.nM);
+                if (V.dlim) live &= block_inside(br, V.slotD, V.dslot, V.dmin, V.dmax);
+                for (int q = skip + (int)k; q > 0; q--) live &= live - 1u;
+                const int s = __ffs(live) - 1;
+                /* the bin's position follows from the block's diagonal starts, as step_in_pixel walks it */
+                const int i0 = (int)(br.x & 0xffffu), j0 = (int)(br.x >> 16);
+                const uint32_t starts = (br.y >> 16) & ((2u << s) - 2u);         /* diagonal starts in bins 1..s */
+                const int d = i0 + j0 + __popc(starts);
+                int i = i0 + s, slot = (int)(br.z & 0xffffu);
+                if (starts) {
+                    i = max(0, d - (V.nM - 1)) + s - (31 - __clz(starts));
+                    slot = d == i0 + j0 + 1 ? (int)(br.z >> 16) : (int)__ldg(V.dslot + d);
+                }
+                const int j = d - i;
+                const float D = __ldg(V.slotD + slot);
+                float mu = __ldg(V.lfm + j) * V.ms[(size_t)pixel * V.nslots + slot];
+                mu *= V.norm;
+                mu *= D * D * D;
+                mu *= K;
+                const float u = GF_MWC_SCALE * (float)xk;
+                if (k < n && !bd_surely_empty(u, mu)) {
+                    if (!(mu < 3.0e38f) && bd_has_stars(u, mu)) {
                         /* an infinite expected count would never leave the sampler's gamma loop */
                         atomicOr(P.err, 1ull);
-                        stop = true;
-                        todo = 0;
+                        c1 = c2 = GF_END_WORD;
+                        px = npx;
                     } else {
-                        k = draw_event(a, wb_ev, mu_ev, V.pixels + pix, w, v_star);
-                        ei = i0; ej = j0;
-                        for (int s = 1; s <= ev_s; s++) gfc::step_in_pixel(ei, ej, V.x, V.y);
+                        const int stars = draw_count(a, wb, u, mu, w);
+                        if (stars > 0) {
+                            EventRecord e;
+                            e.stream = (job << 16) | t;
+                            e.ilb = V.px0 + (int)pixel;
+                            e.im = (int16_t)i;
+                            e.iM = (int16_t)j;
+                            e.k = stars;
+                            e.v_star = w;
+                            evb[atomicAdd(nev, 1)] = e;
+                            w = skip_stars(a, w, stars, (cut.y & 0x10000u) != 0, pix);
+                        }
                     }
                 }
-                /* stage the bins with stars (all lanes converged) */
-                const bool rec = ev && k > 0;
-                const unsigned rm = __ballot_sync(BD_FULL, rec);
-                if (rm) {
-                    if (*nev + __popc(rm) > GF_EVBUF) flush_events(P, evb, nev, lane);      /* leaves *nev = 0 */
-                    if (rec) {
-                        EventRecord e;
-                        e.stream = sid;
-                        e.ilb = pix;
-                        e.im = (int16_t)ei;
-                        e.iM = (int16_t)ej;
-                        e.k = k;
-                        e.nstars = nst;
-                        e.pad = 0;
-                        e.v_star = v_star;
-                        evb[*nev + __popc(rm & ((1u << lane) - 1u))] = e;
-                        nst += k;
-                    }
-                    __syncwarp();
-                    if (lane == 0) *nev += __popc(rm);
-                    __syncwarp();
+                x = (uint32_t)w;
+                c = (uint32_t)(w >> 32);
+                /* the bins after it remain */
+                skip += (int)k + 1;
+                if (k + 1 < n) {
+                    c0 = T | (n - k - 1);
+                } else {
+                    skip = 0;
+                    c0 = c1;
+                    c1 = c2;
+                    c2 = next_word();
                 }
             }
+            __syncwarp();
             if (*nev >= GF_EVBUF / 2) flush_events(P, evb, nev, lane);
-            /* the stream's next block: N blocks further */
-            pix += V.QN;
-            lb += V.RN;
-            if (lb >= V.Bp) { lb -= V.Bp; pix++; }
-            }
         }
-        if (stream_ok && !stop) {
-            rng[NS + t] = (uint32_t)(w >> 32);
-            rng[2 * NS + t] = (uint32_t)w;
+        if (stream_ok) {
+            rng[NS + t] = c;
+            rng[2 * NS + t] = x;
         }
     }
     flush_events(P, evb, nev, lane);
@@ -641,7 +550,7 @@ __global__ void __launch_bounds__(256) expand_kernel(const EventRecord *ev, int6
             s.ilb = E.ilb + J.pix_base;
             s.im = E.im;
             s.iM = E.iM;
-            s.seq = E.nstars + q;
+            s.seq = q;
             s.u[0] = r.uniform();
             s.u[1] = r.uniform();
             float xx = pix.X, yy = pix.Y;
@@ -661,19 +570,6 @@ __global__ void __launch_bounds__(256) expand_kernel(const EventRecord *ev, int6
 
 }  // namespace
 
-cudaError_t launch_slot_density(const SlotDensityParams &P, int model_type, cudaStream_t s)
-{
-    if (P.total_pix <= 0) return cudaSuccess;
-    const long long need = ((long long)P.total_pix + 7) / 8;
-    const int blocks = (int)std::min<long long>(need, (long long)sm_count() * 8);
-    if (model_type == GF_MODEL_EXP_DISK)
-        slot_density_kernel<GF_MODEL_EXP_DISK><<<blocks, 256, 0, s>>>(P);
-    else
-        slot_density_kernel<GF_MODEL_POWER_LAW_ELLIPSOID><<<blocks, 256, 0, s>>>(P);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_block_records(const BlockLfParams &P, cudaStream_t s)
 {
     if (P.total <= 0) return cudaSuccess;
@@ -683,49 +579,52 @@ cudaError_t launch_block_records(const BlockLfParams &P, cudaStream_t s)
     return cudaGetLastError();
 }
 
-size_t batch_draw_warp_bytes(int max_tab, BatchDrawParams *P)
+int block_word_tile(int64_t rows, int max_slots)
 {
-    size_t off = (sizeof(SkyModel) + 15) & ~(size_t)15;
-    P->off_view = (int32_t)off;
-    off += (sizeof(DrawJobView) + 15) & ~(size_t)15;
-    P->off_tab = (int32_t)off;
-    off += ((size_t)4 * max_tab + 15) & ~(size_t)15;
-    P->off_ev = (int32_t)off;
-    off += sizeof(EventRecord) * GF_EVBUF + 16;
-    off = (off + 15) & ~(size_t)15;
-    P->warp_bytes = (int32_t)off;
-    return off;
+    /* as many rows as 96 KB of densities hold, but four tiles an SM while there are fewer rows than that */
+    const int64_t fit = (96 * 1024) / (4 * (int64_t)std::max(max_slots, 1));
+    const int64_t want = std::min<int64_t>(std::min<int64_t>(fit, GF_WORD_TILE), rows / (4 * (int64_t)sm_count()));
+    return (int)std::max<int64_t>(want, 1);
 }
 
-template <int MODEL, bool BOUND>
-cudaError_t launch_batch_draw_t(const BatchDrawParams &P, int warps_per_cta, size_t smem, cudaStream_t s)
+template <int MODEL>
+static cudaError_t launch_block_words_t(const BlockWordParams &P, int max_slots, cudaStream_t s)
 {
-    const int threads = 32 * warps_per_cta;
-    cudaError_t e = cudaFuncSetAttribute(batch_draw_kernel<MODEL, BOUND>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = 4 * (size_t)P.tile * max_slots;
+    cudaError_t e = cudaFuncSetAttribute(block_words_kernel<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     int per_sm = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_draw_kernel<MODEL, BOUND>, threads, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_words_kernel<MODEL>, 256, smem);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    const long long want = ((long long)P.nitems + warps_per_cta - 1) / warps_per_cta;
-    const int blocks = (int)std::min<long long>(want, (long long)sm_count() * per_sm);
-    batch_draw_kernel<MODEL, BOUND><<<blocks, threads, smem, s>>>(P);
+    const int blocks = (int)std::min<long long>(P.total_tiles, (long long)sm_count() * std::max(per_sm, 1));
+    block_words_kernel<MODEL><<<blocks, 256, smem, s>>>(P);
     count_launches(1);
     return cudaGetLastError();
 }
 
-cudaError_t launch_batch_draw(const BatchDrawParams &P, int model_type, int warps_per_cta, bool bound, cudaStream_t s)
+cudaError_t launch_block_words(const BlockWordParams &P, int model_type, int max_slots, cudaStream_t s)
+{
+    if (P.total_tiles <= 0) return cudaSuccess;
+    if (P.tile < 1 || P.tile > GF_WORD_TILE || 4 * (int64_t)P.tile * max_slots > 200 * 1024) return cudaErrorInvalidValue;
+    return model_type == GF_MODEL_EXP_DISK ? launch_block_words_t<GF_MODEL_EXP_DISK>(P, max_slots, s)
+                                           : launch_block_words_t<GF_MODEL_POWER_LAW_ELLIPSOID>(P, max_slots, s);
+}
+
+cudaError_t launch_batch_draw(const BatchDrawParams &P, int warps_per_cta, cudaStream_t s)
 {
     if (P.nitems <= 0) return cudaSuccess;
     if (warps_per_cta < 1 || warps_per_cta > 8) warps_per_cta = 4;
-    const size_t smem = (size_t)warps_per_cta * P.warp_bytes;
-    if (smem > 200 * 1024) return cudaErrorInvalidValue;
+    const size_t smem = (size_t)warps_per_cta * (sizeof(EventRecord) * GF_EVBUF + 16);
     cudaError_t e = cudaMemsetAsync(P.next_item, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return e;
-    if (model_type == GF_MODEL_EXP_DISK)
-        return bound ? launch_batch_draw_t<GF_MODEL_EXP_DISK, true>(P, warps_per_cta, smem, s)
-                     : launch_batch_draw_t<GF_MODEL_EXP_DISK, false>(P, warps_per_cta, smem, s);
-    return bound ? launch_batch_draw_t<GF_MODEL_POWER_LAW_ELLIPSOID, true>(P, warps_per_cta, smem, s)
-                 : launch_batch_draw_t<GF_MODEL_POWER_LAW_ELLIPSOID, false>(P, warps_per_cta, smem, s);
+    const int threads = 32 * warps_per_cta;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_draw_kernel, threads, smem);
+    if (e != cudaSuccess) return e;
+    const long long want = ((long long)P.nitems + warps_per_cta - 1) / warps_per_cta;
+    const int blocks = (int)std::min<long long>(want, (long long)sm_count() * std::max(per_sm, 1));
+    batch_draw_kernel<<<blocks, threads, smem, s>>>(P);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 cudaError_t expand_temp_bytes(int64_t nev, size_t *bytes)

@@ -203,30 +203,55 @@ size_t integ_warp_bytes(int nm_max, int nM_max, int slots_max, IntegPixParams *P
 cudaError_t launch_integrate_pixels(const IntegPixParams &P, int model_type, double2 *tot, cudaStream_t s);
 
 /* the batched draw (gf_batchdraw.cu) */
-struct SlotDensityParams {
-    const CrawlJob *jobs;
-    const unsigned char *const *plans;   /* per request */
-    float2 *const *ms;             /* per request, per pixel, nslots + 1 pairs: (model density, D^3) of each
-                                    * slot, then (first cut apparent-magnitude row as int bits, K = dA POGSON dm dM) */
-    const int32_t *job_list;       /* requests of the launch */
-    const int32_t *pix_off;        /* [njobs + 1] first flat pixel of each listed request */
-    int32_t njobs, total_pix;
+/* Rows of neighbouring pixels: runs of up to GF_ROW_PIXELS pixels of a request with the same first
+ * cut apparent-magnitude row (m0 + dm im + Am > m1).  Per pixel: its row, and the cut row
+ * | 0x10000 when a star of the pixel may lie beyond the projection's edge. */
+#define GF_ROW_PIXELS 4
+/* One request of a draw pass: its tables for the pixels [px0, px0 + npx) of the pass's segment.
+ * Block b of pixel p is the request's (p Bp + b)-th; stream t takes every N-th from the t-th. */
+struct DrawJob {
+    uint32_t *words;               /* [nrows][Bp] block words: number of live bins (bits 0-3), threshold of the largest uniform (above) */
+    float *ms;                     /* [npx][nslots] model density of each slot of the request's plan */
+    uint32_t *roff;                /* [npx] first word of the pixel's row */
+    const uint2 *prow;             /* [pixels] row, cut row | edge flag */
+    const int32_t *rowpx;          /* [rows + 1] first pixel of each row */
+    const uint4 *brec;             /* [Bp] block records (BlockLfParams) */
+    const float *lfm;              /* [nM] LF at each absolute-magnitude row */
+    const uint16_t *dslot;         /* the plan's slot of each diagonal's first bin */
+    const float *slotD;            /* the plan's slot distances */
+    const gf_pencil_beam *pixels;  /* the request's pixels */
+    uint32_t *rng;                 /* the request's streams [3][rng_nstreams] */
+    int32_t rng_nstreams;
+    uint32_t total;                /* npx Bp (below 2^30) */
+    int32_t px0, npx, row0, nrows;
+    int32_t Bp, nslots, N, nM;
+    int32_t QN, RN;                /* N = QN Bp + RN */
+    int32_t first;                 /* (px0 Bp) mod N: the stream that takes the segment's first block */
+    FastDiv fB;                    /* division by Bp */
+    float norm, dm, dM, dmin, dmax;
+    int32_t dlim;                  /* dmin or dmax set */
 };
 struct BlockLfParams {
     const CrawlJob *jobs;
     const unsigned char *const *plans;   /* per request */
     uint4 *const *brec;            /* per request, per block: blk, binfo, bslot | first diagonal-start slot << 16,
-                                    * largest LF value of its bins (float bits, at least 0) */
+                                    * bound of LF D^3 norm over its bins (float bits; NaN: no bound) */
+    float *const *lfm;             /* per request: LF at each absolute-magnitude row */
     const int32_t *job_list;       /* requests of the launch */
     const int64_t *blk_off;        /* [njobs + 1] first flat block of each listed request */
     int32_t njobs;
     int64_t total;
 };
-struct BatchDrawParams {
+#define GF_WORD_TILE 8             /* most rows of a tile of block_words_kernel */
+struct BlockWordParams {
     const CrawlJob *jobs;
-    const unsigned char *const *plans;   /* per request */
-    const float2 *const *ms;       /* per request: slot densities (SlotDensityParams::ms) */
-    const uint4 *const *brec;      /* per request: block records (null: exact test for every bin) */
+    const DrawJob *view;           /* per request */
+    const int32_t *job_list;       /* requests of the launch */
+    const int32_t *tile_off;       /* [njobs + 1] first tile of each listed request (ceil(nrows / tile) tiles each) */
+    int32_t njobs, total_tiles, tile;
+};
+struct BatchDrawParams {
+    const DrawJob *view;           /* per request */
     const uint32_t *items;         /* (request << 16) | first of 32 consecutive streams */
     int32_t nitems;
     uint32_t *next_item;           /* work-queue counter */
@@ -234,14 +259,12 @@ struct BatchDrawParams {
     int64_t ev_capacity;
     unsigned long long *ev_count;  /* events found (may exceed the capacity) */
     unsigned long long *err;       /* set when a bin's expected count is infinite */
-    int32_t off_view, off_tab, off_ev, warp_bytes;   /* per-warp shared-memory layout (batch_draw_warp_bytes) */
 };
-cudaError_t launch_slot_density(const SlotDensityParams &P, int model_type, cudaStream_t s);
 cudaError_t launch_block_records(const BlockLfParams &P, cudaStream_t s);
-size_t batch_draw_warp_bytes(int max_tab, BatchDrawParams *P);
-/* bound: every request of P takes the block bound of its expected counts (see
- * batch_draw_kernel); otherwise every bin is tested exactly */
-cudaError_t launch_batch_draw(const BatchDrawParams &P, int model_type, int warps_per_cta, bool bound, cudaStream_t s);
+/* rows of a tile for a launch over that many rows and plans of at most max_slots slots */
+int block_word_tile(int64_t rows, int max_slots);
+cudaError_t launch_block_words(const BlockWordParams &P, int model_type, int max_slots, cudaStream_t s);
+cudaError_t launch_batch_draw(const BatchDrawParams &P, int warps_per_cta, cudaStream_t s);
 cudaError_t expand_temp_bytes(int64_t nev, size_t *bytes);
 /* star records of the events at offsets from a scan over k; *total = the stars of all events */
 cudaError_t launch_expand_events(const EventRecord *ev, int64_t nev, const CrawlJob *jobs, int64_t *k64, int64_t *off64,

@@ -144,6 +144,13 @@ bool same_cfg(const void *a, const void *b, size_t n)
 /* the kernel template a model type runs in: GF_MODEL_EXP_DISK or GF_MODEL_POWER_LAW_ELLIPSOID */
 int model_kind(int type) { return type == GF_MODEL_EXP_DISK ? GF_MODEL_EXP_DISK : GF_MODEL_POWER_LAW_ELLIPSOID; }
 
+/* room for the Poisson spread of e expected stars (a negative density expects none) */
+double with_spread(double e, double sigmas)
+{
+    const double x = e > 0.0 ? e : 0.0;
+    return x + sigmas * sqrt(x) + 1024.0;
+}
+
 struct ReqInfo {
     std::vector<gfh::HostModel> hm;    /* models in component order */
     std::vector<gf_model_config> mc;
@@ -158,7 +165,40 @@ struct ReqInfo {
     int group = 0;
     int slot = -1;
     double cost = 0;
+    std::vector<int32_t> rowpx;        /* first pixel of each pixel row (GF_ROW_PIXELS), then npixels */
 };
+
+/* The pixel rows of a request: per pixel its row and cut row (gf_launch.h), and each row's first
+ * pixel.  The cut row is the first im with m0 + dm im + Am > m1 in float, as the crawl cuts its bins. */
+void pixel_rows(const SkyModel &m, const gf_job &J, uint2 *prow, std::vector<int32_t> &rowpx)
+{
+    rowpx.clear();
+    rowpx.reserve((size_t)J.npixels / GF_ROW_PIXELS + 64);
+    const bool ext = J.beam_ammin && J.ext.kind != GF_EXT_NONE;
+    float last = -1.f;
+    int icut = -1, prev = -1, in_row = 0;
+    auto cut = [&](int i, float Am) { return m.m0 + m.dm * (float)i + Am > m.m1; };
+    for (int p = 0; p < J.npixels; p++) {
+        const gf_pencil_beam &x = J.pixels[p];
+        const float Am = ext ? J.beam_ammin[x.extIdx] : 0.f;
+        if (icut < 0 || Am != last) {
+            if (icut < 0) icut = m.nm;
+            while (icut < m.nm && !cut(icut, Am)) icut++;
+            while (icut > 0 && cut(icut - 1, Am)) icut--;
+            last = Am;
+        }
+        if (p == 0 || icut != prev || in_row == GF_ROW_PIXELS) {
+            rowpx.push_back(p);
+            in_row = 0;
+        }
+        in_row++;
+        prev = icut;
+        const float ax = fabsf(x.X) + 0.51f * fabsf(x.dx), ay = fabsf(x.Y) + 0.51f * fabsf(x.dx);
+        prow[p].x = (uint32_t)rowpx.size() - 1;
+        prow[p].y = (uint32_t)icut | (ax * ax + ay * ay < 1.9999f ? 0u : 0x10000u);
+    }
+    rowpx.push_back(J.npixels);
+}
 
 /* CrawlState slices of one request inside the arrays of all requests */
 CrawlState slice(const CrawlState &a, size_t off)
@@ -187,6 +227,10 @@ struct MultiWS {
     Grow<CrawlJob> jobs;
     Grow<float> lf;
     Grow<gf_pencil_beam> pix;
+    Grow<uint2> prow;                       /* pixel rows (gf_launch.h): per pixel */
+    Grow<int32_t> rowpx;                    /* first pixel of each row: request j's from its first pixel + j on */
+    Grow<float> lfm;                        /* batched draw: LF at each absolute-magnitude row, per request */
+    Grow<float *> lfmptr;
     Grow<uint64_t> pseed;
     Grow<uint32_t> rng;
     Grow<uint32_t> rng_snap;
@@ -205,9 +249,9 @@ struct MultiWS {
     Grow<const unsigned char *> plans;
     Grow<int32_t> pixoff;
     Grow<gfk::IntegPlanDesc> pdesc;
-    Grow<float2> msbuf;                     /* batched draw: slot densities of the chunk's pixels */
-    Grow<float2 *> msptr;
-    Grow<int32_t> joblist, chunkoff;
+    Grow<uint32_t> tables;                  /* batched draw: block words and slot densities of a segment */
+    Grow<gfk::DrawJob> view;                /* batched draw: per segment and request */
+    Grow<int32_t> joblist, tileoff;
     Grow<EventRecord> ev;
     Grow<int64_t> k64, off64;
     Grow<uint32_t> gitems;                  /* batched draw: (request << 16) | first of 32 streams */
@@ -287,6 +331,10 @@ namespace {
 
 /* ---- host delivery: rows copied to a page-locked ring while the device works on ---- */
 #define GF_RING 3
+
+/* bytes of the draw tables of one segment (see the draw pass): large enough that segments of the
+ * ordinary passes are one, small beside the 180 GB of the card */
+constexpr int64_t kDrawTables = (int64_t)4 << 30;
 
 /* bytes of one row of a table with nb bands, counting the columns in mask (GF_COL_*) */
 size_t row_bytes(int nb, uint32_t mask)
@@ -551,6 +599,9 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         std::stable_sort(q.mc.begin(), q.mc.end(), [](const gf_model_config &a, const gf_model_config &b) { return a.comp < b.comp; });
         if (!gfh::setup_models(J.sky, J.npixels, q.mc.data(), nmod, q.hm, errs[j]) && errs[j].empty()) errs[j] = "invalid model";
         sigs[j] = module_signature(J);
+        if (J.beam_ammin && J.ext.kind == GF_EXT_SCREEN_CSCB)
+            for (int p = 0; p < J.npixels && errs[j].empty(); p++)
+                if (J.pixels[p].extIdx < 0 || J.pixels[p].extIdx >= J.npixels) errs[j] = "pixel extIdx out of range";
     });
     for (int j = 0; j < njobs; j++) {
         const gf_job &J = jobs[j];
@@ -594,12 +645,21 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         /* one page-locked staging area: all pixels, then the per-beam extinction, then the LFs */
         const size_t pb = sizeof(gf_pencil_beam) * (size_t)pix_total, ab = 4 * (size_t)pix_total;
         const size_t lb_ = 4 * (size_t)njobs * nmod * 1024;
-        GF_TRY(ws.h_stage.need(pb + ab + lb_));
+        const size_t rb_ = 8 * (size_t)pix_total, xb = 4 * ((size_t)pix_total + njobs);
+        GF_TRY(ws.prow.need((size_t)pix_total));
+        GF_TRY(ws.rowpx.need((size_t)pix_total + njobs));
+        GF_TRY(ws.h_stage.need(pb + ab + lb_ + rb_ + xb));
         char *h = ws.h_stage.p;
         gf_pencil_beam *hp = (gf_pencil_beam *)h;
         float *ha = (float *)(h + pb), *hl = (float *)(h + pb + ab);
+        uint2 *hr = (uint2 *)(h + pb + ab + lb_);
+        int32_t *hx = (int32_t *)(h + pb + ab + lb_ + rb_);
         memset(hl, 0, lb_);
         parallel_for(njobs, [&](int j) {
+            if (!R[j].plain) {
+                pixel_rows(R[j].hm[0].m, jobs[j], hr + R[j].pix_off, R[j].rowpx);
+                std::copy(R[j].rowpx.begin(), R[j].rowpx.end(), hx + R[j].pix_off + j);
+            }
             memcpy(hp + R[j].pix_off, jobs[j].pixels, sizeof(gf_pencil_beam) * (size_t)jobs[j].npixels);
             if (jobs[j].beam_ammin) memcpy(ha + R[j].pix_off, jobs[j].beam_ammin, 4 * (size_t)jobs[j].npixels);
             else memset(ha + R[j].pix_off, 0, 4 * (size_t)jobs[j].npixels);
@@ -609,6 +669,8 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         GF_CUDA(cudaMemcpyAsync(d_pix, hp, pb, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaMemcpyAsync(d_ammin, ha, ab, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaMemcpyAsync(d_lf, hl, lb_, cudaMemcpyHostToDevice, st));
+        GF_CUDA(cudaMemcpyAsync(ws.prow.p, hr, rb_, cudaMemcpyHostToDevice, st));
+        GF_CUDA(cudaMemcpyAsync(ws.rowpx.p, hx, xb, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaStreamSynchronize(st));
     }
     /* distance tables D[im][iM], shared by the requests with the same magnitude grid */
@@ -732,7 +794,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     /* pixel-by-pixel integrate: anchor plans per magnitude grid (nm * nM is a
      * multiple of 10 for every batched request) */
     std::map<std::tuple<float, float, float, float, int, int>, unsigned char *> plans;
-    std::map<const unsigned char *, int> plan_nslots;
+    std::map<const unsigned char *, gfk::IntegPlanHdr> plan_hdr;
     std::vector<char> plan_used(nmod, 0);
     auto plan_of = [&](int j, int i) -> unsigned char * {
         const SkyModel &m = R[j].hm[i].m;
@@ -794,7 +856,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             for (size_t q = 0; q < uniq.size(); q++) {
                 ok = ok && hh[q].ok;
                 slots_max = std::max(slots_max, hh[q].nslots);
-                plan_nslots[uniq[q]] = hh[q].nslots;
+                plan_hdr[uniq[q]] = hh[q];
             }
             for (int j : integ) {
                 nm_max = std::max(nm_max, R[j].hm[i].m.nm);
@@ -859,8 +921,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         }
         for (int j : integ) {
             /* room for the Poisson spread of the model's stars in one batch */
-            const double e = S[j].expected[i];
-            if (e + ctx->admit_sigma * sqrt(e) + 1024.0 >= (double)jobs[j].capacity) R[j].plain = true;
+            if (with_spread(S[j].expected[i], ctx->admit_sigma) >= (double)jobs[j].capacity) R[j].plain = true;
         }
     }
 
@@ -871,10 +932,10 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     const double kStarBytes = 256.0;
     auto need_of = [&](int j) {
         double mx = 0;
-        for (int i = 0; i < nmod; i++) mx = std::max(mx, S[j].expected[i] + 8.0 * sqrt(S[j].expected[i]) + 1024.0);
+        for (int i = 0; i < nmod; i++) mx = std::max(mx, with_spread(S[j].expected[i], 8.0));
         int ns = 0;
         for (int i = 0; i < nmod; i++)
-            if (plan_used[i] && plan_of(j, i)) ns = std::max(ns, plan_nslots[plan_of(j, i)]);
+            if (plan_used[i] && plan_of(j, i)) ns = std::max(ns, plan_hdr[plan_of(j, i)].nslots);
         return mx * (kStarBytes + 48.0) + 8.0 * (double)jobs[j].npixels * (ns + 1) +
                16.0 * (double)R[j].hm[0].m.nm * R[j].hm[0].m.nM / GF_BLOCK;
     };
@@ -1029,7 +1090,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             for (int j = 0; j < njobs; j++) hj[j] = crawl_job(j, i);
             GF_CUDA(cudaMemcpyAsync(d_jobs, hj.data(), sizeof(CrawlJob) * (size_t)njobs, cudaMemcpyHostToDevice, st));
             double want = 65536;
-            for (int j : batched) want += S[j].expected[i] + 8.0 * sqrt(S[j].expected[i]) + 1024.0;
+            for (int j : batched) want += with_spread(S[j].expected[i], 8.0);
             int64_t cap = (int64_t)want;
             GF_CUDA(cudaMemcpyAsync(d_rng_snap, d_rng, 12 * (size_t)njobs * NS, cudaMemcpyDeviceToDevice, st));
             /* the kernels' model kind: exponential disks, or the ellipsoids (power laws,
@@ -1038,115 +1099,180 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             GF_TRY(rec.need((size_t)cap));
             int64_t nrec = 0;
             if (plan_used[i]) {
-                /* slot densities of the chunk's pixels */
+                /* The draw tables (slot densities a pixel, block words a row; 4 bytes each) of the chunk's requests, in
+                 * segments of every request's pixels when all of them would take more than kDrawTables
+                 * bytes: a segment's words are made, then the streams walk them and stop at its end. */
+                const size_t nb = batched.size();
                 std::vector<const unsigned char *> jp(njobs, nullptr);
-                std::vector<float2 *> jm(njobs, nullptr);
-                std::vector<int32_t> jl, poff;
-                std::vector<int64_t> moff(njobs, 0);
-                int64_t ms_total = 0;
-                int32_t tp = 0;
-                for (int j : batched) {
+                std::vector<uint4 *> lp(njobs, nullptr);
+                std::vector<int32_t> jl(batched.begin(), batched.end());
+                std::vector<int64_t> boff(nb + 1, 0);
+                int64_t pixels = 0, table_words = 0, largest = 1, lfm_n = 0;
+                int slots_max = 1;
+                std::vector<float *> fp(njobs, nullptr);
+                for (size_t q = 0; q < nb; q++) {
+                    const int j = batched[q];
                     jp[j] = plan_of(j, i);
-                    moff[j] = ms_total;
-                    ms_total += (int64_t)jobs[j].npixels * (plan_nslots[jp[j]] + 1);
-                    jl.push_back(j);
-                    poff.push_back(tp);
-                    tp += jobs[j].npixels;
+                    const int64_t Bp = (int64_t)R[j].hm[i].m.nm * R[j].hm[i].m.nM / GF_BLOCK, ns = plan_hdr[jp[j]].nslots;
+                    boff[q + 1] = boff[q] + Bp;
+                    pixels += jobs[j].npixels;
+                    table_words += (int64_t)jobs[j].npixels * (ns + 1) + (int64_t)(R[j].rowpx.size() - 1) * Bp;
+                    largest = std::max(largest, (int64_t)jobs[j].npixels * Bp);
+                    slots_max = std::max(slots_max, (int)ns);
+                    lfm_n += R[j].hm[i].m.nM;
                 }
-                poff.push_back(tp);
-                GF_TRY(ws.msbuf.need((size_t)std::max<int64_t>(ms_total, 1)));
-                for (int j : batched) jm[j] = ws.msbuf.p + moff[j];
-                GF_TRY(ws.msptr.need((size_t)njobs));
-                GF_TRY(ws.joblist.need(jl.size()));
-                GF_TRY(ws.chunkoff.need(poff.size()));
-                GF_CUDA(cudaMemcpyAsync(ws.plans.p, jp.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
-                GF_CUDA(cudaMemcpyAsync(ws.msptr.p, jm.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
-                GF_CUDA(cudaMemcpyAsync(ws.joblist.p, jl.data(), 4 * jl.size(), cudaMemcpyHostToDevice, st));
-                GF_CUDA(cudaMemcpyAsync(ws.chunkoff.p, poff.data(), 4 * poff.size(), cudaMemcpyHostToDevice, st));
-                gfk::SlotDensityParams SD;
-                SD.jobs = d_jobs; SD.plans = ws.plans.p; SD.ms = ws.msptr.p;
-                SD.job_list = ws.joblist.p; SD.pix_off = ws.chunkoff.p;
-                SD.njobs = (int32_t)jl.size(); SD.total_pix = tp;
-                {
-                    ProfScope ps(ctx, GF_PROF_SLOTS);
-                    GF_CUDA(gfk::launch_slot_density(SD, mtype, st));
+                GF_TRY(ws.lfm.need((size_t)lfm_n));
+                lfm_n = 0;
+                for (int j : batched) {
+                    fp[j] = ws.lfm.p + lfm_n;
+                    lfm_n += R[j].hm[i].m.nM;
                 }
-                /* the record of every block of every request (the draw's bound walk) */
-                {
-                    std::vector<uint4 *> lp(njobs, nullptr);
-                    std::vector<int64_t> boff;
-                    int64_t nb_total = 0;
-                    for (int j : batched) {
-                        boff.push_back(nb_total);
-                        nb_total += (int64_t)R[j].hm[i].m.nm * R[j].hm[i].m.nM / GF_BLOCK;
+                int64_t nseg = std::max<int64_t>({1, (4 * table_words + kDrawTables - 1) / kDrawTables, (largest >> 30) + 1});
+                auto seg_px = [&](int j, int64_t k) { return (int32_t)((int64_t)jobs[j].npixels * k / nseg); };
+                /* the row of a pixel, and the rows that the segment's pixels touch */
+                auto row_of = [&](int j, int32_t p) {
+                    const auto &x = R[j].rowpx;
+                    return (int32_t)(std::upper_bound(x.begin(), x.end() - 1, p) - x.begin()) - 1;
+                };
+                auto seg_rows = [&](int j, int64_t k) {
+                    const int32_t a = seg_px(j, k), e = seg_px(j, k + 1);
+                    return e > a ? row_of(j, e - 1) - row_of(j, a) + 1 : 0;
+                };
+                std::vector<gfk::DrawJob> view;
+                std::vector<int32_t> toff;
+                std::vector<int32_t> tiles;
+                int tile = 1;
+                GF_TRY(ws.brec.need((size_t)boff[nb]));
+                for (size_t q = 0; q < nb; q++) lp[batched[q]] = ws.brec.p + boff[q];
+                int64_t rows_max = 0;
+                for (;;) {
+                    int64_t need = 0;
+                    rows_max = 0;
+                    for (int64_t k = 0; k < nseg; k++) {
+                        int64_t n = 0, nr = 0;
+                        for (size_t q = 0; q < nb; q++) {
+                            const int j = batched[q];
+                            const int32_t rows = seg_rows(j, k);
+                            nr += rows;
+                            n += (int64_t)(seg_px(j, k + 1) - seg_px(j, k)) * (plan_hdr[jp[j]].nslots + 1) + rows * (boff[q + 1] - boff[q]);
+                        }
+                        need = std::max(need, n);
+                        rows_max = std::max(rows_max, nr);
                     }
-                    boff.push_back(nb_total);
-                    GF_TRY(ws.brec.need((size_t)std::max<int64_t>(nb_total, 1)));
-                    for (size_t q = 0; q < batched.size(); q++) lp[batched[q]] = ws.brec.p + boff[q];
-                    GF_TRY(ws.brecptr.need((size_t)njobs));
-                    GF_TRY(ws.blkoff.need(boff.size()));
-                    GF_CUDA(cudaMemcpyAsync(ws.brecptr.p, lp.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
-                    GF_CUDA(cudaMemcpyAsync(ws.blkoff.p, boff.data(), 8 * boff.size(), cudaMemcpyHostToDevice, st));
+                    const gf_status as = ws.tables.need((size_t)std::max<int64_t>(need, 1));
+                    if (as == GF_OK) break;
+                    /* less memory than that: more segments, down to a few pixels each */
+                    if (as != GF_E_OOM || nseg * 4 > pixels) return as;
+                    nseg *= 4;
+                }
+                tile = gfk::block_word_tile(rows_max, slots_max);
+                view.resize((size_t)nseg * njobs);
+                toff.resize((size_t)nseg * (nb + 1));
+                tiles.resize((size_t)nseg);
+                for (int64_t k = 0; k < nseg; k++) {
+                    uint32_t *at = ws.tables.p;
+                    int32_t nt = 0;
+                    for (size_t q = 0; q < nb; q++) {
+                        const int j = batched[q];
+                        const gfk::IntegPlanHdr &h = plan_hdr[jp[j]];
+                        const SkyModel &m = R[j].hm[i].m;
+                        gfk::DrawJob &v = view[(size_t)k * njobs + j];
+                        v.px0 = seg_px(j, k);
+                        v.npx = seg_px(j, k + 1) - v.px0;
+                        v.row0 = v.npx ? row_of(j, v.px0) : 0;
+                        v.nrows = seg_rows(j, k);
+                        v.Bp = (int32_t)(boff[q + 1] - boff[q]);
+                        v.nslots = h.nslots;
+                        v.N = N;
+                        v.nM = m.nM;
+                        v.QN = N / v.Bp;
+                        v.RN = N % v.Bp;
+                        v.total = (uint32_t)v.npx * (uint32_t)v.Bp;
+                        v.first = (int32_t)((int64_t)v.px0 * v.Bp % N);
+                        v.fB = make_fastdiv((uint32_t)v.Bp);
+                        v.norm = m.norm; v.dm = m.dm; v.dM = m.dM; v.dmin = m.dmin; v.dmax = m.dmax;
+                        v.dlim = m.dmin != 0.f || m.dmax != 0.f;
+                        v.prow = ws.prow.p + R[j].pix_off;
+                        v.rowpx = ws.rowpx.p + R[j].pix_off + j;
+                        v.brec = lp[j];
+                        v.lfm = fp[j];
+                        v.dslot = (const uint16_t *)(jp[j] + h.off_dslot);
+                        v.slotD = (const float *)(jp[j] + h.off_slot);
+                        v.pixels = d_pix + R[j].pix_off;
+                        v.rng = d_rng + (size_t)j * 3 * NS;
+                        v.rng_nstreams = NS;
+                        v.words = at;
+                        at += (size_t)v.nrows * v.Bp;
+                        v.ms = (float *)at;
+                        at += (size_t)v.npx * h.nslots;
+                        v.roff = at;
+                        at += v.npx;
+                        toff[(size_t)k * (nb + 1) + q] = nt;
+                        nt += (v.nrows + tile - 1) / tile;
+                    }
+                    toff[(size_t)k * (nb + 1) + nb] = nt;
+                    tiles[k] = nt;
+                }
+                GF_TRY(ws.view.need(view.size()));
+                GF_TRY(ws.joblist.need(nb));
+                GF_TRY(ws.tileoff.need(toff.size()));
+                GF_TRY(ws.brecptr.need((size_t)njobs));
+                GF_TRY(ws.lfmptr.need((size_t)njobs));
+                GF_TRY(ws.blkoff.need(nb + 1));
+                GF_CUDA(cudaMemcpyAsync(ws.lfmptr.p, fp.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.plans.p, jp.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.view.p, view.data(), sizeof(gfk::DrawJob) * view.size(), cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.joblist.p, jl.data(), 4 * nb, cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.tileoff.p, toff.data(), 4 * toff.size(), cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.brecptr.p, lp.data(), sizeof(void *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
+                GF_CUDA(cudaMemcpyAsync(ws.blkoff.p, boff.data(), 8 * (nb + 1), cudaMemcpyHostToDevice, st));
+                {
                     gfk::BlockLfParams BL;
-                    BL.jobs = d_jobs; BL.plans = ws.plans.p; BL.brec = ws.brecptr.p;
+                    BL.jobs = d_jobs; BL.plans = ws.plans.p; BL.brec = ws.brecptr.p; BL.lfm = ws.lfmptr.p;
                     BL.job_list = ws.joblist.p; BL.blk_off = ws.blkoff.p;
-                    BL.njobs = (int32_t)batched.size(); BL.total = nb_total;
+                    BL.njobs = (int32_t)nb; BL.total = boff[nb];
                     ProfScope ps(ctx, GF_PROF_SLOTS);
                     GF_CUDA(gfk::launch_block_records(BL, st));
-                    /* the host vectors are read by the copies above before they go out of scope */
-                    GF_CUDA(cudaStreamSynchronize(st));
                 }
+                auto make_words = [&](int64_t k) -> gf_status {
+                    gfk::BlockWordParams W;
+                    W.jobs = d_jobs;
+                    W.view = ws.view.p + (size_t)k * njobs;
+                    W.job_list = ws.joblist.p;
+                    W.tile_off = ws.tileoff.p + (size_t)k * (nb + 1);
+                    W.njobs = (int32_t)nb;
+                    W.total_tiles = tiles[k];
+                    W.tile = tile;
+                    ProfScope ps(ctx, GF_PROF_SLOTS);
+                    GF_CUDA(gfk::launch_block_words(W, mtype, slots_max, st));
+                    return GF_OK;
+                };
                 gfk::BatchDrawParams B;
                 memset(&B, 0, sizeof(B));
-                B.brec = ws.brecptr.p;
-                if (gfk::batch_draw_warp_bytes(max_tab(i, batched), &B) > 200 * 1024)
-                    return fail(GF_E_UNSUPPORTED, "magnitude grid too large for the batched draw");
-                B.jobs = d_jobs; B.plans = ws.plans.p; B.ms = ws.msptr.p;
-                /* work items: 32 consecutive streams of a request, requests in decreasing size;
-                 * first the requests that take the block bound of their expected counts
-                 * (non-negative densities, no distance limits), then the others */
+                /* work items: 32 consecutive streams of a request, requests in decreasing size */
                 const int ngroups = (N + 31) / 32;
-                GF_TRY(ws.gitems.need((size_t)batched.size() * ngroups));
-                int32_t nbound = 0;
+                const int32_t ngitems = (int32_t)(nb * (size_t)ngroups);
+                GF_TRY(ws.gitems.need((size_t)ngitems));
                 {
-                    GF_TRY(ws.h_stage.need(4 * batched.size() * (size_t)ngroups));
+                    GF_TRY(ws.h_stage.need(4 * (size_t)ngitems));
                     uint32_t *gi = (uint32_t *)ws.h_stage.p;
                     size_t q = 0;
-                    for (int pass_bound = 1; pass_bound >= 0; pass_bound--) {
-                        for (int j : batched) {
-                            const SkyModel &mj = R[j].hm[i].m;
-                            const bool bj = mj.dmin == 0.f && mj.dmax == 0.f && mj.f >= 0.f && mj.norm >= 0.f;
-                            if (bj != (pass_bound == 1)) continue;
-                            for (int g = 0; g < ngroups; g++) gi[q++] = ((uint32_t)j << 16) | (uint32_t)(32 * g);
-                        }
-                        if (pass_bound == 1) nbound = (int32_t)q;
-                    }
+                    for (int j : batched)
+                        for (int g = 0; g < ngroups; g++) gi[q++] = ((uint32_t)j << 16) | (uint32_t)(32 * g);
                     GF_CUDA(cudaMemcpyAsync(ws.gitems.p, gi, 4 * q, cudaMemcpyHostToDevice, st));
                     GF_CUDA(cudaStreamSynchronize(st));
                 }
-                const int32_t ngitems = (int32_t)(batched.size() * (size_t)ngroups);
                 B.items = ws.gitems.p; B.nitems = ngitems; B.next_item = d_counter;
                 B.ev_count = ctx->d_counters; B.err = ctx->d_counters + 2;
                 GF_TRY(ws.ev.need((size_t)cap));
                 B.ev = ws.ev.p; B.ev_capacity = (int64_t)ws.ev.n;
-                /* the two launches of a draw pass: bound requests, then exact ones */
-                auto draw_all = [&](const gfk::BatchDrawParams &BB, int wpc) -> gf_status {
-                    gfk::BatchDrawParams X = BB;
-                    X.nitems = nbound;
-                    GF_CUDA(gfk::launch_batch_draw(X, mtype, wpc, true, st));
-                    X.items = BB.items + nbound;
-                    X.nitems = ngitems - nbound;
-                    GF_CUDA(gfk::launch_batch_draw(X, mtype, wpc, false, st));
-                    return GF_OK;
-                };
+                B.view = ws.view.p;
+                GF_TRY(make_words(0));
                 if (ctx->draw_wpc[mtype] == 0) {
                     /* autotuner: time 8, 4, 2 and 1 warps per CTA on the head of the work queue
                      * (the largest requests), from the same stream states, and keep the fastest */
-                    const bool tb = nbound > 0;
                     gfk::BatchDrawParams T = B;
-                    const int32_t avail = tb ? nbound : ngitems;
-                    T.items = B.items + (tb ? 0 : nbound);
-                    T.nitems = std::min<int32_t>(avail, std::max<int32_t>(avail / 16, 148 * 8));
+                    T.nitems = std::min<int32_t>(ngitems, std::max<int32_t>(ngitems / 16, 148 * 8));
                     float best_ms = 0.f;
                     int best = 4;
                     cudaEvent_t e0, e1;
@@ -1156,7 +1282,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                         GF_CUDA(cudaMemcpyAsync(d_rng, d_rng_snap, 12 * (size_t)njobs * NS, cudaMemcpyDeviceToDevice, st));
                         GF_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 24, st));
                         GF_CUDA(cudaEventRecord(e0, st));
-                        GF_CUDA(gfk::launch_batch_draw(T, mtype, wpc, tb, st));
+                        GF_CUDA(gfk::launch_batch_draw(T, wpc, st));
                         GF_CUDA(cudaEventRecord(e1, st));
                         GF_CUDA(cudaEventSynchronize(e1));
                         float ms = 0.f;
@@ -1169,16 +1295,17 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                     GF_CUDA(cudaMemcpyAsync(d_rng, d_rng_snap, 12 * (size_t)njobs * NS, cudaMemcpyDeviceToDevice, st));
                 }
                 int64_t nev = 0;
-                for (;;) {
+                for (bool again = false;; again = true) {
                     GF_CUDA(cudaMemsetAsync(ctx->d_counters, 0, 24, st));
-                    {
+                    for (int64_t k = 0; k < nseg; k++) {
+                        if (k > 0 || (again && nseg > 1)) GF_TRY(make_words(k));
+                        B.view = ws.view.p + (size_t)k * njobs;
                         ProfScope ps(ctx, GF_PROF_BATCH_DRAW);
-                        GF_TRY(draw_all(B, ctx->draw_wpc[mtype]));
+                        GF_CUDA(gfk::launch_batch_draw(B, ctx->draw_wpc[mtype], st));
                     }
                     GF_CUDA(cudaMemcpyAsync(ctx->h_counters, ctx->d_counters, 24, cudaMemcpyDeviceToHost, st));
                     GF_CUDA(cudaStreamSynchronize(st));
                     nev = (int64_t)ctx->h_counters[0];
-                    if (ctx->h_counters[2] & 2ull) return fail(GF_E_STATE, "internal: a request without the block bound in the bound draw");
                     if (ctx->h_counters[2]) return fail(GF_E_INVALID, "a bin has an infinite expected star count");
                     if (nev <= B.ev_capacity) break;
                     /* more bins with stars than the event list holds: restore the streams and draw again */
