@@ -183,15 +183,11 @@ __host__ __device__ __forceinline__ float cube_sample(const SkyModel &m, float x
     return m.cube[((size_t)ix[2] * (size_t)m.cube_n[1] + ix[1]) * (size_t)m.cube_n[0] + ix[0]];
 }
 
-/* Model density at the heliocentric position (x, y, z); MODEL is the
+/* Model density at the position (wx, wy, wz) in the model's frame; MODEL is the
  * compile-time model kind (GF_MODEL_EXP_DISK or GF_MODEL_POWER_LAW_ELLIPSOID). */
 template <int MODEL>
-__device__ __forceinline__ float model_rho(const SkyModel &m, float x, float y, float z)
+__device__ __forceinline__ float model_rho_frame(const SkyModel &m, float wx, float wy, float wz)
 {
-    float vx = x + m.T[0], vy = y + m.T[1], vz = z + m.T[2];
-    float wx = m.M[0] * vx + m.M[1] * vy + m.M[2] * vz;
-    float wy = m.M[3] * vx + m.M[4] * vy + m.M[5] * vz;
-    float wz = m.M[6] * vx + m.M[7] * vy + m.M[8] * vz;
     if (MODEL == GF_MODEL_EXP_DISK) {
         float r2 = wx * wx + wy * wy;
         if (m.r_cut2 != 0.f && r2 + wz * wz > m.r_cut2) return 0.f;
@@ -217,6 +213,17 @@ __device__ __forceinline__ float model_rho(const SkyModel &m, float x, float y, 
         while (k != m.nbreaks && rSq > m.rbreakSq[k]) k++;
         return m.f * m.fArr[k] * gfm::powf_(rSq, 0.5f * m.nArr[k]);
     }
+}
+
+/* Model density at the heliocentric position (x, y, z) */
+template <int MODEL>
+__device__ __forceinline__ float model_rho(const SkyModel &m, float x, float y, float z)
+{
+    float vx = x + m.T[0], vy = y + m.T[1], vz = z + m.T[2];
+    float wx = m.M[0] * vx + m.M[1] * vy + m.M[2] * vz;
+    float wy = m.M[3] * vx + m.M[4] * vy + m.M[5] * vz;
+    float wz = m.M[6] * vx + m.M[7] * vy + m.M[8] * vz;
+    return model_rho_frame<MODEL>(m, wx, wy, wz);
 }
 
 /* Distance of the bin (im, iM): DM = (m0 + im dm) - (M1 - iM dM), D = powf(10, 0.2 DM + 1)

@@ -16,11 +16,13 @@
  *           modulus is the same number rounded in a few different ways, so
  *           the anchors of a diagonal take only 1-4 distinct D; the plan lists
  *           the distinct values (the slots) and maps every anchor to its slot.
- *   pixels  (one warp per pixel) the model density at each slot's distance
- *           along the pixel's direction (the only anchor quantity that depends
- *           on D and the pixel), then one lane per diagonal walks its bins:
- *           mu = (((LF(M) * ms) * norm) * D^3) * K, bins with m + Am > m1 cut.
- *           Per pixel the counts and covered counts are summed in FP64.
+ *   pixels  (two pixels a lane, 64 pixels of a request to a warp) the warp walks
+ *           the plan's diagonals and anchors together: on a diagonal each lane
+ *           forms the model density at the diagonal's slot distances along its own
+ *           pixels' directions (the only anchor quantity that depends on D and the
+ *           pixel), then every bin's mu = (((LF(M) * ms) * norm) * D^3) * K, bins
+ *           with m + Am > m1 cut.  Per pixel the counts and covered counts are
+ *           summed in FP64.
  *   totals  (one CTA per request) the pixel sums in a fixed order.
  *
  * Every bin's mu is bit-identical to the crawl's; the totals differ from a
@@ -59,8 +61,6 @@ __device__ __forceinline__ int first_block_start(long long k0)
 }
 
 #define GF_PLAN_REMEMBER 8          /* distinct distances remembered per diagonal */
-
-constexpr int kIntegChunk = 8;      /* pixels per run a warp takes from the shared counter */
 
 /* distinct anchor distances of diagonal d, in order of first appearance; calls
  * emit(anchor ordinal, slot ordinal on the diagonal, D, local index, i, j) for every anchor */
@@ -205,195 +205,278 @@ __global__ void __launch_bounds__(1024) plan_kernel(const IntegPlanDesc *desc)
     }
 }
 
-/* The lane's diagonals d = lane, lane + 32, ... of one pixel: every uncut bin's mu
- * from its anchor slot, summed in FP64 (and, when COV, mu * cf as well). */
-template <bool COV>
-__device__ __forceinline__ void walk_diagonals(int lane, int nd, int x, int y, int icut, const int2 *diag,
-                                               const uint16_t *anc, const float *LFM, const float2 *Q, float norm,
-                                               float K, float cf, double &cnt, double &cov)
+#define GF_IG_WARPS 4               /* warps of a CTA, all on one request */
+#define GF_IG_SLOTS 8               /* slots of a diagonal kept per lane (a plan has 1-4; further ones are formed anew) */
+
+/* a float's bits as a double: exact for positive normal floats.  One wide multiply-add places the
+ * mantissa and adds the difference of the exponent biases; the conversion instruction runs at an
+ * eighth of the rate of an addition, so a run's bins take the two ways in turn. */
+__device__ __forceinline__ double widen_positive(float v)
 {
-    /* two partial sums per quantity (even and odd bins of each run) halve the chain of
-     * dependent FP64 additions; they are added at the end, in a fixed order */
-    double c0 = 0.0, c1 = 0.0, v0 = 0.0, v1 = 0.0;
-    for (int d = lane; d < nd; d += 32) {
+    return __longlong_as_double((long long)((uint64_t)__float_as_uint(v) * (1ull << 29) + (0x380ull << 52)));
+}
+
+/* the products of two pixels at once (each rounded to nearest, as FMUL) */
+__device__ __forceinline__ float2 mul2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+/* scalar additions: the compiler contracts packed products and packed sums even though both ask for rounding */
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
+
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+
+/* sums of a lane's two pixels: counts, covered counts */
+struct PixelSums {
+    double cx = 0.0, cy = 0.0, vx = 0.0, vy = 0.0;
+};
+
+/* what the lanes of a warp share while they walk a request's diagonals */
+struct DiagonalWalk {
+    const int2 *diag;
+    const uint16_t *anc, *dslot;
+    const float *slotD;
+    int nslots, d0, d1;
+    int icmin, icmax;              /* the lanes' cut rows lie between */
+    const float2 *lf;              /* LF rows reversed (entry k is LF(nM - 1 - k)), each twice; a second copy from entry 1 on, pitch apart */
+    int pitch;
+    float lfmin, lfmax;
+};
+
+/* the directions of a lane's two pixels */
+struct PixelPair {
+    float2 cl, cb, sl, sb;
+};
+
+/* model density of both pixels at distance D (anchor_x's expressions: px = D cl cb ..., then the model's frame) */
+template <int MODEL>
+__device__ __forceinline__ float2 pair_density(const SkyModel &m, const PixelPair &P, float D)
+{
+    const float2 D2 = both(D);
+    const float2 vx = add2(mul2(mul2(D2, P.cl), P.cb), both(m.T[0]));
+    const float2 vy = add2(mul2(mul2(D2, P.sl), P.cb), both(m.T[1]));
+    const float2 vz = add2(mul2(D2, P.sb), both(m.T[2]));
+    const float2 wx = add2(add2(mul2(both(m.M[0]), vx), mul2(both(m.M[1]), vy)), mul2(both(m.M[2]), vz));
+    const float2 wy = add2(add2(mul2(both(m.M[3]), vx), mul2(both(m.M[4]), vy)), mul2(both(m.M[5]), vz));
+    const float2 wz = add2(add2(mul2(both(m.M[6]), vx), mul2(both(m.M[7]), vy)), mul2(both(m.M[8]), vz));
+    return make_float2(gfc::model_rho_frame<MODEL>(m, wx.x, wy.x, wz.x), gfc::model_rho_frame<MODEL>(m, wx.y, wy.y, wz.y));
+}
+
+/* One pair of bins of both pixels (entries lp->xy and lp->zw): products, then the sums; odd: the second bin counts too */
+template <bool COV>
+__device__ __forceinline__ void add_bins(const float4 *lp, float2 ms, float2 D3, float2 K, float2 cf, bool odd, bool turn, PixelSums &sum)
+{
+    const float4 l = *lp;
+    float2 p = mul2({l.x, l.y}, ms), q = mul2({l.z, l.w}, ms);
+    p = mul2(p, D3);
+    q = mul2(q, D3);
+    p = mul2(p, K);
+    q = mul2(q, K);
+    sum.cx += (double)p.x;
+    sum.cy += widen_positive(p.y);
+    if (odd) {
+        sum.cx += widen_positive(q.x);
+        sum.cy += turn ? (double)q.y : widen_positive(q.y);
+    }
+    if (COV) {
+        p = mul2(p, cf);
+        q = mul2(q, cf);
+        sum.vx += (double)p.x;
+        sum.vy += widen_positive(p.y);
+        if (odd) {
+            sum.vx += widen_positive(q.x);
+            sum.vy += turn ? (double)q.y : widen_positive(q.y);
+        }
+    }
+}
+
+/* The diagonals [d0, d1) of the lanes' pixels; K, cf, icut: of each lane's two pixels. */
+template <int MODEL, bool COV>
+__device__ __forceinline__ void walk_diagonals(const SkyModel &m, const DiagonalWalk &W, const PixelPair &pix, int2 icut, float2 K,
+                                               float2 cf, float2 (*s_ms)[32], int lane, PixelSums &sum)
+{
+    const int x = m.nm, y = m.nM, nd = x + y - 1;
+    const float norm = m.norm;
+    const bool dlim = m.dmin != 0.f || m.dmax != 0.f;
+    for (int d = W.d0; d < W.d1; d++) {
         const int i0 = d - (y - 1) > 0 ? d - (y - 1) : 0;
-        int i1 = d < x - 1 ? d : x - 1;
-        i1 = i1 < icut - 1 ? i1 : icut - 1;
-        if (i1 < i0) continue;
-        const int2 dg = diag[d];
-        const uint16_t *ap = anc + dg.x;
-        const float *lf = LFM + (d - i0);           /* LF of bin t of the diagonal: lf[-t] */
-        const int tl = i1 - i0 + 1;
-        int t = 0, seg_end = dg.y < tl ? dg.y : tl;
+        const int len = (d < x - 1 ? d : x - 1) - i0 + 1;
+        const int tmax = min(len, W.icmax - i0);
+        if (tmax <= 0) continue;
+        const int tmin = min(len, W.icmin - i0);
+        const int2 dg = __ldg(W.diag + d);
+        const int s0 = __ldg(W.dslot + d), ns = (d + 1 < nd ? (int)__ldg(W.dslot + d + 1) : W.nslots) - s0;
+        /* The densities, and for which slots every product of the diagonal is a positive normal float in all
+         * lanes' pixels (then the widening by bits is exact). */
+        unsigned plain = 0;
+        for (int k = 0; k < ns && k < GF_IG_SLOTS; k++) {
+            const float D = __ldg(W.slotD + s0 + k);
+            const float2 ms = pair_density<MODEL>(m, pix, D);
+            s_ms[k][lane] = ms;
+            const float f3 = D * D * D;
+            const float fx = ms.x * f3 * K.x * (COV ? cf.x : 1.0f), fy = ms.y * f3 * K.y * (COV ? cf.y : 1.0f);
+            if (__all_sync(0xffffffffu, W.lfmin * fminf(fx, fy) > 1.0e-30f && W.lfmax * fmaxf(fx, fy) < 1.0e30f)) plain |= 1u << k;
+        }
+        if (norm != 1.0f) plain = 0;
+        const int st = (y - 1) - (d - i0);             /* the entry of the diagonal's first bin */
+        const uint16_t *ap = W.anc + dg.x;
+        int t = 0, seg_end = min(dg.y, tmax), slot = __ldg(ap);
         for (;;) {
-            const float2 q = Q[*ap++];
-            if (q.y >= 0.f) {
-                /* One code path for whole and partial segments (no divergence between
-                 * lanes whose segments differ in length): bins u >= len read no LF and
-                 * add an exact +0.0, so the sums take the segment's bins in the order
-                 * of the plain loop (even offsets to c0, odd ones to c1). */
-                const int len = seg_end - t;
-                float mv[GF_BLOCK];
+            const int rel = slot - s0, n = seg_end - t;
+            const float D = __ldg(W.slotD + slot);
+            if (seg_end < tmax) slot = __ldg(++ap);
+            if (!(dlim && (m.dmin > D || m.dmax <= D))) {
+                const float2 ms = rel < GF_IG_SLOTS ? s_ms[rel][lane] : pair_density<MODEL>(m, pix, D);
+                const float2 D3 = both(D * D * D);
+                if (rel < GF_IG_SLOTS && ((plain >> rel) & 1u) && seg_end <= tmin) {
+                    const int at = st + t;
+                    const float4 *lp = (const float4 *)(W.lf + (at & 1) * W.pitch + (at & ~1));
+                    if (n == GF_BLOCK) {
 #pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] = u < len ? lf[-(t + u)] : 0.f;
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] *= q.x;
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] *= norm;
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] *= q.y;
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] *= K;
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u++) mv[u] = u < len ? mv[u] : 0.f;    /* 0 * inf would be NaN */
-#pragma unroll
-                for (int u = 0; u < GF_BLOCK; u += 2) {
-                    c0 += (double)mv[u];
-                    c1 += (double)mv[u + 1];
-                    if (COV) {
-                        v0 += (double)(mv[u] * cf);
-                        v1 += (double)(mv[u + 1] * cf);
+                        for (int u = 0; u < GF_BLOCK / 2; u++) add_bins<COV>(lp + u, ms, D3, K, cf, true, u & 1, sum);
+                    } else {
+#pragma unroll 1
+                        for (int u = 0; u < n; u += 2) add_bins<COV>(lp++, ms, D3, K, cf, u + 1 < n, false, sum);
+                    }
+                } else {
+                    for (int q = t; q < seg_end; q++) {
+                        float2 mu = mul2(W.lf[st + q], ms);
+                        mu = mul2(mu, both(norm));
+                        mu = mul2(mu, D3);
+                        mu = mul2(mu, K);
+                        if (i0 + q < icut.x) {
+                            sum.cx += (double)mu.x;
+                            if (COV) sum.vx += (double)(mu.x * cf.x);
+                        }
+                        if (i0 + q < icut.y) {
+                            sum.cy += (double)mu.y;
+                            if (COV) sum.vy += (double)(mu.y * cf.y);
+                        }
                     }
                 }
             }
             t = seg_end;
-            if (t >= tl) break;
-            seg_end = t + GF_BLOCK < tl ? t + GF_BLOCK : tl;
+            if (t >= tmax) break;
+            seg_end = min(t + GF_BLOCK, tmax);
         }
     }
-    cnt += c0 + c1;
-    if (COV) cov += v0 + v1;
 }
 
-/* One warp per pixel.  Per-warp shared tables: the request's model, LF at every
- * absolute-magnitude row, m at every apparent-magnitude row, and (ms, D^3) of
- * every slot of the pixel (D^3 = -inf marks an anchor outside [dmin, dmax)). */
+/* A warp takes a group of 64 pixels of one request (in P.order: the fully covered ones first, so that
+ * only the groups with partly covered pixels form the covered products) and one of P.splits parts of
+ * their diagonals; a CTA's warps share the request's model and LF table.  The plan's control flow, its
+ * loads and the LF reads are the same for all lanes; per bin and pixel there remain the float products
+ * (two pixels to an instruction), a conversion and an FP64 addition.  Bound by instruction issue: 10 warp
+ * instructions per bin of 32 pixels, 58 % of the slots used (4.3e9 bins: 1.35e9 instructions; with a warp a
+ * pixel and a lane a diagonal 2.57e9, at 22 of 32 lanes, the conversions alone half the time).  Three models:
+ * 256 beams 35.3 -> 29.6 ms, 8 beams 1.43 -> 0.62 ms. */
 template <int MODEL>
-__global__ void __launch_bounds__(256) integrate_pixels_kernel(IntegPixParams P)
+__global__ void __launch_bounds__(32 * GF_IG_WARPS) integrate_pixels_kernel(IntegPixParams P)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    unsigned char *mine = smem + (size_t)wib * P.warp_bytes;
-    SkyModel &m = *(SkyModel *)mine;
-    float *LFM = (float *)(mine + P.off_lf);
-    float *MMr = (float *)(mine + P.off_mr);
-    float2 *Q = (float2 *)(mine + P.off_q);
-    int job = -1;
-    const unsigned char *plan = nullptr;
-    const int2 *diag = nullptr;
-    const float *slotD = nullptr;
-    const uint16_t *anc = nullptr;
-    int nslots = 0;
-    const gf_pencil_beam *pixels = nullptr;
-    SkyGeom g;
-    g.ext_kind = GF_EXT_NONE;
-    g.ammin = nullptr;
-    /* runs of kIntegChunk consecutive pixels (mostly of one request) taken from a
-     * shared counter: the request's tables are set up once per run, not per pixel */
-    int p = 0, pend = 0, job_end = 0;
-    for (;;) {
-        if (p >= pend) {
-            unsigned u0 = 0;
-            if (lane == 0) u0 = atomicAdd(P.next, (unsigned)kIntegChunk);
-            u0 = __shfl_sync(0xffffffffu, u0, 0);
-            if (u0 >= (unsigned)P.total_pix) break;
-            p = (int)u0;
-            pend = p + kIntegChunk < P.total_pix ? p + kIntegChunk : P.total_pix;
-        } else {
-            p++;
-            if (p >= pend) continue;
+    extern __shared__ __align__(16) float2 s_lf[];
+    __shared__ SkyModel m;
+    __shared__ float2 s_ms[GF_IG_WARPS][GF_IG_SLOTS][32];
+    __shared__ float s_ext[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int loaded = -1;
+    for (int cta = blockIdx.x; cta < P.total_ctas; cta += gridDim.x) {
+        int job = 0, hi = P.njobs;
+        while (hi - job > 1) {
+            const int mid = (job + hi) >> 1;
+            if (P.cta_off[mid] <= cta) job = mid; else hi = mid;
         }
-        /* the request of flat pixel p: pix_off is increasing */
-        int lo = job;
-        if (job < 0 || p < P.pix_off[job] || p >= job_end) {
-            lo = 0;
-            int hi = P.njobs;
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (P.pix_off[mid] <= p) lo = mid; else hi = mid;
+        const CrawlJob &J = P.jobs[job];
+        if (job != loaded) {
+            __syncthreads();
+            for (int w = threadIdx.x; w < (int)(sizeof(SkyModel) / 4); w += blockDim.x) ((uint32_t *)&m)[w] = ((const uint32_t *)&J.m)[w];
+            __syncthreads();
+            for (int k = threadIdx.x; k < P.pitch; k += blockDim.x) {
+                const float v = k < m.nM ? gfc::lf_sample(m, m.lf, m.M1 - (float)(m.nM - 1 - k) * m.dM) : 0.f;
+                s_lf[k] = make_float2(v, v);
+                if (k > 0) s_lf[P.pitch + k - 1] = make_float2(v, v);
             }
-        }
-        if (lo != job) {
-            job_end = P.pix_off[lo + 1];
-            job = lo;
-            plan = P.plans[job];
-            if (plan) {
-                __syncwarp();
-                const uint32_t *src = (const uint32_t *)&P.jobs[job].m;
-                for (int w = lane; w < (int)(sizeof(SkyModel) / 4); w += 32) ((uint32_t *)&m)[w] = src[w];
-                __syncwarp();
-                for (int q = lane; q < m.nM; q += 32) LFM[q] = gfc::lf_sample(m, m.lf, m.M1 - (float)q * m.dM);
-                for (int q = lane; q < m.nm; q += 32) MMr[q] = m.m0 + m.dm * (float)q;
-                const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
-                nslots = h->nslots;
-                diag = (const int2 *)(plan + ((sizeof(IntegPlanHdr) + 15) & ~15));
-                slotD = (const float *)(plan + h->off_slot);
-                anc = (const uint16_t *)(plan + h->off_anc);
-                pixels = P.jobs[job].g.pixels;
-                g.ext_kind = P.jobs[job].g.ext_kind;
-                g.ammin = P.jobs[job].g.ammin;
-                __syncwarp();
+            __syncthreads();
+            if (warp == 0) {
+                float lo = s_lf[0].x, up = lo;
+                for (int k = lane; k < m.nM; k += 32) { lo = fminf(lo, s_lf[k].x); up = fmaxf(up, s_lf[k].x); }
+                for (int o = 16; o > 0; o >>= 1) {
+                    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+                    up = fmaxf(up, __shfl_xor_sync(0xffffffffu, up, o));
+                }
+                if (lane == 0) { s_ext[0] = lo; s_ext[1] = up; }
             }
+            __syncthreads();
+            loaded = job;
         }
-        if (!plan) continue;
-        const int ilb = p - (int)P.pix_off[job];
-        const gf_pencil_beam pix = pixels[ilb];
-        const float Am = gfc::beam_extinction(g, pix);
-        const float K = pix.dA * GF_POGSON * m.dm * m.dM;
-        const float cf = pix.coveredFraction;
-        const float norm = m.norm, m1 = m.m1;
+        const unsigned char *plan = P.plans[job];
+        const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
+        const int npix = J.g.npixels, unit = (cta - P.cta_off[job]) * GF_IG_WARPS + warp;
+        const int g = unit / P.splits, sp = unit - g * P.splits;
+        if (g * 64 >= npix) continue;
+        const int qa = g * 64 + lane, qb = qa + 32, base = P.pix_off[job];
+        const uint32_t ia = P.order[base + min(qa, npix - 1)], ib = P.order[base + min(qb, npix - 1)];
+        const gf_pencil_beam pa = J.g.pixels[ia], pb = J.g.pixels[ib];
+        const float2 K = {pa.dA * GF_POGSON * m.dm * m.dM, pb.dA * GF_POGSON * m.dm * m.dM};
+        const float2 cf = {pa.coveredFraction, pb.coveredFraction};
+        const PixelPair pix = {{pa.cl, pb.cl}, {pa.cb, pb.cb}, {pa.sl, pb.sl}, {pa.sb, pb.sb}};
+        const int2 icut = make_int2((int)(P.prow[base + ia].y & 0xffffu), (int)(P.prow[base + ib].y & 0xffffu));
+        /* the diagonals whose first bin lies in the part's share of the bins */
         const int x = m.nm, y = m.nM, nd = x + y - 1;
-        const bool dlim = m.dmin != 0.f || m.dmax != 0.f;
-        /* model density of every slot along this pixel's direction (anchor_x) */
-        for (int s = lane; s < nslots; s += 32) {
-            const float D = slotD[s];
-            const float px = D * pix.cl * pix.cb;
-            const float py = D * pix.sl * pix.cb;
-            const float pz = D * pix.sb;
-            const float ms = gfc::model_rho<MODEL>(m, px, py, pz);
-            const bool dcut = dlim && (m.dmin > D || m.dmax <= D);
-            Q[s] = make_float2(ms, dcut ? -__int_as_float(0x7f800000) : D * D * D);
-        }
-        /* apparent-magnitude rows at and after icut are cut (m0 + dm im is increasing in im) */
-        int icut = x;
-        for (int i = lane; i < x; i += 32)
-            if (MMr[i] + Am > m1) { icut = i; break; }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const int t = __shfl_xor_sync(0xffffffffu, icut, o);
-            icut = t < icut ? t : icut;
-        }
-        __syncwarp();
-        double cnt = 0.0, cov = 0.0;
-        if (cf == 1.0f) {
-            /* fully covered pixel: mu * cf == mu, so the covered sum is the sum */
-            walk_diagonals<false>(lane, nd, x, y, icut, diag, anc, LFM, Q, norm, K, cf, cnt, cov);
-            cov = cnt;
+        auto diagonal_at = [&](long long bin) {
+            int lo = 0, up = nd;
+            while (lo < up) {
+                const int mid = (lo + up) >> 1;
+                if (diag_start(mid, x, y) < bin) lo = mid + 1; else up = mid;
+            }
+            return lo;
+        };
+        const long long bins = (long long)x * y;
+        DiagonalWalk W;
+        W.d0 = sp == 0 ? 0 : diagonal_at(bins * sp / P.splits);
+        W.d1 = sp + 1 == P.splits ? nd : diagonal_at(bins * (sp + 1) / P.splits);
+        W.icmin = __reduce_min_sync(0xffffffffu, min(icut.x, icut.y));
+        W.icmax = __reduce_max_sync(0xffffffffu, max(icut.x, icut.y));
+        W.diag = (const int2 *)(plan + ((sizeof(IntegPlanHdr) + 15) & ~15));
+        W.slotD = (const float *)(plan + h->off_slot);
+        W.anc = (const uint16_t *)(plan + h->off_anc);
+        W.dslot = (const uint16_t *)(plan + h->off_dslot);
+        W.nslots = h->nslots;
+        W.lf = s_lf;
+        W.pitch = P.pitch;
+        W.lfmin = s_ext[0];
+        W.lfmax = s_ext[1];
+        PixelSums sum;
+        if (__all_sync(0xffffffffu, cf.x == 1.0f && cf.y == 1.0f)) {
+            /* fully covered pixels: mu * cf == mu, so the covered sum is the sum */
+            walk_diagonals<MODEL, false>(m, W, pix, icut, K, cf, s_ms[warp], lane, sum);
+            sum.vx = sum.cx;
+            sum.vy = sum.cy;
         } else {
-            walk_diagonals<true>(lane, nd, x, y, icut, diag, anc, LFM, Q, norm, K, cf, cnt, cov);
+            walk_diagonals<MODEL, true>(m, W, pix, icut, K, cf, s_ms[warp], lane, sum);
         }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-            cov += __shfl_xor_sync(0xffffffffu, cov, o);
-        }
-        if (lane == 0) P.pix_sum[p] = make_double2(cnt, cov);
-        __syncwarp();
+        double2 *out = P.pix_sum + (size_t)sp * P.total_pix + base;
+        if (qa < npix) out[ia] = make_double2(sum.cx, sum.vx);
+        if (qb < npix) out[ib] = make_double2(sum.cy, sum.vy);
     }
 }
 
-__global__ void __launch_bounds__(256) job_totals_kernel(const double2 *pix_sum, const int32_t *pix_off,
+__global__ void __launch_bounds__(256) job_totals_kernel(const double2 *pix_sum, const int32_t *pix_off, int splits, int total_pix,
                                                           const unsigned char *const *plans, double2 *tot)
 {
     __shared__ double sc[256], sv[256];
     const int j = blockIdx.x;
     double c = 0.0, v = 0.0;
     if (plans[j])
-        for (int p = pix_off[j] + threadIdx.x; p < pix_off[j + 1]; p += blockDim.x) {
-            const double2 s = pix_sum[p];
-            c += s.x;
-            v += s.y;
-        }
+        for (int sp = 0; sp < splits; sp++)
+            for (int p = pix_off[j] + threadIdx.x; p < pix_off[j + 1]; p += blockDim.x) {
+                const double2 s = pix_sum[(size_t)sp * total_pix + p];
+                c += s.x;
+                v += s.y;
+            }
     sc[threadIdx.x] = c;
     sv[threadIdx.x] = v;
     __syncthreads();
@@ -428,54 +511,43 @@ cudaError_t launch_integ_plans(const IntegPlanDesc *desc_dev, int nplans, cudaSt
     return cudaGetLastError();
 }
 
-size_t integ_warp_bytes(int nm_max, int nM_max, int slots_max, IntegPixParams *P)
+int integ_splits(int64_t groups)
 {
-    size_t off = (sizeof(SkyModel) + 15) & ~(size_t)15;
-    P->off_lf = (int32_t)off;
-    off += ((size_t)4 * nM_max + 15) & ~(size_t)15;
-    P->off_mr = (int32_t)off;
-    off += ((size_t)4 * nm_max + 15) & ~(size_t)15;
-    P->off_q = (int32_t)off;
-    off += (size_t)8 * slots_max;
-    off = (off + 15) & ~(size_t)15;
-    P->warp_bytes = (int32_t)off;
-    return off;
+    /* parts of the diagonals: about 128 warps an SM (several rounds of them, so that a large request does not end last) */
+    const int64_t want = (int64_t)sm_count() * 128;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(32, want / std::max<int64_t>(groups, 1)));
+}
+
+int64_t integ_ctas(int64_t npix, int splits) { return ((npix + 63) / 64 * splits + GF_IG_WARPS - 1) / GF_IG_WARPS; }
+
+size_t integ_smem(int nM_max, int32_t *pitch)
+{
+    *pitch = (int32_t)((nM_max + 15) & ~3);
+    return 16 * (size_t)*pitch;
+}
+
+template <int MODEL>
+static cudaError_t launch_integrate_pixels_t(const IntegPixParams &P, cudaStream_t s)
+{
+    const size_t smem = 16 * (size_t)P.pitch;
+    cudaError_t e = cudaFuncSetAttribute(integrate_pixels_kernel<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, integrate_pixels_kernel<MODEL>, 32 * GF_IG_WARPS, smem);
+    if (e != cudaSuccess) return e;
+    const int blocks = (int)std::min<long long>(P.total_ctas, (long long)sm_count() * std::max(per_sm, 1));
+    integrate_pixels_kernel<MODEL><<<blocks, 32 * GF_IG_WARPS, smem, s>>>(P);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_integrate_pixels(const IntegPixParams &P, int model_type, double2 *tot, cudaStream_t s)
 {
-    if (P.total_pix <= 0) return cudaSuccess;
-    if (!P.next) return cudaErrorInvalidValue;
-    const size_t max_smem = 200 * 1024;
-    int wpb = (int)std::min<size_t>(8, max_smem / (size_t)P.warp_bytes);
-    if (wpb < 1) return cudaErrorInvalidValue;
-    const size_t smem = (size_t)wpb * P.warp_bytes;
-    const int threads = 32 * wpb;
-    cudaError_t e;
-    int per_sm = 0;
-    if (model_type == GF_MODEL_EXP_DISK) {
-        e = cudaFuncSetAttribute(integrate_pixels_kernel<GF_MODEL_EXP_DISK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, integrate_pixels_kernel<GF_MODEL_EXP_DISK>, threads, smem);
-    } else {
-        e = cudaFuncSetAttribute(integrate_pixels_kernel<GF_MODEL_POWER_LAW_ELLIPSOID>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, integrate_pixels_kernel<GF_MODEL_POWER_LAW_ELLIPSOID>, threads, smem);
-    }
+    if (P.total_ctas <= 0) return cudaSuccess;
+    if (16 * (size_t)P.pitch > 200 * 1024 || P.splits < 1) return cudaErrorInvalidValue;
+    cudaError_t e = model_type == GF_MODEL_EXP_DISK ? launch_integrate_pixels_t<GF_MODEL_EXP_DISK>(P, s)
+                                                    : launch_integrate_pixels_t<GF_MODEL_POWER_LAW_ELLIPSOID>(P, s);
     if (e != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    const long long need = ((long long)P.total_pix + wpb * kIntegChunk - 1) / (wpb * kIntegChunk);
-    const int blocks = (int)std::min<long long>(need, (long long)sm_count() * per_sm);
-    e = cudaMemsetAsync(P.next, 0, sizeof(uint32_t), s);
-    if (e != cudaSuccess) return e;
-    if (model_type == GF_MODEL_EXP_DISK)
-        integrate_pixels_kernel<GF_MODEL_EXP_DISK><<<blocks, threads, smem, s>>>(P);
-    else
-        integrate_pixels_kernel<GF_MODEL_POWER_LAW_ELLIPSOID><<<blocks, threads, smem, s>>>(P);
-    count_launches(1);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    job_totals_kernel<<<P.njobs, 256, 0, s>>>(P.pix_sum, P.pix_off, P.plans, tot);
+    job_totals_kernel<<<P.njobs, 256, 0, s>>>(P.pix_sum, P.pix_off, P.splits, P.total_pix, P.plans, tot);
     count_launches(1);
     return cudaGetLastError();
 }

@@ -191,14 +191,19 @@ struct IntegPixParams {
     const CrawlJob *jobs;          /* per request: model, geometry (pixels, extinction) */
     const unsigned char *const *plans;   /* per request: plan of its grid, or null (request skipped) */
     const int32_t *pix_off;        /* [njobs + 1] first flat pixel of each request */
-    int32_t njobs, total_pix;
-    double2 *pix_sum;              /* [total_pix] (expected, expected covered) */
-    int32_t off_lf, off_mr, off_q, warp_bytes;   /* per-warp shared-memory layout (integ_warp_bytes) */
-    uint32_t *next;                /* device counter of the pixel runs handed out (reset by the launch) */
+    const int32_t *cta_off;        /* [njobs + 1] first CTA of each request (integ_ctas each, none if skipped) */
+    const uint32_t *order;         /* [total_pix] per request its pixels, the fully covered ones first */
+    const uint2 *prow;             /* [total_pix] cut row of each pixel (pixel rows, below) */
+    int32_t njobs, total_pix, total_ctas, splits;
+    double2 *pix_sum;              /* [splits][total_pix] (expected, expected covered) of each part of the diagonals */
+    int32_t pitch;                 /* entries of a copy of the LF table (integ_smem) */
 };
 size_t integ_plan_bytes(int nm, int nM, int *max_anchors, int *max_slots);
 cudaError_t launch_integ_plans(const IntegPlanDesc *desc_dev, int nplans, cudaStream_t s);
-size_t integ_warp_bytes(int nm_max, int nM_max, int slots_max, IntegPixParams *P);
+/* parts of the diagonals for that many groups of 64 pixels; CTAs of a request; shared memory of a CTA */
+int integ_splits(int64_t groups);
+int64_t integ_ctas(int64_t npix, int splits);
+size_t integ_smem(int nM_max, int32_t *pitch);
 /* per-pixel sums into P.pix_sum, then per-request totals into tot[njobs] */
 cudaError_t launch_integrate_pixels(const IntegPixParams &P, int model_type, double2 *tot, cudaStream_t s);
 

@@ -169,9 +169,15 @@ struct ReqInfo {
 };
 
 /* The pixel rows of a request: per pixel its row and cut row (gf_launch.h), and each row's first
- * pixel.  The cut row is the first im with m0 + dm im + Am > m1 in float, as the crawl cuts its bins. */
-void pixel_rows(const SkyModel &m, const gf_job &J, uint2 *prow, std::vector<int32_t> &rowpx)
+ * pixel; and the pixels with the fully covered ones first.  The cut row is the first im with
+ * m0 + dm im + Am > m1 in float, as the crawl cuts its bins. */
+void pixel_rows(const SkyModel &m, const gf_job &J, uint2 *prow, uint32_t *order, std::vector<int32_t> &rowpx)
 {
+    /* the integrate's order: fully covered pixels first */
+    uint32_t full = 0;
+    for (int p = 0; p < J.npixels; p++) full += J.pixels[p].coveredFraction == 1.0f;
+    uint32_t nf = 0, npart = full;
+    for (int p = 0; p < J.npixels; p++) order[J.pixels[p].coveredFraction == 1.0f ? nf++ : npart++] = (uint32_t)p;
     rowpx.clear();
     rowpx.reserve((size_t)J.npixels / GF_ROW_PIXELS + 64);
     const bool ext = J.beam_ammin && J.ext.kind != GF_EXT_NONE;
@@ -228,6 +234,8 @@ struct MultiWS {
     Grow<float> lf;
     Grow<gf_pencil_beam> pix;
     Grow<uint2> prow;                       /* pixel rows (gf_launch.h): per pixel */
+    Grow<uint32_t> order;                   /* pixel-by-pixel integrate: pixels, the fully covered ones first */
+    Grow<int32_t> ctaoff;
     Grow<int32_t> rowpx;                    /* first pixel of each row: request j's from its first pixel + j on */
     Grow<float> lfm;                        /* batched draw: LF at each absolute-magnitude row, per request */
     Grow<float *> lfmptr;
@@ -645,19 +653,21 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         /* one page-locked staging area: all pixels, then the per-beam extinction, then the LFs */
         const size_t pb = sizeof(gf_pencil_beam) * (size_t)pix_total, ab = 4 * (size_t)pix_total;
         const size_t lb_ = 4 * (size_t)njobs * nmod * 1024;
-        const size_t rb_ = 8 * (size_t)pix_total, xb = 4 * ((size_t)pix_total + njobs);
+        const size_t rb_ = 8 * (size_t)pix_total, xb = 4 * ((size_t)pix_total + njobs), ob = 4 * (size_t)pix_total;
         GF_TRY(ws.prow.need((size_t)pix_total));
         GF_TRY(ws.rowpx.need((size_t)pix_total + njobs));
-        GF_TRY(ws.h_stage.need(pb + ab + lb_ + rb_ + xb));
+        GF_TRY(ws.order.need((size_t)pix_total));
+        GF_TRY(ws.h_stage.need(pb + ab + lb_ + rb_ + xb + ob));
         char *h = ws.h_stage.p;
         gf_pencil_beam *hp = (gf_pencil_beam *)h;
         float *ha = (float *)(h + pb), *hl = (float *)(h + pb + ab);
         uint2 *hr = (uint2 *)(h + pb + ab + lb_);
         int32_t *hx = (int32_t *)(h + pb + ab + lb_ + rb_);
+        uint32_t *ho = (uint32_t *)(h + pb + ab + lb_ + rb_ + xb);
         memset(hl, 0, lb_);
         parallel_for(njobs, [&](int j) {
             if (!R[j].plain) {
-                pixel_rows(R[j].hm[0].m, jobs[j], hr + R[j].pix_off, R[j].rowpx);
+                pixel_rows(R[j].hm[0].m, jobs[j], hr + R[j].pix_off, ho + R[j].pix_off, R[j].rowpx);
                 std::copy(R[j].rowpx.begin(), R[j].rowpx.end(), hx + R[j].pix_off + j);
             }
             memcpy(hp + R[j].pix_off, jobs[j].pixels, sizeof(gf_pencil_beam) * (size_t)jobs[j].npixels);
@@ -671,6 +681,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         GF_CUDA(cudaMemcpyAsync(d_lf, hl, lb_, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaMemcpyAsync(ws.prow.p, hr, rb_, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaMemcpyAsync(ws.rowpx.p, hx, xb, cudaMemcpyHostToDevice, st));
+        GF_CUDA(cudaMemcpyAsync(ws.order.p, ho, ob, cudaMemcpyHostToDevice, st));
         GF_CUDA(cudaStreamSynchronize(st));
     }
     /* distance tables D[im][iM], shared by the requests with the same magnitude grid */
@@ -803,15 +814,26 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     };
     std::vector<double2> htot(njobs);
     const bool pixel_integrate = pix_total < (int64_t)INT32_MAX;
+    int splits = 1;
+    int32_t total_ctas = 0;
     if (pixel_integrate && !integ.empty()) {
         std::vector<int32_t> off(njobs + 1);
         for (int j = 0; j < njobs; j++) off[j] = (int32_t)R[j].pix_off;
         off[njobs] = (int32_t)pix_total;
         GF_TRY(ws.pixoff.need((size_t)njobs + 1));
         GF_CUDA(cudaMemcpyAsync(ws.pixoff.p, off.data(), 4 * ((size_t)njobs + 1), cudaMemcpyHostToDevice, st));
-        GF_TRY(ws.pixsum.need((size_t)std::max<int64_t>(pix_total, 1)));
         GF_TRY(ws.tot.need((size_t)njobs));
         GF_TRY(ws.plans.need((size_t)njobs));
+        int64_t groups = 0;
+        for (int j : integ) groups += (jobs[j].npixels + 63) / 64;
+        splits = gfk::integ_splits(groups);
+        GF_TRY(ws.pixsum.need((size_t)std::max<int64_t>(pix_total, 1) * splits));
+        std::vector<int32_t> coff(njobs + 1, 0);
+        for (int j = 0; j < njobs; j++)
+            coff[j + 1] = coff[j] + (R[j].plain ? 0 : (int32_t)gfk::integ_ctas(jobs[j].npixels, splits));
+        total_ctas = coff[njobs];
+        GF_TRY(ws.ctaoff.need((size_t)njobs + 1));
+        GF_CUDA(cudaMemcpyAsync(ws.ctaoff.p, coff.data(), 4 * ((size_t)njobs + 1), cudaMemcpyHostToDevice, st));
     }
     setup_time.stop();
     for (int i = 0; i < nmod && !integ.empty(); i++) {
@@ -852,27 +874,27 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 GF_CUDA(cudaMemcpyAsync(hh + q, uniq[q], sizeof(gfk::IntegPlanHdr), cudaMemcpyDeviceToHost, st));
             GF_CUDA(cudaStreamSynchronize(st));
             bool ok = true;
-            int slots_max = 1, nm_max = 1, nM_max = 1;
+            int nM_max = 1;
             for (size_t q = 0; q < uniq.size(); q++) {
                 ok = ok && hh[q].ok;
-                slots_max = std::max(slots_max, hh[q].nslots);
                 plan_hdr[uniq[q]] = hh[q];
             }
-            for (int j : integ) {
-                nm_max = std::max(nm_max, R[j].hm[i].m.nm);
-                nM_max = std::max(nM_max, R[j].hm[i].m.nM);
-            }
+            for (int j : integ) nM_max = std::max(nM_max, R[j].hm[i].m.nM);
             gfk::IntegPixParams P;
             memset(&P, 0, sizeof(P));
-            if (ok && gfk::integ_warp_bytes(nm_max, nM_max, slots_max, &P) <= 200 * 1024) {
+            if (ok && gfk::integ_smem(nM_max, &P.pitch) <= 200 * 1024) {
                 GF_CUDA(cudaMemcpyAsync(ws.plans.p, job_plan.data(), sizeof(unsigned char *) * (size_t)njobs, cudaMemcpyHostToDevice, st));
                 P.jobs = d_jobs;
                 P.plans = ws.plans.p;
                 P.pix_off = ws.pixoff.p;
+                P.cta_off = ws.ctaoff.p;
+                P.order = ws.order.p;
+                P.prow = ws.prow.p;
                 P.njobs = njobs;
                 P.total_pix = (int32_t)pix_total;
+                P.total_ctas = total_ctas;
+                P.splits = splits;
                 P.pix_sum = ws.pixsum.p;
-                P.next = d_counter;
                 {
                     ProfScope ps(ctx, GF_PROF_INTEGRATE);
                     GF_CUDA(gfk::launch_integrate_pixels(P, model_kind(R[integ[0]].hm[i].m.type), ws.tot.p, st));
