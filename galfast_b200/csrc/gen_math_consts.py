@@ -115,6 +115,18 @@ def main():
         los.append(hexd(lo))
     w("#define GFM_ATAN_TAB_HI_LIST { " + ", ".join(his) + " }")
     w("#define GFM_ATAN_TAB_LO_LIST { " + ", ".join(los) + " }")
+    # table-driven exp: 2^(k/32), and ln2/32 as 36 bits and the rest
+    step = LN2 / 32
+    sh = chop(step, 36)
+    w(f"#define GFM_EXPT_INV {hexd(1 / step)}")
+    w(f"#define GFM_EXPT_HI {hexd(sh)}")
+    w(f"#define GFM_EXPT_LO {hexd(step - Decimal(sh))}")
+    w("#define GFM_EXPT_LIST { " + ", ".join(hexd((step * k).exp()) for k in range(32)) + " }")
+    # table-driven log: 64/j and log(j/64) for j = 45..91, and the series of log(1 + r) to r^8
+    w("#define GFM_LOGT_LIST { " + ", ".join(
+        "{ %s, %s }" % (hexd(Decimal(64) / j), hexd((Decimal(j) / 64).ln() if j != 64 else Decimal(0))) for j in range(45, 92)) + " }")
+    for k in range(2, 9):
+        w(f"#define GFM_LOGT_C{k} {hexd(Fraction((-1) ** (k + 1), k))}")
     print("\n".join(out))
 
 

@@ -23,6 +23,15 @@
  *         atan2 and asin are built on it.
  * The float entry points evaluate the double kernel and round once, so they
  * are correctly rounded except within ~2^-50 of a rounding boundary.
+ *
+ * On the device expf, logf, log10f, exp10f and powf first take a table-driven
+ * exp and log (Tang, "Table-driven implementation of the exponential function
+ * in IEEE floating-point arithmetic", 1989, and of the logarithm, 1990): 11 and
+ * 14 double operations and a table entry, against 22 and 26 with a division.
+ * Their doubles differ from the kernels' by a few units in the last place, so
+ * they round to the same float unless they lie that near to a rounding
+ * boundary; a result within a wider window of one (1e-7 to 4e-6 of all) takes
+ * the kernel.  Every float argument is checked by tests/cpp/fast_math_check.cu.
  */
 #pragma once
 #include <stdint.h>
@@ -260,10 +269,109 @@ GFM_HD double asin_d(double x)
 
 /* ---------------- single-precision entry points ---------------- */
 
-GFM_HD float expf_(float x) { return (float)exp_d((double)x); }
-GFM_HD float logf_(float x) { return (float)log_d((double)x); }
-GFM_HD float log10f_(float x) { return (float)(log_d((double)x) * GFM_INV_LN10); }
-GFM_HD float exp10f_(float x) { return (float)exp_d((double)x * GFM_LN10_HI); }
+GFM_HD float expf_kernel(float x) { return (float)exp_d((double)x); }
+GFM_HD float logf_kernel(float x) { return (float)log_d((double)x); }
+GFM_HD float log10f_kernel(float x) { return (float)(log_d((double)x) * GFM_INV_LN10); }
+GFM_HD float exp10f_kernel(float x) { return (float)exp_d((double)x * GFM_LN10_HI); }
+
+#if defined(__CUDACC__)
+static __device__ const double gfm_expt_dev[32] = GFM_EXPT_LIST;
+static __device__ const double gfm_logt_dev[47][2] = GFM_LOGT_LIST;
+
+/* exp(x) for |x| < 700: x = (32 n + j) ln2/32 + r with |r| <= ln2/64, exp(x) = 2^n 2^(j/32) (1 + r + ... + r^6/720) */
+static __device__ __forceinline__ double exp_t(double x)
+{
+    const double t = dfma(x, GFM_EXPT_INV, 0x1.8p52);          /* rint in the low bits */
+    const int k = __double2loint(t);
+    const double n = t - 0x1.8p52;
+    double r = dfma(-n, GFM_EXPT_HI, x);
+    r = dfma(-n, GFM_EXPT_LO, r);
+    double p = GFM_EXP_C6;
+    p = dfma(p, r, GFM_EXP_C5);
+    p = dfma(p, r, GFM_EXP_C4);
+    p = dfma(p, r, GFM_EXP_C3);
+    p = dfma(p, r, GFM_EXP_C2);
+    p = dfma(p, r, GFM_EXP_C1);
+    const double T = __ldg(gfm_expt_dev + (k & 31));
+    const double y = dfma(T * r, p, T);
+    return __hiloint2double(__double2hiint(y) + ((k >> 5) << 20), __double2loint(y));
+}
+
+/* log(x) for a positive normal x: x = 2^e m with m in (sqrt(1/2), sqrt 2], c = rint(64 m)/64, r = (m - c)/c;
+ * c = 1 around x = 1, where the result is r's own series */
+static __device__ __forceinline__ double log_t(double x)
+{
+    int hi = __double2hiint(x), e = (hi >> 20) - 1023;
+    hi = (hi & 0x000fffff) | 0x3ff00000;
+    if (hi > 0x3ff6a09e) { hi -= 0x00100000; e++; }
+    const double m = __hiloint2double(hi, __double2loint(x));
+    const double t = dfma(m, 64.0, 0x1.8p52);
+    const double *T = gfm_logt_dev[__double2loint(t) - 45];
+    const double r = dfma(t - 0x1.8p52, -0.015625, m) * __ldg(T);
+    double p = GFM_LOGT_C8;
+    p = dfma(p, r, GFM_LOGT_C7);
+    p = dfma(p, r, GFM_LOGT_C6);
+    p = dfma(p, r, GFM_LOGT_C5);
+    p = dfma(p, r, GFM_LOGT_C4);
+    p = dfma(p, r, GFM_LOGT_C3);
+    p = dfma(p, r, GFM_LOGT_C2);
+    const double s = dfma(r * r, p, r), de = (double)e;
+    return dfma(de, GFM_LN2_HI, __ldg(T + 1)) + dfma(de, GFM_LN2_LO, s);
+}
+
+/* does every double within w units in the last place of y (a normal float's range) round to the same float? */
+static __device__ __forceinline__ bool rounds_alike(double y, int w)
+{
+    return (unsigned)((__double2loint(y) & 0x1fffffff) - 0x10000000 + w) > (unsigned)(2 * w);
+}
+
+static __device__ __noinline__ float expf_far(float x) { return expf_kernel(x); }
+static __device__ __noinline__ float logf_far(float x) { return logf_kernel(x); }
+static __device__ __noinline__ float log10f_far(float x) { return log10f_kernel(x); }
+static __device__ __noinline__ float exp10f_far(float x) { return exp10f_kernel(x); }
+#endif
+
+GFM_HD float expf_(float x)
+{
+#if defined(__CUDA_ARCH__)
+    if (x <= -104.f) return 0.f;                /* below half the smallest float */
+    const double y = exp_t((double)x);
+    if (x > -87.f && x < 88.f && rounds_alike(y, 16)) return (float)y;
+    return expf_far(x);
+#else
+    return expf_kernel(x);
+#endif
+}
+GFM_HD float logf_(float x)
+{
+#if defined(__CUDA_ARCH__)
+    const double y = log_t((double)x);
+    if (x > 0.f && x < finf() && rounds_alike(y, 16)) return (float)y;
+    return logf_far(x);
+#else
+    return logf_kernel(x);
+#endif
+}
+GFM_HD float log10f_(float x)
+{
+#if defined(__CUDA_ARCH__)
+    const double y = log_t((double)x) * GFM_INV_LN10;
+    if (x > 0.f && x < finf() && rounds_alike(y, 16)) return (float)y;
+    return log10f_far(x);
+#else
+    return log10f_kernel(x);
+#endif
+}
+GFM_HD float exp10f_(float x)
+{
+#if defined(__CUDA_ARCH__)
+    const double y = exp_t((double)x * GFM_LN10_HI);
+    if (x > -37.f && x < 38.f && rounds_alike(y, 16)) return (float)y;
+    return exp10f_far(x);
+#else
+    return exp10f_kernel(x);
+#endif
+}
 GFM_HD float sinf_(float x) { return (float)sin_d((double)x); }
 GFM_HD float cosf_(float x) { return (float)cos_d((double)x); }
 GFM_HD float tanf_(float x)
@@ -285,7 +393,7 @@ GFM_HD bool f_is_int(float y, bool *odd)
 }
 
 /* powf(x, y) with the C99 special cases */
-GFM_HD float powf_(float x, float y)
+GFM_HD float powf_kernel(float x, float y)
 {
     if (y == 0.f) return 1.f;
     if (x == 1.f) return 1.f;
@@ -313,6 +421,28 @@ GFM_HD float powf_(float x, float y)
     if (xneg && !yint) return fnan();
     float r = (float)exp_d((double)y * log_d((double)ax));
     return (xneg && odd) ? -r : r;
+}
+
+#if defined(__CUDACC__)
+static __device__ __noinline__ float powf_far(float x, float y) { return powf_kernel(x, y); }
+#endif
+
+GFM_HD float powf_(float x, float y)
+{
+#if defined(__CUDA_ARCH__)
+    if (y == 0.f) return 1.f;
+    /* z's error (3 units of log's last place) is at most 2^-44 here, and so is the result's, relatively */
+    if (x > 0.f && x < finf()) {
+        const double z = (double)y * log_t((double)x);
+        if (fabs(z) < 86.0) {
+            const double r = exp_t(z);
+            if (rounds_alike(r, 1024)) return (float)r;
+        }
+    }
+    return powf_far(x, y);
+#else
+    return powf_kernel(x, y);
+#endif
 }
 
 } /* namespace gfm */
