@@ -39,6 +39,52 @@ void release_caches(gf_ctx *ctx)
     gf_table_free(ctx, &ctx->plain_table);
     free_multi_ws(ctx);
     free_rec_cache(ctx);
+    free_blocks(ctx);
+}
+
+static const size_t kBlockMin = 4096, kBlockMax = (size_t)64 << 20, kBlocksHeld = (size_t)512 << 20;
+
+/* blocks come in powers of two, so that requests of similar sizes share them */
+static size_t block_class(size_t bytes)
+{
+    size_t c = kBlockMin;
+    while (c < bytes) c <<= 1;
+    return c;
+}
+
+gf_status kept_alloc(gf_ctx *ctx, void **p, size_t bytes)
+{
+    *p = nullptr;
+    const size_t c = bytes > kBlockMax ? bytes : block_class(bytes);
+    auto it = ctx->blocks.find(c);
+    if (it != ctx->blocks.end() && !it->second.empty()) {
+        *p = it->second.back();
+        it->second.pop_back();
+        ctx->blocks_held -= c;
+        return GF_OK;
+    }
+    GF_CUDA(device_malloc(p, c));
+    return GF_OK;
+}
+
+void kept_free(gf_ctx *ctx, void *p, size_t bytes)
+{
+    if (!p) return;
+    const size_t c = bytes > kBlockMax ? bytes : block_class(bytes);
+    if (c > kBlockMax || ctx->blocks_held + c > kBlocksHeld) {
+        cudaFree(p);
+        return;
+    }
+    ctx->blocks[c].push_back(p);
+    ctx->blocks_held += c;
+}
+
+void free_blocks(gf_ctx *ctx)
+{
+    for (auto &k : ctx->blocks)
+        for (void *p : k.second) cudaFree(p);
+    ctx->blocks.clear();
+    ctx->blocks_held = 0;
 }
 
 cudaError_t device_malloc(void **p, size_t bytes)
@@ -146,6 +192,7 @@ struct ModelState {
 
 struct gf_skygen {
     gf_ctx *ctx = nullptr;
+    std::vector<std::pair<void *, size_t>> kept;      /* its blocks (kept_alloc), given back with it */
     gf_skygen_config cfg{};
     SkyGeom geom{};
     gf_pencil_beam *d_pixels = nullptr;
@@ -153,7 +200,6 @@ struct gf_skygen {
     std::vector<ModelState> models;
     /* per-launch buffers */
     int64_t *d_limits = nullptr;
-    int64_t *h_nstars = nullptr;         /* pinned [nthreads] */
     uint32_t *d_rng_snap = nullptr;      /* [3][nthreads] */
     StarRecord *d_rec = nullptr, *d_rec2 = nullptr;
     float *d_rec_am = nullptr, *d_rec_am2 = nullptr;   /* GF_EXT_MAPS: anchor extinction per record */
@@ -179,13 +225,23 @@ struct gf_skygen {
 
 namespace {
 
+/* device memory of a generator, until gf_skygen_destroy */
+template <typename T>
+gf_status own_alloc(gf_skygen *s, T **p, size_t n)
+{
+    GF_TRY(gfa::kept_alloc(s->ctx, p, n));
+    if (*p) s->kept.push_back({(void *)*p, n * sizeof(T)});
+    return GF_OK;
+}
+
 /* CrawlState arrays carved from one allocation */
 size_t crawl_state_bytes(int n) { return (size_t)n * (8 * 4 + 16 + 8) + 256; }
 
-gf_status alloc_crawl_state(int n, CrawlState &st, void **mem)
+gf_status alloc_crawl_state(gf_skygen *s, int n, CrawlState &st, void **mem)
 {
-    GF_CUDA(gfa::device_malloc(mem, crawl_state_bytes(n)));
-    char *p = (char *)*mem;
+    char *p = nullptr;
+    GF_TRY(own_alloc(s, &p, crawl_state_bytes(n)));
+    *mem = p;
     auto take = [&](size_t bytes) { char *r = p; p += (bytes + 15) & ~(size_t)15; return r; };
     st.anc = (AnchorX *)take(16 * (size_t)n);
     st.nstars = (int64_t *)take(8 * (size_t)n);
@@ -497,7 +553,9 @@ gf_status gf_ctx_destroy(gf_ctx *ctx)
     cudaStreamSynchronize(ctx->stream);
     gfa::free_multi_ws(ctx);
     gfa::free_rec_cache(ctx);
+    gfa::free_blocks(ctx);
     gf_table_free(ctx, &ctx->plain_table);
+    if (ctx->h_streams) cudaFreeHost(ctx->h_streams);
     dev_free(ctx->d_rng);
     dev_free(ctx->d_mult);
     dev_free(ctx->jt.lo);
@@ -574,17 +632,15 @@ gf_status gf_rng_init(gf_ctx *ctx, uint32_t seed48, int32_t nstreams)
     GF_TRY(check_ctx(ctx));
     if (nstreams <= 0 || nstreams > GF_MAX_STREAMS) return fail(GF_E_INVALID, "nstreams must be in [1, 65536]");
     if (nstreams % 64) nstreams += 64 - nstreams % 64;     /* roundUpModulo (cuda_rng.h:468) */
-    const std::vector<uint32_t> &mult = gfh::multipliers();
     GF_TRY(gfa::ensure_multipliers(ctx));
-    std::vector<uint32_t> h(3 * (size_t)nstreams);
-    gfh::seed_streams(seed48, nstreams, mult.data(), h.data());
-    if (ctx->rng_nstreams != nstreams) {
+    if (ctx->rng_nstreams != nstreams || !ctx->d_rng) {
+        GF_CUDA(cudaStreamSynchronize(ctx->stream));
         dev_free(ctx->d_rng);
+        ctx->rng_nstreams = 0;
         GF_TRY(dev_alloc(&ctx->d_rng, 3 * (size_t)nstreams));
         ctx->rng_nstreams = nstreams;
     }
-    GF_CUDA(cudaMemcpyAsync(ctx->d_rng, h.data(), 4 * h.size(), cudaMemcpyHostToDevice, ctx->stream));
-    GF_CUDA(cudaStreamSynchronize(ctx->stream));
+    GF_CUDA(gfk::launch_seed_streams(nullptr, seed48, 1, ctx->d_mult, nstreams, ctx->d_rng, ctx->stream));
     return GF_OK;
 }
 
@@ -655,8 +711,10 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
     s->nthreads = cfg->nthreads;
     gf_status st = GF_OK;
     auto bail = [&](gf_status code) { gf_skygen_destroy(s); return code; };
-    if ((st = dev_alloc(&s->d_pixels, npixels)) != GF_OK) return bail(st);
-    cudaMemcpy(s->d_pixels, pixels, sizeof(gf_pencil_beam) * (size_t)npixels, cudaMemcpyHostToDevice);
+    /* uploads go through the generator's stream, behind whatever used its blocks before */
+    auto up = [&](void *d, const void *h, size_t bytes) { cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, ctx->stream); };
+    if ((st = own_alloc(s, &s->d_pixels, npixels)) != GF_OK) return bail(st);
+    up(s->d_pixels, pixels, sizeof(gf_pencil_beam) * (size_t)npixels);
     /* 3-D extinction maps: device copies and the per-beam rows of nz minima */
     size_t ammin_per_beam = 1;
     if (ext && ext->kind == GF_EXT_MAPS) {
@@ -669,8 +727,8 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
                 return bail(fail(GF_E_INVALID, "invalid extinction map (or north/south depths differ)"));
             nz = e.n[2];
             const size_t n = (size_t)e.n[0] * e.n[1] * e.n[2];
-            if ((st = dev_alloc(&s->d_map[h], n)) != GF_OK) return bail(st);
-            cudaMemcpy(s->d_map[h], e.A, 4 * n, cudaMemcpyHostToDevice);
+            if ((st = own_alloc(s, &s->d_map[h], n)) != GF_OK) return bail(st);
+            up(s->d_map[h], e.A, 4 * n);
             s->geom.map[h] = s->d_map[h];
             for (int a = 0; a < 3; a++) {
                 s->geom.map_n[h][a] = e.n[a];
@@ -690,8 +748,8 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
         ammin_per_beam = (size_t)nz;
     }
     if (beam_ammin) {
-        if ((st = dev_alloc(&s->d_ammin, ammin_per_beam * (size_t)npixels)) != GF_OK) return bail(st);
-        cudaMemcpy(s->d_ammin, beam_ammin, 4 * ammin_per_beam * (size_t)npixels, cudaMemcpyHostToDevice);
+        if ((st = own_alloc(s, &s->d_ammin, ammin_per_beam * (size_t)npixels)) != GF_OK) return bail(st);
+        up(s->d_ammin, beam_ammin, 4 * ammin_per_beam * (size_t)npixels);
     }
     s->geom.pixels = s->d_pixels;
     s->geom.npixels = npixels;
@@ -704,22 +762,27 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
     for (int i = 0; i < nmodels; i++) {
         ModelState &ms = s->models[i];
         ms.hm = hms[i];
-        if ((st = dev_alloc(&ms.d_lf, ms.hm.lf.size())) != GF_OK) return bail(st);
-        cudaMemcpy(ms.d_lf, ms.hm.lf.data(), 4 * ms.hm.lf.size(), cudaMemcpyHostToDevice);
+        if ((st = own_alloc(s, &ms.d_lf, ms.hm.lf.size())) != GF_OK) return bail(st);
+        up(ms.d_lf, ms.hm.lf.data(), 4 * ms.hm.lf.size());
         if (ms.hm.cube) {
-            if ((st = dev_alloc(&ms.d_cube, ms.hm.cube_size)) != GF_OK) return bail(st);
-            cudaMemcpy(ms.d_cube, ms.hm.cube, 4 * ms.hm.cube_size, cudaMemcpyHostToDevice);
+            if ((st = own_alloc(s, &ms.d_cube, ms.hm.cube_size)) != GF_OK) return bail(st);
+            up(ms.d_cube, ms.hm.cube, 4 * ms.hm.cube_size);
             ms.hm.m.cube = ms.d_cube;
         }
-        if ((st = dev_alloc(&ms.d_Dtab, (size_t)ms.hm.m.nm * ms.hm.m.nM)) != GF_OK) return bail(st);
+        if ((st = own_alloc(s, &ms.d_Dtab, (size_t)ms.hm.m.nm * ms.hm.m.nM)) != GF_OK) return bail(st);
         if (gfk::launch_dtab(ms.hm.m, ms.d_Dtab, ctx->stream) != cudaSuccess) return bail(fail(GF_E_CUDA, "distance table"));
-        if ((st = alloc_crawl_state(s->nthreads, ms.st, &ms.st_mem)) != GF_OK) return bail(st);
-        if ((st = alloc_crawl_state(s->nthreads, ms.snap, &ms.snap_mem)) != GF_OK) return bail(st);
+        if ((st = alloc_crawl_state(s, s->nthreads, ms.st, &ms.st_mem)) != GF_OK) return bail(st);
+        if ((st = alloc_crawl_state(s, s->nthreads, ms.snap, &ms.snap_mem)) != GF_OK) return bail(st);
     }
-    if ((st = dev_alloc(&s->d_limits, s->nthreads)) != GF_OK) return bail(st);
-    if ((st = dev_alloc(&s->d_rng_snap, 3 * (size_t)s->nthreads)) != GF_OK) return bail(st);
-    if (cudaMallocHost(&s->h_nstars, 8 * (size_t)s->nthreads) != cudaSuccess) return bail(fail(GF_E_OOM, "pinned allocation"));
-    cudaError_t ce = cudaGetLastError();
+    if ((st = own_alloc(s, &s->d_limits, s->nthreads)) != GF_OK) return bail(st);
+    if ((st = own_alloc(s, &s->d_rng_snap, 3 * (size_t)s->nthreads)) != GF_OK) return bail(st);
+    if (!ctx->h_streams && cudaMallocHost(&ctx->h_streams, 8 * (size_t)GF_MAX_STREAMS) != cudaSuccess) {
+        ctx->h_streams = nullptr;
+        return bail(fail(GF_E_OOM, "pinned allocation"));
+    }
+    /* the caller's arrays have been read */
+    cudaError_t ce = cudaStreamSynchronize(ctx->stream);
+    if (ce == cudaSuccess) ce = cudaGetLastError();
     if (ce != cudaSuccess) return bail(fail(GF_E_CUDA, cudaGetErrorString(ce)));
     *out = s;
     return GF_OK;
@@ -730,16 +793,7 @@ gf_status gf_skygen_destroy(gf_skygen *s)
     if (!s) return GF_OK;
     cudaSetDevice(s->ctx->device);
     cudaStreamSynchronize(s->ctx->stream);
-    for (auto &ms : s->models) {
-        dev_free(ms.d_lf);
-        dev_free(ms.d_cube);
-        dev_free(ms.d_Dtab);
-        if (ms.st_mem) cudaFree(ms.st_mem);
-        if (ms.snap_mem) cudaFree(ms.snap_mem);
-    }
-    dev_free(s->d_pixels); dev_free(s->d_ammin); dev_free(s->d_limits); dev_free(s->d_rng_snap);
-    if (s->h_nstars) cudaFreeHost(s->h_nstars);
-    dev_free(s->d_map[0]); dev_free(s->d_map[1]);
+    for (auto &k : s->kept) gfa::kept_free(s->ctx, k.first, k.second);
     /* the record and placement buffers go to the context for its next generator
      * (the larger set is kept) */
     if (!s->ctx->rec_cache) s->ctx->rec_cache = new RecView();
@@ -748,7 +802,6 @@ gf_status gf_skygen_destroy(gf_skygen *s)
     move_recs(mine, *s);
     if (mine.rec_cap > c.rec_cap) std::swap(mine, c);
     free_recs(mine);
-    dev_free(s->d_ck); dev_free(s->d_ck_count); dev_free(s->d_ck_sel); dev_free(s->d_keep);
     delete s;
     return GF_OK;
 }
@@ -791,9 +844,19 @@ gf_status gf_skygen_integrate(gf_skygen *s, int32_t model, double *expected, dou
     const int N = s->nthreads;
     const int npix = s->geom.npixels;
     double *d_counts = nullptr, *d_cov = nullptr, *d_pp = nullptr;
-    GF_TRY(dev_alloc(&d_counts, N));
-    GF_TRY(dev_alloc(&d_cov, N));
-    if (per_pixel) GF_TRY(dev_alloc(&d_pp, npix));
+    struct Blocks {
+        gf_ctx *ctx;
+        std::vector<std::pair<void *, size_t>> v;
+        ~Blocks() { for (auto &k : v) gfa::kept_free(ctx, k.first, k.second); }
+    } blocks{s->ctx, {}};
+    auto take = [&](double **p, size_t n) -> gf_status {
+        GF_TRY(gfa::kept_alloc(s->ctx, p, n));
+        blocks.v.push_back({(void *)*p, 8 * n});
+        return GF_OK;
+    };
+    GF_TRY(take(&d_counts, N));
+    GF_TRY(take(&d_cov, N));
+    if (per_pixel) GF_TRY(take(&d_pp, npix));
     GF_CUDA(cudaMemsetAsync(d_counts, 0, 8 * (size_t)N, st));
     GF_CUDA(cudaMemsetAsync(d_cov, 0, 8 * (size_t)N, st));
     if (d_pp) GF_CUDA(cudaMemsetAsync(d_pp, 0, 8 * (size_t)npix, st));
@@ -827,7 +890,6 @@ gf_status gf_skygen_integrate(gf_skygen *s, int32_t model, double *expected, dou
     GF_CUDA(cudaMemcpyAsync(hv.data(), d_cov, 8 * (size_t)N, cudaMemcpyDeviceToHost, st));
     if (per_pixel) GF_CUDA(cudaMemcpyAsync(per_pixel, d_pp, 8 * (size_t)npix, cudaMemcpyDeviceToHost, st));
     GF_CUDA(cudaStreamSynchronize(st));
-    dev_free(d_counts); dev_free(d_cov); dev_free(d_pp);
     double e = 0, ec = 0;
     for (int i = 0; i < N; i++) { e += hc[i]; ec += hv[i]; }
     if (kmax % GF_BLOCK == 0) ms.stream_expected = hc;   /* the draw crawl assigns the same bins to the same streams */
@@ -920,14 +982,13 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
     {
         const int64_t want = (int64_t)N + (C + C / 2 + 65536) / kCkEvery + 4096;
         if (want > s->ck_cap) {
-            dev_free(s->d_ck);
-            GF_TRY(dev_alloc(&s->d_ck, (size_t)want));
+            GF_TRY(own_alloc(s, &s->d_ck, (size_t)want));
             s->ck_cap = (int32_t)want;
         }
         if (!s->d_ck_count) {
-            GF_TRY(dev_alloc(&s->d_ck_count, 4));
-            GF_TRY(dev_alloc(&s->d_ck_sel, 1));
-            GF_TRY(dev_alloc(&s->d_keep, 1));
+            GF_TRY(own_alloc(s, &s->d_ck_count, 4));
+            GF_TRY(own_alloc(s, &s->d_ck_sel, 1));
+            GF_TRY(own_alloc(s, &s->d_keep, 1));
         }
     }
 
@@ -975,7 +1036,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
             }
             GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters, s->ctx->d_counters, 8, cudaMemcpyDeviceToHost, st));
             GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters + 4, s->d_ck_count, 4, cudaMemcpyDeviceToHost, st));
-            GF_CUDA(cudaMemcpyAsync(s->h_nstars + w_lo, ms.st.nstars + w_lo, 8 * (size_t)(w_hi - w_lo), cudaMemcpyDeviceToHost, st));
+            GF_CUDA(cudaMemcpyAsync(s->ctx->h_streams + w_lo, ms.st.nstars + w_lo, 8 * (size_t)(w_hi - w_lo), cudaMemcpyDeviceToHost, st));
             GF_CUDA(cudaStreamSynchronize(st));
             int64_t total = (int64_t)s->ctx->h_counters[0];
             if (total <= s->rec_cap) break;
@@ -986,8 +1047,8 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
             GF_CUDA(cudaMemcpyAsync(s->ctx->d_counters, &rb, 8, cudaMemcpyHostToDevice, st));
         }
         for (int i = w_lo; i < w_hi; i++) {
-            if (cum + s->h_nstars[i] >= C) { t = i; break; }
-            cum += s->h_nstars[i];
+            if (cum + s->ctx->h_streams[i] >= C) { t = i; break; }
+            cum += s->ctx->h_streams[i];
         }
         if (t >= 0) break;
         w_lo = w_hi;
@@ -999,7 +1060,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         GF_CUDA(cudaStreamSynchronize(st));
         nbatch = (int64_t)s->ctx->h_counters[0];
         generated_all = true;
-        for (int i = ms.first_active; i < N; i++) ms.stream_drawn[i] += s->h_nstars[i];
+        for (int i = ms.first_active; i < N; i++) ms.stream_drawn[i] += s->ctx->h_streams[i];
         ms.first_active = N;
     } else {
         /* The batch ends inside stream t: it keeps the stars of the streams before
@@ -1054,7 +1115,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         nbatch = (int64_t)s->ctx->h_counters[0];
         if (nbatch != C) return fail(GF_E_CUDA, "batch rerun produced an unexpected star count");
         generated_all = false;
-        for (int i = ms.first_active; i < t; i++) ms.stream_drawn[i] += s->h_nstars[i];
+        for (int i = ms.first_active; i < t; i++) ms.stream_drawn[i] += s->ctx->h_streams[i];
         ms.stream_drawn[t] += Lt;
         ms.first_active = t;
     }
@@ -1304,7 +1365,10 @@ gf_status gf_module_bond2010(gf_ctx *ctx, const gf_bond2010_config *cfg, gf_tabl
     return GF_OK;
 }
 
-gf_status gf_photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, gf_photometry **out)
+}  /* extern "C" */
+
+namespace gfa {
+gf_status photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, bool kept, gf_photometry **out)
 {
     GF_TRY(check_ctx(ctx));
     if (!cfg || !out || cfg->nbands < 2 || cfg->nbands > GF_MAX_BANDS || cfg->bidx < 0 || cfg->bidx >= cfg->nbands ||
@@ -1312,12 +1376,21 @@ gf_status gf_photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, gf_
         return fail(GF_E_INVALID, "invalid photometry configuration");
     gf_photometry *p = new gf_photometry();
     size_t n = (size_t)(cfg->nbands - 1) * cfg->nMr * cfg->nFeH;
-    if (dev_alloc(&p->d_colors, n) != GF_OK || dev_alloc(&p->d_eflags, n) != GF_OK) {
-        dev_free(p->d_colors); dev_free(p->d_eflags); delete p;
+    p->cache = kept ? ctx : nullptr;
+    p->n = n;
+    if ((kept ? kept_alloc(ctx, &p->d_colors, n) : dev_alloc(&p->d_colors, n)) != GF_OK ||
+        (kept ? kept_alloc(ctx, &p->d_eflags, n) : dev_alloc(&p->d_eflags, n)) != GF_OK) {
+        gf_photometry_destroy(p);
         return fail(GF_E_OOM, "photometry tables");
     }
-    cudaMemcpy(p->d_colors, cfg->colors, 4 * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(p->d_eflags, cfg->eflags, n, cudaMemcpyHostToDevice);
+    cudaError_t e = cudaMemcpyAsync(p->d_colors, cfg->colors, 4 * n, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(p->d_eflags, cfg->eflags, n, cudaMemcpyHostToDevice, ctx->stream);
+    /* an object of the caller's may be used on other contexts */
+    if (e == cudaSuccess && !kept) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) {
+        gf_photometry_destroy(p);
+        return fail(GF_E_CUDA, cudaGetErrorString(e));
+    }
     gfk::PhotTables &T = p->tab;
     T.nbands = cfg->nbands; T.bidx = cfg->bidx; T.nFeH = cfg->nFeH; T.nMr = cfg->nMr;
     for (int i = 0; i < GF_MAX_BANDS; i++) T.reddening[i] = cfg->reddening[i];
@@ -1326,11 +1399,24 @@ gf_status gf_photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, gf_
     *out = p;
     return GF_OK;
 }
+}  // namespace gfa
+
+extern "C" {
+
+gf_status gf_photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, gf_photometry **out)
+{
+    return gfa::photometry_create(ctx, cfg, false, out);
+}
 
 gf_status gf_photometry_destroy(gf_photometry *p)
 {
     if (!p) return GF_OK;
-    dev_free(p->d_colors); dev_free(p->d_eflags);
+    if (p->cache) {
+        gfa::kept_free(p->cache, p->d_colors, 4 * p->n);
+        gfa::kept_free(p->cache, p->d_eflags, p->n);
+    } else {
+        dev_free(p->d_colors); dev_free(p->d_eflags);
+    }
     delete p;
     return GF_OK;
 }
@@ -1346,19 +1432,23 @@ gf_status gf_module_photometry(gf_ctx *ctx, const gf_photometry *p, gf_table *t,
     return GF_OK;
 }
 
-gf_status gf_photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, gf_photoerr **out)
+}  /* extern "C" */
+
+namespace gfa {
+gf_status photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, bool kept, gf_photoerr **out)
 {
     GF_TRY(check_ctx(ctx));
     if (!cfg || !out || cfg->nbands < 1 || cfg->nbands > GF_MAX_BANDS || cfg->nknots < 2 || !cfg->mag || !cfg->sigma)
         return fail(GF_E_INVALID, "invalid photometric error configuration");
     gf_photoerr *p = new gf_photoerr();
-    size_t n = (size_t)cfg->nbands * cfg->nknots;
-    if (dev_alloc(&p->d_mag, n) != GF_OK || dev_alloc(&p->d_sigma, n) != GF_OK) {
-        dev_free(p->d_mag); dev_free(p->d_sigma); delete p;
-        return fail(GF_E_OOM, "photometric error tables");
-    }
-    cudaMemcpy(p->d_mag, cfg->mag, 8 * n, cudaMemcpyHostToDevice);
-    cudaMemcpy(p->d_sigma, cfg->sigma, 8 * n, cudaMemcpyHostToDevice);
+    const size_t n = (size_t)cfg->nbands * cfg->nknots;
+    p->cache = kept ? ctx : nullptr;
+    p->n = n;
+    auto take = [&](auto **q, size_t k) { return kept ? kept_alloc(ctx, q, k) : dev_alloc(q, k); };
+    auto failed = [&]() { gf_photoerr_destroy(p); return fail(GF_E_OOM, "photometric error tables"); };
+    if (take(&p->d_mag, n) != GF_OK || take(&p->d_sigma, n) != GF_OK) return failed();
+    cudaError_t e = cudaMemcpyAsync(p->d_mag, cfg->mag, 8 * n, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(p->d_sigma, cfg->sigma, 8 * n, cudaMemcpyHostToDevice, ctx->stream);
     p->tab.nbands = cfg->nbands; p->tab.nknots = cfg->nknots; p->tab.mag = p->d_mag; p->tab.sigma = p->d_sigma;
     p->tab.seed = cfg->seed;
     p->tab.guide = nullptr;
@@ -1372,35 +1462,45 @@ gf_status gf_photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, gf_phot
         for (int i = 0; i < nk && mono; i++) mono = std::isfinite(xa[i]) && (i == 0 || xa[i] > xa[i - 1]);
     }
     if (mono) {
-        const int G = nk;
-        std::vector<int32_t> guide((size_t)cfg->nbands * G);
         for (int b = 0; b < cfg->nbands; b++) {
             const double *xa = cfg->mag + (size_t)b * nk;
-            const double x0 = xa[0], inv = (double)G / (xa[nk - 1] - xa[0]);
-            p->tab.gx0[b] = x0;
-            p->tab.ginv[b] = inv;
-            int last = 0, i = 0;
-            for (int g = 0; g < G; g++) {
-                while (i <= nk - 2 && gfk::perr_cell(xa[i], x0, inv, G) < g) last = i++;
-                guide[(size_t)b * G + g] = last;
-            }
+            p->tab.gx0[b] = xa[0];
+            p->tab.ginv[b] = (double)nk / (xa[nk - 1] - xa[0]);
         }
-        if (dev_alloc(&p->d_guide, guide.size()) != GF_OK) {
-            dev_free(p->d_mag); dev_free(p->d_sigma); delete p;
-            return fail(GF_E_OOM, "photometric error tables");
-        }
-        cudaMemcpy(p->d_guide, guide.data(), 4 * guide.size(), cudaMemcpyHostToDevice);
+        p->nguide = n;
+        if (take(&p->d_guide, n) != GF_OK) return failed();
+        p->tab.nguide = nk;
+        if (e == cudaSuccess) e = gfk::launch_perr_guide(p->tab, p->d_guide, ctx->stream);
         p->tab.guide = p->d_guide;
-        p->tab.nguide = G;
+    }
+    /* an object of the caller's may be used on other contexts */
+    if (e == cudaSuccess && !kept) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) {
+        gf_photoerr_destroy(p);
+        return fail(GF_E_CUDA, cudaGetErrorString(e));
     }
     *out = p;
     return GF_OK;
+}
+}  // namespace gfa
+
+extern "C" {
+
+gf_status gf_photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, gf_photoerr **out)
+{
+    return gfa::photoerr_create(ctx, cfg, false, out);
 }
 
 gf_status gf_photoerr_destroy(gf_photoerr *p)
 {
     if (!p) return GF_OK;
-    dev_free(p->d_mag); dev_free(p->d_sigma); dev_free(p->d_guide);
+    if (p->cache) {
+        gfa::kept_free(p->cache, p->d_mag, 8 * p->n);
+        gfa::kept_free(p->cache, p->d_sigma, 8 * p->n);
+        gfa::kept_free(p->cache, p->d_guide, 4 * p->nguide);
+    } else {
+        dev_free(p->d_mag); dev_free(p->d_sigma); dev_free(p->d_guide);
+    }
     delete p;
     return GF_OK;
 }
@@ -1480,13 +1580,12 @@ static gf_status catalog_run_once(gf_ctx *ctx, const gf_job *job, gf_batch_callb
     if (ctx->plain_table.capacity == job->capacity && ctx->plain_table.nbands == job->nbands) {
         g.t = ctx->plain_table;
         memset(&ctx->plain_table, 0, sizeof(gf_table));
-        g.t.size = 0;
-        GF_TRY(zero_module_columns(ctx, &g.t));
+        g.t.size = 0;          /* each batch zeroes the module columns of its own rows */
     } else {
         GF_TRY(gf_table_alloc(ctx, job->capacity, job->nbands, &g.t));
     }
-    if (job->phot) GF_TRY(gf_photometry_create(ctx, job->phot, &g.ph));
-    if (job->perr) GF_TRY(gf_photoerr_create(ctx, job->perr, &g.pe));
+    if (job->phot) GF_TRY(gfa::photometry_create(ctx, job->phot, true, &g.ph));
+    if (job->perr) GF_TRY(gfa::photoerr_create(ctx, job->perr, true, &g.pe));
     int64_t row_offset = 0;
     for (int i = 0; i < (int)models.size(); i++) {
         int32_t done = 0;

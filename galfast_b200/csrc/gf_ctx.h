@@ -4,6 +4,7 @@
  */
 #pragma once
 #include <chrono>
+#include <map>
 #include <cuda_runtime.h>
 #include <string>
 #include <utility>
@@ -58,6 +59,24 @@ gf_status dev_alloc(T **p, size_t n)
 }
 }  // namespace gfa
 
+struct gf_ctx;
+
+namespace gfa {
+/* Device memory of one call (or one generator) from the blocks that the context keeps from earlier
+ * ones: cudaMalloc and cudaFree synchronise the device and take locks of the whole machine, and a
+ * request makes dozens of small tables.  A block is used and reused on the context's stream only,
+ * or given back after that stream has been waited for; at most kBlocksHeld bytes are kept, blocks
+ * above kBlockMax are not, and release_caches and gf_ctx_destroy give all back. */
+gf_status kept_alloc(gf_ctx *ctx, void **p, size_t bytes);
+void kept_free(gf_ctx *ctx, void *p, size_t bytes);
+template <typename T>
+gf_status kept_alloc(gf_ctx *ctx, T **p, size_t n)
+{
+    *p = nullptr;
+    return n ? kept_alloc(ctx, (void **)p, n * sizeof(T)) : GF_OK;
+}
+}  // namespace gfa
+
 struct gf_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
@@ -77,6 +96,9 @@ struct gf_ctx {
     int64_t multi_budget = 0;            /* device bytes per multi-request chunk (0: 60% of free memory) */
     MultiWS *multi_ws = nullptr;         /* buffers of gf_catalog_run_multi kept between calls */
     gf_table plain_table = {};           /* output table of gf_catalog_run, kept for the next call of the same shape */
+    std::map<size_t, std::vector<void *>> blocks;   /* device blocks kept for the next call, by size (kept_alloc) */
+    size_t blocks_held = 0;
+    int64_t *h_streams = nullptr;        /* pinned: stars per stream of a draw window */
     void *rec_cache = nullptr;           /* star-record and placement buffers of a finished generator, for the next one */
     int32_t draw_wpc[3] = {0, 0, 0};      /* warps per CTA of the batched draw, by model kind (0: not tuned yet) */
     uint32_t host_cols = GF_COL_ALL;     /* columns gf_catalog_run_multi_host copies to host memory */
@@ -84,12 +106,16 @@ struct gf_ctx {
 };
 
 struct gf_photometry {
+    gf_ctx *cache = nullptr;             /* tables from this context's kept blocks (an object of one call), or allocated */
+    size_t n = 0;
     gfk::PhotTables tab;
     float *d_colors = nullptr;
     uint8_t *d_eflags = nullptr;
 };
 
 struct gf_photoerr {
+    gf_ctx *cache = nullptr;             /* as gf_photometry */
+    size_t n = 0, nguide = 0;
     gfk::PerrTables tab;
     double *d_mag = nullptr, *d_sigma = nullptr;
     int32_t *d_guide = nullptr;
@@ -113,6 +139,10 @@ gf_status catalog_run_multi_admitted(gf_ctx *ctx, const gf_job *jobs, int32_t nj
                                      gf_catalog_stats *stats, Admission *adm);
 
 gf_status check_ctx(gf_ctx *ctx);
+/* photometry and photometric-error tables of one call (kept blocks of the context) */
+gf_status photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, bool kept, gf_photometry **out);
+gf_status photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, bool kept, gf_photoerr **out);
+void free_blocks(gf_ctx *ctx);
 /* zero the module columns (FeH, vcyl, mags, photoflags, obsmags, pm, radec) of rows
  * [0, n): rows a module skips (hidden stars) read zero whatever the table held before */
 gf_status zero_module_rows(gf_ctx *ctx, const gf_table *t, int64_t n);

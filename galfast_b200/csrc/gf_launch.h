@@ -99,7 +99,8 @@ cudaError_t sort_temp_bytes(int64_t n, size_t *bytes);
 cudaError_t launch_sort_gather(const LaunchSort &L, cudaStream_t s);
 cudaError_t launch_dtab(const SkyModel &m, float *D, cudaStream_t s);
 cudaError_t launch_jump_tables(const uint32_t *mult, int n, uint64_t *lo, uint64_t *hi, cudaStream_t s);
-cudaError_t launch_seed_streams(const uint32_t *seeds, int njobs, const uint32_t *mult, int NS, uint32_t *rng, cudaStream_t s);
+/* seeds: per request (device), or null: seed0 */
+cudaError_t launch_seed_streams(const uint32_t *seeds, uint32_t seed0, int njobs, const uint32_t *mult, int NS, uint32_t *rng, cudaStream_t s);
 cudaError_t launch_crawl_multi(const LaunchCrawlMulti &L, int draw, cudaStream_t s);
 cudaError_t sort_temp_bytes_multi(int64_t n, size_t *bytes);
 cudaError_t launch_place_sort_multi(const LaunchPlaceMulti &L, cudaStream_t s);
@@ -153,6 +154,8 @@ __host__ __device__ inline int perr_cell(double x, double x0, double inv, int n)
     const double t = (x - x0) * inv;
     return t < 0.0 ? 0 : (t >= (double)n ? n - 1 : (int)t);
 }
+/* the bracket guide of c's knots (c.nguide cells a band, gx0 and ginv set) into guide */
+cudaError_t launch_perr_guide(const PerrTables &c, int32_t *guide, cudaStream_t s);
 cudaError_t launch_photoerrors(const PerrTables &c, int64_t row_offset, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
 cudaError_t launch_vel2pm(const gf_vel2pm_config &c, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
 cudaError_t launch_gal2other(int32_t coordsys, gf_table t, int64_t begin, int64_t end, cudaStream_t s);

@@ -901,6 +901,29 @@ __device__ __forceinline__ double linear_eval(const double *xa, const double *ya
     return 0.0;
 }
 
+/* guide cell g of a band: its last knot (at most nknots - 2) whose own cell is before g, or 0 */
+__global__ void perr_guide_kernel(PerrTables c, int32_t *guide)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= c.nbands * c.nguide) return;
+    const int b = k / c.nguide, g = k - b * c.nguide;
+    const double *xa = c.mag + (size_t)b * c.nknots;
+    int lo = 0, hi = c.nknots - 1;          /* knots before lo: cell < g; from hi on: not (or out of range) */
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (perr_cell(xa[mid], c.gx0[b], c.ginv[b], c.nguide) < g) lo = mid + 1; else hi = mid;
+    }
+    guide[k] = lo > 0 ? lo - 1 : 0;
+}
+
+cudaError_t launch_perr_guide(const PerrTables &c, int32_t *guide, cudaStream_t s)
+{
+    const int n = c.nbands * c.nguide;
+    perr_guide_kernel<<<(n + 255) / 256, 256, 0, s>>>(c, guide);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 /* observed magnitudes of one row; catalog_row numbers the row within its request's catalog */
 __device__ __forceinline__ void photoerr_row(const PerrTables &c, uint64_t seed, int64_t catalog_row, gf_table &t, int64_t row)
 {

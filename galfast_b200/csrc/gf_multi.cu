@@ -44,19 +44,20 @@ using gfa::ProfScope;
 
 namespace {
 
-/* device allocations released together */
+/* device tables of one call, from the context's kept blocks (used on its stream only) */
 struct Pool {
-    std::vector<void *> ptrs;
+    gf_ctx *ctx;
+    std::vector<std::pair<void *, size_t>> ptrs;
     template <typename T>
     gf_status alloc(T **p, size_t n)
     {
-        GF_TRY(dev_alloc(p, n));
-        if (*p) ptrs.push_back((void *)*p);
+        GF_TRY(gfa::kept_alloc(ctx, p, n));
+        if (*p) ptrs.push_back({(void *)*p, n * sizeof(T)});
         return GF_OK;
     }
     ~Pool()
     {
-        for (void *p : ptrs) cudaFree(p);
+        for (auto &k : ptrs) gfa::kept_free(ctx, k.first, k.second);
     }
 };
 
@@ -638,7 +639,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         q.group = it->second;
     }
 
-    Pool pool;
+    Pool pool{ctx, {}};
     if (!ctx->multi_ws) ctx->multi_ws = new MultiWS();
     MultiWS &ws = *ctx->multi_ws;
     gf_pencil_beam *d_pix = nullptr;
@@ -716,7 +717,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         std::vector<uint32_t> seeds(njobs);
         for (int j = 0; j < njobs; j++) seeds[j] = jobs[j].seed48;
         GF_CUDA(cudaMemcpyAsync(d_seeds, seeds.data(), 4 * (size_t)njobs, cudaMemcpyHostToDevice, st));
-        GF_CUDA(gfk::launch_seed_streams(d_seeds, njobs, ctx->d_mult, NS, d_rng, st));
+        GF_CUDA(gfk::launch_seed_streams(d_seeds, 0u, njobs, ctx->d_mult, NS, d_rng, st));
     }
 
     /* ---- per-(request, stream) state ---- */
@@ -1053,8 +1054,8 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     if (!batched_all.empty())
         for (int g = 0; g < (int)group_rep.size(); g++) {
             const gf_job &J = jobs[group_rep[g]];
-            if (J.phot) GF_TRY(gf_photometry_create(ctx, J.phot, &gm[g].ph));
-            if (J.perr) GF_TRY(gf_photoerr_create(ctx, J.perr, &gm[g].pe));
+            if (J.phot) GF_TRY(gfa::photometry_create(ctx, J.phot, true, &gm[g].ph));
+            if (J.perr) GF_TRY(gfa::photoerr_create(ctx, J.perr, true, &gm[g].pe));
         }
 
     /* growing buffers of the draw passes */

@@ -1157,12 +1157,12 @@ __device__ __forceinline__ uint64_t lcg48_jump(uint64_t x0, uint64_t n)
 /* The stream states of many requests at once, identical to gfh::seed_streams:
  * srand48(seed); per stream i in order: c = (int)(drand48() * a_i) (x86 gives
  * INT_MIN out of range), x = lrand48() (cux.cpp:404-414). */
-__global__ void seed_streams_kernel(const uint32_t *seeds, int njobs, const uint32_t *mult, int NS, uint32_t *rng)
+__global__ void seed_streams_kernel(const uint32_t *seeds, uint32_t seed0, int njobs, const uint32_t *mult, int NS, uint32_t *rng)
 {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= (int64_t)njobs * NS) return;
     const int j = (int)(g / NS), i = (int)(g % NS);
-    const uint64_t x0 = ((uint64_t)seeds[j] << 16) | 0x330Eull;
+    const uint64_t x0 = ((uint64_t)(seeds ? seeds[j] : seed0) << 16) | 0x330Eull;
     const uint64_t x1 = lcg48_jump(x0, 2ull * i + 1);
     const uint64_t x2 = (0x5DEECE66Dull * x1 + 0xBull) & ((1ull << 48) - 1);
     const uint32_t prime = mult[i];
@@ -1174,11 +1174,11 @@ __global__ void seed_streams_kernel(const uint32_t *seeds, int njobs, const uint
     r[2 * NS + i] = (uint32_t)(x2 >> 17);
 }
 
-cudaError_t launch_seed_streams(const uint32_t *seeds, int njobs, const uint32_t *mult, int NS, uint32_t *rng, cudaStream_t s)
+cudaError_t launch_seed_streams(const uint32_t *seeds, uint32_t seed0, int njobs, const uint32_t *mult, int NS, uint32_t *rng, cudaStream_t s)
 {
     const int64_t n = (int64_t)njobs * NS;
     if (n <= 0) return cudaSuccess;
-    seed_streams_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(seeds, njobs, mult, NS, rng);
+    seed_streams_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(seeds, seed0, njobs, mult, NS, rng);
     count_launches(1);
     return cudaGetLastError();
 }
