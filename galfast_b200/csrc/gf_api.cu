@@ -198,6 +198,9 @@ struct gf_skygen {
     gf_pencil_beam *d_pixels = nullptr;
     float *d_ammin = nullptr;
     std::vector<ModelState> models;
+    /* integrate by pixels: cut rows and order of the pixels (gfa::pixel_rows); null: by streams only */
+    uint2 *d_prow = nullptr;
+    uint32_t *d_order = nullptr;
     /* per-launch buffers */
     int64_t *d_limits = nullptr;
     uint32_t *d_rng_snap = nullptr;      /* [3][nthreads] */
@@ -774,6 +777,20 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
         if ((st = alloc_crawl_state(s, s->nthreads, ms.st, &ms.st_mem)) != GF_OK) return bail(st);
         if ((st = alloc_crawl_state(s, s->nthreads, ms.snap, &ms.snap_mem)) != GF_OK) return bail(st);
     }
+    std::vector<uint2> prow;
+    std::vector<uint32_t> order;
+    if (!s->maps && hms[0].m.nm <= 16384) {
+        std::vector<int32_t> rowpx;
+        prow.resize(npixels);
+        order.resize(npixels);
+        gfa::pixel_rows(hms[0].m, pixels, npixels, s->geom.ext_kind != GF_EXT_NONE ? beam_ammin : nullptr, prow.data(), order.data(), rowpx);
+        if (own_alloc(s, &s->d_prow, npixels) == GF_OK && own_alloc(s, &s->d_order, npixels) == GF_OK) {
+            up(s->d_prow, prow.data(), sizeof(uint2) * (size_t)npixels);
+            up(s->d_order, order.data(), 4 * (size_t)npixels);
+        } else {
+            s->d_prow = nullptr;
+        }
+    }
     if ((st = own_alloc(s, &s->d_limits, s->nthreads)) != GF_OK) return bail(st);
     if ((st = own_alloc(s, &s->d_rng_snap, 3 * (size_t)s->nthreads)) != GF_OK) return bail(st);
     if (!ctx->h_streams && cudaMallocHost(&ctx->h_streams, 8 * (size_t)GF_MAX_STREAMS) != cudaSuccess) {
@@ -835,6 +852,99 @@ gf_status gf_skygen_set_norm(gf_skygen *s, int32_t model, float norm)
     return GF_OK;
 }
 
+}  /* extern "C" */
+
+namespace {
+/* kept blocks of one call */
+struct Blocks {
+    gf_ctx *ctx;
+    std::vector<std::pair<void *, size_t>> v;
+    template <typename T>
+    gf_status take(T **p, size_t n)
+    {
+        GF_TRY(gfa::kept_alloc(ctx, p, n));
+        v.push_back({(void *)*p, sizeof(T) * n});
+        return GF_OK;
+    }
+    ~Blocks() { for (auto &k : v) gfa::kept_free(ctx, k.first, k.second); }
+};
+
+/* The integrate of one model by pixels instead of by streams (gf_integrate.cu): the same bins and
+ * anchors when blocks of bins never straddle pixels.  *done is false, and nothing has changed, where it
+ * does not apply: other grids, 3-D extinction maps (anchors' extinction by distance), density cubes,
+ * an anchor plan that does not fit, or few bins.  The plan and the sums cost some 0.16 ms a model, the crawl
+ * 0.04 ms and 0.5 ms more for 1e8 bins (5e6 bins: 0.07 ms a model by streams, 0.17 by pixels; 4.6e7: 0.26
+ * and 0.17; 7.5e8: 3.5 and 0.54). */
+constexpr long long kPixelIntegrateBins = 25000000;
+gf_status integrate_by_pixels(gf_skygen *s, ModelState &ms, double *expected, double *expected_covered, double *per_pixel, bool *done)
+{
+    const SkyModel &m = ms.hm.m;
+    const long long kmax = (long long)m.nm * m.nM;
+    gfk::IntegPixParams P;
+    memset(&P, 0, sizeof(P));
+    if (!s->d_prow || kmax % GF_BLOCK != 0 || m.nm + m.nM > 16384 || m.type == GF_MODEL_DENSITY_CUBE ||
+        kmax * s->geom.npixels < kPixelIntegrateBins || gfk::integ_smem(m.nM, &P.pitch) > 200 * 1024)
+        return GF_OK;
+    gf_ctx *ctx = s->ctx;
+    cudaStream_t st = ctx->stream;
+    const int npix = s->geom.npixels;
+    /* what the kernels read: one upload */
+    struct Setup {
+        CrawlJob job;
+        gfk::IntegPlanDesc desc;
+        const unsigned char *plan;
+        int32_t pix_off[2], cta_off[2];
+    } h, *d = nullptr;
+    memset((void *)&h, 0, sizeof(h));
+    Blocks blocks{ctx, {}};
+    const size_t plan_bytes = gfk::integ_plan_bytes(m.nm, m.nM, &h.desc.max_anchors, &h.desc.max_slots);
+    P.splits = gfk::integ_splits((npix + 63) / 64);
+    P.total_ctas = (int32_t)gfk::integ_ctas(npix, P.splits);
+    P.njobs = 1;
+    P.total_pix = npix;
+    double2 *tot = nullptr;
+    double *pp = nullptr;
+    GF_TRY(blocks.take(&h.desc.plan, plan_bytes));
+    GF_TRY(blocks.take(&d, 1));
+    GF_TRY(blocks.take(&P.pix_sum, (size_t)npix * P.splits));
+    GF_TRY(blocks.take(&tot, gfk::integ_totals(1)));
+    if (per_pixel) GF_TRY(blocks.take(&pp, npix));
+    h.desc.Dtab = ms.d_Dtab;
+    h.desc.nm = m.nm; h.desc.nM = m.nM; h.desc.nM_tab = m.nM;
+    h.plan = h.desc.plan;
+    h.pix_off[1] = npix;
+    h.cta_off[1] = P.total_ctas;
+    h.job.m = m;
+    h.job.m.lf = ms.d_lf;
+    h.job.g = s->geom;
+    h.job.Dtab = ms.d_Dtab;
+    P.jobs = &d->job; P.plans = &d->plan; P.pix_off = d->pix_off; P.cta_off = d->cta_off;
+    P.order = s->d_order; P.prow = s->d_prow;
+    gfk::IntegPlanHdr hdr;
+    double2 sums;
+    ProfScope ps(ctx, GF_PROF_INTEGRATE);
+    GF_CUDA(cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    GF_CUDA(gfk::launch_integ_plans(&d->desc, 1, st));
+    GF_CUDA(gfk::launch_integrate_pixels(P, m.type, tot, st));
+    if (per_pixel) GF_CUDA(gfk::launch_pixel_counts(P, pp, st));
+    GF_CUDA(cudaMemcpyAsync(&hdr, h.desc.plan, sizeof(hdr), cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaMemcpyAsync(&sums, tot, sizeof(sums), cudaMemcpyDeviceToHost, st));
+    if (per_pixel) GF_CUDA(cudaMemcpyAsync(per_pixel, pp, 8 * (size_t)npix, cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaStreamSynchronize(st));
+    if (!hdr.ok) return GF_OK;     /* (nothing was summed) */
+    /* blocks of bins go to the streams in turn: an even share predicts the draw's windows */
+    ms.stream_expected.assign(s->nthreads, sums.x / s->nthreads);
+    ms.expected = sums.x;
+    ms.expected_covered = sums.y;
+    if (expected) *expected = sums.x;
+    if (expected_covered) *expected_covered = sums.y;
+    *done = true;
+    return GF_OK;
+}
+}  // namespace
+
+extern "C" {
+
 gf_status gf_skygen_integrate(gf_skygen *s, int32_t model, double *expected, double *expected_covered, double *per_pixel)
 {
     if (!s || model < 0 || model >= (int)s->models.size()) return fail(GF_E_INVALID, "invalid model");
@@ -843,20 +953,15 @@ gf_status gf_skygen_integrate(gf_skygen *s, int32_t model, double *expected, dou
     cudaStream_t st = s->ctx->stream;
     const int N = s->nthreads;
     const int npix = s->geom.npixels;
+    bool done = false;
+    const gf_status by_pixels = integrate_by_pixels(s, ms, expected, expected_covered, per_pixel, &done);
+    if (by_pixels != GF_OK && by_pixels != GF_E_OOM) return by_pixels;   /* the crawl needs less memory */
+    if (done) return GF_OK;
     double *d_counts = nullptr, *d_cov = nullptr, *d_pp = nullptr;
-    struct Blocks {
-        gf_ctx *ctx;
-        std::vector<std::pair<void *, size_t>> v;
-        ~Blocks() { for (auto &k : v) gfa::kept_free(ctx, k.first, k.second); }
-    } blocks{s->ctx, {}};
-    auto take = [&](double **p, size_t n) -> gf_status {
-        GF_TRY(gfa::kept_alloc(s->ctx, p, n));
-        blocks.v.push_back({(void *)*p, 8 * n});
-        return GF_OK;
-    };
-    GF_TRY(take(&d_counts, N));
-    GF_TRY(take(&d_cov, N));
-    if (per_pixel) GF_TRY(take(&d_pp, npix));
+    Blocks blocks{s->ctx, {}};
+    GF_TRY(blocks.take(&d_counts, N));
+    GF_TRY(blocks.take(&d_cov, N));
+    if (per_pixel) GF_TRY(blocks.take(&d_pp, npix));
     GF_CUDA(cudaMemsetAsync(d_counts, 0, 8 * (size_t)N, st));
     GF_CUDA(cudaMemsetAsync(d_cov, 0, 8 * (size_t)N, st));
     if (d_pp) GF_CUDA(cudaMemsetAsync(d_pp, 0, 8 * (size_t)npix, st));

@@ -139,6 +139,11 @@ gf_status catalog_run_multi_admitted(gf_ctx *ctx, const gf_job *jobs, int32_t nj
                                      gf_catalog_stats *stats, Admission *adm);
 
 gf_status check_ctx(gf_ctx *ctx);
+/* Of one request: per pixel its pixel row and cut row (gf_launch.h), each row's first pixel (then
+ * npixels), and the pixels with the fully covered ones first.  ammin: the least extinction of each
+ * beam, null for none. */
+void pixel_rows(const SkyModel &m, const gf_pencil_beam *pixels, int32_t npixels, const float *ammin, uint2 *prow,
+                uint32_t *order, std::vector<int32_t> &rowpx);
 /* photometry and photometric-error tables of one call (kept blocks of the context) */
 gf_status photometry_create(gf_ctx *ctx, const gf_photometry_config *cfg, bool kept, gf_photometry **out);
 gf_status photoerr_create(gf_ctx *ctx, const gf_photoerr_config *cfg, bool kept, gf_photoerr **out);

@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(32 * GF_IG_WARPS) integrate_pixels_kernel(Inte
         const IntegPlanHdr *h = (const IntegPlanHdr *)plan;
         const int npix = J.g.npixels, unit = (cta - P.cta_off[job]) * GF_IG_WARPS + warp;
         const int g = unit / P.splits, sp = unit - g * P.splits;
-        if (g * 64 >= npix) continue;
+        if (g * 64 >= npix || !h->ok) continue;
         const int qa = g * 64 + lane, qb = qa + 32, base = P.pix_off[job];
         const uint32_t ia = P.order[base + min(qa, npix - 1)], ib = P.order[base + min(qb, npix - 1)];
         const gf_pencil_beam pa = J.g.pixels[ia], pb = J.g.pixels[ib];
@@ -464,15 +464,19 @@ __global__ void __launch_bounds__(32 * GF_IG_WARPS) integrate_pixels_kernel(Inte
     }
 }
 
+/* GF_TOTAL_PARTS CTAs a request sum its pixels, one more launch their sums: a single large request
+ * (20k pixels in 32 parts: 10 MB) is latency-bound with one CTA. */
+#define GF_TOTAL_PARTS 32
+
 __global__ void __launch_bounds__(256) job_totals_kernel(const double2 *pix_sum, const int32_t *pix_off, int splits, int total_pix,
-                                                          const unsigned char *const *plans, double2 *tot)
+                                                          const unsigned char *const *plans, double2 *part)
 {
     __shared__ double sc[256], sv[256];
-    const int j = blockIdx.x;
+    const int j = blockIdx.y;
     double c = 0.0, v = 0.0;
     if (plans[j])
         for (int sp = 0; sp < splits; sp++)
-            for (int p = pix_off[j] + threadIdx.x; p < pix_off[j + 1]; p += blockDim.x) {
+            for (int p = pix_off[j] + blockIdx.x * blockDim.x + threadIdx.x; p < pix_off[j + 1]; p += GF_TOTAL_PARTS * blockDim.x) {
                 const double2 s = pix_sum[(size_t)sp * total_pix + p];
                 c += s.x;
                 v += s.y;
@@ -487,7 +491,28 @@ __global__ void __launch_bounds__(256) job_totals_kernel(const double2 *pix_sum,
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) tot[j] = make_double2(sc[0], sv[0]);
+    if (threadIdx.x == 0) part[(size_t)j * GF_TOTAL_PARTS + blockIdx.x] = make_double2(sc[0], sv[0]);
+}
+
+__global__ void __launch_bounds__(256) sum_totals_kernel(const double2 *part, int njobs, double2 *tot)
+{
+    const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (j >= njobs) return;
+    double2 s = part[(size_t)j * GF_TOTAL_PARTS + lane];
+    for (int o = 16; o > 0; o >>= 1) {
+        s.x += __shfl_down_sync(0xffffffffu, s.x, o);
+        s.y += __shfl_down_sync(0xffffffffu, s.y, o);
+    }
+    if (lane == 0) tot[j] = s;
+}
+
+__global__ void __launch_bounds__(256) pixel_counts_kernel(const double2 *pix_sum, int splits, int npix, double *out)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= npix) return;
+    double v = 0.0;
+    for (int sp = 0; sp < splits; sp++) v += pix_sum[(size_t)sp * npix + p].y;
+    out[p] = v;
 }
 
 }  // namespace
@@ -547,7 +572,18 @@ cudaError_t launch_integrate_pixels(const IntegPixParams &P, int model_type, dou
     cudaError_t e = model_type == GF_MODEL_EXP_DISK ? launch_integrate_pixels_t<GF_MODEL_EXP_DISK>(P, s)
                                                     : launch_integrate_pixels_t<GF_MODEL_POWER_LAW_ELLIPSOID>(P, s);
     if (e != cudaSuccess) return e;
-    job_totals_kernel<<<P.njobs, 256, 0, s>>>(P.pix_sum, P.pix_off, P.splits, P.total_pix, P.plans, tot);
+    double2 *part = tot + P.njobs;
+    job_totals_kernel<<<dim3(GF_TOTAL_PARTS, P.njobs), 256, 0, s>>>(P.pix_sum, P.pix_off, P.splits, P.total_pix, P.plans, part);
+    sum_totals_kernel<<<(P.njobs + 7) / 8, 256, 0, s>>>(part, P.njobs, tot);
+    count_launches(2);
+    return cudaGetLastError();
+}
+
+size_t integ_totals(int njobs) { return (size_t)njobs * (1 + GF_TOTAL_PARTS); }
+
+cudaError_t launch_pixel_counts(const IntegPixParams &P, double *out, cudaStream_t s)
+{
+    pixel_counts_kernel<<<(P.total_pix + 255) / 256, 256, 0, s>>>(P.pix_sum, P.splits, P.total_pix, out);
     count_launches(1);
     return cudaGetLastError();
 }

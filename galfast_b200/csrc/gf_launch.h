@@ -207,8 +207,11 @@ cudaError_t launch_integ_plans(const IntegPlanDesc *desc_dev, int nplans, cudaSt
 int integ_splits(int64_t groups);
 int64_t integ_ctas(int64_t npix, int splits);
 size_t integ_smem(int nM_max, int32_t *pitch);
-/* per-pixel sums into P.pix_sum, then per-request totals into tot[njobs] */
+/* per-pixel sums into P.pix_sum, then per-request totals into tot[0 .. njobs); tot holds integ_totals(njobs) */
+size_t integ_totals(int njobs);
 cudaError_t launch_integrate_pixels(const IntegPixParams &P, int model_type, double2 *tot, cudaStream_t s);
+/* out[p] = the expected covered stars of pixel p, over the parts of P.pix_sum */
+cudaError_t launch_pixel_counts(const IntegPixParams &P, double *out, cudaStream_t s);
 
 /* the batched draw (gf_batchdraw.cu) */
 /* Rows of neighbouring pixels: runs of up to GF_ROW_PIXELS pixels of a request with the same first

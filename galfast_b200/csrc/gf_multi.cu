@@ -169,25 +169,37 @@ struct ReqInfo {
     std::vector<int32_t> rowpx;        /* first pixel of each pixel row (GF_ROW_PIXELS), then npixels */
 };
 
-/* The pixel rows of a request: per pixel its row and cut row (gf_launch.h), and each row's first
- * pixel; and the pixels with the fully covered ones first.  The cut row is the first im with
- * m0 + dm im + Am > m1 in float, as the crawl cuts its bins. */
-void pixel_rows(const SkyModel &m, const gf_job &J, uint2 *prow, uint32_t *order, std::vector<int32_t> &rowpx)
+
+/* CrawlState slices of one request inside the arrays of all requests */
+CrawlState slice(const CrawlState &a, size_t off)
+{
+    CrawlState s;
+    s.status = a.status + off; s.blk_ilb = a.blk_ilb + off; s.blk_k = a.blk_k + off; s.pos = a.pos + off;
+    s.ndraw = a.ndraw + off; s.cur_ilb = a.cur_ilb + off; s.cur_im = a.cur_im + off; s.cur_iM = a.cur_iM + off;
+    s.anc = a.anc + off; s.nstars = a.nstars + off;
+    return s;
+}
+
+}  // namespace
+
+namespace gfa {
+/* The cut row is the first im with m0 + dm im + Am > m1 in float, as the crawl cuts its bins. */
+void pixel_rows(const SkyModel &m, const gf_pencil_beam *pixels, int32_t npixels, const float *ammin, uint2 *prow,
+                uint32_t *order, std::vector<int32_t> &rowpx)
 {
     /* the integrate's order: fully covered pixels first */
     uint32_t full = 0;
-    for (int p = 0; p < J.npixels; p++) full += J.pixels[p].coveredFraction == 1.0f;
+    for (int p = 0; p < npixels; p++) full += pixels[p].coveredFraction == 1.0f;
     uint32_t nf = 0, npart = full;
-    for (int p = 0; p < J.npixels; p++) order[J.pixels[p].coveredFraction == 1.0f ? nf++ : npart++] = (uint32_t)p;
+    for (int p = 0; p < npixels; p++) order[pixels[p].coveredFraction == 1.0f ? nf++ : npart++] = (uint32_t)p;
     rowpx.clear();
-    rowpx.reserve((size_t)J.npixels / GF_ROW_PIXELS + 64);
-    const bool ext = J.beam_ammin && J.ext.kind != GF_EXT_NONE;
+    rowpx.reserve((size_t)npixels / GF_ROW_PIXELS + 64);
     float last = -1.f;
     int icut = -1, prev = -1, in_row = 0;
     auto cut = [&](int i, float Am) { return m.m0 + m.dm * (float)i + Am > m.m1; };
-    for (int p = 0; p < J.npixels; p++) {
-        const gf_pencil_beam &x = J.pixels[p];
-        const float Am = ext ? J.beam_ammin[x.extIdx] : 0.f;
+    for (int p = 0; p < npixels; p++) {
+        const gf_pencil_beam &x = pixels[p];
+        const float Am = ammin ? ammin[x.extIdx] : 0.f;
         if (icut < 0 || Am != last) {
             if (icut < 0) icut = m.nm;
             while (icut < m.nm && !cut(icut, Am)) icut++;
@@ -204,20 +216,9 @@ void pixel_rows(const SkyModel &m, const gf_job &J, uint2 *prow, uint32_t *order
         prow[p].x = (uint32_t)rowpx.size() - 1;
         prow[p].y = (uint32_t)icut | (ax * ax + ay * ay < 1.9999f ? 0u : 0x10000u);
     }
-    rowpx.push_back(J.npixels);
+    rowpx.push_back(npixels);
 }
-
-/* CrawlState slices of one request inside the arrays of all requests */
-CrawlState slice(const CrawlState &a, size_t off)
-{
-    CrawlState s;
-    s.status = a.status + off; s.blk_ilb = a.blk_ilb + off; s.blk_k = a.blk_k + off; s.pos = a.pos + off;
-    s.ndraw = a.ndraw + off; s.cur_ilb = a.cur_ilb + off; s.cur_im = a.cur_im + off; s.cur_iM = a.cur_iM + off;
-    s.anc = a.anc + off; s.nstars = a.nstars + off;
-    return s;
-}
-
-}  // namespace
+}  // namespace gfa
 
 /* Device buffers of gf_catalog_run_multi, kept by the context between calls
  * (they only grow), so that repeated runs do not allocate. */
@@ -254,7 +255,7 @@ struct MultiWS {
     Grow<uint64_t> key, key_b;
     Grow<uint32_t> idx_a, idx_b;
     Grow<char> temp;
-    Grow<double2> pixsum, tot;              /* pixel-by-pixel integrate: per pixel, per request */
+    Grow<double2> pixsum, tot;              /* pixel-by-pixel integrate: per pixel; per request, then its parts */
     Grow<const unsigned char *> plans;
     Grow<int32_t> pixoff;
     Grow<gfk::IntegPlanDesc> pdesc;
@@ -668,7 +669,9 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         memset(hl, 0, lb_);
         parallel_for(njobs, [&](int j) {
             if (!R[j].plain) {
-                pixel_rows(R[j].hm[0].m, jobs[j], hr + R[j].pix_off, ho + R[j].pix_off, R[j].rowpx);
+                const float *am = jobs[j].ext.kind != GF_EXT_NONE ? jobs[j].beam_ammin : nullptr;
+                gfa::pixel_rows(R[j].hm[0].m, jobs[j].pixels, jobs[j].npixels, am, hr + R[j].pix_off, ho + R[j].pix_off,
+                                R[j].rowpx);
                 std::copy(R[j].rowpx.begin(), R[j].rowpx.end(), hx + R[j].pix_off + j);
             }
             memcpy(hp + R[j].pix_off, jobs[j].pixels, sizeof(gf_pencil_beam) * (size_t)jobs[j].npixels);
@@ -823,7 +826,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         off[njobs] = (int32_t)pix_total;
         GF_TRY(ws.pixoff.need((size_t)njobs + 1));
         GF_CUDA(cudaMemcpyAsync(ws.pixoff.p, off.data(), 4 * ((size_t)njobs + 1), cudaMemcpyHostToDevice, st));
-        GF_TRY(ws.tot.need((size_t)njobs));
+        GF_TRY(ws.tot.need(gfk::integ_totals(njobs)));
         GF_TRY(ws.plans.need((size_t)njobs));
         int64_t groups = 0;
         for (int j : integ) groups += (jobs[j].npixels + 63) / 64;
