@@ -241,6 +241,7 @@ struct DrawJob {
     FastDiv fB;                    /* division by Bp */
     float norm, dm, dM, dmin, dmax;
     int32_t dlim;                  /* dmin or dmax set */
+    int32_t lanes;                 /* streams of a work item (a warp) of the draw: at most 32 */
 };
 struct BlockLfParams {
     const CrawlJob *jobs;
@@ -263,9 +264,10 @@ struct BlockWordParams {
 };
 struct BatchDrawParams {
     const DrawJob *view;           /* per request */
-    const uint32_t *items;         /* (request << 16) | first of 32 consecutive streams */
+    const uint32_t *items;         /* (request << 16) | first of the item's consecutive streams, the largest requests first */
     int32_t nitems;
     uint32_t *next_item;           /* work-queue counter */
+    int32_t sms;                   /* SMs of the device (set by the launch) */
     EventRecord *ev;
     int64_t ev_capacity;
     unsigned long long *ev_count;  /* events found (may exceed the capacity) */

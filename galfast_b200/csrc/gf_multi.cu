@@ -264,8 +264,8 @@ struct MultiWS {
     Grow<int32_t> joblist, tileoff;
     Grow<EventRecord> ev;
     Grow<int64_t> k64, off64;
-    Grow<uint32_t> gitems;                  /* batched draw: (request << 16) | first of 32 streams */
-    Grow<uint4> brec;                       /* batched draw: per request and block, the bound walk's record */
+    Grow<uint32_t> gitems;                  /* batched draw: (request << 16) | an item's first stream */
+    Grow<uint4> brec;                       /* batched draw: block records, per request and block */
     Grow<uint4 *> brecptr;
     Grow<int64_t> blkoff;
     gf_table out;
@@ -1192,6 +1192,18 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                     nseg *= 4;
                 }
                 tile = gfk::block_word_tile(rows_max, slots_max);
+                /* Streams of a work item: 16 instead of 32 for the requests with more than an eighth of the
+                 * call's blocks.  Their streams are the longest chains, the call ends with them, and a warp's
+                 * services hold up all its streams: twelve requests up to a quarter of the call 13.7 -> 12.1 ms,
+                 * eight beams 2.7 -> 2.5 ms; on the largest of 64 beams, a thirteenth of the call, 10.0 -> 10.4 ms. */
+                std::vector<int32_t> lanes(nb, 32);
+                {
+                    double all = 0.0;
+                    std::vector<double> blocks(nb);
+                    for (size_t q = 0; q < nb; q++) all += blocks[q] = (double)jobs[batched[q]].npixels * (double)(boff[q + 1] - boff[q]);
+                    for (size_t q = 0; q < nb; q++)
+                        if (blocks[q] > all / 8.0) lanes[q] = 16;
+                }
                 view.resize((size_t)nseg * njobs);
                 toff.resize((size_t)nseg * (nb + 1));
                 tiles.resize((size_t)nseg);
@@ -1210,6 +1222,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                         v.Bp = (int32_t)(boff[q + 1] - boff[q]);
                         v.nslots = h.nslots;
                         v.N = N;
+                        v.lanes = lanes[q];
                         v.nM = m.nM;
                         v.QN = N / v.Bp;
                         v.RN = N % v.Bp;
@@ -1275,16 +1288,16 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 };
                 gfk::BatchDrawParams B;
                 memset(&B, 0, sizeof(B));
-                /* work items: 32 consecutive streams of a request, requests in decreasing size */
-                const int ngroups = (N + 31) / 32;
-                const int32_t ngitems = (int32_t)(nb * (size_t)ngroups);
+                /* work items: consecutive streams of a request, requests in decreasing size */
+                int32_t ngitems = 0;
+                for (size_t q = 0; q < nb; q++) ngitems += (N + lanes[q] - 1) / lanes[q];
                 GF_TRY(ws.gitems.need((size_t)ngitems));
                 {
                     GF_TRY(ws.h_stage.need(4 * (size_t)ngitems));
                     uint32_t *gi = (uint32_t *)ws.h_stage.p;
                     size_t q = 0;
-                    for (int j : batched)
-                        for (int g = 0; g < ngroups; g++) gi[q++] = ((uint32_t)j << 16) | (uint32_t)(32 * g);
+                    for (size_t k = 0; k < nb; k++)
+                        for (int t = 0; t < N; t += lanes[k]) gi[q++] = ((uint32_t)batched[k] << 16) | (uint32_t)t;
                     GF_CUDA(cudaMemcpyAsync(ws.gitems.p, gi, 4 * q, cudaMemcpyHostToDevice, st));
                     GF_CUDA(cudaStreamSynchronize(st));
                 }
@@ -1296,9 +1309,9 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 GF_TRY(make_words(0));
                 if (ctx->draw_wpc[mtype] == 0) {
                     /* autotuner: time 8, 4, 2 and 1 warps per CTA on the head of the work queue
-                     * (the largest requests), from the same stream states, and keep the fastest */
+                     * (the largest requests, as many as are on the chip together), from the same stream states, and keep the fastest */
                     gfk::BatchDrawParams T = B;
-                    T.nitems = std::min<int32_t>(ngitems, std::max<int32_t>(ngitems / 16, 148 * 8));
+                    T.nitems = std::min<int32_t>(ngitems, std::max<int32_t>(ngitems / 16, 148 * 24));
                     float best_ms = 0.f;
                     int best = 4;
                     cudaEvent_t e0, e1;
