@@ -42,6 +42,9 @@ void release_caches(gf_ctx *ctx)
     free_blocks(ctx);
 }
 
+/* block words of a generator's draw: the largest tables, and the largest kept for the next generator (words of 4 bytes) */
+static const int64_t kWordsMost = (int64_t)4 << 30;
+static const size_t kWordsKept = (size_t)256 << 20;
 static const size_t kBlockMin = 4096, kBlockMax = (size_t)64 << 20, kBlocksHeld = (size_t)512 << 20;
 
 /* blocks come in powers of two, so that requests of similar sizes share them */
@@ -185,6 +188,9 @@ struct ModelState {
     void *st_mem = nullptr, *snap_mem = nullptr;
     double expected = 0, expected_covered = 0;
     int64_t drawn = 0;
+    unsigned char *d_plan = nullptr;         /* anchor plan of its grid (IntegPlanDesc), and its header */
+    gfk::IntegPlanHdr plan{};
+    bool planned = false;
     std::vector<double> stream_expected;     /* per-stream expected stars (integrate pass) */
     std::vector<int64_t> stream_drawn;       /* stars drawn per stream so far */
     int first_active = 0;                    /* streams before it have finished */
@@ -201,6 +207,16 @@ struct gf_skygen {
     /* integrate by pixels: cut rows and order of the pixels (gfa::pixel_rows); null: by streams only */
     uint2 *d_prow = nullptr;
     uint32_t *d_order = nullptr;
+    /* draw by block words: first pixels of the pixel rows; the tables of model words_model */
+    std::vector<int32_t> rowpx;
+    int32_t *d_rowpx = nullptr;
+    uint32_t *d_words = nullptr;
+    size_t words_cap = 0;
+    int words_model = -1;
+    struct WordSetup *d_setup = nullptr;
+    uint4 *d_brec = nullptr;
+    float *d_lfm = nullptr;
+    size_t brec_cap = 0, lfm_cap = 0;
     /* per-launch buffers */
     int64_t *d_limits = nullptr;
     uint32_t *d_rng_snap = nullptr;      /* [3][nthreads] */
@@ -289,10 +305,14 @@ struct RecView {
     void *d_sort_temp = nullptr;
     size_t sort_temp_bytes = 0;
     int64_t rec_cap = 0;
+    uint32_t *d_words = nullptr;      /* block words, slot densities and row offsets of a draw */
+    size_t words_cap = 0;
 };
 
 void free_recs(RecView &v)
 {
+    dev_free(v.d_words);
+    v.words_cap = 0;
     dev_free(v.d_rec); dev_free(v.d_rec2); dev_free(v.d_rec_am); dev_free(v.d_rec_am2);
     dev_free(v.d_lb); dev_free(v.d_projIdx); dev_free(v.d_hidden);
     dev_free(v.d_projXY); dev_free(v.d_DM); dev_free(v.d_absmag); dev_free(v.d_XYZ);
@@ -780,11 +800,13 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
     std::vector<uint2> prow;
     std::vector<uint32_t> order;
     if (!s->maps && hms[0].m.nm <= 16384) {
-        std::vector<int32_t> rowpx;
         prow.resize(npixels);
         order.resize(npixels);
-        gfa::pixel_rows(hms[0].m, pixels, npixels, s->geom.ext_kind != GF_EXT_NONE ? beam_ammin : nullptr, prow.data(), order.data(), rowpx);
-        if (own_alloc(s, &s->d_prow, npixels) == GF_OK && own_alloc(s, &s->d_order, npixels) == GF_OK) {
+        gfa::pixel_rows(hms[0].m, pixels, npixels, s->geom.ext_kind != GF_EXT_NONE ? beam_ammin : nullptr, prow.data(), order.data(),
+                        s->rowpx);
+        if (own_alloc(s, &s->d_prow, npixels) == GF_OK && own_alloc(s, &s->d_order, npixels) == GF_OK &&
+            own_alloc(s, &s->d_rowpx, s->rowpx.size()) == GF_OK) {
+            up(s->d_rowpx, s->rowpx.data(), 4 * s->rowpx.size());
             up(s->d_prow, prow.data(), sizeof(uint2) * (size_t)npixels);
             up(s->d_order, order.data(), 4 * (size_t)npixels);
         } else {
@@ -817,7 +839,16 @@ gf_status gf_skygen_destroy(gf_skygen *s)
     RecView &c = *(RecView *)s->ctx->rec_cache;
     RecView mine;
     move_recs(mine, *s);
-    if (mine.rec_cap > c.rec_cap) std::swap(mine, c);
+    if (mine.rec_cap > c.rec_cap) {
+        std::swap(mine.d_words, c.d_words);
+        std::swap(mine.words_cap, c.words_cap);
+        std::swap(mine, c);
+    }
+    if (s->words_cap > c.words_cap && s->words_cap <= gfa::kWordsKept) {
+        std::swap(s->d_words, c.d_words);
+        std::swap(s->words_cap, c.words_cap);
+    }
+    dev_free(s->d_words);
     free_recs(mine);
     delete s;
     return GF_OK;
@@ -847,6 +878,7 @@ gf_status gf_skygen_set_norm(gf_skygen *s, int32_t model, float norm)
     if (!s || model < 0 || model >= (int)s->models.size()) return fail(GF_E_INVALID, "invalid model");
     ModelState &ms = s->models[model];
     ms.hm.m.norm = norm;
+    s->words_model = -1;           /* (its thresholds) */
     ms.expected *= norm;
     ms.expected_covered *= norm;
     return GF_OK;
@@ -869,6 +901,24 @@ struct Blocks {
     ~Blocks() { for (auto &k : v) gfa::kept_free(ctx, k.first, k.second); }
 };
 
+/* the model's anchor plan, made on the context's stream; its header is read once that has been waited for */
+gf_status start_plan(gf_skygen *s, ModelState &ms)
+{
+    const SkyModel &m = ms.hm.m;
+    gfk::IntegPlanDesc h, *d = nullptr;
+    memset(&h, 0, sizeof(h));
+    const size_t bytes = gfk::integ_plan_bytes(m.nm, m.nM, &h.max_anchors, &h.max_slots);
+    Blocks blocks{s->ctx, {}};
+    GF_TRY(blocks.take(&d, 1));
+    if (!ms.d_plan) GF_TRY(own_alloc(s, &ms.d_plan, bytes));
+    h.plan = ms.d_plan;
+    h.Dtab = ms.d_Dtab;
+    h.nm = m.nm; h.nM = m.nM; h.nM_tab = m.nM;
+    GF_CUDA(cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, s->ctx->stream));
+    GF_CUDA(gfk::launch_integ_plans(d, 1, s->ctx->stream));
+    return GF_OK;
+}
+
 /* The integrate of one model by pixels instead of by streams (gf_integrate.cu): the same bins and
  * anchors when blocks of bins never straddle pixels.  *done is false, and nothing has changed, where it
  * does not apply: other grids, 3-D extinction maps (anchors' extinction by distance), density cubes,
@@ -876,42 +926,43 @@ struct Blocks {
  * 0.04 ms and 0.5 ms more for 1e8 bins (5e6 bins: 0.07 ms a model by streams, 0.17 by pixels; 4.6e7: 0.26
  * and 0.17; 7.5e8: 3.5 and 0.54). */
 constexpr long long kPixelIntegrateBins = 25000000;
+bool by_pixels(const gf_skygen *s, const SkyModel &m)
+{
+    const long long kmax = (long long)m.nm * m.nM;
+    return s->d_prow && kmax % GF_BLOCK == 0 && m.nm + m.nM <= 16384 && m.type != GF_MODEL_DENSITY_CUBE &&
+           kmax * s->geom.npixels >= kPixelIntegrateBins;
+}
+
 gf_status integrate_by_pixels(gf_skygen *s, ModelState &ms, double *expected, double *expected_covered, double *per_pixel, bool *done)
 {
     const SkyModel &m = ms.hm.m;
-    const long long kmax = (long long)m.nm * m.nM;
     gfk::IntegPixParams P;
     memset(&P, 0, sizeof(P));
-    if (!s->d_prow || kmax % GF_BLOCK != 0 || m.nm + m.nM > 16384 || m.type == GF_MODEL_DENSITY_CUBE ||
-        kmax * s->geom.npixels < kPixelIntegrateBins || gfk::integ_smem(m.nM, &P.pitch) > 200 * 1024)
-        return GF_OK;
+    if (!by_pixels(s, m) || gfk::integ_smem(m.nM, &P.pitch) > 200 * 1024) return GF_OK;
     gf_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     const int npix = s->geom.npixels;
     /* what the kernels read: one upload */
     struct Setup {
         CrawlJob job;
-        gfk::IntegPlanDesc desc;
         const unsigned char *plan;
         int32_t pix_off[2], cta_off[2];
     } h, *d = nullptr;
     memset((void *)&h, 0, sizeof(h));
     Blocks blocks{ctx, {}};
-    const size_t plan_bytes = gfk::integ_plan_bytes(m.nm, m.nM, &h.desc.max_anchors, &h.desc.max_slots);
+    ProfScope ps(ctx, GF_PROF_INTEGRATE);
+    if (!ms.planned) GF_TRY(start_plan(s, ms));
     P.splits = gfk::integ_splits((npix + 63) / 64);
     P.total_ctas = (int32_t)gfk::integ_ctas(npix, P.splits);
     P.njobs = 1;
     P.total_pix = npix;
     double2 *tot = nullptr;
     double *pp = nullptr;
-    GF_TRY(blocks.take(&h.desc.plan, plan_bytes));
     GF_TRY(blocks.take(&d, 1));
     GF_TRY(blocks.take(&P.pix_sum, (size_t)npix * P.splits));
     GF_TRY(blocks.take(&tot, gfk::integ_totals(1)));
     if (per_pixel) GF_TRY(blocks.take(&pp, npix));
-    h.desc.Dtab = ms.d_Dtab;
-    h.desc.nm = m.nm; h.desc.nM = m.nM; h.desc.nM_tab = m.nM;
-    h.plan = h.desc.plan;
+    h.plan = ms.d_plan;
     h.pix_off[1] = npix;
     h.cta_off[1] = P.total_ctas;
     h.job.m = m;
@@ -920,18 +971,16 @@ gf_status integrate_by_pixels(gf_skygen *s, ModelState &ms, double *expected, do
     h.job.Dtab = ms.d_Dtab;
     P.jobs = &d->job; P.plans = &d->plan; P.pix_off = d->pix_off; P.cta_off = d->cta_off;
     P.order = s->d_order; P.prow = s->d_prow;
-    gfk::IntegPlanHdr hdr;
     double2 sums;
-    ProfScope ps(ctx, GF_PROF_INTEGRATE);
     GF_CUDA(cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, st));
-    GF_CUDA(gfk::launch_integ_plans(&d->desc, 1, st));
     GF_CUDA(gfk::launch_integrate_pixels(P, m.type, tot, st));
     if (per_pixel) GF_CUDA(gfk::launch_pixel_counts(P, pp, st));
-    GF_CUDA(cudaMemcpyAsync(&hdr, h.desc.plan, sizeof(hdr), cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaMemcpyAsync(&ms.plan, ms.d_plan, sizeof(ms.plan), cudaMemcpyDeviceToHost, st));
     GF_CUDA(cudaMemcpyAsync(&sums, tot, sizeof(sums), cudaMemcpyDeviceToHost, st));
     if (per_pixel) GF_CUDA(cudaMemcpyAsync(per_pixel, pp, 8 * (size_t)npix, cudaMemcpyDeviceToHost, st));
     GF_CUDA(cudaStreamSynchronize(st));
-    if (!hdr.ok) return GF_OK;     /* (nothing was summed) */
+    ms.planned = true;
+    if (!ms.plan.ok) return GF_OK;     /* (nothing was summed) */
     /* blocks of bins go to the streams in turn: an even share predicts the draw's windows */
     ms.stream_expected.assign(s->nthreads, sums.x / s->nthreads);
     ms.expected = sums.x;
@@ -1061,6 +1110,118 @@ gf_status gf_skygen_precision(gf_skygen *s, int32_t model, gf_precision_report *
     return GF_OK;
 }
 
+}  /* extern "C" */
+
+/* what the kernels that make a generator's block words read, and the view of its draw */
+struct WordSetup {
+    CrawlJob job;
+    gfk::DrawJob view;
+    const unsigned char *plan;
+    uint4 *brec;
+    float *lfm;
+    int32_t job_list, tile_off[2];
+    int64_t blk_off[2];
+};
+
+namespace {
+/* The block words (gf_batchdraw.cu) of one model over all pixels of a generator, for
+ * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
+ * integrate_by_pixels says the same, and tables above 4 GB or that do not fit the device.
+ * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
+ * of 71524 pixels (2.7e9 bins a model, 8 windows) 67.9 -> 38.9 ms for three models (tables 1.3),
+ * 1600 pixels (4.6e7 bins) 2.05 -> 0.70 (tables 0.17). */
+gf_status ensure_words(gf_skygen *s, int model, bool *ok)
+{
+    *ok = false;
+    ModelState &ms = s->models[model];
+    const SkyModel &m = ms.hm.m;
+    if (!by_pixels(s, m)) return GF_OK;
+    if (s->words_model == model) { *ok = true; return GF_OK; }
+    gf_ctx *ctx = s->ctx;
+    cudaStream_t st = ctx->stream;
+    if (!ms.planned) {
+        GF_TRY(start_plan(s, ms));
+        GF_CUDA(cudaMemcpyAsync(&ms.plan, ms.d_plan, sizeof(ms.plan), cudaMemcpyDeviceToHost, st));
+        GF_CUDA(cudaStreamSynchronize(st));
+        ms.planned = true;
+    }
+    const int64_t npix = s->geom.npixels, Bp = (int64_t)m.nm * m.nM / GF_BLOCK, nrows = (int64_t)s->rowpx.size() - 1;
+    const int64_t nslots = ms.plan.nslots, n = nrows * Bp + npix * (nslots + 1);
+    const int tile = ms.plan.ok ? gfk::block_word_tile(nrows, (int)nslots) : 0;
+    if (!ms.plan.ok || npix * Bp >= (1 << 30) || nrows * Bp >= ((int64_t)1 << 32) || 4 * n > gfa::kWordsMost ||
+        4 * (int64_t)tile * nslots > 200 * 1024)
+        return GF_OK;
+    if ((size_t)n > s->words_cap) {
+        GF_CUDA(cudaStreamSynchronize(st));
+        dev_free(s->d_words);
+        s->words_cap = 0;
+        s->words_model = -1;
+        RecView *c = (RecView *)ctx->rec_cache;
+        if (c && c->words_cap >= (size_t)n) {
+            std::swap(s->d_words, c->d_words);
+            std::swap(s->words_cap, c->words_cap);
+        } else {
+            const gf_status as = dev_alloc(&s->d_words, (size_t)n);
+            if (as == GF_E_OOM) return GF_OK;
+            GF_TRY(as);
+            s->words_cap = (size_t)n;
+        }
+    }
+    if (!s->d_setup) GF_TRY(own_alloc(s, &s->d_setup, 1));
+    if (s->brec_cap < (size_t)Bp) {
+        GF_TRY(own_alloc(s, &s->d_brec, (size_t)Bp));
+        s->brec_cap = (size_t)Bp;
+    }
+    if (s->lfm_cap < (size_t)m.nM) {
+        GF_TRY(own_alloc(s, &s->d_lfm, (size_t)m.nM));
+        s->lfm_cap = (size_t)m.nM;
+    }
+    s->words_model = -1;
+    WordSetup h;
+    memset((void *)&h, 0, sizeof(h));
+    h.job.m = m;
+    h.job.m.lf = ms.d_lf;
+    h.job.g = s->geom;
+    h.job.Dtab = ms.d_Dtab;
+    h.plan = ms.d_plan;
+    h.brec = s->d_brec;
+    h.lfm = s->d_lfm;
+    h.tile_off[1] = (int32_t)((nrows + tile - 1) / tile);
+    h.blk_off[1] = Bp;
+    gfk::DrawJob &v = h.view;
+    v.npx = (int32_t)npix;
+    v.nrows = (int32_t)nrows;
+    v.Bp = (int32_t)Bp;
+    v.nslots = (int32_t)nslots;
+    v.prow = s->d_prow;
+    v.rowpx = s->d_rowpx;
+    v.brec = s->d_brec;
+    v.lfm = s->d_lfm;
+    v.dslot = (const uint16_t *)(ms.d_plan + ms.plan.off_dslot);
+    v.slotD = (const float *)(ms.d_plan + ms.plan.off_slot);
+    v.words = s->d_words;
+    v.ms = (float *)(s->d_words + nrows * Bp);
+    v.roff = s->d_words + nrows * Bp + npix * nslots;
+    WordSetup *d = s->d_setup;
+    GF_CUDA(cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, st));
+    gfk::BlockLfParams BL;
+    BL.jobs = &d->job; BL.plans = &d->plan; BL.brec = &d->brec; BL.lfm = &d->lfm;
+    BL.job_list = &d->job_list; BL.blk_off = d->blk_off;
+    BL.njobs = 1; BL.total = Bp;
+    gfk::BlockWordParams W;
+    W.jobs = &d->job; W.view = &d->view; W.job_list = &d->job_list; W.tile_off = d->tile_off;
+    W.njobs = 1; W.total_tiles = h.tile_off[1]; W.tile = tile;
+    ProfScope ps(ctx, GF_PROF_SLOTS);
+    GF_CUDA(gfk::launch_block_records(BL, st));
+    GF_CUDA(gfk::launch_block_words(W, m.type, (int)nslots, st));
+    s->words_model = model;
+    *ok = true;
+    return GF_OK;
+}
+}  // namespace
+
+extern "C" {
+
 gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_generated, int32_t *done)
 {
     if (!s || model < 0 || model >= (int)s->models.size() || !out || !n_generated || !done) return fail(GF_E_INVALID, "invalid arguments");
@@ -1078,6 +1239,11 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         ms.crawl_init = true;
         ms.stream_drawn.assign(N, 0);
     }
+    bool words = false;
+    GF_TRY(ensure_words(s, model, &words));
+    auto draw = [&](const gfk::LaunchCrawl &L) {
+        return words ? gfk::launch_stream_draw(L, &s->d_setup->view, st) : gfk::launch_crawl(L, 1, st);
+    };
     GF_CUDA(cudaMemsetAsync(ms.st.nstars, 0, 8 * (size_t)N, st));
     GF_CUDA(cudaMemsetAsync(s->ctx->d_counters, 0, 24, st));
     GF_TRY(ensure_rec_capacity(s, C + C / 2 + 65536, 0));
@@ -1137,7 +1303,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
             L.ck_every = kCkEvery;
             {
                 ProfScope ps(s->ctx, GF_PROF_DRAW_WINDOW);
-                GF_CUDA(gfk::launch_crawl(L, 1, st));
+                GF_CUDA(draw(L));
             }
             GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters, s->ctx->d_counters, 8, cudaMemcpyDeviceToHost, st));
             GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters + 4, s->d_ck_count, 4, cudaMemcpyDeviceToHost, st));
@@ -1213,7 +1379,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         L.stream_end = r_hi;
         {
             ProfScope ps(s->ctx, GF_PROF_DRAW_RERUN);
-            GF_CUDA(gfk::launch_crawl(L, 1, st));
+            GF_CUDA(draw(L));
         }
         GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters, s->ctx->d_counters, 8, cudaMemcpyDeviceToHost, st));
         GF_CUDA(cudaStreamSynchronize(st));

@@ -40,9 +40,6 @@ namespace {
 #define BD_FULL 0xffffffffu
 #define GF_EVBUF 64                /* events staged in shared memory per warp (a pass over the parked lanes adds at most 32) */
 #define GF_BINS 0x3ffu             /* the bins of a block as bits */
-#define GF_NLIVE 0xfu              /* a block word: number of live bins below, threshold / 16 above */
-#define GF_DEAD_WORD 0xfffffff0u   /* no live bins, nothing reaches the threshold */
-#define GF_END_WORD 0xffffffffu    /* past the stream's last block */
 
 /* one MWC step; returns the new x (the uniform is 2^-32 x) */
 __device__ __forceinline__ uint32_t bd_mwc_x(uint64_t &v, uint32_t a)
@@ -316,46 +313,6 @@ __device__ __forceinline__ void flush_events(const BatchDrawParams &P, EventReco
     __syncwarp();
 }
 
-/* n (at most 10) MWC steps from (c, x); returns the largest x of them.  Every lane takes the
- * first six unconditionally (most) when all have as many bins: on this chip a step is a wide
- * multiply-add, a move and a maximum, 7 cycles of a scheduler, and 5 more when predicated or
- * selected.  Lanes with fewer bins are blocks that the magnitude cut crosses. */
-__device__ __forceinline__ uint32_t walk_bins(uint32_t &x, uint32_t &c, uint32_t a, uint32_t n)
-{
-    uint32_t mx = 0;
-    auto step = [&](uint32_t &xs, uint32_t &cs) {
-        asm("{\n\t.reg .u64 t;\n\tmov.b64 t, {%1, %4};\n\tmad.wide.u32 t, %2, %3, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
-            : "=r"(xs), "+r"(cs) : "r"(xs), "r"(a), "r"(0u));
-    };
-    if (__all_sync(BD_FULL, n >= 6u)) {
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            step(x, c);
-            mx = max(mx, x);
-        }
-    } else {
-#pragma unroll
-        for (int s = 0; s < 6; s++) {
-            uint32_t x1 = x, c1 = c;
-            step(x1, c1);
-            const bool on = s < (int)n;
-            x = on ? x1 : x;
-            c = on ? c1 : c;
-            mx = max(mx, on ? x1 : 0u);
-        }
-    }
-#pragma unroll
-    for (int s = 6; s < GF_BLOCK; s++) {
-        uint32_t x1 = x, c1 = c;
-        step(x1, c1);
-        const bool on = s < (int)n;
-        x = on ? x1 : x;
-        c = on ? c1 : c;
-        mx = max(mx, on ? x1 : 0u);
-    }
-    return mx;
-}
-
 /* One warp per item of up to 32 consecutive streams of a request, one lane per stream.  A step of a lane
  * is one block: its word (loaded three steps ahead), at most 10 MWC steps, one comparison.
  * Almost every block is empty, and the few lanes that find a candidate bin would hold up
@@ -420,7 +377,7 @@ __global__ void __launch_bounds__(256, 3) batch_draw_kernel(BatchDrawParams P)
             for (int u = 0; u < 4; u++) {
                 const bool act = !parked && c0 != GF_END_WORD;
                 uint32_t x1 = x, cc = c;
-                const uint32_t mx = walk_bins(x1, cc, a, act ? c0 & GF_NLIVE : (uint32_t)GF_BLOCK);
+                const uint32_t mx = gfc::walk_bins(x1, cc, a, act ? c0 & GF_NLIVE : (uint32_t)GF_BLOCK);
                 if (act) {
                     if (mx >= (c0 & ~GF_NLIVE)) {
                         parked = true;

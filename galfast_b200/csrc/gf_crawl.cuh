@@ -290,4 +290,44 @@ __device__ __forceinline__ float bin_mu_x(const AnchorX &a, float lfv, float mro
     return (mrow + a.Am > m1) ? cut_marker() : rho;
 }
 
+/* n (at most 10) MWC steps from (c, x); returns the largest x of them.  Every lane takes the
+ * first six unconditionally (most) when all have as many bins: on this chip a step is a wide
+ * multiply-add, a move and a maximum, 7 cycles of a scheduler, and 5 more when predicated or
+ * selected.  Lanes with fewer bins are blocks that the magnitude cut crosses. */
+__device__ __forceinline__ uint32_t walk_bins(uint32_t &x, uint32_t &c, uint32_t a, uint32_t n)
+{
+    uint32_t mx = 0;
+    auto step = [&](uint32_t &xs, uint32_t &cs) {
+        asm("{\n\t.reg .u64 t;\n\tmov.b64 t, {%1, %4};\n\tmad.wide.u32 t, %2, %3, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
+            : "=r"(xs), "+r"(cs) : "r"(xs), "r"(a), "r"(0u));
+    };
+    if (__all_sync(0xffffffffu, n >= 6u)) {
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            step(x, c);
+            mx = max(mx, x);
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < 6; s++) {
+            uint32_t x1 = x, c1 = c;
+            step(x1, c1);
+            const bool on = s < (int)n;
+            x = on ? x1 : x;
+            c = on ? c1 : c;
+            mx = max(mx, on ? x1 : 0u);
+        }
+    }
+#pragma unroll
+    for (int s = 6; s < GF_BLOCK; s++) {
+        uint32_t x1 = x, c1 = c;
+        step(x1, c1);
+        const bool on = s < (int)n;
+        x = on ? x1 : x;
+        c = on ? c1 : c;
+        mx = max(mx, on ? x1 : 0u);
+    }
+    return mx;
+}
+
 }  // namespace gfc

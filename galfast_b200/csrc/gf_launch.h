@@ -220,6 +220,9 @@ cudaError_t launch_pixel_counts(const IntegPixParams &P, double *out, cudaStream
 #define GF_ROW_PIXELS 4
 /* One request of a draw pass: its tables for the pixels [px0, px0 + npx) of the pass's segment.
  * Block b of pixel p is the request's (p Bp + b)-th; stream t takes every N-th from the t-th. */
+#define GF_NLIVE 0xfu              /* a block word: number of live bins below, threshold / 16 above */
+#define GF_DEAD_WORD 0xfffffff0u   /* no live bins, nothing reaches the threshold */
+#define GF_END_WORD 0xffffffffu    /* past the stream's last block */
 struct DrawJob {
     uint32_t *words;               /* [nrows][Bp] block words: number of live bins (bits 0-3), threshold of the largest uniform (above) */
     float *ms;                     /* [npx][nslots] model density of each slot of the request's plan */
@@ -277,6 +280,8 @@ cudaError_t launch_block_records(const BlockLfParams &P, cudaStream_t s);
 /* rows of a tile for a launch over that many rows and plans of at most max_slots slots */
 int block_word_tile(int64_t rows, int max_slots);
 cudaError_t launch_block_words(const BlockWordParams &P, int model_type, int max_slots, cudaStream_t s);
+/* a draw launch (launch_crawl) of one request through the block words of all its pixels; view is on the device */
+cudaError_t launch_stream_draw(const LaunchCrawl &L, const DrawJob *view, cudaStream_t s);
 cudaError_t launch_batch_draw(const BatchDrawParams &P, int warps_per_cta, cudaStream_t s);
 cudaError_t expand_temp_bytes(int64_t nev, size_t *bytes);
 /* star records of the events at offsets from a scan over k; *total = the stars of all events */

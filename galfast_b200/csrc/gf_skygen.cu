@@ -27,6 +27,7 @@
  * Results are bin-for-bin and draw-for-draw those of the reference CPU path.
  */
 #include "gf_crawl.cuh"
+#include "gf_launch.h"
 #include "gf_rng.h"
 #include <cub/cub.cuh>
 #include <atomic>
@@ -151,6 +152,20 @@ struct CrawlSmem {
     long long nstars, limit;
     int next_ck, flag, fL, es;
     double red[2][CW];
+};
+
+/* a stream drawn by one warp from block words (stream_draw_kernel): the anchors of one block */
+template <>
+struct CrawlSmem<1, 0> {
+    CrawlJob job;
+    float4 slot[GF_BLOCK];
+    StarRecord recbuf[GF_RECBUF];
+    float ambuf[GF_RECBUF];
+    int nrec;
+    Cursor cur;
+    unsigned long long v, mult;
+    long long nstars, limit;
+    int next_ck, flag, fL, es;
 };
 
 /* Write the staged star records to the global buffer (one warp, all lanes). */
@@ -730,6 +745,188 @@ __global__ void __launch_bounds__(CW * 32, DRAW ? 16 / CW : 24 / CW) crawl_kerne
     }
 }
 
+/* The bins of one block from bin pos on, bin s on lane s, from state v: expected counts as the crawl
+ * forms them, then the bins with stars one after another (handle_event).  Leaves the state after
+ * the last bin in v; stars: whether any had some; returns handle_event's flag. */
+template <int MODEL>
+__device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S, const float *lfm, int sid, int lane, int ilb,
+                                       int lb, int pos, uint64_t &v, bool &stars, uint32_t a, const uint64_t *jlo,
+                                       const uint64_t *jhi)
+{
+    const CrawlJob &J = S.job;
+    const SkyModel &m = J.m;
+    const int x = m.nm, y = m.nM, k0 = lb * GF_BLOCK;
+    int i0, j0;
+    gfc::diag_to_ij_fast(k0, x, y, J.fx, J.fy, i0, j0);
+    int i = i0, j = j0, n = 0;
+    bool anchor = lane == 0;
+    for (int s = 1; s < GF_BLOCK; s++)
+        if (s <= lane) {
+            anchor = gfc::step_in_pixel(i, j, x, y);
+            n += anchor ? 1 : 0;
+        }
+    __syncwarp();
+    if (anchor && lane < GF_BLOCK) {
+        const AnchorX ax = gfc::anchor_x<MODEL>(m, J.g, J.Dtab, ilb, i, j);
+        S.slot[n] = make_float4(ax.Am, ax.ms, ax.D3, ax.K);
+    }
+    __syncwarp();
+    float mus = gfc::cut_marker();
+    if (lane >= pos && lane < GF_BLOCK)
+        mus = gfc::bin_mu_x(ax_from(S.slot[n]), __ldg(lfm + j), m.m0 + m.dm * (float)i, m.norm, m.m1);
+    uint32_t live = __ballot_sync(FULLMASK, !gfc::is_cut(mus));
+    stars = false;
+    for (;;) {
+        uint64_t w = v, wb = v;
+        bool ev = false;
+        if ((live >> lane) & 1u) {
+            for (int q = __popc(live & ((1u << lane) - 1u)); q > 0; q--) (void)mwc_step(w, a);
+            wb = w;
+            const float u = mwc_step(w, a);
+            ev = !surely_empty(u, mus) && has_stars(u, mus);
+        }
+        const unsigned evm = __ballot_sync(FULLMASK, ev);
+        if (!evm) {
+            if (live) v = shfl64(w, 31 - __clz(live));
+            return 0;
+        }
+        const int es = __ffs(evm) - 1;
+        const uint64_t vb = shfl64(wb, es);
+        const float emu = __shfl_sync(FULLMASK, mus, es);
+        handle_event<1, MODEL, 0>(P, S, sid, lane, 0, es, vb, emu, ilb, k0, i0, j0, true, a, jlo, jhi);
+        v = S.v;
+        stars = true;
+        if (S.flag) return S.flag;
+        live &= ~((2u << es) - 1u);
+        __syncwarp();
+    }
+}
+
+/* The draw crawl of one stream by one warp, where the request has block words (gf_batchdraw.cu): the
+ * crawl's states, limits, checkpoints and records.  Lane L takes the L-th next block of the stream,
+ * jumps to the state its first bin has if no bin before it has stars, and walks it against the
+ * block's threshold; only blocks with a candidate are scanned bin by bin, in order, and a block that
+ * did have stars starts the window again right after it.
+ * Bound by instruction issue; per window of 32 blocks a walk, two modular products and a scan. */
+template <int MODEL>
+__global__ void __launch_bounds__(32, 20) stream_draw_kernel(CrawlParams P, const DrawJob *view)
+{
+    __shared__ CrawlSmem<1, 0> S;
+    const int lane = threadIdx.x, tid = P.stream_begin + blockIdx.x;
+    for (int q = lane; q < (int)(sizeof(CrawlJob) / 4); q += 32) ((int *)&S.job)[q] = ((const int *)&P.job0)[q];
+    __syncwarp();
+    const CrawlJob &J = S.job;
+    const CrawlState &st = J.st;
+    const int status = st.status[tid];
+    if (status == 2) return;
+    const int NS = J.rng_nstreams, sid = (J.job_id << 16) | tid;
+    const uint32_t N = (uint32_t)J.m.nthreads, Bp = (uint32_t)view->Bp, npx = (uint32_t)view->npx;
+    const uint32_t *words = view->words, *roff = view->roff;
+    const float *lfm = view->lfm;
+    uint64_t v = ((uint64_t)J.rng[NS + tid] << 32) | J.rng[2 * NS + tid];
+    if (lane == 0) {
+        Cursor &c = S.cur;
+        if (status == 0) {
+            c.blk_ilb = (int)((uint32_t)tid / Bp);
+            c.blk_k = (int)((uint32_t)tid % Bp) * GF_BLOCK;
+            c.pos = 0;
+            c.ndraw = 0;
+            c.cur_ilb = c.cur_im = c.cur_iM = 0;
+            c.anc.Am = c.anc.ms = c.anc.D3 = c.anc.K = 0.f;
+        } else {
+            c.blk_ilb = st.blk_ilb[tid]; c.blk_k = st.blk_k[tid]; c.pos = st.pos[tid];
+            c.ndraw = st.ndraw[tid];
+            c.cur_ilb = st.cur_ilb[tid]; c.cur_im = st.cur_im[tid]; c.cur_iM = st.cur_iM[tid];
+            c.anc = st.anc[tid];
+        }
+        S.v = v;
+        S.nstars = st.nstars[tid];
+        S.limit = J.limits ? J.limits[tid] : J.limit_all;
+        S.next_ck = (int)S.nstars;
+        S.nrec = 0;
+    }
+    __syncwarp();
+    const uint32_t a = J.rng[tid];
+    const uint64_t *jlo = P.jt.lo + (size_t)tid * 32, *jhi = P.jt.hi + (size_t)tid * GF_JUMP_HI;
+    if (S.cur.ndraw) {
+        finish_pending<1, 0>(P, S, sid, lane, a);
+        v = S.v;
+    }
+    uint32_t ilb = (uint32_t)S.cur.blk_ilb, lb = (uint32_t)S.cur.blk_k / GF_BLOCK;
+    int pos = S.cur.pos;
+    const bool pending = S.cur.ndraw != 0;
+    __syncwarp();
+    if (lane == 0 && !pending) S.cur.pos = 0;      /* what handle_event reads: blocks are scanned with all their anchors */
+    __syncwarp();
+    /* blocks of the stream are N apart; this lane's is lane N after the window's first */
+    const uint32_t QN = N / Bp, RN = N % Bp, qL = (uint32_t)lane * N / Bp, rL = (uint32_t)lane * N % Bp, QW = 32u * N / Bp,
+                   RW = 32u * N % Bp;
+    auto ahead = [&](uint32_t &p, uint32_t &b, uint32_t q, uint32_t r) {
+        p += q;
+        b += r;
+        if (b >= Bp) { b -= Bp; p++; }
+    };
+    bool finished = false;
+    int flag = pending ? 1 : 0;
+    while (!flag) {
+        bool stars;
+        if (pos > 0) {
+            /* the rest of a block that the last batch ended in */
+            if (ilb < npx) flag = scan_block<MODEL>(P, S, lfm, sid, lane, (int)ilb, (int)lb, pos, v, stars, a, jlo, jhi);
+            pos = 0;
+            ahead(ilb, lb, QN, RN);
+            continue;
+        }
+        uint32_t pL = ilb, bL = lb;
+        ahead(pL, bL, qL, rL);
+        const bool end = pL >= npx;
+        const uint32_t word = end ? GF_DEAD_WORD : __ldg(words + (__ldg(roff + pL) + bL));
+        const int n = (int)(word & GF_NLIVE);
+        const int inc = warp_incl_scan(n, lane);
+        const uint64_t w0 = jump(v, inc - n, jlo, jhi, a);
+        uint32_t x = (uint32_t)w0, c = (uint32_t)(w0 >> 32);
+        const uint32_t mx = gfc::walk_bins(x, c, a, n ? (uint32_t)n : (uint32_t)GF_BLOCK);
+        unsigned cand = __ballot_sync(FULLMASK, n != 0 && mx >= (word & ~GF_NLIVE));
+        const uint64_t w1 = n ? ((uint64_t)c << 32) | x : w0;
+        bool again = false;
+        for (; cand && !flag && !again; cand &= cand - 1u) {
+            const int f = __ffs(cand) - 1;
+            uint64_t vf = shfl64(w0, f);
+            const uint32_t pf = __shfl_sync(FULLMASK, pL, f), bf = __shfl_sync(FULLMASK, bL, f);
+            flag = scan_block<MODEL>(P, S, lfm, sid, lane, (int)pf, (int)bf, 0, vf, stars, a, jlo, jhi);
+            if (stars) {
+                v = vf;
+                ilb = pf;
+                lb = bf;
+                ahead(ilb, lb, QN, RN);
+                again = true;
+            }
+        }
+        if (flag || again) continue;
+        v = shfl64(w1, 31);
+        if (__any_sync(FULLMASK, end)) {
+            finished = true;
+            break;
+        }
+        ahead(ilb, lb, QW, RW);
+    }
+    flush_records<1, 0>(P, S, lane);
+    if (lane == 0) {
+        const Cursor &c = S.cur;
+        const bool paused = c.ndraw != 0;
+        st.status[tid] = finished ? 2 : 1;
+        st.blk_ilb[tid] = paused ? c.blk_ilb : (int)ilb;
+        st.blk_k[tid] = paused ? c.blk_k : (int)lb * GF_BLOCK;
+        st.pos[tid] = paused ? c.pos : pos;
+        st.ndraw[tid] = c.ndraw;
+        st.cur_ilb[tid] = c.cur_ilb; st.cur_im[tid] = c.cur_im; st.cur_iM[tid] = c.cur_iM;
+        st.anc[tid] = c.anc;
+        st.nstars[tid] = S.nstars;
+        J.rng[NS + tid] = (uint32_t)(v >> 32);
+        J.rng[2 * NS + tid] = (uint32_t)v;
+    }
+}
+
 /* D[im][iM] = powf(10, 0.2 DM + 1) with DM = (m0 + im dm) - (M1 - iM dM), skygen.cu.h:219-222 */
 __global__ void dtab_kernel(SkyModel m, float *D)
 {
@@ -1022,9 +1219,8 @@ cudaError_t dispatch_crawl(int draw, int model_type, int cw, bool persistent, co
 template <int DRAW, int MODEL, int CW>
 static cudaError_t start_crawl_persistent(const CrawlParams &P, size_t smem, cudaStream_t s);
 
-cudaError_t launch_crawl(const LaunchCrawl &L, int draw, cudaStream_t s)
+static void fill_params(CrawlParams &P, const LaunchCrawl &L)
 {
-    CrawlParams P;
     memset(&P, 0, sizeof(P));
     fill_job(P.job0, L);
     P.nitems = L.stream_end - L.stream_begin;
@@ -1039,6 +1235,23 @@ cudaError_t launch_crawl(const LaunchCrawl &L, int draw, cudaStream_t s)
     P.ck_count = L.ck_count;
     P.ck_capacity = L.ck_capacity;
     P.ck_every = L.ck_every > 0 ? L.ck_every : 64;
+}
+
+cudaError_t launch_stream_draw(const LaunchCrawl &L, const DrawJob *view, cudaStream_t s)
+{
+    CrawlParams P;
+    fill_params(P, L);
+    if (P.nitems <= 0) return cudaSuccess;
+    if (L.m.type == GF_MODEL_EXP_DISK) stream_draw_kernel<GF_MODEL_EXP_DISK><<<P.nitems, 32, 0, s>>>(P, view);
+    else stream_draw_kernel<GF_MODEL_POWER_LAW_ELLIPSOID><<<P.nitems, 32, 0, s>>>(P, view);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_crawl(const LaunchCrawl &L, int draw, cudaStream_t s)
+{
+    CrawlParams P;
+    fill_params(P, L);
     if (P.nitems <= 0) return cudaSuccess;
     const size_t smem = (size_t)(L.m.nm + L.m.nM) * sizeof(float);
     if (smem > 64 * 1024) return cudaErrorInvalidValue;
