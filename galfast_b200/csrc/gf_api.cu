@@ -1128,8 +1128,8 @@ namespace {
  * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
  * integrate_by_pixels says the same, and tables above 4 GB or that do not fit the device.
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
- * of 71524 pixels (2.7e9 bins a model, 8 windows) 67.9 -> 38.9 ms for three models (tables 1.3),
- * 1600 pixels (4.6e7 bins) 2.05 -> 0.70 (tables 0.17). */
+ * of 71524 pixels (2.7e9 bins a model, 8 windows) 67.9 -> 28.0 ms for three models (tables 1.3),
+ * 1600 pixels (4.6e7 bins) 2.05 -> 0.67 (tables 0.17). */
 gf_status ensure_words(gf_skygen *s, int model, bool *ok)
 {
     *ok = false;

@@ -290,6 +290,20 @@ __device__ __forceinline__ float bin_mu_x(const AnchorX &a, float lfv, float mro
     return (mrow + a.Am > m1) ? cut_marker() : rho;
 }
 
+/* ten MWC steps from (c, x); returns the largest x of them */
+__device__ __forceinline__ uint32_t walk_ten(uint32_t &x, uint32_t &c, uint32_t a)
+{
+    uint32_t mx = 0;
+#pragma unroll
+    for (int s = 0; s < GF_BLOCK; s++) {
+        const uint64_t t = (uint64_t)a * x + c;
+        x = (uint32_t)t;
+        c = (uint32_t)(t >> 32);
+        mx = max(mx, x);
+    }
+    return mx;
+}
+
 /* n (at most 10) MWC steps from (c, x); returns the largest x of them.  Every lane takes the
  * first six unconditionally (most) when all have as many bins: on this chip a step is a wide
  * multiply-add, a move and a maximum, 7 cycles of a scheduler, and 5 more when predicated or

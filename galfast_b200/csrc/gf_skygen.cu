@@ -310,17 +310,19 @@ __device__ __noinline__ void handle_event(const CrawlParams &P, CrawlSmem<DRAW, 
         draw_stars<DRAW, CW>(P, S, sid, lane, r, nd, ns, S.limit, e_ilb, e_im, e_iM, anc_es.Am);
         vnew = r.v();
         if (nd) flag = 1;             /* the stream reached its limit: pause right after the bin */
-        /* The walk assumed one uniform for this bin; it drew r.used >= 1.  Every later
-         * bin's start state moves by a^(used-1): the scaled multiplier of that power. */
-        const uint64_t p = ((uint64_t)a << 32) - 1;
-        uint32_t n = r.used - 1;
-        uint64_t ms = __ldg(jlo);                                 /* scaled a^0 */
-        if (n >= 2048) {
-            const uint64_t m2047 = gfr::mwc_mulmod_scaled(__ldg(jlo + 31), __ldg(jhi + 63), a, p);
-            while (n >= 2047) { ms = gfr::mwc_mulmod_scaled(ms, m2047, a, p); n -= 2047; }
+        if (CW > 0) {                 /* (stream_draw_kernel jumps from the state itself) */
+            /* The walk assumed one uniform for this bin; it drew r.used >= 1.  Every later
+             * bin's start state moves by a^(used-1): the scaled multiplier of that power. */
+            const uint64_t p = ((uint64_t)a << 32) - 1;
+            uint32_t n = r.used - 1;
+            uint64_t ms = __ldg(jlo);                                 /* scaled a^0 */
+            if (n >= 2048) {
+                const uint64_t m2047 = gfr::mwc_mulmod_scaled(__ldg(jlo + 31), __ldg(jhi + 63), a, p);
+                while (n >= 2047) { ms = gfr::mwc_mulmod_scaled(ms, m2047, a, p); n -= 2047; }
+            }
+            ms = gfr::mwc_mulmod_scaled(ms, gfr::mwc_mulmod_scaled(__ldg(jlo + (n & 31)), __ldg(jhi + (n >> 5)), a, p), a, p);
+            if (lane == 0) S.mult = ms;
         }
-        ms = gfr::mwc_mulmod_scaled(ms, gfr::mwc_mulmod_scaled(__ldg(jlo + (n & 31)), __ldg(jhi + (n >> 5)), a, p), a, p);
-        if (lane == 0) S.mult = ms;
     }
     __syncwarp();
     if (lane == 0) {
@@ -749,22 +751,22 @@ __global__ void __launch_bounds__(CW * 32, DRAW ? 16 / CW : 24 / CW) crawl_kerne
  * forms them, then the bins with stars one after another (handle_event).  Leaves the state after
  * the last bin in v; stars: whether any had some; returns handle_event's flag. */
 template <int MODEL>
-__device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S, const float *lfm, int sid, int lane, int ilb,
+__device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S, const uint4 *brec, const float *lfm, int sid, int lane, int ilb,
                                        int lb, int pos, uint64_t &v, bool &stars, uint32_t a, const uint64_t *jlo,
                                        const uint64_t *jhi)
 {
     const CrawlJob &J = S.job;
     const SkyModel &m = J.m;
-    const int x = m.nm, y = m.nM, k0 = lb * GF_BLOCK;
-    int i0, j0;
-    gfc::diag_to_ij_fast(k0, x, y, J.fx, J.fy, i0, j0);
-    int i = i0, j = j0, n = 0;
-    bool anchor = lane == 0;
-    for (int s = 1; s < GF_BLOCK; s++)
-        if (s <= lane) {
-            anchor = gfc::step_in_pixel(i, j, x, y);
-            n += anchor ? 1 : 0;
-        }
+    const int y = m.nM, k0 = lb * GF_BLOCK;
+    /* the block's first bin and which of its bins start a diagonal (its block record) */
+    const uint4 br = __ldg(brec + lb);
+    const int i0 = (int)(br.x & 0xffffu), j0 = (int)(br.x >> 16);
+    const int s = min(lane, GF_BLOCK - 1);
+    const uint32_t starts = (br.y >> 16) & ((2u << s) - 2u);         /* in bins 1..s */
+    const int n = __popc(starts), d = i0 + j0 + n;
+    const int i = starts ? max(0, d - (y - 1)) + s - (31 - __clz(starts)) : i0 + s, j = d - i;
+    const bool anchor = s == 0 || ((starts >> s) & 1u);
+    const float lfv = __ldg(lfm + j);      /* (in flight while the anchors are formed) */
     __syncwarp();
     if (anchor && lane < GF_BLOCK) {
         const AnchorX ax = gfc::anchor_x<MODEL>(m, J.g, J.Dtab, ilb, i, j);
@@ -773,7 +775,7 @@ __device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S,
     __syncwarp();
     float mus = gfc::cut_marker();
     if (lane >= pos && lane < GF_BLOCK)
-        mus = gfc::bin_mu_x(ax_from(S.slot[n]), __ldg(lfm + j), m.m0 + m.dm * (float)i, m.norm, m.m1);
+        mus = gfc::bin_mu_x(ax_from(S.slot[n]), lfv, m.m0 + m.dm * (float)i, m.norm, m.m1);
     uint32_t live = __ballot_sync(FULLMASK, !gfc::is_cut(mus));
     stars = false;
     for (;;) {
@@ -803,13 +805,18 @@ __device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S,
 }
 
 /* The draw crawl of one stream by one warp, where the request has block words (gf_batchdraw.cu): the
- * crawl's states, limits, checkpoints and records.  Lane L takes the L-th next block of the stream,
- * jumps to the state its first bin has if no bin before it has stars, and walks it against the
- * block's threshold; only blocks with a candidate are scanned bin by bin, in order, and a block that
- * did have stars starts the window again right after it.
- * Bound by instruction issue; per window of 32 blocks a walk, two modular products and a scan. */
+ * crawl's states, limits, checkpoints and records.  Lane L takes two of the stream's next 64 blocks,
+ * jumps to the state their first bin has if no bin before it has stars, and walks them against
+ * their thresholds; only blocks with a candidate are scanned bin by bin, in order, and a block that
+ * did have stars has the window's later blocks walked again from the state after it.
+ * Bound by the longest stream: blocks of a stream lie at the same place of the grid when N is a
+ * multiple of a pixel's blocks, and a stream of the dense bins has ten times the stars of the others, at
+ * some 5000 cycles a scan (half of it the density anchors).  So warps with room beat many of them: 71524
+ * pixels, three models, 28.0 ms at 16 CTAs an SM and 128 registers; at 20 and 96, 33 ms, at 12, 30 ms.
+ * With a block a lane, its word loaded in its own window and the window begun again after each star
+ * 38.9 ms; with a CTA of four warps a stream and every bin's expected count formed 67.9 ms. */
 template <int MODEL>
-__global__ void __launch_bounds__(32, 20) stream_draw_kernel(CrawlParams P, const DrawJob *view)
+__global__ void __launch_bounds__(32, 16) stream_draw_kernel(CrawlParams P, const DrawJob *view)
 {
     __shared__ CrawlSmem<1, 0> S;
     const int lane = threadIdx.x, tid = P.stream_begin + blockIdx.x;
@@ -823,6 +830,7 @@ __global__ void __launch_bounds__(32, 20) stream_draw_kernel(CrawlParams P, cons
     const uint32_t N = (uint32_t)J.m.nthreads, Bp = (uint32_t)view->Bp, npx = (uint32_t)view->npx;
     const uint32_t *words = view->words, *roff = view->roff;
     const float *lfm = view->lfm;
+    const uint4 *brec = view->brec;
     uint64_t v = ((uint64_t)J.rng[NS + tid] << 32) | J.rng[2 * NS + tid];
     if (lane == 0) {
         Cursor &c = S.cur;
@@ -858,57 +866,115 @@ __global__ void __launch_bounds__(32, 20) stream_draw_kernel(CrawlParams P, cons
     __syncwarp();
     if (lane == 0 && !pending) S.cur.pos = 0;      /* what handle_event reads: blocks are scanned with all their anchors */
     __syncwarp();
-    /* blocks of the stream are N apart; this lane's is lane N after the window's first */
-    const uint32_t QN = N / Bp, RN = N % Bp, qL = (uint32_t)lane * N / Bp, rL = (uint32_t)lane * N % Bp, QW = 32u * N / Bp,
-                   RW = 32u * N % Bp;
+    /* Blocks of the stream are N apart; the lane's two are 2 lane N and (2 lane + 1) N after the window's
+     * first.  The words of the next window are in flight or here, as are the row offsets of the one after:
+     * neither load fits into one window. */
+    const uint32_t QN = N / Bp, RN = N % Bp, qL = 2u * lane * N / Bp, rL = 2u * lane * N % Bp, QW = 64u * N / Bp, RW = 64u * N % Bp;
     auto ahead = [&](uint32_t &p, uint32_t &b, uint32_t q, uint32_t r) {
         p += q;
         b += r;
         if (b >= Bp) { b -= Bp; p++; }
     };
+    auto row_at = [&](uint32_t p) { return p < npx ? __ldg(roff + p) : GF_END_WORD; };
+    auto word_in = [&](uint32_t row, uint32_t b) { return row != GF_END_WORD ? __ldg(words + (row + b)) : GF_END_WORD; };
+    /* the multiplier of ten bins in each block before the lane's, the windows' usual case */
+    const uint64_t pmod = ((uint64_t)a << 32) - 1;
+    const int nL = 2 * lane * GF_BLOCK;
+    const uint64_t mL = gfr::mwc_mulmod_scaled(__ldg(jlo + (nL & 31)), __ldg(jhi + (nL >> 5)), a, pmod);
+    uint32_t wa, wb, va, vb, p2, b2, ra, rb;       /* words of this window and the next; the lane's first block two windows on */
+    auto rows_on = [&]() {
+        uint32_t q = p2, b = b2;
+        ahead(q, b, QN, RN);
+        ra = row_at(p2);
+        rb = row_at(q);
+    };
+    auto words_on = [&](uint32_t &x, uint32_t &y) {
+        uint32_t b = b2 + RN;
+        if (b >= Bp) b -= Bp;
+        x = word_in(ra, b2);
+        y = word_in(rb, b);
+        ahead(p2, b2, QW, RW);
+        rows_on();
+    };
+    auto start_window = [&]() {
+        p2 = ilb;
+        b2 = lb;
+        ahead(p2, b2, qL, rL);
+        rows_on();
+        words_on(wa, wb);
+        words_on(va, vb);
+    };
     bool finished = false;
     int flag = pending ? 1 : 0;
-    while (!flag) {
+    if (!flag && pos > 0) {
+        /* the rest of the block that the last batch ended in */
         bool stars;
-        if (pos > 0) {
-            /* the rest of a block that the last batch ended in */
-            if (ilb < npx) flag = scan_block<MODEL>(P, S, lfm, sid, lane, (int)ilb, (int)lb, pos, v, stars, a, jlo, jhi);
-            pos = 0;
-            ahead(ilb, lb, QN, RN);
-            continue;
+        if (ilb < npx) flag = scan_block<MODEL>(P, S, brec, lfm, sid, lane, (int)ilb, (int)lb, pos, v, stars, a, jlo, jhi);
+        pos = 0;
+        ahead(ilb, lb, QN, RN);
+    }
+    start_window();
+    while (!flag) {
+        uint32_t xa, xb;
+        words_on(xa, xb);
+        const bool end = wa == GF_END_WORD || wb == GF_END_WORD;
+        int na = wa == GF_END_WORD ? 0 : (int)(wa & GF_NLIVE), nb = wb == GF_END_WORD ? 0 : (int)(wb & GF_NLIVE);
+        bool stars = __all_sync(FULLMASK, na == GF_BLOCK && nb == GF_BLOCK);
+        uint64_t w0, w1;               /* the state before the lane's blocks, and between them */
+        uint32_t x, c, ma, mb;
+        if (stars) {
+            w0 = gfr::mwc_mulmod_scaled(mL, v, a, pmod);
+            x = (uint32_t)w0;
+            c = (uint32_t)(w0 >> 32);
+            ma = gfc::walk_ten(x, c, a);
+            w1 = ((uint64_t)c << 32) | x;
+            mb = gfc::walk_ten(x, c, a);
         }
-        uint32_t pL = ilb, bL = lb;
-        ahead(pL, bL, qL, rL);
-        const bool end = pL >= npx;
-        const uint32_t word = end ? GF_DEAD_WORD : __ldg(words + (__ldg(roff + pL) + bL));
-        const int n = (int)(word & GF_NLIVE);
-        const int inc = warp_incl_scan(n, lane);
-        const uint64_t w0 = jump(v, inc - n, jlo, jhi, a);
-        uint32_t x = (uint32_t)w0, c = (uint32_t)(w0 >> 32);
-        const uint32_t mx = gfc::walk_bins(x, c, a, n ? (uint32_t)n : (uint32_t)GF_BLOCK);
-        unsigned cand = __ballot_sync(FULLMASK, n != 0 && mx >= (word & ~GF_NLIVE));
-        const uint64_t w1 = n ? ((uint64_t)c << 32) | x : w0;
-        bool again = false;
-        for (; cand && !flag && !again; cand &= cand - 1u) {
-            const int f = __ffs(cand) - 1;
-            uint64_t vf = shfl64(w0, f);
-            const uint32_t pf = __shfl_sync(FULLMASK, pL, f), bf = __shfl_sync(FULLMASK, bL, f);
-            flag = scan_block<MODEL>(P, S, lfm, sid, lane, (int)pf, (int)bf, 0, vf, stars, a, jlo, jhi);
-            if (stars) {
-                v = vf;
-                ilb = pf;
-                lb = bf;
-                ahead(ilb, lb, QN, RN);
-                again = true;
+        for (bool walked = stars;; walked = false) {
+            if (!walked) {
+                const int inc = warp_incl_scan(na + nb, lane);
+                w0 = jump(v, inc - na - nb, jlo, jhi, a);
+                x = (uint32_t)w0;
+                c = (uint32_t)(w0 >> 32);
+                ma = gfc::walk_bins(x, c, a, (uint32_t)na);
+                w1 = ((uint64_t)c << 32) | x;
+                mb = gfc::walk_bins(x, c, a, (uint32_t)nb);
             }
+            const unsigned ca = __ballot_sync(FULLMASK, na != 0 && ma >= (wa & ~GF_NLIVE));
+            const unsigned cb = __ballot_sync(FULLMASK, nb != 0 && mb >= (wb & ~GF_NLIVE));
+            stars = false;
+            for (unsigned cand = ca | cb; cand && !flag && !stars; cand &= cand - 1u) {
+                const int f = __ffs(cand) - 1;
+                for (int second = 0; second < 2 && !flag && !stars; second++) {
+                    if (!(((second ? cb : ca) >> f) & 1u)) continue;
+                    uint64_t vf = shfl64(second ? w1 : w0, f);
+                    uint32_t pf = ilb, bf = lb;
+                    ahead(pf, bf, __shfl_sync(FULLMASK, qL, f), __shfl_sync(FULLMASK, rL, f));
+                    if (second) ahead(pf, bf, QN, RN);
+                    flag = scan_block<MODEL>(P, S, brec, lfm, sid, lane, (int)pf, (int)bf, 0, vf, stars, a, jlo, jhi);
+                    if (stars) {
+                        /* the blocks after it are walked again, from the state after its stars */
+                        v = vf;
+                        if (lane <= f) {
+                            na = 0;
+                            if (lane < f || second) nb = 0;
+                        }
+                    }
+                }
+            }
+            if (flag || !stars) break;
         }
-        if (flag || again) continue;
-        v = shfl64(w1, 31);
+        if (flag) break;
+        v = shfl64(((uint64_t)c << 32) | x, 31);
         if (__any_sync(FULLMASK, end)) {
             finished = true;
             break;
         }
         ahead(ilb, lb, QW, RW);
+        wa = va;
+        wb = vb;
+        va = xa;
+        vb = xb;
     }
     flush_records<1, 0>(P, S, lane);
     if (lane == 0) {
