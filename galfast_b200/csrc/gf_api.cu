@@ -191,6 +191,7 @@ struct ModelState {
     unsigned char *d_plan = nullptr;         /* anchor plan of its grid (IntegPlanDesc), and its header */
     gfk::IntegPlanHdr plan{};
     bool planned = false;
+    double total = -1.0;                     /* expected stars of an integrate by pixels, which has no sums per stream */
     std::vector<double> stream_expected;     /* per-stream expected stars (integrate pass) */
     std::vector<int64_t> stream_drawn;       /* stars drawn per stream so far */
     int first_active = 0;                    /* streams before it have finished */
@@ -981,8 +982,8 @@ gf_status integrate_by_pixels(gf_skygen *s, ModelState &ms, double *expected, do
     GF_CUDA(cudaStreamSynchronize(st));
     ms.planned = true;
     if (!ms.plan.ok) return GF_OK;     /* (nothing was summed) */
-    /* blocks of bins go to the streams in turn: an even share predicts the draw's windows */
-    ms.stream_expected.assign(s->nthreads, sums.x / s->nthreads);
+    ms.stream_expected.clear();    /* predict_streams, when a draw needs them */
+    ms.total = sums.x;
     ms.expected = sums.x;
     ms.expected_covered = sums.y;
     if (expected) *expected = sums.x;
@@ -1046,6 +1047,7 @@ gf_status gf_skygen_integrate(gf_skygen *s, int32_t model, double *expected, dou
     GF_CUDA(cudaStreamSynchronize(st));
     double e = 0, ec = 0;
     for (int i = 0; i < N; i++) { e += hc[i]; ec += hv[i]; }
+    ms.total = -1.0;
     if (kmax % GF_BLOCK == 0) ms.stream_expected = hc;   /* the draw crawl assigns the same bins to the same streams */
     ms.expected = e;
     ms.expected_covered = ec;
@@ -1112,6 +1114,38 @@ gf_status gf_skygen_precision(gf_skygen *s, int32_t model, gf_precision_report *
 
 }  /* extern "C" */
 
+namespace {
+/* Expected stars of each stream after an integrate by pixels, for the draw's windows (they decide how much
+ * is drawn ahead, not what).  Stream t takes blocks t, t + N, ...: the blocks of the grid that are t modulo
+ * g = gcd(N, blocks of a pixel), each as often as the others; their shares of the total come from 256
+ * pixels.  With an even share the 18 batches of a full sky took 14.2 s, with these 9.1 (10.7 with the crawl's
+ * integrate): N is a multiple of a pixel's blocks there, and the streams of the bright bins have far
+ * fewer stars than the others.  A stripe of the survey: 8 windows and 28.0 ms of draws, now 6 and 23.2. */
+gf_status predict_streams(gf_skygen *s, ModelState &ms)
+{
+    const SkyModel &m = ms.hm.m;
+    const int N = s->nthreads, Bp = m.nm * m.nM / GF_BLOCK;
+    cudaStream_t st = s->ctx->stream;
+    double *d_E = nullptr;
+    Blocks blocks{s->ctx, {}};
+    GF_TRY(blocks.take(&d_E, Bp));
+    GF_CUDA(cudaMemsetAsync(d_E, 0, 8 * (size_t)Bp, st));
+    GF_CUDA(gfk::launch_block_expect(crawl_launch(s, ms), std::min(s->geom.npixels, 256), d_E, st));
+    std::vector<double> E(Bp);
+    GF_CUDA(cudaMemcpyAsync(E.data(), d_E, 8 * (size_t)Bp, cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaStreamSynchronize(st));
+    int g = N, r = Bp;
+    while (r) { const int q = g % r; g = r; r = q; }
+    std::vector<double> share(g, 0.0);
+    double all = 0.0;
+    for (int b = 0; b < Bp; b++) { share[b % g] += E[b]; all += E[b]; }
+    ms.stream_expected.resize(N);
+    for (int t = 0; t < N; t++)
+        ms.stream_expected[t] = all > 0.0 ? ms.total * (share[t % g] / all) * ((double)g / N) : ms.total / N;
+    return GF_OK;
+}
+}  // namespace
+
 /* what the kernels that make a generator's block words read, and the view of its draw */
 struct WordSetup {
     CrawlJob job;
@@ -1126,9 +1160,9 @@ struct WordSetup {
 namespace {
 /* The block words (gf_batchdraw.cu) of one model over all pixels of a generator, for
  * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
- * integrate_by_pixels says the same, and tables above 4 GB or that do not fit the device.
+ * integrate_by_pixels says the same, and tables above 4 GB or half of the device's free memory.
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
- * of 71524 pixels (2.7e9 bins a model, 8 windows) 67.9 -> 28.0 ms for three models (tables 1.3),
+ * of 71524 pixels (2.7e9 bins a model, 6 windows) 67.9 -> 23.2 ms for three models (tables 1.3),
  * 1600 pixels (4.6e7 bins) 2.05 -> 0.67 (tables 0.17). */
 gf_status ensure_words(gf_skygen *s, int model, bool *ok)
 {
@@ -1161,6 +1195,10 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
             std::swap(s->d_words, c->d_words);
             std::swap(s->words_cap, c->words_cap);
         } else {
+            /* half of what is free stays free for the records, and for other contexts */
+            size_t fr = 0, all = 0;
+            GF_CUDA(cudaMemGetInfo(&fr, &all));
+            if (8 * (size_t)n > fr) return GF_OK;
             const gf_status as = dev_alloc(&s->d_words, (size_t)n);
             if (as == GF_E_OOM) return GF_OK;
             GF_TRY(as);
@@ -1267,6 +1305,9 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
      * emulated threads one after another).  Streams run speculatively in
      * windows predicted from their expected counts; the window that reaches
      * the capacity fixes the boundary stream t. */
+    const bool sampled = ms.total >= 0.0;
+    if (sampled && ms.stream_expected.empty() && ms.total * (double)ms.hm.m.norm - (double)ms.drawn > 0.8 * (double)C)
+        GF_TRY(predict_streams(s, ms));
     const bool have_pred = (int)ms.stream_expected.size() == N;
     int64_t cum = 0;          /* stars of streams before the current window position */
     int t = -1;
@@ -1276,6 +1317,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         int64_t room = C - cum;
         if (have_pred) {
             double need = (double)room + 6.0 * sqrt((double)room) + 256.0, acc = 0.0;
+            if (sampled) need += (double)room / 64.0;
             w_hi = w_lo;
             while (w_hi < N && acc < need) {
                 double rem = ms.stream_expected[w_hi] * (double)ms.hm.m.norm - (double)ms.stream_drawn[w_hi];

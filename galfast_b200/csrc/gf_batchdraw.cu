@@ -15,7 +15,7 @@
  *                   up to 4 neighbouring pixels with the same cut: how many bins are live
  *                   (not cut), and a threshold that no uniform of an empty block's bins
  *                   reaches in any of the row's pixels.
- *   draw            one warp per 32 consecutive streams, one lane per stream.  Stream t
+ *   draw            one warp per up to 32 consecutive streams, one lane per stream.  Stream t
  *                   takes blocks t, t + N, t + 2N, ... of the request: a step loads the
  *                   word of the lane's next block, steps the MWC over the live bins and
  *                   compares the largest uniform with the threshold.  A lane whose block
@@ -23,6 +23,8 @@
  *                   first candidate bin together, test it exactly, run the reference's
  *                   Poisson sampler and the star uniforms, record the bin (an event: its k
  *                   and the stream state at its first star) and go on with the bins after it.
+ *                   (A single request's generator walks the same words with a warp a stream:
+ *                   stream_draw_kernel, gf_skygen.cu.)
  *   expand          (thread per event) the star records of each event, regenerated
  *                   from its stream state, at offsets from a scan over k.
  *

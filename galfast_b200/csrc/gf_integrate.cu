@@ -23,7 +23,7 @@
  *           pixel), then every bin's mu = (((LF(M) * ms) * norm) * D^3) * K, bins
  *           with m + Am > m1 cut.  Per pixel the counts and covered counts are
  *           summed in FP64.
- *   totals  (one CTA per request) the pixel sums in a fixed order.
+ *   totals  (32 CTAs per request, then their sums) the pixel sums in a fixed order.
  *
  * Every bin's mu is bit-identical to the crawl's; the totals differ from a
  * per-stream summation only by the order of the FP64 additions.

@@ -280,6 +280,8 @@ cudaError_t launch_block_records(const BlockLfParams &P, cudaStream_t s);
 /* rows of a tile for a launch over that many rows and plans of at most max_slots slots */
 int block_word_tile(int64_t rows, int max_slots);
 cudaError_t launch_block_words(const BlockWordParams &P, int model_type, int max_slots, cudaStream_t s);
+/* E[b] += the expected stars of block b of L's grid over that many pixels spread over the request */
+cudaError_t launch_block_expect(const LaunchCrawl &L, int samples, double *E, cudaStream_t s);
 /* a draw launch (launch_crawl) of one request through the block words of all its pixels; view is on the device */
 cudaError_t launch_stream_draw(const LaunchCrawl &L, const DrawJob *view, cudaStream_t s);
 cudaError_t launch_batch_draw(const BatchDrawParams &P, int warps_per_cta, cudaStream_t s);

@@ -8,9 +8,10 @@
  * once:
  *
  *   seeding     the 65536 streams of every request, on the GPU (seed_streams_kernel)
- *   integrate   one persistent crawl per model over the (request, stream) work queue
- *   draw        one persistent crawl per model over the same queue, requests in
- *               decreasing size so that the queue ends on small work
+ *   integrate   pixel by pixel over all requests (gf_integrate.cu)
+ *   draw        block words of every request's pixels, then a lane a stream over all
+ *               requests in decreasing size (gf_batchdraw.cu); a grid whose anchor plan
+ *               does not fit takes one persistent crawl per model for both instead
  *   place/sort  all records at once, sorted by (request, star_comp order)
  *   modules     one launch per module over the rows of all requests; Bond2010 and
  *               the photometric errors use each row's own request (its streams,

@@ -3,6 +3,7 @@
  *
  *   crawl_kernel<DRAW>   integrate pass (DRAW = 0) and Poisson draw pass (DRAW = 1)
  *                        of skygenGPU<T>::kernel (src/skygen/skygen.cu.h:469-618)
+ *   stream_draw_kernel   the draw of a request that has block words, a warp a stream
  *   place_kernel         per-star placement of draw_stars (skygen.cu.h:366-457)
  *   batch sort           star_comp ordering and truncation (skyconfig_impl.h:34-68, 467-515)
  *
@@ -811,10 +812,11 @@ __device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S,
  * did have stars has the window's later blocks walked again from the state after it.
  * Bound by the longest stream: blocks of a stream lie at the same place of the grid when N is a
  * multiple of a pixel's blocks, and a stream of the dense bins has ten times the stars of the others, at
- * some 5000 cycles a scan (half of it the density anchors).  So warps with room beat many of them: 71524
- * pixels, three models, 28.0 ms at 16 CTAs an SM and 128 registers; at 20 and 96, 33 ms, at 12, 30 ms.
- * With a block a lane, its word loaded in its own window and the window begun again after each star
- * 38.9 ms; with a CTA of four warps a stream and every bin's expected count formed 67.9 ms. */
+ * some 5000 cycles a scan (half of it the density anchors).  So fewer warps beat more of them: 71524
+ * pixels, three models, 30.6 ms at 16 CTAs an SM and 128 registers, 34.9 at 20, 32.2 at 12 (28.0 once a
+ * scan took a block's bins from its record instead of stepping to them).  With a block a lane, its word
+ * loaded in its own window and the window begun again after each star 38.9 ms; with a CTA of four warps
+ * a stream and every bin's expected count formed 67.9 ms. */
 template <int MODEL>
 __global__ void __launch_bounds__(32, 16) stream_draw_kernel(CrawlParams P, const DrawJob *view)
 {
@@ -991,6 +993,32 @@ __global__ void __launch_bounds__(32, 16) stream_draw_kernel(CrawlParams P, cons
         J.rng[NS + tid] = (uint32_t)(v >> 32);
         J.rng[2 * NS + tid] = (uint32_t)v;
     }
+}
+
+/* Expected stars of each block of the grid (kmax a multiple of 10), summed over `samples` pixels spread
+ * over the request: the streams' shares of the blocks, for the draw's windows.  GF_EXPECT_PIXELS a thread. */
+#define GF_EXPECT_PIXELS 16
+template <int MODEL>
+__global__ void __launch_bounds__(128) block_expect_kernel(CrawlJob J, int samples, double *E)
+{
+    const SkyModel &m = J.m;
+    const int lb = blockIdx.x * blockDim.x + threadIdx.x;
+    if (lb >= m.nm * m.nM / GF_BLOCK) return;
+    int i0, j0;
+    gfc::diag_to_ij_fast(lb * GF_BLOCK, m.nm, m.nM, J.fx, J.fy, i0, j0);
+    double e = 0.0;
+    const int q1 = min(samples, (int)(blockIdx.y + 1) * GF_EXPECT_PIXELS);
+    for (int q = blockIdx.y * GF_EXPECT_PIXELS; q < q1; q++) {
+        const int ilb = (int)((long long)q * J.g.npixels / samples);
+        int i = i0, j = j0;
+        AnchorX A = gfc::anchor_x<MODEL>(m, J.g, J.Dtab, ilb, i, j);
+        for (int s = 0; s < GF_BLOCK; s++) {
+            if (s > 0 && gfc::step_in_pixel(i, j, m.nm, m.nM)) A = gfc::anchor_x<MODEL>(m, J.g, J.Dtab, ilb, i, j);
+            const float mus = gfc::bin_mu_x(A, gfc::lf_sample(m, m.lf, m.M1 - (float)j * m.dM), m.m0 + m.dm * (float)i, m.norm, m.m1);
+            if (!gfc::is_cut(mus)) e += (double)mus;
+        }
+    }
+    atomicAdd(E + lb, e);
 }
 
 /* D[im][iM] = powf(10, 0.2 DM + 1) with DM = (m0 + im dm) - (M1 - iM dM), skygen.cu.h:219-222 */
@@ -1301,6 +1329,17 @@ static void fill_params(CrawlParams &P, const LaunchCrawl &L)
     P.ck_count = L.ck_count;
     P.ck_capacity = L.ck_capacity;
     P.ck_every = L.ck_every > 0 ? L.ck_every : 64;
+}
+
+cudaError_t launch_block_expect(const LaunchCrawl &L, int samples, double *E, cudaStream_t s)
+{
+    CrawlJob J;
+    fill_job(J, L);
+    const dim3 grid((L.m.nm * L.m.nM / GF_BLOCK + 127) / 128, (samples + GF_EXPECT_PIXELS - 1) / GF_EXPECT_PIXELS);
+    if (L.m.type == GF_MODEL_EXP_DISK) block_expect_kernel<GF_MODEL_EXP_DISK><<<grid, 128, 0, s>>>(J, samples, E);
+    else block_expect_kernel<GF_MODEL_POWER_LAW_ELLIPSOID><<<grid, 128, 0, s>>>(J, samples, E);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_stream_draw(const LaunchCrawl &L, const DrawJob *view, cudaStream_t s)

@@ -617,7 +617,7 @@ enum {
  * src/pipeline.cpp:199-289), applied before the copy instead of when writing. */
 gf_status gf_multi_set_host_columns(gf_ctx *ctx, uint32_t columns);
 
-/* Warps per CTA of the batched draw kernel (one warp per stream), by model kind
+/* Warps per CTA of the batched draw kernel (a lane per stream), by model kind
  * (GF_MODEL_*): 1, 2, 4 or 8.  The first gf_catalog_run_multi pass of each kind
  * times the four on the head of its work queue and keeps the fastest for the
  * context (0 = not tuned yet); gf_tuning_set fixes the choice, or with 0 asks
