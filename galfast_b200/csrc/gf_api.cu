@@ -43,7 +43,7 @@ void release_caches(gf_ctx *ctx)
 }
 
 /* block words of a generator's draw: the largest tables, and the largest kept for the next generator (words of 4 bytes) */
-static const int64_t kWordsMost = (int64_t)4 << 30;
+static const int64_t kWordsMost = (int64_t)16 << 30;
 static const size_t kWordsKept = (size_t)256 << 20;
 static const size_t kBlockMin = 4096, kBlockMax = (size_t)64 << 20, kBlocksHeld = (size_t)512 << 20;
 
@@ -306,7 +306,7 @@ struct RecView {
     void *d_sort_temp = nullptr;
     size_t sort_temp_bytes = 0;
     int64_t rec_cap = 0;
-    uint32_t *d_words = nullptr;      /* block words, slot densities and row offsets of a draw */
+    uint32_t *d_words = nullptr;      /* block words and row offsets of a draw */
     size_t words_cap = 0;
 };
 
@@ -1160,7 +1160,7 @@ struct WordSetup {
 namespace {
 /* The block words (gf_batchdraw.cu) of one model over all pixels of a generator, for
  * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
- * integrate_by_pixels says the same, and tables above 4 GB or half of the device's free memory.
+ * integrate_by_pixels says the same, and tables above 16 GB or half of the device's free memory.
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
  * of 71524 pixels (2.7e9 bins a model, 6 windows) 67.9 -> 23.2 ms for three models (tables 1.3),
  * 1600 pixels (4.6e7 bins) 2.05 -> 0.67 (tables 0.17). */
@@ -1180,9 +1180,9 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
         ms.planned = true;
     }
     const int64_t npix = s->geom.npixels, Bp = (int64_t)m.nm * m.nM / GF_BLOCK, nrows = (int64_t)s->rowpx.size() - 1;
-    const int64_t nslots = ms.plan.nslots, n = nrows * Bp + npix * (nslots + 1);
+    const int64_t nslots = ms.plan.nslots, n = nrows * Bp + npix;
     const int tile = ms.plan.ok ? gfk::block_word_tile(nrows, (int)nslots) : 0;
-    if (!ms.plan.ok || npix * Bp >= (1 << 30) || nrows * Bp >= ((int64_t)1 << 32) || 4 * n > gfa::kWordsMost ||
+    if (!ms.plan.ok || nrows * Bp >= 0xffffffffll || 4 * n > gfa::kWordsMost ||
         4 * (int64_t)tile * nslots > 200 * 1024)
         return GF_OK;
     if ((size_t)n > s->words_cap) {
@@ -1238,8 +1238,7 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
     v.dslot = (const uint16_t *)(ms.d_plan + ms.plan.off_dslot);
     v.slotD = (const float *)(ms.d_plan + ms.plan.off_slot);
     v.words = s->d_words;
-    v.ms = (float *)(s->d_words + nrows * Bp);
-    v.roff = s->d_words + nrows * Bp + npix * nslots;
+    v.roff = s->d_words + nrows * Bp;
     WordSetup *d = s->d_setup;
     GF_CUDA(cudaMemcpyAsync(d, &h, sizeof(h), cudaMemcpyHostToDevice, st));
     gfk::BlockLfParams BL;

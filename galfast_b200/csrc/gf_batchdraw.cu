@@ -204,7 +204,7 @@ __global__ void __launch_bounds__(256) block_words_kernel(BlockWordParams P)
                     const float py = D * pix.sl * pix.cb;
                     const float pz = D * pix.sb;
                     const float ms = gfc::model_rho<MODEL>(m, px, py, pz);
-                    ms_row[s] = ms;
+                    if (V.ms) ms_row[s] = ms;
                     s_ms[q * nslots + s] = p == pa ? ms : fmaxf(s_ms[q * nslots + s], ms);
                 }
             }

@@ -225,7 +225,7 @@ cudaError_t launch_pixel_counts(const IntegPixParams &P, double *out, cudaStream
 #define GF_END_WORD 0xffffffffu    /* past the stream's last block */
 struct DrawJob {
     uint32_t *words;               /* [nrows][Bp] block words: number of live bins (bits 0-3), threshold of the largest uniform (above) */
-    float *ms;                     /* [npx][nslots] model density of each slot of the request's plan */
+    float *ms;                     /* [npx][nslots] model density of each slot of the request's plan, or null: not wanted */
     uint32_t *roff;                /* [npx] first word of the pixel's row */
     const uint2 *prow;             /* [pixels] row, cut row | edge flag */
     const int32_t *rowpx;          /* [rows + 1] first pixel of each row */
