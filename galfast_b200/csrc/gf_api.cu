@@ -1170,6 +1170,8 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
     ModelState &ms = s->models[model];
     const SkyModel &m = ms.hm.m;
     if (!by_pixels(s, m)) return GF_OK;
+    /* no bound on the expected counts: every block would be scanned, for longer than the crawl takes */
+    if (!(m.f >= 0.f && m.norm >= 0.f)) return GF_OK;
     if (s->words_model == model) { *ok = true; return GF_OK; }
     gf_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
