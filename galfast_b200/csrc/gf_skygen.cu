@@ -814,7 +814,7 @@ __device__ __noinline__ int scan_block(const CrawlParams &P, CrawlSmem<1, 0> &S,
  * multiple of a pixel's blocks, and a stream of the dense bins has ten times the stars of the others, at
  * some 5000 cycles a scan (half of it the density anchors).  So fewer warps beat more of them: 71524
  * pixels, three models, 30.6 ms at 16 CTAs an SM and 128 registers, 34.9 at 20, 32.2 at 12 (28.0 once a
- * scan took a block's bins from its record instead of stepping to them).  With a block a lane, its word
+ * scan took a block's bins from its record instead of stepping to them, 23.2 in 6 windows instead of 8).  With a block a lane, its word
  * loaded in its own window and the window begun again after each star 38.9 ms; with a CTA of four warps
  * a stream and every bin's expected count formed 67.9 ms. */
 template <int MODEL>
