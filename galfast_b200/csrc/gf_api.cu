@@ -143,14 +143,16 @@ gf_status ensure_multipliers(gf_ctx *ctx)
     if (ctx->d_mult) return GF_OK;
     const std::vector<uint32_t> &mult = gfh::multipliers();
     /* the context takes the three tables together, when all are there: a failed
-     * allocation leaves none, and the next call makes them again */
+     * allocation leaves none, and the next call makes them again.  The upload goes through the
+     * context's stream, in front of the kernels that read it: a copy from pageable memory may return before its
+     * last part has arrived, and the legacy stream is not ordered with this one. */
     uint32_t *d_mult = nullptr;
     JumpTables jt = {nullptr, nullptr};
     auto make = [&]() -> gf_status {
         GF_TRY(dev_alloc(&d_mult, GF_MAX_STREAMS));
         GF_TRY(dev_alloc(&jt.lo, (size_t)GF_MAX_STREAMS * 32));
         GF_TRY(dev_alloc(&jt.hi, (size_t)GF_MAX_STREAMS * GF_JUMP_HI));
-        GF_CUDA(cudaMemcpy(d_mult, mult.data(), 4 * (size_t)GF_MAX_STREAMS, cudaMemcpyHostToDevice));
+        GF_CUDA(cudaMemcpyAsync(d_mult, mult.data(), 4 * (size_t)GF_MAX_STREAMS, cudaMemcpyHostToDevice, ctx->stream));
         GF_CUDA(gfk::launch_jump_tables(d_mult, GF_MAX_STREAMS, jt.lo, jt.hi, ctx->stream));
         return GF_OK;
     };
@@ -1433,7 +1435,8 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
         ms.stream_drawn[t] += Lt;
         ms.first_active = t;
     }
-    GF_CUDA(cudaMemcpy(s->ctx->h_counters + 2, s->ctx->d_counters + 2, 8, cudaMemcpyDeviceToHost));
+    GF_CUDA(cudaMemcpyAsync(s->ctx->h_counters + 2, s->ctx->d_counters + 2, 8, cudaMemcpyDeviceToHost, st));
+    GF_CUDA(cudaStreamSynchronize(st));
     if (s->ctx->h_counters[2]) return fail(GF_E_INVALID, "a bin has an infinite expected star count");
     /* placement, sort by (hidden, l, b, DM, M, Am), truncation at the first hidden row */
     GF_CUDA(cudaMemsetAsync(s->ctx->d_counters + 1, 0, 8, st));
