@@ -4,6 +4,7 @@
  */
 #include "gf_ctx.h"
 #include "gf_host.h"
+#include "gf_rng.h"
 #include "gf_safeprimes.h"
 
 #include <cuda_runtime.h>
@@ -45,6 +46,7 @@ void release_caches(gf_ctx *ctx)
 /* block words of a generator's draw: the largest tables, and the largest kept for the next generator (words of 4 bytes) */
 static const int64_t kWordsMost = (int64_t)16 << 30;
 static const size_t kWordsKept = (size_t)256 << 20;
+static const int kStuckWord = 7;        /* of h_counters */
 static const size_t kBlockMin = 4096, kBlockMax = (size_t)64 << 20, kBlocksHeld = (size_t)512 << 20;
 
 /* blocks come in powers of two, so that requests of similar sizes share them */
@@ -137,6 +139,16 @@ gf_status check_ctx(gf_ctx *ctx)
     GF_CUDA(cudaSetDevice(ctx->device));
     return GF_OK;
 }
+
+gf_status check_streams(gf_ctx *ctx)
+{
+    volatile unsigned long long *stuck = ctx->h_counters + kStuckWord;
+    if (!*stuck) return GF_OK;
+    *stuck = 0;
+    return fail(GF_E_TIMEOUT, "a random stream repeats its state: its rows were left undrawn");
+}
+
+gfk::StreamPowers stream_powers(gf_ctx *ctx) { return {ctx->jt, ctx->d_mult, ctx->h_counters + kStuckWord}; }
 
 gf_status ensure_multipliers(gf_ctx *ctx)
 {
@@ -564,6 +576,7 @@ gf_status gf_ctx_create(int device, gf_ctx **out)
     cudaError_t ce = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = gfa::device_malloc((void **)&c->d_counters, 64);
     if (ce == cudaSuccess) ce = cudaMallocHost(&c->h_counters, 64);
+    if (ce == cudaSuccess) memset(c->h_counters, 0, 64);
     if (ce != cudaSuccess) {
         delete c;
         return fail(GF_E_CUDA, std::string("context setup: ") + cudaGetErrorString(ce));
@@ -600,7 +613,7 @@ gf_status gf_ctx_sync(gf_ctx *ctx)
 {
     GF_TRY(check_ctx(ctx));
     GF_CUDA(cudaStreamSynchronize(ctx->stream));
-    return GF_OK;
+    return gfa::check_streams(ctx);
 }
 
 gf_status gf_ctx_mark(gf_ctx *ctx, int32_t slot)
@@ -676,13 +689,16 @@ gf_status gf_rng_get_state(gf_ctx *ctx, uint32_t *host_state, int32_t nstreams)
     if (nstreams != ctx->rng_nstreams) return fail(GF_E_INVALID, "stream count mismatch");
     GF_CUDA(cudaMemcpyAsync(host_state, ctx->d_rng, 12 * (size_t)nstreams, cudaMemcpyDeviceToHost, ctx->stream));
     GF_CUDA(cudaStreamSynchronize(ctx->stream));
-    return GF_OK;
+    return gfa::check_streams(ctx);
 }
 
 gf_status gf_rng_set_state(gf_ctx *ctx, const uint32_t *host_state, int32_t nstreams)
 {
     GF_TRY(check_ctx(ctx));
     if (nstreams != ctx->rng_nstreams) return fail(GF_E_INVALID, "stream count mismatch");
+    for (int32_t i = 0; i < nstreams; i++)
+        if (gfr::mwc_fixed(host_state[i], host_state[(size_t)nstreams + i], host_state[2 * (size_t)nstreams + i]))
+            return fail(GF_E_INVALID, "a stream state that never changes (carry and x both 0, or a - 1 and 2^32 - 1)");
     GF_CUDA(cudaMemcpyAsync(ctx->d_rng, host_state, 12 * (size_t)nstreams, cudaMemcpyHostToDevice, ctx->stream));
     GF_CUDA(cudaStreamSynchronize(ctx->stream));
     return GF_OK;
@@ -693,6 +709,7 @@ gf_status gf_rng_poisson(gf_ctx *ctx, uint32_t state[3], const float *mu, int32_
     GF_TRY(check_ctx(ctx));
     if (!state || n < 0 || (n > 0 && (!mu || !out))) return fail(GF_E_INVALID, "invalid gf_rng_poisson arguments");
     if (state[0] == 0) return fail(GF_E_INVALID, "stream multiplier must be nonzero");
+    if (gfr::mwc_fixed(state[0], state[1], state[2])) return fail(GF_E_INVALID, "a stream state that never changes");
     for (int32_t i = 0; i < n; i++)
         if (!(mu[i] >= 0.f && mu[i] < 1e7f)) return fail(GF_E_INVALID, "Poisson means must be in [0, 1e7)");
     uint32_t *d_st = nullptr, *d_out = nullptr;
@@ -1582,6 +1599,7 @@ gf_status gf_table_download_rows(gf_ctx *ctx, const gf_table *dev, int64_t begin
     GF_TRY(cp(host->absmagSys, dev->absmagSys, 4, 2));
     GF_TRY(cp(host->absmagSysNcomp, dev->absmagSysNcomp, 4, 1));
     GF_CUDA(cudaStreamSynchronize(st));
+    GF_TRY(gfa::check_streams(ctx));
     host->size = end - begin;
     host->systems = dev->systems;
     return GF_OK;
@@ -1635,7 +1653,7 @@ static gf_status module_feh(gf_ctx *ctx, const gf_feh_config *fp, const gf_gauss
     const int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_FEH);
-    GF_CUDA(gfk::launch_feh(fp, gp, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_feh(fp, gp, gfa::stream_powers(ctx), ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     return GF_OK;
 }
 
@@ -1652,7 +1670,7 @@ gf_status gf_module_multiples(gf_ctx *ctx, const gf_multiples_config *cfg, gf_ta
     const int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_FEH);
-    GF_CUDA(gfk::launch_multiples(*cfg, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_multiples(*cfg, gfa::stream_powers(ctx), ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     t->systems = 1;
     return GF_OK;
 }
@@ -1678,7 +1696,7 @@ gf_status gf_module_bond2010(gf_ctx *ctx, const gf_bond2010_config *cfg, gf_tabl
     int64_t n = end - begin;
     if ((n + 255) / 256 > ctx->rng_nstreams) return fail(GF_E_INVALID, "more than 256 rows per stream");
     ProfScope ps(ctx, GF_PROF_BOND2010);
-    GF_CUDA(gfk::launch_bond2010(*cfg, {ctx->jt, ctx->d_mult}, ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
+    GF_CUDA(gfk::launch_bond2010(*cfg, gfa::stream_powers(ctx), ctx->d_rng, ctx->rng_nstreams, *t, begin, end, ctx->stream));
     return GF_OK;
 }
 
@@ -1927,6 +1945,7 @@ static gf_status catalog_run_once(gf_ctx *ctx, const gf_job *job, gf_batch_callb
             if (job->v2pm) GF_TRY(gf_module_vel2pm(ctx, job->v2pm, &g.t, 0, n));
             if (job->gal2other) GF_TRY(gf_module_gal2other(ctx, job->gal2other, &g.t, 0, n));
             GF_CUDA(cudaStreamSynchronize(ctx->stream));
+            GF_TRY(gfa::check_streams(ctx));
             S.stored[i] += n;
             if (cb && cb(user, models[i].comp, &g.t, row_offset) != 0) return fail(GF_E_STATE, "stopped by the batch callback");
             row_offset += n;

@@ -139,6 +139,10 @@ gf_status catalog_run_multi_admitted(gf_ctx *ctx, const gf_job *jobs, int32_t nj
                                      gf_catalog_stats *stats, Admission *adm);
 
 gf_status check_ctx(gf_ctx *ctx);
+/* Once the context's stream has been waited for: whether a module's stream went on without an accepted pair
+ * (StreamPowers::stuck, the last of h_counters).  GF_E_TIMEOUT then, once. */
+gf_status check_streams(gf_ctx *ctx);
+gfk::StreamPowers stream_powers(gf_ctx *ctx);
 /* Of one request: per pixel its pixel row and cut row (gf_launch.h), each row's first pixel (then
  * npixels), and the pixels with the fully covered ones first.  ammin: the least extinction of each
  * beam, null for none. */

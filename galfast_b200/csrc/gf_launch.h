@@ -110,12 +110,13 @@ cudaError_t launch_tie_place_multi(const LaunchPlaceMulti &L, const int64_t *row
 /* modules (gf_modules.cu) */
 cudaError_t launch_clipper(const gf_footprint &foot, gf_table t, int64_t begin, int64_t end, cudaStream_t s);
 cudaError_t launch_poisson_stream(uint32_t *st, const float *mu, int32_t n, uint32_t *out, cudaStream_t s);
-/* os_FeH (fp) or os_GaussianFeH (gp): the one that is not NULL */
 /* the context's multipliers and their powers, with which a warp jumps along a stream */
 struct StreamPowers {
     JumpTables jt;
     const uint32_t *mult;
+    unsigned long long *stuck;     /* host word, page-locked: set when a stream yields no accepted pair (gfa::check_streams) */
 };
+/* os_FeH (fp) or os_GaussianFeH (gp): the one that is not NULL */
 cudaError_t launch_feh(const gf_feh_config *fp, const gf_gaussfeh_config *gp, const StreamPowers &pw,
     uint32_t *rng, int32_t NS, gf_table t,
                        int64_t begin, int64_t end, cudaStream_t s);

@@ -144,6 +144,7 @@ cudaError_t launch_fixedfeh(const gf_fixedfeh_config &c, gf_table t, int64_t beg
  * a stream, 0.06 ms now (latency of one chunk); 4.0e6 rows 0.94 -> 0.39 ms, 6.2e7 rows 5.7 -> 6.0 ms
  * (instruction issue: 56 % of slots, 16e3 warp instructions a chunk, half of them the rows' functions).
  */
+#define GF_PAIR_TRIES 4096              /* pairs of a row's Gaussians (one in 4.7 is rejected): no stream that steps comes near */
 #define GF_RUN_LANE 26                  /* uniforms of a lane in a run (even): three runs serve 256 rows of three Gaussians */
 #define GF_RUN_PITCH 33
 #define GF_RUN_END 0xffffu
@@ -178,13 +179,13 @@ struct RowJump {
     bool ok;                            /* the multiplier is within the bounds of mwc_fold3 */
 };
 
-__device__ __forceinline__ RowJump row_jump(const JumpTables &jt, const uint32_t *mult, const uint32_t *rng, int64_t th)
+__device__ __forceinline__ RowJump row_jump(const StreamPowers &pw, const uint32_t *rng, int64_t th)
 {
     RowJump j;
     j.a = rng[th];
-    const bool same = j.a == mult[th];
-    j.lo = same ? jt.lo + (size_t)th * 32 : nullptr;
-    j.hi = same ? jt.hi + (size_t)th * GF_JUMP_HI : nullptr;
+    const bool same = j.a == pw.mult[th];
+    j.lo = same ? pw.jt.lo + (size_t)th * 32 : nullptr;
+    j.hi = same ? pw.jt.hi + (size_t)th * GF_JUMP_HI : nullptr;
     j.ok = j.a >= 16u && j.a <= 0xfffffff0u;
     return j;
 }
@@ -318,7 +319,7 @@ __device__ __forceinline__ int rows_of_run(const RowJump &j, uint64_t &v, int r0
 
 /* the rows [begin + 256 th, ...) of one chunk with stream th, on one warp */
 template <class Ops>
-__device__ __forceinline__ void chunk_rows(const Ops &ops, const JumpTables &jt, const uint32_t *mult, uint32_t *rng, int32_t NS,
+__device__ __forceinline__ void chunk_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS,
                                            gf_table &t, int64_t begin, int64_t end, int64_t th, RowStream &S)
 {
     constexpr int NG = Ops::NG, R = GF_RUN_LANE;
@@ -338,7 +339,7 @@ __device__ __forceinline__ void chunk_rows(const Ops &ops, const JumpTables &jt,
     __syncwarp();
     if (na == 0) return;
     const int lead = leads == na ? 1 : leads == 0 ? 0 : -1;
-    const RowJump j = row_jump(jt, mult, rng, th);
+    const RowJump j = row_jump(pw, rng, th);
     uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
     int r0 = 0;
     while (r0 < na) {
@@ -347,17 +348,26 @@ __device__ __forceinline__ void chunk_rows(const Ops &ops, const JumpTables &jt,
             /* a state outside the Lehmer range, or a row longer than a run: its uniforms one after
              * another, the accepted ones laid out as the first of a run */
             const int kind = S.list[r0] >> 8;
-            int q = 0;
+            int q = 0, tries = 0;
+            __syncwarp();                                  /* (the run's tables have been read) */
             if (kind) {
                 S.u[0] = row_step(v, j.a);
                 q = GF_RUN_PITCH;
             }
             for (int g = 0; g < NG; g++, q += 2 * GF_RUN_PITCH) {
                 float u0, u1, y;
+                bool accepted;
                 do {
                     u0 = row_step(v, j.a);
                     u1 = row_step(v, j.a);
-                } while (!pair_accepted(pair_r2(u0, u1, y)));
+                    accepted = pair_accepted(pair_r2(u0, u1, y));
+                } while (!accepted && ++tries < GF_PAIR_TRIES);
+                if (!accepted) {
+                    /* a state that repeats itself (v = 0, a 2^32 - 1, or any of a multiplier 0): the rows left keep
+                     * what they hold, and the caller learns of it at its next synchronisation */
+                    if (lane == 0) *(volatile unsigned long long *)pw.stuck = 1ull;
+                    return;
+                }
                 S.u[q] = u0;
                 S.u[q + GF_RUN_PITCH] = u1;
                 S.next[q] = (uint16_t)(q + 2 * GF_RUN_PITCH);
@@ -396,18 +406,18 @@ __device__ __forceinline__ void chunk_rows(const Ops &ops, const JumpTables &jt,
 #define GF_ROW_WARPS 4
 
 template <class Ops>
-__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_kernel(const Ops ops, JumpTables jt, const uint32_t *mult, uint32_t *rng, int32_t NS, gf_table t,
+__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng, int32_t NS, gf_table t,
                                                                         int64_t begin, int64_t end, int64_t nchunks)
 {
     __shared__ RowStream S[GF_ROW_WARPS];
     const int64_t th = (int64_t)blockIdx.x * GF_ROW_WARPS + (threadIdx.x >> 5);
     if (th >= nchunks) return;
-    chunk_rows(ops, jt, mult, rng, NS, t, begin, end, th, S[threadIdx.x >> 5]);
+    chunk_rows(ops, pw, rng, NS, t, begin, end, th, S[threadIdx.x >> 5]);
 }
 
 /* the 256-row chunks of every request of a pass, each drawing from its request's streams */
 template <class Ops>
-__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel(const Ops ops, JumpTables jt, const uint32_t *mult, uint32_t *rng_all, int32_t NS,
+__global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng_all, int32_t NS,
                                                                               MultiRows R, const int64_t *slot_chunk_begin,
                                                                               int32_t nslots, int64_t nchunks,
                                                                               const int64_t *slot_rows, gf_table t)
@@ -421,7 +431,7 @@ __global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel
         if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
     }
     const int64_t b = R.slot_row_begin[lo];
-    chunk_rows(ops, jt, mult, rng_all + (size_t)R.slot_job[lo] * 3 * NS, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo],
+    chunk_rows(ops, pw, rng_all + (size_t)R.slot_job[lo] * 3 * NS, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo],
                S[threadIdx.x >> 5]);
 }
 
@@ -430,7 +440,7 @@ cudaError_t launch_stream_rows(const Ops &ops, const StreamPowers &pw, uint32_t 
                                int64_t nchunks, cudaStream_t s)
 {
     stream_rows_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
-        ops, pw.jt, pw.mult, rng, NS, t, begin, end, nchunks);
+        ops, pw, rng, NS, t, begin, end, nchunks);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -440,7 +450,7 @@ cudaError_t launch_stream_rows_multi(const Ops &ops, const StreamPowers &pw, uin
                                      int32_t nslots, int64_t nchunks, const int64_t *slot_rows, gf_table t, cudaStream_t s)
 {
     stream_rows_multi_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
-        ops, pw.jt, pw.mult, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
+        ops, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -691,7 +701,7 @@ struct MultOps {
 
 /* rows [begin + 256 th, ...) with stream th on one warp: at most two uniforms a row, so one run of 512 serves
  * the chunk; the walk over the rows only counts them, the magnitudes are formed by all lanes */
-__device__ __forceinline__ void chunk_rows(const MultOps &ops, const JumpTables &jt, const uint32_t *mult, uint32_t *rng,
+__device__ __forceinline__ void chunk_rows(const MultOps &ops, const StreamPowers &pw, uint32_t *rng,
                                            int32_t NS, gf_table &t, int64_t begin, int64_t end, int64_t th, RowStream &S)
 {
     const int lane = threadIdx.x & 31;
@@ -714,7 +724,7 @@ __device__ __forceinline__ void chunk_rows(const MultOps &ops, const JumpTables 
     }
     if (na == 0) return;
     const bool two = ops.c.algo != GF_MULT_EQUAL_MASS;
-    const RowJump j = row_jump(jt, mult, rng, th);
+    const RowJump j = row_jump(pw, rng, th);
     uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
     constexpr int R = 16;
     uint64_t w0;

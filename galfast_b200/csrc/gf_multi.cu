@@ -1482,7 +1482,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             GF_TRY(gfa::zero_module_rows(ctx, &out, total));
             out.systems = J0.multiples ? 1 : 0;
             /* the module chain in pipeline order (pipeline.h:75-88) over every request's rows */
-            const gfk::StreamPowers powers = {ctx->jt, ctx->d_mult};
+            const gfk::StreamPowers powers = gfa::stream_powers(ctx);
             gfk::MultiRows MR;
             MR.row_slot = row_slot.p; MR.slot_row_begin = d_row_begin; MR.slot_job = d_slot_job;
             if (total > 0) {
@@ -1530,6 +1530,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 if (hd.stop.load()) return fail(GF_E_STATE, "stopped by the host callback");
             } else {
                 GF_CUDA(cudaStreamSynchronize(st));
+                GF_TRY(gfa::check_streams(ctx));
                 if (cb) {
                     std::vector<int64_t> rb(njobs, 0), rc(njobs, 0);
                     for (int s = 0; s < nslots; s++) { rb[slot_job[s]] = row_begin[s]; rc[slot_job[s]] = slot_rows[s]; }
@@ -1571,6 +1572,8 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     if (to_host) {
         GF_CUDA(cudaStreamSynchronize(ws.copy_stream));
         if (hd.stop.load()) return fail(GF_E_STATE, "stopped by the host callback");
+        GF_CUDA(cudaStreamSynchronize(st));
+        GF_TRY(gfa::check_streams(ctx));
     }
     return GF_OK;
 }

@@ -36,6 +36,13 @@ namespace gfr {
 /* 2.32830643708e-10f == 2^-32 exactly */
 #define GF_MWC_SCALE 2.32830643708e-10f
 
+/* Does the stream (a, c, x) stay where it is for ever?  v = 0 and v = p = a 2^32 - 1 (c = a - 1, x = 2^32 - 1) do: its
+ * uniforms are all 0 or all 1, and no sampler that rejects would end.  (A multiplier of 0 marks a stream that is not used.) */
+GFR_HD bool mwc_fixed(uint32_t a, uint32_t c, uint32_t x)
+{
+    return a != 0u && ((c == 0u && x == 0u) || (c == a - 1u && x == 0xffffffffu));
+}
+
 struct Mwc {
     uint32_t a, c, x;
     uint32_t used;          /* uniforms drawn since the caller last cleared it */

@@ -343,7 +343,9 @@ const char *gf_last_error(void);
 /* Create a context on CUDA device `device`. */
 gf_status gf_ctx_create(int device, gf_ctx **out);
 gf_status gf_ctx_destroy(gf_ctx *ctx);
-/* Block until all work queued on the context's stream is done. */
+/* Block until all work queued on the context's stream is done.  GF_E_TIMEOUT when a module drew from a
+ * stream whose uniforms never gave an accepted pair (4096 tries a row): the rows left of that stream's 256 keep
+ * what they held.  The calls that wait for the stream and deliver rows or states report it too, once. */
 gf_status gf_ctx_sync(gf_ctx *ctx);
 /* Device-side timing on the context's stream: record event `slot` (0..15),
  * and read the elapsed milliseconds between two recorded slots. */
@@ -383,6 +385,8 @@ gf_status gf_rng_init(gf_ctx *ctx, uint32_t seed48, int32_t nstreams);
 uint32_t gf_rng_seed48_from_cli_seed(uint64_t seed);
 /* Copy the stream states to/from host memory: [3][nstreams] words a, c, x. */
 gf_status gf_rng_get_state(gf_ctx *ctx, uint32_t *host_state, int32_t nstreams);
+/* GF_E_INVALID, with no stream changed, when a stream of a nonzero multiplier would never leave
+ * its state: c = x = 0, or c = a - 1 with x = 2^32 - 1. */
 gf_status gf_rng_set_state(gf_ctx *ctx, const uint32_t *host_state, int32_t nstreams);
 
 /* n Poisson deviates drawn one after another from ONE stream on the device:
