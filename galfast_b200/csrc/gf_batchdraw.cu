@@ -410,8 +410,8 @@ __global__ void __launch_bounds__(256, 3) batch_draw_kernel(BatchDrawParams P)
                 const gf_pencil_beam *pix = V.pixels + V.px0 + pixel;
                 const float dA = __ldg(&pix->dA);
                 /* its first candidate bin, the states before and after it */
-                const uint32_t n = c0 & GF_NLIVE, T = c0 & ~GF_NLIVE;
-                uint32_t k = 0, xk = 0;
+                uint32_t n = c0 & GF_NLIVE, k = 0, xk = 0;
+                const uint32_t T = c0 & ~GF_NLIVE;
                 w = ((uint64_t)c << 32) | x;
                 uint64_t wb = w;
                 for (; k < n; k++) {
@@ -442,8 +442,10 @@ __global__ void __launch_bounds__(256, 3) batch_draw_kernel(BatchDrawParams P)
                 const float u = GF_MWC_SCALE * (float)xk;
                 if (k < n && !bd_surely_empty(u, mu)) {
                     if (!(mu < 3.0e38f) && bd_has_stars(u, mu)) {
-                        /* an infinite expected count would never leave the sampler's gamma loop */
+                        /* an infinite expected count would never leave the sampler's gamma loop: the stream ends
+                         * here, its block's later bins too (px no longer tells which block a word is of) */
                         atomicOr(P.err, 1ull);
+                        n = k + 1;
                         c1 = c2 = GF_END_WORD;
                         px = npx;
                     } else {

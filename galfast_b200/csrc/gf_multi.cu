@@ -947,8 +947,11 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             }
         }
         for (int j : integ) {
-            /* room for the Poisson spread of the model's stars in one batch */
-            if (with_spread(S[j].expected[i], ctx->admit_sigma) >= (double)jobs[j].capacity) R[j].plain = true;
+            /* room for the Poisson spread of the model's stars in one batch.  A total that is no number (an infinite
+             * density where the luminosity function is zero) says nothing of the room, and takes the
+             * plain path with the infinite ones, which says what is wrong with such a request. */
+            const double e = S[j].expected[i];
+            if (!std::isfinite(e) || with_spread(e, ctx->admit_sigma) >= (double)jobs[j].capacity) R[j].plain = true;
         }
     }
 
