@@ -1203,8 +1203,7 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
     const int64_t npix = s->geom.npixels, Bp = (int64_t)m.nm * m.nM / GF_BLOCK, nrows = (int64_t)s->rowpx.size() - 1;
     const int64_t nslots = ms.plan.nslots, n = nrows * Bp + npix;
     const int tile = ms.plan.ok ? gfk::block_word_tile(nrows, (int)nslots) : 0;
-    if (!ms.plan.ok || nrows * Bp >= 0xffffffffll || 4 * n > gfa::kWordsMost ||
-        4 * (int64_t)tile * nslots > 200 * 1024)
+    if (!ms.plan.ok || nrows * Bp >= 0xffffffffll || 4 * n > gfa::kWordsMost || !gfk::block_words_fit(tile, nslots))
         return GF_OK;
     if ((size_t)n > s->words_cap) {
         GF_CUDA(cudaStreamSynchronize(st));

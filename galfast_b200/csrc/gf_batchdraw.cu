@@ -556,7 +556,7 @@ template <int MODEL>
 static cudaError_t launch_block_words_t(const BlockWordParams &P, int max_slots, cudaStream_t s)
 {
     const size_t smem = 4 * (size_t)P.tile * max_slots;
-    cudaError_t e = cudaFuncSetAttribute(block_words_kernel<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaError_t e = cudaFuncSetAttribute(block_words_kernel<MODEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, GF_WORD_SMEM);
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, block_words_kernel<MODEL>, 256, smem);
     if (e != cudaSuccess) return e;
@@ -569,7 +569,7 @@ static cudaError_t launch_block_words_t(const BlockWordParams &P, int max_slots,
 cudaError_t launch_block_words(const BlockWordParams &P, int model_type, int max_slots, cudaStream_t s)
 {
     if (P.total_tiles <= 0) return cudaSuccess;
-    if (P.tile < 1 || P.tile > GF_WORD_TILE || 4 * (int64_t)P.tile * max_slots > 200 * 1024) return cudaErrorInvalidValue;
+    if (P.tile < 1 || P.tile > GF_WORD_TILE || !block_words_fit(P.tile, max_slots)) return cudaErrorInvalidValue;
     return model_type == GF_MODEL_EXP_DISK ? launch_block_words_t<GF_MODEL_EXP_DISK>(P, max_slots, s)
                                            : launch_block_words_t<GF_MODEL_POWER_LAW_ELLIPSOID>(P, max_slots, s);
 }

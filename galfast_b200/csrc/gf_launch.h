@@ -259,6 +259,10 @@ struct BlockLfParams {
     int64_t total;
 };
 #define GF_WORD_TILE 8             /* most rows of a tile of block_words_kernel */
+#define GF_WORD_SMEM (200 * 1024)  /* most shared memory of its CTA */
+/* whether the densities of a tile's rows fit, a float a slot: plans of more than 51200 slots (grids of some 15000
+ * diagonals) do not, even a row at a time, and their requests crawl */
+inline bool block_words_fit(int64_t tile, int64_t nslots) { return 4 * tile * nslots <= GF_WORD_SMEM; }
 struct BlockWordParams {
     const CrawlJob *jobs;
     const DrawJob *view;           /* per request */

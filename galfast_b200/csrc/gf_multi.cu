@@ -870,7 +870,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 GF_CUDA(cudaMemcpyAsync(ws.pdesc.p, nd.data(), sizeof(gfk::IntegPlanDesc) * nd.size(), cudaMemcpyHostToDevice, st));
                 GF_CUDA(gfk::launch_integ_plans(ws.pdesc.p, (int)nd.size(), st));
             }
-            /* every plan's header: slot count, and whether it fitted */
+            /* every plan's header: slot count, and whether it fitted (and will the draw's words) */
             std::vector<unsigned char *> uniq;
             for (auto &kv : plans) uniq.push_back(kv.second);
             GF_TRY(ws.h_stage.need(sizeof(gfk::IntegPlanHdr) * uniq.size()));
@@ -881,7 +881,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             bool ok = true;
             int nM_max = 1;
             for (size_t q = 0; q < uniq.size(); q++) {
-                ok = ok && hh[q].ok;
+                ok = ok && hh[q].ok && gfk::block_words_fit(1, hh[q].nslots);
                 plan_hdr[uniq[q]] = hh[q];
             }
             for (int j : integ) nM_max = std::max(nM_max, R[j].hm[i].m.nM);
