@@ -92,16 +92,41 @@ void free_blocks(gf_ctx *ctx)
     ctx->blocks_held = 0;
 }
 
+/* whether an allocation from here on is one that gf_debug_fail_allocations arranged to fail */
+static bool fails_by_arrangement()
+{
+    const long long after = g_fail_after.load();
+    if (after < 0) return false;
+    const long long k = g_alloc_seen.fetch_add(1);
+    const long long cnt = g_fail_count.load();
+    return k >= after && (cnt == 0 || k < after + cnt);
+}
+
+/* A failed allocation stays the thread's last error until it is asked for, and every launch asks: a caller that
+ * goes on without the memory would find it behind its next launch.  It is taken here. */
+static cudaError_t allocated(cudaError_t e, void **p)
+{
+    if (e == cudaSuccess) return e;
+    *p = nullptr;
+    (void)cudaGetLastError();
+    return e;
+}
+
 cudaError_t device_malloc(void **p, size_t bytes)
 {
     *p = nullptr;
-    const long long after = g_fail_after.load();
-    if (after >= 0) {
-        const long long k = g_alloc_seen.fetch_add(1);
-        const long long cnt = g_fail_count.load();
-        if (k >= after && (cnt == 0 || k < after + cnt)) return cudaErrorMemoryAllocation;
+    if (fails_by_arrangement()) {
+        /* a real failure: a request that no device can meet */
+        (void)allocated(cudaMalloc(p, ~(size_t)0 >> 1), p);
+        return cudaErrorMemoryAllocation;
     }
-    return cudaMalloc(p, bytes);
+    return allocated(cudaMalloc(p, bytes), p);
+}
+
+cudaError_t host_malloc(void **p, size_t bytes)
+{
+    *p = nullptr;
+    return allocated(cudaMallocHost(p, bytes), p);
 }
 
 gf_status fail(gf_status s, const std::string &msg)
@@ -575,7 +600,7 @@ gf_status gf_ctx_create(int device, gf_ctx **out)
     c->device = device;
     cudaError_t ce = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (ce == cudaSuccess) ce = gfa::device_malloc((void **)&c->d_counters, 64);
-    if (ce == cudaSuccess) ce = cudaMallocHost(&c->h_counters, 64);
+    if (ce == cudaSuccess) ce = gfa::host_malloc((void **)&c->h_counters, 64);
     if (ce == cudaSuccess) memset(c->h_counters, 0, 64);
     if (ce != cudaSuccess) {
         delete c;
@@ -835,10 +860,8 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
     }
     if ((st = own_alloc(s, &s->d_limits, s->nthreads)) != GF_OK) return bail(st);
     if ((st = own_alloc(s, &s->d_rng_snap, 3 * (size_t)s->nthreads)) != GF_OK) return bail(st);
-    if (!ctx->h_streams && cudaMallocHost(&ctx->h_streams, 8 * (size_t)GF_MAX_STREAMS) != cudaSuccess) {
-        ctx->h_streams = nullptr;
+    if (!ctx->h_streams && gfa::host_malloc((void **)&ctx->h_streams, 8 * (size_t)GF_MAX_STREAMS) != cudaSuccess)
         return bail(fail(GF_E_OOM, "pinned allocation"));
-    }
     /* the caller's arrays have been read */
     cudaError_t ce = cudaStreamSynchronize(ctx->stream);
     if (ce == cudaSuccess) ce = cudaGetLastError();

@@ -43,9 +43,10 @@ void dev_free(T *&p)
     } while (0)
 
 namespace gfa {
-/* Every device allocation of the library goes through here: cudaMalloc, or the
- * out-of-memory error that gf_debug_fail_allocations arranges, without calling it. */
+/* Every device allocation of the library goes through here: cudaMalloc, of a size that no device has where
+ * gf_debug_fail_allocations arranges a failure.  A failure does not stay the thread's last error. */
 cudaError_t device_malloc(void **p, size_t bytes);
+cudaError_t host_malloc(void **p, size_t bytes);      /* page-locked, likewise */
 /* gf_debug_fail_allocations */
 void set_alloc_failures(long long after, long long count);
 

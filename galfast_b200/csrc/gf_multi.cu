@@ -108,7 +108,7 @@ struct HostGrow {
         if (p) cudaFreeHost(p);
         p = nullptr;
         n = 0;
-        GF_CUDA(cudaMallocHost((void **)&p, m * sizeof(T)));
+        GF_CUDA(gfa::host_malloc((void **)&p, m * sizeof(T)));
         n = m;
         return GF_OK;
     }

@@ -754,8 +754,8 @@ int gf_textout_multi_sink(void *set, int32_t model, const gf_table *host, const 
 /* ---- failure injection (tests) ---- */
 
 /* Make the library's device allocations fail as if the device were out of
- * memory, without calling cudaMalloc for them: the allocations after the next
- * `after` ones fail, `count` of them (0: every one), then allocations succeed
+ * memory, by asking cudaMalloc for more than any device has: the allocations after
+ * the next `after` ones fail, `count` of them (0: every one), then allocations succeed
  * again; after < 0 turns it off.  Process-wide.  gf_catalog_run and
  * gf_catalog_run_multi answer an out-of-memory failure before their first
  * delivered rows by freeing the context's cached buffers and running once more
