@@ -293,6 +293,23 @@ gf_status own_alloc(gf_skygen *s, T **p, size_t n)
     return GF_OK;
 }
 
+/* *p with room for n instead of *cap: the old block goes back.  Without the memory there is none, and *cap is 0. */
+template <typename T, typename N>
+gf_status own_grow(gf_skygen *s, T **p, N *cap, size_t n)
+{
+    for (size_t k = 0; *p && k < s->kept.size(); k++)
+        if (s->kept[k].first == (void *)*p) {
+            gfa::kept_free(s->ctx, s->kept[k].first, s->kept[k].second);
+            s->kept.erase(s->kept.begin() + k);
+            break;
+        }
+    *p = nullptr;
+    *cap = 0;
+    GF_TRY(own_alloc(s, p, n));
+    *cap = (N)n;
+    return GF_OK;
+}
+
 /* CrawlState arrays carved from one allocation */
 size_t crawl_state_bytes(int n) { return (size_t)n * (8 * 4 + 16 + 8) + 256; }
 
@@ -391,27 +408,29 @@ gf_status ensure_rec_capacity(gf_skygen *s, int64_t need, int64_t keep)
     }
     int64_t cap = std::max<int64_t>(need, s->rec_cap * 3 / 2);
     cap = std::max<int64_t>(cap, 4096);
-    StarRecord *old = s->d_rec;
-    float *old_am = s->d_rec_am;
-    s->d_rec = nullptr;
-    s->d_rec_am = nullptr;
-    if (keep > 0 && old) {
+    if (keep > 0 && s->d_rec) {
+        /* the kept records move first: without the memory for that they stay where they are */
         StarRecord *nr = nullptr;
+        float *na = nullptr;
         GF_TRY(dev_alloc(&nr, cap));
-        GF_CUDA(cudaMemcpyAsync(nr, old, sizeof(StarRecord) * (size_t)keep, cudaMemcpyDeviceToDevice, s->ctx->stream));
-        if (s->maps && old_am) {
-            float *na = nullptr;
-            GF_TRY(dev_alloc(&na, cap));
-            GF_CUDA(cudaMemcpyAsync(na, old_am, 4 * (size_t)keep, cudaMemcpyDeviceToDevice, s->ctx->stream));
-            s->d_rec_am = na;
+        if (s->maps && s->d_rec_am) {
+            const gf_status as = dev_alloc(&na, cap);
+            if (as != GF_OK) {
+                dev_free(nr);
+                return as;
+            }
+            GF_CUDA(cudaMemcpyAsync(na, s->d_rec_am, 4 * (size_t)keep, cudaMemcpyDeviceToDevice, s->ctx->stream));
         }
+        GF_CUDA(cudaMemcpyAsync(nr, s->d_rec, sizeof(StarRecord) * (size_t)keep, cudaMemcpyDeviceToDevice, s->ctx->stream));
         GF_CUDA(cudaStreamSynchronize(s->ctx->stream));
-        dev_free(old);
+        dev_free(s->d_rec);
+        dev_free(s->d_rec_am);
         s->d_rec = nr;
+        s->d_rec_am = na;
     } else {
-        dev_free(old);
+        dev_free(s->d_rec);
+        dev_free(s->d_rec_am);
     }
-    dev_free(old_am);
     dev_free(s->d_rec2);
     dev_free(s->d_rec_am2);
     dev_free(s->d_lb); dev_free(s->d_projIdx); dev_free(s->d_hidden);
@@ -1170,12 +1189,15 @@ gf_status predict_streams(gf_skygen *s, ModelState &ms)
     cudaStream_t st = s->ctx->stream;
     double *d_E = nullptr;
     Blocks blocks{s->ctx, {}};
-    GF_TRY(blocks.take(&d_E, Bp));
-    GF_CUDA(cudaMemsetAsync(d_E, 0, 8 * (size_t)Bp, st));
-    GF_CUDA(gfk::launch_block_expect(crawl_launch(s, ms), std::min(s->geom.npixels, 256), d_E, st));
-    std::vector<double> E(Bp);
-    GF_CUDA(cudaMemcpyAsync(E.data(), d_E, 8 * (size_t)Bp, cudaMemcpyDeviceToHost, st));
-    GF_CUDA(cudaStreamSynchronize(st));
+    std::vector<double> E(Bp, 0.0);
+    const gf_status as = blocks.take(&d_E, Bp);
+    if (as != GF_OK && as != GF_E_OOM) return as;
+    if (as == GF_OK) {             /* (an even share without the memory) */
+        GF_CUDA(cudaMemsetAsync(d_E, 0, 8 * (size_t)Bp, st));
+        GF_CUDA(gfk::launch_block_expect(crawl_launch(s, ms), std::min(s->geom.npixels, 256), d_E, st));
+        GF_CUDA(cudaMemcpyAsync(E.data(), d_E, 8 * (size_t)Bp, cudaMemcpyDeviceToHost, st));
+        GF_CUDA(cudaStreamSynchronize(st));
+    }
     int g = N, r = Bp;
     while (r) { const int q = g % r; g = r; r = q; }
     std::vector<double> share(g, 0.0);
@@ -1206,7 +1228,7 @@ namespace {
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
  * of 71524 pixels (2.7e9 bins a model, 6 windows) 67.9 -> 23.2 ms for three models (tables 1.3),
  * 1600 pixels (4.6e7 bins) 2.05 -> 0.67 (tables 0.17). */
-gf_status ensure_words(gf_skygen *s, int model, bool *ok)
+gf_status make_words(gf_skygen *s, int model, bool *ok)
 {
     *ok = false;
     ModelState &ms = s->models[model];
@@ -1215,6 +1237,7 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
     /* no bound on the expected counts: every block would be scanned, for longer than the crawl takes */
     if (!(m.f >= 0.f && m.norm >= 0.f)) return GF_OK;
     if (s->words_model == model) { *ok = true; return GF_OK; }
+    s->words_model = -1;           /* (the view of another model may lose its tables below) */
     gf_ctx *ctx = s->ctx;
     cudaStream_t st = ctx->stream;
     if (!ms.planned) {
@@ -1232,7 +1255,6 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
         GF_CUDA(cudaStreamSynchronize(st));
         dev_free(s->d_words);
         s->words_cap = 0;
-        s->words_model = -1;
         RecView *c = (RecView *)ctx->rec_cache;
         if (c && c->words_cap >= (size_t)n) {
             std::swap(s->d_words, c->d_words);
@@ -1249,15 +1271,8 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
         }
     }
     if (!s->d_setup) GF_TRY(own_alloc(s, &s->d_setup, 1));
-    if (s->brec_cap < (size_t)Bp) {
-        GF_TRY(own_alloc(s, &s->d_brec, (size_t)Bp));
-        s->brec_cap = (size_t)Bp;
-    }
-    if (s->lfm_cap < (size_t)m.nM) {
-        GF_TRY(own_alloc(s, &s->d_lfm, (size_t)m.nM));
-        s->lfm_cap = (size_t)m.nM;
-    }
-    s->words_model = -1;
+    if (s->brec_cap < (size_t)Bp) GF_TRY(own_grow(s, &s->d_brec, &s->brec_cap, (size_t)Bp));
+    if (s->lfm_cap < (size_t)m.nM) GF_TRY(own_grow(s, &s->d_lfm, &s->lfm_cap, (size_t)m.nM));
     WordSetup h;
     memset((void *)&h, 0, sizeof(h));
     h.job.m = m;
@@ -1298,6 +1313,26 @@ gf_status ensure_words(gf_skygen *s, int model, bool *ok)
     *ok = true;
     return GF_OK;
 }
+
+/* the crawl needs none of the memory */
+gf_status ensure_words(gf_skygen *s, int model, bool *ok)
+{
+    const gf_status as = make_words(s, model, ok);
+    return as == GF_E_OOM ? GF_OK : as;
+}
+
+/* Memory is short: the block words and what the context keeps for its next calls go back, and the model crawls
+ * from here on (its states and checkpoints are the crawl's). */
+void give_back(gf_skygen *s, bool *words)
+{
+    cudaStreamSynchronize(s->ctx->stream);
+    dev_free(s->d_words);
+    s->words_cap = 0;
+    s->words_model = -1;
+    *words = false;
+    gfa::free_rec_cache(s->ctx);
+    gfa::free_blocks(s->ctx);
+}
 }  // namespace
 
 extern "C" {
@@ -1326,21 +1361,22 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
     };
     GF_CUDA(cudaMemsetAsync(ms.st.nstars, 0, 8 * (size_t)N, st));
     GF_CUDA(cudaMemsetAsync(s->ctx->d_counters, 0, 24, st));
-    GF_TRY(ensure_rec_capacity(s, C + C / 2 + 65536, 0));
+    auto records = [&](int64_t need, int64_t keep) -> gf_status {
+        const gf_status as = ensure_rec_capacity(s, need, keep);
+        if (as != GF_E_OOM) return as;
+        give_back(s, &words);
+        return ensure_rec_capacity(s, need, keep);
+    };
+    GF_TRY(records(C + C / 2 + 65536, 0));
     const int fb = (N + 255) / 256;
     /* checkpoints: one at each stream's first bin with stars and one every kCkEvery stars */
     const int kCkEvery = 64;
     {
         const int64_t want = (int64_t)N + (C + C / 2 + 65536) / kCkEvery + 4096;
-        if (want > s->ck_cap) {
-            GF_TRY(own_alloc(s, &s->d_ck, (size_t)want));
-            s->ck_cap = (int32_t)want;
-        }
-        if (!s->d_ck_count) {
-            GF_TRY(own_alloc(s, &s->d_ck_count, 4));
-            GF_TRY(own_alloc(s, &s->d_ck_sel, 1));
-            GF_TRY(own_alloc(s, &s->d_keep, 1));
-        }
+        if (want > s->ck_cap) GF_TRY(own_grow(s, &s->d_ck, &s->ck_cap, (size_t)want));
+        if (!s->d_ck_count) GF_TRY(own_alloc(s, &s->d_ck_count, 4));
+        if (!s->d_ck_sel) GF_TRY(own_alloc(s, &s->d_ck_sel, 1));
+        if (!s->d_keep) GF_TRY(own_alloc(s, &s->d_keep, 1));
     }
 
     /* The batch is filled by streams in stream order (the CPU path runs the
@@ -1397,7 +1433,7 @@ gf_status gf_skygen_draw(gf_skygen *s, int32_t model, gf_table *out, int64_t *n_
             if (total <= s->rec_cap) break;
             /* the window drew more stars than the record buffer holds: grow it and redo the window */
             GF_TRY(snapshot_range(s, ms, w_lo, w_hi, true));
-            GF_TRY(ensure_rec_capacity(s, total + total / 4, (int64_t)rec_before));
+            GF_TRY(records(total + total / 4, (int64_t)rec_before));
             unsigned long long rb = rec_before;
             GF_CUDA(cudaMemcpyAsync(s->ctx->d_counters, &rb, 8, cudaMemcpyHostToDevice, st));
         }
