@@ -1224,7 +1224,8 @@ struct WordSetup {
 namespace {
 /* The block words (gf_batchdraw.cu) of one model over all pixels of a generator, for
  * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
- * integrate_by_pixels says the same, and tables above 16 GB or half of the device's free memory.
+ * integrate_by_pixels says the same, and tables above 16 GB, half of the device's free memory, or what a
+ * many-request call or its server leaves them.
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
  * of 71524 pixels (2.7e9 bins a model, 6 windows) 67.9 -> 23.2 ms for three models (tables 1.3),
  * 1600 pixels (4.6e7 bins) 2.05 -> 0.67 (tables 0.17). */
@@ -1260,6 +1261,8 @@ gf_status make_words(gf_skygen *s, int model, bool *ok)
             std::swap(s->d_words, c->d_words);
             std::swap(s->words_cap, c->words_cap);
         } else {
+            if (ctx->words_most > 0 && 4 * n > ctx->words_most) return GF_OK;
+            if (ctx->adm && ctx->adm->extra && !ctx->adm->extra(ctx->adm->user, 4 * n)) return GF_OK;
             /* half of what is free stays free for the records, and for other contexts */
             size_t fr = 0, all = 0;
             GF_CUDA(cudaMemGetInfo(&fr, &all));

@@ -63,6 +63,7 @@ gf_status dev_alloc(T **p, size_t n)
 struct gf_ctx;
 
 namespace gfa {
+struct Admission;
 /* Device memory of one call (or one generator) from the blocks that the context keeps from earlier
  * ones: cudaMalloc and cudaFree synchronise the device and take locks of the whole machine, and a
  * request makes dozens of small tables.  A block is used and reused on the context's stream only,
@@ -94,6 +95,8 @@ struct gf_ctx {
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> prof_pending;
     double prof_ms[GF_PROF_NPHASES] = {};
     int64_t prof_n[GF_PROF_NPHASES] = {};
+    gfa::Admission *adm = nullptr;       /* of the many-request call whose plain requests are under way, or null */
+    int64_t words_most = 0;              /* bytes that their generators' block words may take (0: no limit was set) */
     int64_t multi_budget = 0;            /* device bytes per multi-request chunk (0: 60% of free memory) */
     MultiWS *multi_ws = nullptr;         /* buffers of gf_catalog_run_multi kept between calls */
     gf_table plain_table = {};           /* output table of gf_catalog_run, kept for the next call of the same shape */
@@ -133,6 +136,8 @@ namespace gfa {
  * always generated. */
 struct Admission {
     int32_t (*admit)(void *user, const double *need, int32_t n, int64_t *budget) = nullptr;
+    /* reserves that many bytes for the block words of a request on the plain path, if they are free now; false: it crawls */
+    bool (*extra)(void *user, int64_t bytes) = nullptr;
     void *user = nullptr;
     std::vector<char> deferred;
 };

@@ -344,8 +344,8 @@ namespace {
 #define GF_RING 3
 
 /* bytes of the draw tables of one segment (see the draw pass): large enough that segments of the
- * ordinary passes are one, small beside the 180 GB of the card */
-constexpr int64_t kDrawTables = (int64_t)4 << 30;
+ * ordinary passes are one, small beside the 180 GB of the card; and the least that a budget cuts them to */
+constexpr int64_t kDrawTables = (int64_t)4 << 30, kDrawTablesLeast = (int64_t)64 << 20;
 
 /* bytes of one row of a table with nb bands, counting the columns in mask (GF_COL_*) */
 size_t row_bytes(int nb, uint32_t mask)
@@ -958,16 +958,27 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     /* ---- requests generated together ---- */
     /* device memory of a batched request's draw passes: records, sort keys and
      * output columns take about kStarBytes per star of its largest model, events 48
-     * bytes per star at most, and the slot densities of its pixels */
+     * bytes per star at most; and the draw tables, 4 bytes per slot and pixel and per block and
+     * pixel row (a chunk's requests hold at most kDrawTables bytes of them at a time) */
     const double kStarBytes = 256.0;
+    struct Need {
+        double stars = 0, tables = 0;
+        double bytes() const { return stars + std::min(tables, (double)kDrawTables); }
+    };
     auto need_of = [&](int j) {
-        double mx = 0;
-        for (int i = 0; i < nmod; i++) mx = std::max(mx, with_spread(S[j].expected[i], 8.0));
-        int ns = 0;
-        for (int i = 0; i < nmod; i++)
-            if (plan_used[i] && plan_of(j, i)) ns = std::max(ns, plan_hdr[plan_of(j, i)].nslots);
-        return mx * (kStarBytes + 48.0) + 8.0 * (double)jobs[j].npixels * (ns + 1) +
-               16.0 * (double)R[j].hm[0].m.nm * R[j].hm[0].m.nM / GF_BLOCK;
+        Need q;
+        double mx = 0, records = 0;
+        for (int i = 0; i < nmod; i++) {
+            const SkyModel &m = R[j].hm[i].m;
+            const double Bp = (double)m.nm * m.nM / GF_BLOCK;
+            mx = std::max(mx, with_spread(S[j].expected[i], 8.0));
+            records = std::max(records, 16.0 * Bp + 4.0 * m.nM);
+            if (plan_used[i] && plan_of(j, i))
+                q.tables = std::max(q.tables, 4.0 * ((double)jobs[j].npixels * (plan_hdr[plan_of(j, i)].nslots + 1) +
+                                                     (double)(R[j].rowpx.size() - 1) * Bp));
+        }
+        q.stars = mx * (kStarBytes + 48.0) + records;
+        return q;
     };
     int64_t budget = ctx->multi_budget;
     if (adm && adm->admit) {
@@ -979,7 +990,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             if (!R[j].plain) cand.push_back(j);
         if (!cand.empty()) {
             std::vector<double> need(cand.size());
-            for (size_t k = 0; k < cand.size(); k++) need[k] = need_of(cand[k]);
+            for (size_t k = 0; k < cand.size(); k++) need[k] = need_of(cand[k]).bytes();
             int64_t granted = 0;
             int32_t take = adm->admit(adm->user, need.data(), (int32_t)cand.size(), &granted);
             take = std::max<int32_t>(1, std::min<int32_t>(take, (int32_t)cand.size()));
@@ -1000,18 +1011,26 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     }
     /* chunks of requests whose draw passes fit the memory budget */
     std::vector<std::vector<int>> chunks;
-    {
-        double used = 0;
-        for (int j : batched_all) {
-            const double need = need_of(j);
-            if (chunks.empty() || (used + need > (double)budget && !chunks.back().empty())) {
-                chunks.emplace_back();
-                used = 0;
+    std::vector<Need> chunk_need;
+    for (int j : batched_all) {
+        const Need q = need_of(j);
+        if (!chunks.empty()) {
+            Need &c = chunk_need.back();
+            const Need sum = {c.stars + q.stars, c.tables + q.tables};
+            if (sum.bytes() <= (double)budget) {
+                c = sum;
+                chunks.back().push_back(j);
+                continue;
             }
-            chunks.back().push_back(j);
-            used += need;
         }
+        chunks.push_back({j});
+        chunk_need.push_back(q);
     }
+    /* what of the budget a chunk's stars leave for its draw tables; a segment of kDrawTablesLeast costs little more */
+    auto tables_most = [&](size_t c) {
+        const double left = (double)budget - chunk_need[c].stars;
+        return (int64_t)std::max(std::min(left, (double)kDrawTables), (double)kDrawTablesLeast);
+    };
 
     std::vector<int32_t> job_slot(njobs, 0);
     int32_t *d_job_slot = nullptr, *d_slot_job = nullptr, *d_slot_comp = nullptr;
@@ -1104,7 +1123,8 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
     } copy_drain{&ws, to_host};
     int pass = 0;
 
-    for (const std::vector<int> &batched : chunks) {
+    for (size_t chunk = 0; chunk < chunks.size(); chunk++) {
+        const std::vector<int> &batched = chunks[chunk];
         /* output order of the chunk: by module group, then request */
         std::vector<int> slot_job = batched;
         std::stable_sort(slot_job.begin(), slot_job.end(), [&](int a, int b) { return R[a].group != R[b].group ? R[a].group < R[b].group : a < b; });
@@ -1130,8 +1150,10 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
             int64_t nrec = 0;
             if (plan_used[i]) {
                 /* The draw tables (slot densities a pixel, block words a row; 4 bytes each) of the chunk's requests, in
-                 * segments of every request's pixels when all of them would take more than kDrawTables
+                 * segments of every request's pixels when all of them would take more than tables_most
                  * bytes: a segment's words are made, then the streams walk them and stop at its end. */
+                const int64_t most = tables_most(chunk);
+                GF_TRY(ws.ev.need((size_t)cap));
                 const size_t nb = batched.size();
                 std::vector<const unsigned char *> jp(njobs, nullptr);
                 std::vector<uint4 *> lp(njobs, nullptr);
@@ -1157,7 +1179,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                     fp[j] = ws.lfm.p + lfm_n;
                     lfm_n += R[j].hm[i].m.nM;
                 }
-                int64_t nseg = std::max<int64_t>({1, (4 * table_words + kDrawTables - 1) / kDrawTables, (largest >> 30) + 1});
+                int64_t nseg = std::max<int64_t>({1, (4 * table_words + most - 1) / most, (largest >> 30) + 1});
                 auto seg_px = [&](int j, int64_t k) { return (int32_t)((int64_t)jobs[j].npixels * k / nseg); };
                 /* the row of a pixel, and the rows that the segment's pixels touch */
                 auto row_of = [&](int j, int32_t p) {
@@ -1307,7 +1329,6 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                 }
                 B.items = ws.gitems.p; B.nitems = ngitems; B.next_item = d_counter;
                 B.ev_count = ctx->d_counters; B.err = ctx->d_counters + 2;
-                GF_TRY(ws.ev.need((size_t)cap));
                 B.ev = ws.ev.p; B.ev_capacity = (int64_t)ws.ev.n;
                 B.view = ws.view.p;
                 GF_TRY(make_words(0));
@@ -1551,6 +1572,12 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
      * stream (deliveries stay in order) while the device generates them. */
     {
         gfa::ProfScope plain_time(ctx, GF_PROF_PLAIN);
+        /* their block words stay within a budget that was set, and are asked for where others share one */
+        struct PlainMemory {
+            gf_ctx *ctx;
+            PlainMemory(gf_ctx *c, gfa::Admission *adm) : ctx(c) { ctx->adm = adm; ctx->words_most = ctx->multi_budget; }
+            ~PlainMemory() { ctx->adm = nullptr; ctx->words_most = 0; }
+        } plain_memory(ctx, adm);
         for (int j = 0; j < njobs; j++) {
             if (!R[j].plain || R[j].deferred) continue;
             if (to_host) {

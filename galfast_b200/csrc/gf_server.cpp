@@ -216,7 +216,7 @@ int forward_rows(void *u, int32_t model, const gf_table *dev, const int64_t *row
 
 struct Reservation {
     gf_server *s;
-    int64_t bytes = 0;
+    int64_t bytes = 0, words = 0;        /* words: the part for block words of requests on the plain path */
     bool held = false;
 };
 
@@ -229,7 +229,7 @@ void release(Reservation &r)
         r.s->running--;
     }
     r.held = false;
-    r.bytes = 0;
+    r.bytes = r.words = 0;
     r.s->cv_budget.notify_all();
 }
 
@@ -256,6 +256,26 @@ int32_t admit(void *u, const double *need, int32_t n, int64_t *budget)
     s->info.peak_running = std::max(s->info.peak_running, s->running);
     *budget = std::max<int64_t>(r.bytes, 1);
     return k;
+}
+
+/* the block words of a request on the plain path: without waiting, since without them it crawls.  One
+ * request of a call has them at a time, so the largest counts. */
+bool extra(void *u, int64_t bytes)
+{
+    Reservation &r = *(Reservation *)u;
+    gf_server *s = r.s;
+    std::lock_guard<std::mutex> g(s->mu);
+    const int64_t more = bytes - r.words;
+    if (more <= 0) return true;
+    if (s->budget - s->reserved < more) return false;
+    r.words = bytes;
+    r.bytes += more;
+    s->reserved += more;
+    if (!r.held) s->running++;
+    r.held = true;
+    s->info.peak_reserved = std::max(s->info.peak_reserved, s->reserved);
+    s->info.peak_running = std::max(s->info.peak_running, s->running);
+    return true;
 }
 
 void worker_main(gf_server *s)
@@ -295,6 +315,7 @@ void worker_main(gf_server *s)
         res.s = s;
         gfa::Admission adm;
         adm.admit = admit;
+        adm.extra = extra;
         adm.user = &res;
         st = ctx ? gfa::catalog_run_multi_admitted(ctx, jobs.data(), (int32_t)jobs.size(), forward_rows, &f, stats.data(), &adm)
                  : GF_E_STATE;

@@ -578,9 +578,11 @@ gf_status gf_catalog_run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, g
 gf_status gf_multi_set_admission(gf_ctx *ctx, double sigmas);
 
 /* Device memory that one chunk of a multi-request run may use for its draw
- * passes (records, placement, sort and output columns, about 320 bytes per
- * expected star of a request's largest model).  Requests are generated in
- * consecutive chunks that fit; the callback then sees each chunk's rows.
+ * passes: records, placement, sort and output columns, about 300 bytes per
+ * expected star of a request's largest model, and draw tables of 4 bytes per slot (some 500) and pixel
+ * and per block of ten bins and row of up to four pixels, in segments of at most 4 GB and at least 64 MB.
+ * Requests are generated in consecutive chunks that fit; the callback then sees each chunk's rows.
+ * A request that runs alone holds its block words to a budget that was set, too.
  * 0 (the default) = 60% of the free device memory at the start of the run. */
 gf_status gf_multi_set_memory_budget(gf_ctx *ctx, int64_t bytes);
 
