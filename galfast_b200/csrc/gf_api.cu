@@ -984,15 +984,18 @@ gf_status start_plan(gf_skygen *s, ModelState &ms)
 /* The integrate of one model by pixels instead of by streams (gf_integrate.cu): the same bins and
  * anchors when blocks of bins never straddle pixels.  *done is false, and nothing has changed, where it
  * does not apply: other grids, 3-D extinction maps (anchors' extinction by distance), density cubes,
- * an anchor plan that does not fit, or few bins.  The plan and the sums cost some 0.16 ms a model, the crawl
- * 0.04 ms and 0.5 ms more for 1e8 bins (5e6 bins: 0.07 ms a model by streams, 0.17 by pixels; 4.6e7: 0.26
- * and 0.17; 7.5e8: 3.5 and 0.54). */
+ * an anchor plan that does not fit, or few bins or pixels.  The plan and the sums cost some 0.16 ms a model, the
+ * crawl 0.04 ms and 0.5 ms more for 1e8 bins (5e6 bins: 0.07 ms a model by streams, 0.17 by pixels; 4.6e7: 0.26
+ * and 0.17; 7.5e8: 3.5 and 0.54).  Few pixels of a fine grid leave a few warps that walk it for 80 ns a bin
+ * and 32nd part (480000 bins a pixel, 234 pixels: 0.57 ms a model by streams, 1.4 by pixels; 1.2e7 and 20:
+ * 1.5 and 28; 120000 and 756: 0.48 and 0.38), and its block words as few CTAs. */
 constexpr long long kPixelIntegrateBins = 25000000;
+constexpr int kPixelIntegratePixels = 512;
 bool by_pixels(const gf_skygen *s, const SkyModel &m)
 {
     const long long kmax = (long long)m.nm * m.nM;
     return s->d_prow && kmax % GF_BLOCK == 0 && m.nm + m.nM <= 16384 && m.type != GF_MODEL_DENSITY_CUBE &&
-           kmax * s->geom.npixels >= kPixelIntegrateBins;
+           s->geom.npixels >= kPixelIntegratePixels && kmax * s->geom.npixels >= kPixelIntegrateBins;
 }
 
 gf_status integrate_by_pixels(gf_skygen *s, ModelState &ms, double *expected, double *expected_covered, double *per_pixel, bool *done)
@@ -1224,7 +1227,7 @@ struct WordSetup {
 namespace {
 /* The block words (gf_batchdraw.cu) of one model over all pixels of a generator, for
  * launch_stream_draw; *ok is false where the draw crawls instead: the grids and requests of which
- * integrate_by_pixels says the same, and tables above 16 GB, half of the device's free memory, or what a
+ * by_pixels says the same, and tables above 16 GB, half of the device's free memory, or what a
  * many-request call or its server leaves them.
  * Thresholds of all blocks against the densities and bins of each block of each window: a stripe
  * of 71524 pixels (2.7e9 bins a model, 6 windows) 67.9 -> 23.2 ms for three models (tables 1.3),

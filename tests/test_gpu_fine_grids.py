@@ -31,3 +31,25 @@ def test_grid_above_the_slots_of_the_block_words_crawls(ctx, lib, multipliers):
         for got in (many[0, m], many[1, m], one[m]):
             for c in COLS:
                 assert np.array_equal(np.concatenate([p[c] for p in got], axis=-1), np.concatenate([p[c] for p in v], axis=-1)), (m, c)
+
+
+@pytest.mark.parametrize("radius,words", [(0.85, False), (1.35, True)])       # 0.01 mag rows: about 230 and 580 pixels
+def test_few_pixels_of_a_fine_grid_crawl(ctx, lib, multipliers, radius, words):
+    """Both have 1e8 bins and more; the fewer pixels leave the pixel integrate and the block words a few warps only."""
+    w = W.build_workload(lib, foot=W.cap_footprint(60.0, 40.0, radius), dx_deg=0.1, m0=16.0, m1=19.0, seed48=22, capacity=1 << 20,
+                         with_modules=False)
+    w.sky.dm = 0.01
+    assert (w.npixels >= 512) == words and w.npixels > 200
+    ctx.profile()
+    ctx.profile_read()
+    one = {}
+    G.run_catalog(ctx, w, sink=lambda m, t, off: one.setdefault(m, []).append(t.as_dict(COLS)))
+    phases = ctx.profile_read()
+    ctx.profile(False)
+    assert ("slot_density" in phases) == words
+    want = {}
+    O.run_catalog(w, multipliers, threads=8, sink=lambda m, t, off: want.setdefault(m, []).append(t.as_dict(COLS)))
+    assert sorted(one) == sorted(want) == [0, 1, 2]
+    for m, v in want.items():
+        for c in COLS:
+            assert np.array_equal(np.concatenate([p[c] for p in one[m]], axis=-1), np.concatenate([p[c] for p in v], axis=-1)), (m, c)
