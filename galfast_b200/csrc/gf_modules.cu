@@ -6,7 +6,7 @@
  *
  *   clipper_kernel     os_clipper::process (src/skygen/os_skygen.cpp:999-1044), analytic footprints
  *   fixedfeh_kernel    os_fixedFeH_kernel (src/modules/fixedFeH_gpu.cu.h:34-50)
- *   stream_rows_kernel with
+ *   stream_rows_kernel, and thread_rows_kernel for many chunks, with
  *     BondOps          os_Bond2010_kernel (src/modules/Bond2010_gpu.cu.h:81-218)
  *     FehOps           os_FeH_kernel (src/modules/FeH_gpu.cu.h:43-87)
  *     GaussFehOps      os_GaussianFeH_kernel (src/modules/GaussianFeH_gpu.cu.h:42-73)
@@ -141,8 +141,9 @@ cudaError_t launch_fixedfeh(const gf_fixedfeh_config &c, gf_table t, int64_t beg
  *   3  walks the rows through fh, one shared-memory read a row;
  *   4  forms the rows' values, 32 rows at a time, reading and writing whole lines.
  * A row that the run ends in begins the next run.  Measured (Bond2010): 20001 rows 0.73 ms as one thread
- * a stream, 0.06 ms now (latency of one chunk); 4.0e6 rows 0.94 -> 0.39 ms, 6.2e7 rows 5.7 -> 6.0 ms
- * (instruction issue: 56 % of slots, 16e3 warp instructions a chunk, half of them the rows' functions).
+ * a stream, 0.06 ms now (latency of one chunk); 4.0e6 rows 0.94 -> 0.39 ms (instruction issue: 56 % of slots,
+ * 16e3 warp instructions a chunk, half of them the rows' functions).  Many chunks take a thread each instead
+ * (thread_rows).
  */
 #define GF_PAIR_TRIES 4096              /* pairs of a row's Gaussians (one in 4.7 is rejected): no stream that steps comes near */
 #define GF_RUN_LANE 26                  /* uniforms of a lane in a run (even): three runs serve 256 rows of three Gaussians */
@@ -415,6 +416,17 @@ __global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_kernel(const
     chunk_rows(ops, pw, rng, NS, t, begin, end, th, S[threadIdx.x >> 5]);
 }
 
+/* the last slot whose first chunk is at or before c */
+__device__ __forceinline__ int slot_of_chunk(const int64_t *slot_chunk_begin, int nslots, int64_t c)
+{
+    int lo = 0, hi = nslots - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
+    }
+    return lo;
+}
+
 /* the 256-row chunks of every request of a pass, each drawing from its request's streams */
 template <class Ops>
 __global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng_all, int32_t NS,
@@ -425,21 +437,81 @@ __global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel
     __shared__ RowStream S[GF_ROW_WARPS];
     const int64_t c = (int64_t)blockIdx.x * GF_ROW_WARPS + (threadIdx.x >> 5);
     if (c >= nchunks) return;
-    int lo = 0, hi = nslots - 1;          /* last slot whose first chunk is <= c */
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (slot_chunk_begin[mid] <= c) lo = mid; else hi = mid - 1;
-    }
-    const int64_t b = R.slot_row_begin[lo];
-    chunk_rows(ops, pw, rng_all + (size_t)R.slot_job[lo] * 3 * NS, NS, t, b, b + slot_rows[lo], c - slot_chunk_begin[lo],
+    const int slot = slot_of_chunk(slot_chunk_begin, nslots, c);
+    const int64_t b = R.slot_row_begin[slot];
+    chunk_rows(ops, pw, rng_all + (size_t)R.slot_job[slot] * 3 * NS, NS, t, b, b + slot_rows[slot], c - slot_chunk_begin[slot],
                S[threadIdx.x >> 5]);
+}
+
+/* The rows of a chunk on one thread, one row after another: the better arrangement once there are enough
+ * chunks to fill the chip with threads, since it makes no tables (a warp's 16e3 instructions a chunk are 500
+ * for a thread's share).  A warp a CTA spreads 65536 chunks evenly (13.8 warps an SM; with 128 threads 3.4
+ * CTAs).  Threads against warps, one component: Bond2010 10e6 rows 1.03 and 0.93 ms, 12e6 1.08 and
+ * 1.11, 16.7e6 1.24 and 1.53, a pass of 6.2e7 4.6 and 5.1; FeH 10e6 0.43 and 0.44, 16.7e6 0.53 and 0.71; GaussianFeH of
+ * two components 12e6 0.62 and 0.62, 16.7e6 0.66 and 0.83; multiples 8e6 0.46 and 0.47, 16.7e6 0.70 and 0.94.  So
+ * 11.5e6 rows are the line, for the multiples, whose walk reads every row's fraction, 8e6 (THREADS_FROM, in chunks). */
+template <class Ops>
+__device__ __forceinline__ void thread_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table &t,
+                                            int64_t begin, int64_t end, int64_t th)
+{
+    const uint32_t a = rng[th];
+    uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
+    const int64_t rb = begin + 256 * th, re = rb + 256 < end ? rb + 256 : end;
+    for (int64_t row = rb; row < re; row++) {
+        const int kind = ops.kind(t, row);
+        if (kind < 0) continue;
+        const float pu = kind ? row_step(v, a) : 0.f;
+        float ys[Ops::NG], ss[Ops::NG];
+        int tries = 0;
+#pragma unroll
+        for (int g = 0; g < Ops::NG; g++) {
+            float r2;
+            bool accepted;
+            do {
+                const float u0 = row_step(v, a), u1 = row_step(v, a);
+                r2 = pair_r2(u0, u1, ys[g]);
+                accepted = pair_accepted(r2);
+            } while (!accepted && ++tries < GF_PAIR_TRIES);
+            if (!accepted) {
+                *(volatile unsigned long long *)pw.stuck = 1ull;
+                return;
+            }
+            ss[g] = sqrtf(-2.0f * gfm::logf_(r2) / r2);
+        }
+        ops.apply(t, row, kind, pu, ys, ss);
+    }
+    rng[NS + th] = (uint32_t)(v >> 32);
+    rng[2 * NS + th] = (uint32_t)v;
+}
+
+template <class Ops>
+__global__ void __launch_bounds__(32) thread_rows_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng, int32_t NS, gf_table t,
+                                                          int64_t begin, int64_t end, int64_t nchunks)
+{
+    const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (th < nchunks) thread_rows(ops, pw, rng, NS, t, begin, end, th);
+}
+
+template <class Ops>
+__global__ void __launch_bounds__(32) thread_rows_multi_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng_all, int32_t NS,
+                                                                MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots,
+                                                                int64_t nchunks, const int64_t *slot_rows, gf_table t)
+{
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= nchunks) return;
+    const int slot = slot_of_chunk(slot_chunk_begin, nslots, c);
+    const int64_t b = R.slot_row_begin[slot];
+    thread_rows(ops, pw, rng_all + (size_t)R.slot_job[slot] * 3 * NS, NS, t, b, b + slot_rows[slot], c - slot_chunk_begin[slot]);
 }
 
 template <class Ops>
 cudaError_t launch_stream_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
                                int64_t nchunks, cudaStream_t s)
 {
-    stream_rows_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
+    if (nchunks >= Ops::THREADS_FROM)
+        thread_rows_kernel<Ops><<<(unsigned)((nchunks + 31) / 32), 32, 0, s>>>(ops, pw, rng, NS, t, begin, end, nchunks);
+    else
+        stream_rows_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
         ops, pw, rng, NS, t, begin, end, nchunks);
     count_launches(1);
     return cudaGetLastError();
@@ -449,7 +521,11 @@ template <class Ops>
 cudaError_t launch_stream_rows_multi(const Ops &ops, const StreamPowers &pw, uint32_t *rng_all, int32_t NS, MultiRows R, const int64_t *slot_chunk_begin,
                                      int32_t nslots, int64_t nchunks, const int64_t *slot_rows, gf_table t, cudaStream_t s)
 {
-    stream_rows_multi_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
+    if (nchunks >= Ops::THREADS_FROM)
+        thread_rows_multi_kernel<Ops><<<(unsigned)((nchunks + 31) / 32), 32, 0, s>>>(ops, pw, rng_all, NS, R, slot_chunk_begin, nslots,
+                                                                                       nchunks, slot_rows, t);
+    else
+        stream_rows_multi_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
         ops, pw, rng_all, NS, R, slot_chunk_begin, nslots, nchunks, slot_rows, t);
     count_launches(1);
     return cudaGetLastError();
@@ -493,6 +569,7 @@ __device__ __forceinline__ void draw_moments(float v[3], float R2, float Z, cons
 struct BondOps {
     gf_bond2010_config par;
     static constexpr int NG = 3;
+    static constexpr int64_t THREADS_FROM = 45000;
 
     __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
     {
@@ -559,6 +636,7 @@ cudaError_t launch_bond2010(const gf_bond2010_config &c, const StreamPowers &pw,
 struct FehOps {
     gf_feh_config par;
     static constexpr int NG = 1;
+    static constexpr int64_t THREADS_FROM = 45000;
 
     __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
     {
@@ -592,6 +670,7 @@ struct FehOps {
 struct GaussFehOps {
     gf_gaussfeh_config par;
     static constexpr int NG = 1;
+    static constexpr int64_t THREADS_FROM = 45000;
 
     __device__ __forceinline__ int kind(const gf_table &t, int64_t row) const
     {
@@ -655,6 +734,7 @@ __device__ __forceinline__ float mult_tex(const float *tab, int n, float x0, flo
  * luminosity function, a second one */
 struct MultOps {
     gf_multiples_config c;
+    static constexpr int64_t THREADS_FROM = 31000;
 
     __device__ __forceinline__ bool active(const gf_table &t, int64_t row) const
     {
@@ -762,6 +842,25 @@ __device__ __forceinline__ void chunk_rows(const MultOps &ops, const StreamPower
         rng[NS + th] = (uint32_t)(ve >> 32);
         rng[2 * NS + th] = (uint32_t)ve;
     }
+}
+
+__device__ __forceinline__ void thread_rows(const MultOps &ops, const StreamPowers &, uint32_t *rng, int32_t NS, gf_table &t,
+                                            int64_t begin, int64_t end, int64_t th)
+{
+    const bool two = ops.c.algo != GF_MULT_EQUAL_MASS;
+    const uint32_t a = rng[th];
+    uint64_t v = ((uint64_t)rng[NS + th] << 32) | rng[2 * NS + th];
+    const int64_t rb = begin + 256 * th, re = rb + 256 < end ? rb + 256 : end;
+    for (int64_t row = rb; row < re; row++) {
+        if (!ops.active(t, row)) {
+            ops.single(t, row);
+            continue;
+        }
+        const bool companion = !(row_step(v, a) > ops.fraction(t, row));
+        ops.apply(t, row, companion, companion && two ? row_step(v, a) : 0.f);
+    }
+    rng[NS + th] = (uint32_t)(v >> 32);
+    rng[2 * NS + th] = (uint32_t)v;
 }
 
 cudaError_t launch_multiples(const gf_multiples_config &c, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,

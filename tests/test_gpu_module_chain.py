@@ -1,7 +1,7 @@
 """The postprocessing modules over as many rows and streams as a large batch has, on contexts of their
 own (so that the tables of stream powers are made anew), against the oracle: the whole chain on 4000003
-rows, and Bond2010 on some rows of every one of the 65536 streams.  Stream states and columns must be
-equal bit for bit (the same portable math on both sides)."""
+rows, and the modules that draw on some rows of every stream, with a warp and with a thread to a chunk of 256
+rows.  Stream states and columns must be equal bit for bit (the same portable math on both sides)."""
 import ctypes as C
 
 import numpy as np
@@ -96,31 +96,37 @@ def test_chain_on_four_million_rows_equals_oracle(lib, multipliers):
         ctx.close()
 
 
-def test_rows_of_every_stream_equal_oracle(lib, multipliers):
-    """24 visible rows in each chunk of 256: every stream's powers are used (a run is 832 uniforms, the rows
-    take some 200), the other rows stay as they are."""
-    n = 256 * NS
+@pytest.mark.parametrize("chunks", [30999, 44999, NS])       # a warp a chunk; the multiples, then all modules, a thread a chunk
+def test_rows_of_every_stream_equal_oracle(lib, multipliers, chunks):
+    """24 visible rows in each chunk of 256, of several components: the powers of every stream are used (a run is
+    832 uniforms, the rows take some 200), the other rows stay as they are."""
+    n = 256 * chunks - 5
     host = G.HostTable(n, 0)
     a = host.arrays
     rng = np.random.default_rng(3)
     a["hidden"][0] = 1
-    rows = (256 * np.arange(NS)[:, None] + np.sort(rng.integers(0, 256, (NS, 24)), axis=1)).ravel()
+    rows = np.minimum(256 * np.arange(chunks)[:, None] + np.sort(rng.integers(0, 256, (chunks, 24)), axis=1), n - 1).ravel()
     a["hidden"][0, rows] = 0
-    a["comp"][0, rows] = rng.integers(0, 3, len(rows))
+    a["comp"][0, rows] = rng.integers(0, 4, len(rows))
     a["XYZ"][:, rows] = rng.normal(size=(3, len(rows))) * 3000.0
-    cfg = W.bond2010_config()
+    a["absmag"][0, rows] = rng.uniform(3, 15, len(rows))
+    L = O.load("p")
+    modules = [("gf_module_feh", L.or_module_feh, W.feh_config()), ("gf_module_gaussfeh", L.or_module_gaussfeh, W.gaussfeh_config(comp_mask=0b100)),
+               ("gf_module_multiples", L.or_module_multiples, W.multiples_config(lib, comp_mask=0b011, fraction=W.MULT_FRACTION, lf=W.MULT_LF)),
+               ("gf_module_bond2010", L.or_module_bond2010, W.bond2010_config())]
     state = O.seed_streams(77, multipliers, NS)
     ctx = G.Context(0)
     dev = G.DeviceTable(ctx, n, 0)
     try:
-        upload(dev, host, ["hidden", "comp", "XYZ"])
+        upload(dev, host, ["hidden", "comp", "XYZ", "absmag"])
         ctx.rng_init(77, NS)
-        G.check(lib.gf_module_bond2010(ctx.h, C.byref(cfg), C.byref(dev.t), 0, n))
-        ctx.sync()
-        assert O.load("p").or_module_bond2010(C.addressof(cfg), state.ctypes.data, NS, C.addressof(host.t), 0, n) == 0
-        assert np.array_equal(ctx.rng_state(), state)
-        got = column(dev.t, host, "vcyl").cpu().numpy()
-        assert np.array_equal(got, a["vcyl"], equal_nan=True)
+        for fn, orfn, cfg in modules:
+            G.check(getattr(lib, fn)(ctx.h, C.byref(cfg), C.byref(dev.t), 0, n))
+            assert orfn(C.addressof(cfg), state.ctypes.data, NS, C.addressof(host.t), 0, n) == 0
+            assert np.array_equal(ctx.rng_state(), state), fn
+        for name in ("FeH", "FeH_comp", "absmag", "absmagSys", "absmagSysNcomp", "vcyl"):
+            got = column(dev.t, host, name).cpu().numpy()
+            assert np.array_equal(got, a[name], equal_nan=got.dtype.kind == "f"), name
     finally:
         dev.free()
         ctx.close()
