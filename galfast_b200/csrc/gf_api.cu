@@ -68,7 +68,12 @@ gf_status kept_alloc(gf_ctx *ctx, void **p, size_t bytes)
         ctx->blocks_held -= c;
         return GF_OK;
     }
-    GF_CUDA(device_malloc(p, c));
+    cudaError_t e = device_malloc(p, c);
+    if (e == cudaErrorMemoryAllocation && ctx->blocks_held) {
+        free_blocks(ctx);
+        e = device_malloc(p, c);
+    }
+    GF_CUDA(e);
     return GF_OK;
 }
 
@@ -383,6 +388,19 @@ void free_recs(RecView &v)
 }  // namespace
 
 namespace gfa {
+/* the blocks and block words kept for the next call; whether there were any */
+static bool give_back_kept(gf_ctx *ctx)
+{
+    RecView *c = (RecView *)ctx->rec_cache;
+    const bool any = ctx->blocks_held || (c && c->d_words);
+    if (c) {
+        dev_free(c->d_words);
+        c->words_cap = 0;
+    }
+    free_blocks(ctx);
+    return any;
+}
+
 void free_rec_cache(gf_ctx *ctx)
 {
     if (!ctx || !ctx->rec_cache) return;
@@ -1603,6 +1621,12 @@ gf_status gf_table_alloc(gf_ctx *ctx, int64_t capacity, int32_t nbands, gf_table
     t->capacity = capacity;
     t->nbands = nbands;
     gf_status st = table_alloc_columns(t, (size_t)capacity, nbands);
+    if (st == GF_E_OOM && gfa::give_back_kept(ctx)) {
+        gf_table_free(ctx, t);
+        t->capacity = capacity;
+        t->nbands = nbands;
+        st = table_alloc_columns(t, (size_t)capacity, nbands);
+    }
     if (st != GF_OK) {
         const std::string msg = gfa::g_err;
         gf_table_free(ctx, t);         /* no partial table is left behind */

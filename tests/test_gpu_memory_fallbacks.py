@@ -110,3 +110,24 @@ def test_generator_draws_without_the_memory_of_its_block_words(lib_hook, fail_in
                     assert np.array_equal(rows[c], want[k][c]), (after, k, c)
     # the tables of the block words and of the records are done without or got at the second try; a few small ones are not
     assert sum(outcomes) <= 6 and not all(outcomes)
+
+
+def test_what_a_context_keeps_goes_back_before_an_allocation_fails(lib_hook):
+    """A catalog leaves blocks and block words with its context; the allocation that fails after it takes them back first."""
+    w = beam(lib_hook, 10.0, 45.0, 5.0, 16.0, 19.0, 0.2)
+    for what in ("table", "generator"):
+        ctx = G.Context(0)
+        want = G.run_catalog(ctx, w)
+        assert lib_hook.gf_debug_fail_allocations(0, 1) == 0
+        if what == "table":
+            G.DeviceTable(ctx, 1000, 5).free()
+        else:
+            # 3.5e6 pixels: more than any kept block holds, so that the first allocation is a new one
+            big = beam(lib_hook, 10.0, 45.0, 5.0, 16.0, 19.0, 0.2)
+            n = 3500000 // big.npixels
+            big.pixels, big.ammin, big.npixels = bytearray(bytes(big.pixels) * n), np.tile(big.ammin, n), big.npixels * n
+            G.Skygen(ctx, big).close()
+        lib_hook.gf_debug_fail_allocations(-1, 0)
+        got = G.run_catalog(ctx, w)
+        assert list(got.generated[:3]) == list(want.generated[:3])
+        ctx.close()
