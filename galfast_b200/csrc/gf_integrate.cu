@@ -373,7 +373,11 @@ __device__ __forceinline__ void walk_diagonals(const SkyModel &m, const Diagonal
  * (two pixels to an instruction), a conversion and an FP64 addition.  Bound by instruction issue: 10 warp
  * instructions per bin of 32 pixels, 58 % of the slots used (4.3e9 bins: 1.35e9 instructions; with a warp a
  * pixel and a lane a diagonal 2.57e9, at 22 of 32 lanes, the conversions alone half the time).  Three models:
- * 256 beams 35.3 -> 29.6 ms, 8 beams 1.43 -> 0.62 ms. */
+ * 256 beams 35.3 -> 29.6 ms (27.0 with the exponentials rounded from a table), 8 beams 1.43 -> 0.62 ms.
+ * The runs of two pixels to an instruction need every LF row of the model positive and a normalisation of 1
+ * (the widening by bits holds for positive normal products only): one zero row anywhere, or a norm that was
+ * set, sends all bins through the general loop.  19600 pixels, three models: 1.59 ms, and 1.91 with zero rows or a
+ * norm (11.5 by streams); 64 beams 7.3 ms, and 9.6 with zero rows (9.5 before this kernel). */
 template <int MODEL>
 __global__ void __launch_bounds__(32 * GF_IG_WARPS) integrate_pixels_kernel(IntegPixParams P)
 {

@@ -237,7 +237,6 @@ struct DrawJob {
     const gf_pencil_beam *pixels;  /* the request's pixels */
     uint32_t *rng;                 /* the request's streams [3][rng_nstreams] */
     int32_t rng_nstreams;
-    uint32_t total;                /* npx Bp (below 2^30) */
     int32_t px0, npx, row0, nrows;
     int32_t Bp, nslots, N, nM;
     int32_t QN, RN;                /* N = QN Bp + RN */

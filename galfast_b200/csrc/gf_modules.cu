@@ -226,7 +226,7 @@ __device__ __forceinline__ uint64_t stream_state_at(uint32_t a, uint64_t w0, int
     return ((uint64_t)hi << 32) | lo;
 }
 
-/* gaussian()'s test of a pair of uniforms (cuda_rng.h:165-182) */
+/* the polar Box-Muller test of a pair of uniforms (gaussian, cuda_rng.h:165-182) */
 __device__ __forceinline__ float pair_r2(float u0, float u1, float &y)
 {
     const float x = -1.f + 2.f * u0;

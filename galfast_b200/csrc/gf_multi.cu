@@ -1252,7 +1252,6 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
                         v.nM = m.nM;
                         v.QN = N / v.Bp;
                         v.RN = N % v.Bp;
-                        v.total = (uint32_t)v.npx * (uint32_t)v.Bp;
                         v.first = (int32_t)((int64_t)v.px0 * v.Bp % N);
                         v.fB = make_fastdiv((uint32_t)v.Bp);
                         v.norm = m.norm; v.dm = m.dm; v.dM = m.dM; v.dmin = m.dmin; v.dmax = m.dmax;

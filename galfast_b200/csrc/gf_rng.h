@@ -11,9 +11,9 @@
  * after n steps v_n = a^n v_0 mod p.  mwc_mulmod() reduces a 128-bit product
  * modulo p with the same "a*lo + hi" folding the generator itself performs.
  *
- * The samplers restate src/common/cuda_rng.h:158-376 (GSL-derived Poisson,
- * Gaussian by the polar Box-Muller method, gamma, beta, binomial) with the
- * portable functions of gf_math.h, so host and device results agree.
+ * The samplers restate src/common/cuda_rng.h:158-376 (GSL-derived Poisson, gamma,
+ * beta, binomial) with the portable functions of gf_math.h, so host and device results
+ * agree; the Gaussians (polar Box-Muller) are drawn by the rows' kernels, gf_modules.cu.
  */
 #pragma once
 #include <stdint.h>
@@ -65,18 +65,6 @@ struct Mwc {
         float u;
         do { u = uniform(); } while (u == 0.f);
         return u;
-    }
-
-    /* gaussian: cuda_rng.h:165-182 (polar Box-Muller) */
-    GFR_HD float gaussian(const float sigma)
-    {
-        float x, y, r2;
-        do {
-            x = -1.f + 2.f * uniform();
-            y = -1.f + 2.f * uniform();
-            r2 = x * x + y * y;
-        } while (r2 > 1.0f || r2 == 0.f || r2 == 4.f);
-        return sigma * y * sqrtf(-2.0f * gfm::logf_(r2) / r2);
     }
 
     /* gamma_large: cuda_rng.h:185-208 */

@@ -362,7 +362,7 @@ enum {
     GF_PROF_INTEGRATE = 0, GF_PROF_DRAW_WINDOW = 1, GF_PROF_DRAW_RERUN = 2, GF_PROF_PLACE = 3,
     GF_PROF_SORT = 4, GF_PROF_CLIPPER = 5, GF_PROF_FEH = 6, GF_PROF_BOND2010 = 7, GF_PROF_PHOTOMETRY = 8,
     GF_PROF_PHOTOERR = 9, GF_PROF_VEL2PM = 10, GF_PROF_GAL2OTHER = 11,
-    GF_PROF_SLOTS = 12,          /* batched draw: model density at the slot distances of each pixel */
+    GF_PROF_SLOTS = 12,          /* block records and words of a draw, and the batched draw's model density at the slot distances of each pixel */
     GF_PROF_EXPAND = 13,         /* batched draw: star records of the bins with stars */
     GF_PROF_BATCH_DRAW = 14,     /* batched draw: the Poisson draw of every stream (one launch per model pass) */
     GF_PROF_SETUP = 15,          /* many-request calls: host wall time from the call to the integrate pass (checks,
