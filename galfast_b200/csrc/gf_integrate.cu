@@ -319,7 +319,9 @@ __device__ __forceinline__ void walk_diagonals(const SkyModel &m, const Diagonal
             s_ms[k][lane] = ms;
             const float f3 = D * D * D;
             const float fx = ms.x * f3 * K.x * (COV ? cf.x : 1.0f), fy = ms.y * f3 * K.y * (COV ? cf.y : 1.0f);
-            if (__all_sync(0xffffffffu, W.lfmin * fminf(fx, fy) > 1.0e-30f && W.lfmax * fmaxf(fx, fy) < 1.0e30f)) plain |= 1u << k;
+            /* (each factor for itself: a minimum of two drops the one that is no number) */
+            const bool in = W.lfmin * fx > 1.0e-30f && W.lfmin * fy > 1.0e-30f && W.lfmax * fx < 1.0e30f && W.lfmax * fy < 1.0e30f;
+            if (__all_sync(0xffffffffu, in)) plain |= 1u << k;
         }
         if (norm != 1.0f) plain = 0;
         const int st = (y - 1) - (d - i0);             /* the entry of the diagonal's first bin */
@@ -406,7 +408,13 @@ __global__ void __launch_bounds__(32 * GF_IG_WARPS) integrate_pixels_kernel(Inte
             __syncthreads();
             if (warp == 0) {
                 float lo = s_lf[0].x, up = lo;
-                for (int k = lane; k < m.nM; k += 32) { lo = fminf(lo, s_lf[k].x); up = fmaxf(up, s_lf[k].x); }
+                bool number = true;
+                for (int k = lane; k < m.nM; k += 32) {
+                    lo = fminf(lo, s_lf[k].x);
+                    up = fmaxf(up, s_lf[k].x);
+                    number = number && s_lf[k].x == s_lf[k].x;
+                }
+                if (!__all_sync(0xffffffffu, number)) lo = -1.0f;         /* no slot is plain */
                 for (int o = 16; o > 0; o >>= 1) {
                     lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
                     up = fmaxf(up, __shfl_xor_sync(0xffffffffu, up, o));
