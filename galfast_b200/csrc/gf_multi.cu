@@ -610,7 +610,7 @@ gf_status run_multi(gf_ctx *ctx, const gf_job *jobs, int32_t njobs, gf_multi_cal
         std::stable_sort(q.mc.begin(), q.mc.end(), [](const gf_model_config &a, const gf_model_config &b) { return a.comp < b.comp; });
         if (!gfh::setup_models(J.sky, J.npixels, q.mc.data(), nmod, q.hm, errs[j]) && errs[j].empty()) errs[j] = "invalid model";
         sigs[j] = module_signature(J);
-        if (J.beam_ammin && J.ext.kind == GF_EXT_SCREEN_CSCB)
+        if (J.beam_ammin && J.ext.kind != GF_EXT_NONE)       /* (pixel_rows looks them up) */
             for (int p = 0; p < J.npixels && errs[j].empty(); p++)
                 if (J.pixels[p].extIdx < 0 || J.pixels[p].extIdx >= J.npixels) errs[j] = "pixel extIdx out of range";
     });
