@@ -445,11 +445,14 @@ __global__ void __launch_bounds__(32 * GF_ROW_WARPS, 6) stream_rows_multi_kernel
 
 /* The rows of a chunk on one thread, one row after another: the better arrangement once there are enough
  * chunks to fill the chip with threads, since it makes no tables (a warp's 16e3 instructions a chunk are 500
- * for a thread's share).  A warp a CTA spreads 65536 chunks evenly (13.8 warps an SM; with 128 threads 3.4
- * CTAs).  Threads against warps, one component: Bond2010 10e6 rows 1.03 and 0.93 ms, 12e6 1.08 and
- * 1.11, 16.7e6 1.24 and 1.53, a pass of 6.2e7 4.6 and 5.1; FeH 10e6 0.43 and 0.44, 16.7e6 0.53 and 0.71; GaussianFeH of
- * two components 12e6 0.62 and 0.62, 16.7e6 0.66 and 0.83; multiples 8e6 0.46 and 0.47, 16.7e6 0.70 and 0.94.  So
- * 11.5e6 rows are the line, for the multiples, whose walk reads every row's fraction, 8e6 (THREADS_FROM, in chunks). */
+ * for a thread's share).  Threads against warps, one component: Bond2010 10e6 rows 1.03 and 0.93 ms, 12e6
+ * 1.08 and 1.11, 16.7e6 1.25 and 1.53; FeH 10e6 0.43 and 0.44, 16.7e6 0.53 and 0.71; GaussianFeH of two components
+ * 12e6 0.62 and 0.62, 16.7e6 0.65 and 0.83; multiples 8e6 0.46 and 0.47, 16.7e6 0.69 and 0.94.  So 11.5e6 rows are the
+ * line, for the multiples, whose walk reads every row's fraction, 8e6 (THREADS_FROM, in chunks).
+ * CTAs are of one warp, so that a call's spread evenly, and at most GF_THREAD_CTAS to an SM: each thread holds a
+ * line of every column that it walks, 1 KB of them, and with 16 warps an SM (78 MB) they stay in L2.  Bond2010
+ * over the passes of 2048 requests (5.3e8 rows, the largest 2.4e8): 8 warps 52.8 ms, 12 40.5, 16 37.0, 24 58.1, as
+ * many as fit 62; a warp a chunk 47.3. */
 template <class Ops>
 __device__ __forceinline__ void thread_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table &t,
                                             int64_t begin, int64_t end, int64_t th)
@@ -488,8 +491,8 @@ template <class Ops>
 __global__ void __launch_bounds__(32) thread_rows_kernel(const Ops ops, const StreamPowers pw, uint32_t *rng, int32_t NS, gf_table t,
                                                           int64_t begin, int64_t end, int64_t nchunks)
 {
-    const int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (th < nchunks) thread_rows(ops, pw, rng, NS, t, begin, end, th);
+    for (int64_t th = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; th < nchunks; th += (int64_t)gridDim.x * blockDim.x)
+        thread_rows(ops, pw, rng, NS, t, begin, end, th);
 }
 
 template <class Ops>
@@ -497,19 +500,22 @@ __global__ void __launch_bounds__(32) thread_rows_multi_kernel(const Ops ops, co
                                                                 MultiRows R, const int64_t *slot_chunk_begin, int32_t nslots,
                                                                 int64_t nchunks, const int64_t *slot_rows, gf_table t)
 {
-    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nchunks) return;
-    const int slot = slot_of_chunk(slot_chunk_begin, nslots, c);
-    const int64_t b = R.slot_row_begin[slot];
-    thread_rows(ops, pw, rng_all + (size_t)R.slot_job[slot] * 3 * NS, NS, t, b, b + slot_rows[slot], c - slot_chunk_begin[slot]);
+    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < nchunks; c += (int64_t)gridDim.x * blockDim.x) {
+        const int slot = slot_of_chunk(slot_chunk_begin, nslots, c);
+        const int64_t b = R.slot_row_begin[slot];
+        thread_rows(ops, pw, rng_all + (size_t)R.slot_job[slot] * 3 * NS, NS, t, b, b + slot_rows[slot], c - slot_chunk_begin[slot]);
+    }
 }
+
+#define GF_THREAD_CTAS 16
+inline unsigned thread_ctas(int64_t nchunks) { return (unsigned)std::min<int64_t>((nchunks + 31) / 32, (int64_t)sm_count() * GF_THREAD_CTAS); }
 
 template <class Ops>
 cudaError_t launch_stream_rows(const Ops &ops, const StreamPowers &pw, uint32_t *rng, int32_t NS, gf_table t, int64_t begin, int64_t end,
                                int64_t nchunks, cudaStream_t s)
 {
     if (nchunks >= Ops::THREADS_FROM)
-        thread_rows_kernel<Ops><<<(unsigned)((nchunks + 31) / 32), 32, 0, s>>>(ops, pw, rng, NS, t, begin, end, nchunks);
+        thread_rows_kernel<Ops><<<thread_ctas(nchunks), 32, 0, s>>>(ops, pw, rng, NS, t, begin, end, nchunks);
     else
         stream_rows_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
         ops, pw, rng, NS, t, begin, end, nchunks);
@@ -522,7 +528,7 @@ cudaError_t launch_stream_rows_multi(const Ops &ops, const StreamPowers &pw, uin
                                      int32_t nslots, int64_t nchunks, const int64_t *slot_rows, gf_table t, cudaStream_t s)
 {
     if (nchunks >= Ops::THREADS_FROM)
-        thread_rows_multi_kernel<Ops><<<(unsigned)((nchunks + 31) / 32), 32, 0, s>>>(ops, pw, rng_all, NS, R, slot_chunk_begin, nslots,
+        thread_rows_multi_kernel<Ops><<<thread_ctas(nchunks), 32, 0, s>>>(ops, pw, rng_all, NS, R, slot_chunk_begin, nslots,
                                                                                        nchunks, slot_rows, t);
     else
         stream_rows_multi_kernel<Ops><<<(unsigned)((nchunks + GF_ROW_WARPS - 1) / GF_ROW_WARPS), 32 * GF_ROW_WARPS, 0, s>>>(
