@@ -555,14 +555,14 @@ def bench_multi(args, G, W, ctx, rank, world, dist):
                                 integ_ms, integ_launches, args.steps, ipk,
                                 "per bin 8 FP32 (4 products, 2 cuts, 2 sums); per diagonal 60 FP32 + 6 SFU")
     pk, pk_kind = peaks()
-    draw_bytes = 48.0 * nmod * sum(ws[j].npixels for j in batched) + 32.0 * sum(
+    draw_bytes = 48.0 * nmod * sum(ws[j].npixels for j in batched) + 24.0 * sum(
         stats[j].generated[i] for j in batched for i in range(nmod))
     roofline_hbm = None
     if draw_ms:
         ach = draw_bytes / (draw_ms / args.steps / 1e3) / 1e9
         roofline_hbm = {"bound": "hbm", "kernel": "batch_draw_kernel", "achieved": ach, "peak": pk["hbm_gbs"], "unit": "GB/s",
                         "frac": ach / pk["hbm_gbs"], "peak_source": pk_kind,
-                        "work_model": "48 B per beam read + 32 B per star event written"}
+                        "work_model": "48 B per beam read + 24 B per star event written"}
 
     cpu = None
     if rank == 0 and not args.no_cpu_baseline and world == 1:
