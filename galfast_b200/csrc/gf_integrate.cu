@@ -319,8 +319,9 @@ __device__ __forceinline__ void walk_diagonals(const SkyModel &m, const Diagonal
             s_ms[k][lane] = ms;
             const float f3 = D * D * D;
             const float fx = ms.x * f3 * K.x * (COV ? cf.x : 1.0f), fy = ms.y * f3 * K.y * (COV ? cf.y : 1.0f);
-            /* (each factor for itself: a minimum of two drops the one that is no number) */
-            const bool in = W.lfmin * fx > 1.0e-30f && W.lfmin * fy > 1.0e-30f && W.lfmax * fx < 1.0e30f && W.lfmax * fy < 1.0e30f;
+            /* (each factor for itself: a minimum of two drops the one that is no number; with a row that is not
+             * positive, bounds of negative products would pass) */
+            const bool in = W.lfmin > 0.0f && W.lfmin * fx > 1.0e-30f && W.lfmin * fy > 1.0e-30f && W.lfmax * fx < 1.0e30f && W.lfmax * fy < 1.0e30f;
             if (__all_sync(0xffffffffu, in)) plain |= 1u << k;
         }
         if (norm != 1.0f) plain = 0;

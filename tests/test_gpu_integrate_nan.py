@@ -1,5 +1,5 @@
-"""Expected counts that are no numbers, in the pixel-by-pixel integrate: densities that are none in some pixels
-and rows of a luminosity function that are none.  The same pixels as on the CPU path have no number, and the others
+"""Expected counts that are no positive numbers, in the pixel-by-pixel integrate: densities that are none in some pixels
+and rows of a luminosity function that are none, and factors of both signs.  The same pixels as on the CPU path have no number, and the others
 its counts."""
 import ctypes as C
 
@@ -65,3 +65,21 @@ def test_bins_without_a_number_draw_nothing(ctx, lib, multipliers):
     m.type, m.n, m.l, m.ba, m.ca, m.f = A.GF_MODEL_LCBULGE, 1.3, 2000.0, 1.0, 1.0, 1e-6
     _, total = draw_all(ctx, w, multipliers, 20000)
     assert total > 10000
+
+
+@pytest.mark.parametrize("grid", sorted(GRIDS))
+def test_negative_densities_over_luminosity_functions_of_both_signs(ctx, lib, grid):
+    """Products of two negative factors are among the bins, beside negative ones."""
+    w = beam(lib, *GRIDS[grid])
+    M, phi = W.lf_table()
+    phi = phi * np.where(M < 9.0, -1.0, 0.5)
+    w.models[1].lf_M, w.models[1].lf_phi = (v.ctypes.data_as(C.POINTER(C.c_double)) for v in (M, phi))
+    w.models[1].f = -0.12
+    (e, ec, pp), (oe, oc, op) = counts(ctx, w, 1)
+    # sums with cancellation: a part in 1e6 of what the same grid counts with positive factors
+    w.models[1].f = 0.12
+    phi[:] = np.abs(phi)
+    sky = G.Skygen(ctx, w)
+    pe, pc, ppos = sky.integrate_counts(1, per_pixel=True)
+    assert np.all(np.abs(pp - op) <= 1e-6 * ppos)
+    assert abs(e - oe) <= 1e-11 * pe and abs(ec - oc) <= 1e-11 * pc
