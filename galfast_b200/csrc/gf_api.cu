@@ -166,6 +166,7 @@ gf_status zero_module_rows(gf_ctx *ctx, const gf_table *t, int64_t n)
 gf_status check_ctx(gf_ctx *ctx)
 {
     if (!ctx) return fail(GF_E_INVALID, "null context");
+    if (ctx->destroyed) return fail(GF_E_STATE, "the generator's context was destroyed");
     GF_CUDA(cudaSetDevice(ctx->device));
     return GF_OK;
 }
@@ -649,7 +650,7 @@ gf_status gf_ctx_create(int device, gf_ctx **out)
 
 gf_status gf_ctx_destroy(gf_ctx *ctx)
 {
-    if (!ctx) return GF_OK;
+    if (!ctx || ctx->destroyed) return GF_OK;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     gfa::free_multi_ws(ctx);
@@ -667,7 +668,8 @@ gf_status gf_ctx_destroy(gf_ctx *ctx)
     for (auto &p : ctx->prof_pending) { cudaEventDestroy(p.second.first); cudaEventDestroy(p.second.second); }
     for (auto &e : ctx->ev_pool) cudaEventDestroy(e);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
-    delete ctx;
+    ctx->destroyed = true;
+    if (ctx->generators == 0) delete ctx;       /* else with the last of them */
     return GF_OK;
 }
 
@@ -812,6 +814,7 @@ gf_status gf_skygen_create(gf_ctx *ctx, const gf_skygen_config *cfg, const gf_pe
     if (!gfh::setup_models(*cfg, npixels, models, nmodels, hms, err)) return fail(GF_E_INVALID, err);
     gf_skygen *s = new gf_skygen();
     s->ctx = ctx;
+    ctx->generators++;
     s->cfg = *cfg;
     s->nthreads = cfg->nthreads;
     gf_status st = GF_OK;
@@ -911,14 +914,24 @@ gf_status gf_skygen_destroy(gf_skygen *s)
 {
     if (!s) return GF_OK;
     cudaSetDevice(s->ctx->device);
+    RecView mine;
+    move_recs(mine, *s);
+    s->ctx->generators--;
+    if (s->ctx->destroyed) {
+        /* (its stream was waited for then) */
+        for (auto &k : s->kept) cudaFree(k.first);
+        dev_free(s->d_words);
+        free_recs(mine);
+        if (s->ctx->generators == 0) delete s->ctx;
+        delete s;
+        return GF_OK;
+    }
     cudaStreamSynchronize(s->ctx->stream);
     for (auto &k : s->kept) gfa::kept_free(s->ctx, k.first, k.second);
     /* the record and placement buffers go to the context for its next generator
      * (the larger set is kept) */
     if (!s->ctx->rec_cache) s->ctx->rec_cache = new RecView();
     RecView &c = *(RecView *)s->ctx->rec_cache;
-    RecView mine;
-    move_recs(mine, *s);
     if (mine.rec_cap > c.rec_cap) {
         std::swap(mine.d_words, c.d_words);
         std::swap(mine.words_cap, c.words_cap);

@@ -82,6 +82,8 @@ gf_status kept_alloc(gf_ctx *ctx, T **p, size_t n)
 struct gf_ctx {
     int device = 0;
     cudaStream_t stream = nullptr;
+    int generators = 0;                  /* not destroyed yet; they hold blocks of this context */
+    bool destroyed = false;              /* by the user, before its generators: they give their memory back themselves */
     uint32_t *d_rng = nullptr;           /* persistent streams [3][rng_nstreams] */
     int32_t rng_nstreams = 0;
     uint32_t *d_mult = nullptr;

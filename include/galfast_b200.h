@@ -342,6 +342,7 @@ const char *gf_last_error(void);
 
 /* Create a context on CUDA device `device`. */
 gf_status gf_ctx_create(int device, gf_ctx **out);
+/* Generators of the context that are not destroyed yet can only be destroyed after it (GF_E_STATE otherwise). */
 gf_status gf_ctx_destroy(gf_ctx *ctx);
 /* Block until all work queued on the context's stream is done.  GF_E_TIMEOUT when a module drew from a
  * stream whose uniforms never gave an accepted pair (4096 tries a row): the rows left of that stream's 256 keep
